@@ -1,6 +1,8 @@
-"""Compile the CUDA sources into `deconver_b200/libndc_b200.so` for sm_100a with nvcc.
+"""Compile the CUDA sources into `deconver_b200/libndc_b200.so` for sm_100a with nvcc, and the
+layer's native host path (`csrc/ndc_torch.cpp`, on that library and PyTorch's C++ API) into
+`deconver_b200/_ndc_torch.so` with the host compiler.
 
-The library is built in-tree (next to this file) so that it travels with the source tree.
+Both are built in-tree (next to this file) so that they travel with the source tree.
 nvcc cross-compiles without a GPU.  The tiled kernels are compiled as six translation units
 (forward / backward of volumes / backward of images, each for float32 and bfloat16) next to the
 ABI unit and the instance-norm and bias units, in parallel, then linked.  Run as `python -m deconver_b200._build [--force]`.
@@ -9,6 +11,7 @@ ABI unit and the instance-norm and bias units, in parallel, then linked.  Run as
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
@@ -16,6 +19,8 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(PKG, "libndc_b200.so")
+EXT = os.path.join(PKG, "_ndc_torch.so")
+EXT_SRC = os.path.join(CSRC, "ndc_torch.cpp")
 OBJ = os.path.join(PKG, "_obj")
 
 NVCC_FLAGS = [
@@ -26,7 +31,8 @@ NVCC_FLAGS = [
 ]
 
 # (object name, source, extra defines)
-UNITS = [("abi", "ndc_abi.cu", []), ("inorm", "ndc_inorm.cu", []), ("bias", "ndc_bias.cu", [])] + [
+UNITS = [("abi", "ndc_abi.cu", []), ("inorm", "ndc_inorm.cu", []), ("bias", "ndc_bias.cu", []),
+         ("proj", "ndc_proj.cu", [])] + [
     ("dw4_p%d_t%d" % (part, t), "ndc_dw4_inst.cu", ["-DNDC_DW4_PART=%d" % part, "-DNDC_DW4_T=%d" % t])
     for part in (1, 2, 0) for t in (0, 1)   # the longest units first
 ]
@@ -39,19 +45,61 @@ def sources():
     return deps
 
 
-def is_stale():
-    if not os.path.exists(LIB):
+def _older(target, deps):
+    if not os.path.exists(target):
         return True
-    built = os.path.getmtime(LIB)
-    return any(os.path.getmtime(s) > built for s in sources())
+    built = os.path.getmtime(target)
+    return any(os.path.getmtime(s) > built for s in deps)
+
+
+def is_stale():
+    return _older(LIB, sources())
+
+
+def ext_is_stale():
+    return _older(EXT, [EXT_SRC, os.path.join(INCLUDE, "ndc_b200.h")])
+
+
+def _compile_ext():
+    """Object of the host extension, and the command that links it once the library is there."""
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    obj = os.path.join(OBJ, "ndc_torch.o")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
+           "-DTORCH_EXTENSION_NAME=_ndc_torch", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I", INCLUDE, "-I", os.path.join(root, "include"),
+           "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"], "-c", EXT_SRC, "-o", obj]
+    link = [cmd[0], "-shared", obj, "-o", EXT, "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L", PKG, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    return subprocess.run(cmd, cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True), link
 
 
 def build_library(force=False, verbose=False, extra_flags=()):
-    """Build the shared library if it is missing or older than a source file."""
-    if not (force or is_stale()):
+    """Build the shared library and the host extension if missing or older than a source file."""
+    if not (force or is_stale() or ext_is_stale()):
         return LIB
-    nvcc = os.environ.get("NVCC", "nvcc")
     os.makedirs(OBJ, exist_ok=True)
+    with ThreadPoolExecutor(max_workers=1) as pool:   # the extension compiles next to the library
+        ext = pool.submit(_compile_ext) if force or ext_is_stale() else None
+        if force or is_stale():
+            _build_cuda(verbose, extra_flags)
+        if ext is not None:
+            res, link = ext.result()
+            if res.stdout and (verbose or res.returncode):
+                print(res.stdout, end="", flush=True)
+            if res.returncode:
+                raise subprocess.CalledProcessError(res.returncode, res.args)
+            if verbose:
+                print(" ".join(link), flush=True)
+            subprocess.check_call(link, cwd=ROOT)
+    return LIB
+
+
+def _build_cuda(verbose, extra_flags):
+    nvcc = os.environ.get("NVCC", "nvcc")
 
     def compile_unit(unit):
         name, src, defines = unit
@@ -75,7 +123,6 @@ def build_library(force=False, verbose=False, extra_flags=()):
     if verbose:
         print(" ".join(link), flush=True)
     subprocess.check_call(link, cwd=ROOT)
-    return LIB
 
 
 if __name__ == "__main__":

@@ -5,9 +5,10 @@ raises; nothing falls back to PyTorch or to the CPU.
 """
 
 import ctypes
+import importlib.util
 import os
 
-from ._build import LIB
+from ._build import EXT, LIB
 
 NDC_F32, NDC_BF16 = 0, 1
 NDC_OK = 0
@@ -21,7 +22,8 @@ SYMBOLS = (
     "ndc_fwd", "ndc_bwd_workspace_bytes", "ndc_bwd", "ndc_bwd_static", "ndc_gconv",
     "ndc_probe_fp32_fma", "ndc_inorm_workspace_bytes", "ndc_inorm_last_error", "ndc_inorm_fwd",
     "ndc_inorm_bwd", "ndc_bias_grad_workspace_bytes", "ndc_bias_last_error", "ndc_bias_add",
-    "ndc_bias_grad", "ndc_bias_gelu_fwd", "ndc_bias_gelu_bwd",
+    "ndc_bias_grad", "ndc_bias_gelu_fwd", "ndc_bias_gelu_bwd", "ndc_proj_wgrad_workspace_bytes",
+    "ndc_proj_last_error", "ndc_proj_wgrad", "ndc_proj_sum", "ndc_params_prepare", "ndc_params_grad",
 )
 
 
@@ -103,8 +105,37 @@ def load():
     lib.ndc_bias_gelu_bwd.restype = ctypes.c_int
     lib.ndc_bias_gelu_bwd.argtypes = [ctypes.c_int32, ctypes.c_int32, ctypes.c_int64, ctypes.c_int32, vp,
                                       vp, fp, vp, fp, vp, ctypes.c_size_t, vp]
+    lib.ndc_proj_wgrad_workspace_bytes.restype = ctypes.c_size_t
+    lib.ndc_proj_wgrad_workspace_bytes.argtypes = [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int64]
+    lib.ndc_proj_last_error.restype = ctypes.c_char_p
+    lib.ndc_proj_wgrad.restype = ctypes.c_int
+    lib.ndc_proj_wgrad.argtypes = [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int64, ctypes.c_int32,
+                                   ctypes.c_int32, vp, vp, vp, vp, ctypes.c_size_t, vp]
+    lib.ndc_proj_sum.restype = ctypes.c_int
+    lib.ndc_proj_sum.argtypes = [ctypes.c_int32, ctypes.c_int64, ctypes.c_int32, fp, vp, vp]
+    lib.ndc_params_prepare.restype = ctypes.c_int
+    lib.ndc_params_prepare.argtypes = [ctypes.c_int32, vp, ctypes.c_int64, fp, vp, ctypes.c_int64, fp, vp]
+    lib.ndc_params_grad.restype = ctypes.c_int
+    lib.ndc_params_grad.argtypes = [ctypes.c_int32, vp, fp, ctypes.c_int64, vp, fp, ctypes.c_int64, vp, vp]
     _lib = lib
     return lib
+
+
+_ext = None
+
+
+def load_ext():
+    """Load the native host path of the layer (once); it is built next to the library."""
+    global _ext
+    if _ext is None:
+        if not os.path.exists(EXT):
+            raise RuntimeError(f"{EXT} has not been built; run `python -m deconver_b200._build`.")
+        load()
+        spec = importlib.util.spec_from_file_location("_ndc_torch", EXT)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _ext = module
+    return _ext
 
 
 def check(status):

@@ -1,0 +1,345 @@
+// The layer's host path in native code: one autograd node for the whole `Deconv` layer
+// (parameters -> float32, 1x1 projection, multiplicative updates), on the C ABI of
+// libndc_b200.so and cuBLAS.
+//
+// What bounds the layer at the deep stages and on single images is not the GPU: at 512 channels
+// x 8^3 a forward and backward are 0.16 ms of kernels, and issuing them from Python through
+// separate autograd nodes took 0.60 ms.  One node, one pass over the parameters in each
+// direction, and no intermediate tensor that the update kernels do not read.
+#include <ATen/Context.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/ops/empty.h>
+#include <ATen/ops/relu.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <cublas_v2.h>
+#include <torch/extension.h>
+
+#include <mutex>
+#include <vector>
+
+#include "ndc_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? NDC_BF16 : NDC_F32; }
+bool kernel_dtype(const Tensor& t) { return t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16; }
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
+void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+
+void check(int status, const char* message) {
+    TORCH_CHECK(status == NDC_OK, "ndc_b200 status ", status, ": ", message);
+}
+
+// ---- optional CUDA-event timing of ndc_fwd / ndc_bwd on the stream they are issued on ----------
+struct Timing {
+    std::mutex mu;
+    bool enabled = false;
+    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> spans[2];   // forward, backward
+} g_timing;
+
+struct Span {
+    cudaEvent_t start = nullptr, stop = nullptr;
+    int kind;
+    explicit Span(int k) : kind(k) {
+        if (!g_timing.enabled) return;
+        C10_CUDA_CHECK(cudaEventCreate(&start));
+        C10_CUDA_CHECK(cudaEventCreate(&stop));
+        C10_CUDA_CHECK(cudaEventRecord(start, (cudaStream_t)stream()));
+    }
+    ~Span() {
+        if (!start) return;
+        (void)cudaEventRecord(stop, (cudaStream_t)stream());
+        std::lock_guard<std::mutex> lock(g_timing.mu);
+        g_timing.spans[kind].emplace_back(start, stop);
+    }
+};
+
+void timing_enable() {
+    std::lock_guard<std::mutex> lock(g_timing.mu);
+    for (auto& v : g_timing.spans) {
+        for (auto& s : v) { (void)cudaEventDestroy(s.first); (void)cudaEventDestroy(s.second); }
+        v.clear();
+    }
+    g_timing.enabled = true;
+}
+
+// Stops collecting; the caller has synchronised.  {forward ms, backward ms}
+std::vector<std::vector<float>> timing_collect() {
+    std::lock_guard<std::mutex> lock(g_timing.mu);
+    g_timing.enabled = false;
+    std::vector<std::vector<float>> out(2);
+    for (int k = 0; k < 2; ++k) {
+        for (auto& s : g_timing.spans[k]) {
+            float ms = 0.0f;
+            C10_CUDA_CHECK(cudaEventElapsedTime(&ms, s.first, s.second));
+            out[k].push_back(ms);
+            (void)cudaEventDestroy(s.first);
+            (void)cudaEventDestroy(s.second);
+        }
+        g_timing.spans[k].clear();
+    }
+    return out;
+}
+
+// ---- 1x1 projections -------------------------------------------------------------------------
+// The precision the framework gives convolutions of float32 tensors: TF32 unless switched off.
+bool conv_tf32() { return at::globalContext().allowTF32CuDNN(at::Float32Op::CONV); }
+
+// y[b] = op(w) x[b] (+ y[b] if `accumulate`) for a (Co, Ci) matrix `w`, op = transpose if
+// `transpose`, and contiguous (B, channels, N) tensors: one strided batched library GEMM with the
+// matrix repeated by a zero batch stride; no tensor is converted or copied.
+void channel_gemm(const Tensor& w, bool transpose, const Tensor& x, Tensor& y, int64_t batch, int64_t n,
+                  bool accumulate) {
+    const int64_t co = w.size(0), ci = w.size(1);
+    const int64_t out = transpose ? ci : co, in = transpose ? co : ci;
+    if (!batch || !n || !out || !in) return;
+    const bool bf16 = x.scalar_type() == at::kBFloat16;
+    const bool tf32 = !bf16 && conv_tf32();
+    const float one = 1.0f, beta = accumulate ? 1.0f : 0.0f;
+    const cudaDataType_t type = bf16 ? CUDA_R_16BF : CUDA_R_32F;
+    const cublasComputeType_t compute = tf32 ? CUBLAS_COMPUTE_32F_FAST_TF32 : CUBLAS_COMPUTE_32F;
+    at::NoTF32Guard plain;   // the handle's own mode; `compute` says what this product uses
+    cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
+    // column-major view: (n x out) = (n x in) * (in x out)
+    const cublasStatus_t st = cublasGemmStridedBatchedEx(
+        handle, CUBLAS_OP_N, transpose ? CUBLAS_OP_T : CUBLAS_OP_N, (int)n, (int)out, (int)in, &one, x.data_ptr(),
+        type, (int)n, (long long)(in * n), w.data_ptr(), type, (int)ci, 0LL, &beta, y.data_ptr(), type, (int)n,
+        (long long)(out * n), (int)batch, compute, CUBLAS_GEMM_DEFAULT);
+    TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection GEMM failed (cuBLAS status ", (int)st, ")");
+}
+
+Tensor weight_grad(const Tensor& gy, const Tensor& x, const Tensor& w, int64_t batch, int64_t n) {
+    Tensor gw = at::empty(w.sizes(), w.options());
+    const int64_t co = w.size(0), ci = w.size(1);
+    if (!batch || !n) return gw.zero_();
+    const bool bf16 = gy.scalar_type() == at::kBFloat16;
+    // The library's tcgen05 GEMM is the faster one where it can load whole vectors and fill the GPU:
+    // its positions cut into `slices` per sample (views of the tensors as they lie), or, from 192
+    // input channels on, where the product is bound by the tensor cores (co * ci / (co + ci)
+    // multiply-adds per value read), one product per sample.  Everything else - rows that are not
+    // whole vectors, many samples of few channels - runs on the kernel of ndc_proj_wgrad.
+    int64_t slices = 1;
+    while (slices < 32 && n % (slices * 16) == 0 && n / (slices * 2) >= 2048) slices *= 2;
+    if (n % (bf16 ? 8 : 4) == 0 && (ci >= 192 || (batch <= 4 && slices > 1))) {
+        if (ci >= 192 && batch * ((co + 127) / 128) * ((ci + 127) / 128) >= 64) slices = 1;
+        Tensor partial = at::empty({batch * slices, co, ci}, w.options().dtype(at::kFloat));
+        const float one = 1.0f, zero = 0.0f;
+        const cudaDataType_t type = bf16 ? CUDA_R_16BF : CUDA_R_32F;
+        const cublasComputeType_t compute = !bf16 && conv_tf32() ? CUBLAS_COMPUTE_32F_FAST_TF32 : CUBLAS_COMPUTE_32F;
+        at::NoTF32Guard plain;
+        cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
+        const int64_t calls = slices > 1 ? batch : 1, length = n / slices;
+        for (int64_t b = 0; b < calls; ++b) {
+            const size_t e = bf16 ? 2 : 4;
+            const cublasStatus_t st = cublasGemmStridedBatchedEx(
+                handle, CUBLAS_OP_T, CUBLAS_OP_N, (int)ci, (int)co, (int)length, &one,
+                static_cast<const char*>(x.data_ptr()) + b * ci * n * e, type, (int)n, (long long)(slices > 1 ? length : ci * n),
+                static_cast<const char*>(gy.data_ptr()) + b * co * n * e, type, (int)n, (long long)(slices > 1 ? length : co * n),
+                &zero, fptr(partial) + b * slices * co * ci, CUDA_R_32F, (int)ci, (long long)(co * ci),
+                (int)(slices > 1 ? slices : batch), compute, CUBLAS_GEMM_DEFAULT);
+            TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection gradient failed (cuBLAS status ", (int)st, ")");
+        }
+        if (batch * slices == 1 && !bf16) return partial.view(w.sizes());
+        check(ndc_proj_sum((int)(batch * slices), co * ci, dtype_code(gy), fptr(partial), ptr(gw), stream()), ndc_proj_last_error());
+        return gw;
+    }
+    const size_t bytes = ndc_proj_wgrad_workspace_bytes((int)batch, (int)co, (int)ci, n);
+    Tensor ws = at::empty({(int64_t)bytes}, w.options().dtype(at::kByte));
+    check(ndc_proj_wgrad((int)batch, (int)co, (int)ci, n, dtype_code(gy), conv_tf32() ? 1 : 0, ptr(gy), ptr(x),
+                         ptr(gw), ptr(ws), bytes, stream()), ndc_proj_last_error());
+    return gw;
+}
+
+// ---- the layer -------------------------------------------------------------------------------
+struct Config {
+    int64_t groups, m, sc;
+    double eps;
+    int64_t iters, grad_iters, flags;
+};
+
+NdcDesc make_desc(const Tensor& x, const Tensor& h0, const Config& c, bool relu) {
+    NdcDesc d;
+    int64_t sp[3] = {1, 1, 1}, k[3] = {1, 1, 1};
+    const int64_t rank = x.dim() - 2;
+    for (int64_t i = 0; i < rank; ++i) { sp[3 - rank + i] = x.size(2 + i); k[3 - rank + i] = h0.size(2 + i); }
+    d.batch = (int)x.size(0); d.groups = (int)c.groups; d.m = (int)c.m; d.sc = (int)c.sc;
+    d.D = (int)sp[0]; d.H = (int)sp[1]; d.W = (int)sp[2];
+    d.kD = (int)k[0]; d.kH = (int)k[1]; d.kW = (int)k[2];
+    d.eps = (float)c.eps; d.relu_input = relu ? 1 : 0; d.dtype = dtype_code(x); d.flags = (int)c.flags;
+    return d;
+}
+
+// relu(h0) and the bias as the kernels take them
+void prepare_params(const Tensor& h0, const Tensor& bias, Tensor& h, Tensor& b) {
+    const auto f32 = h0.options().dtype(at::kFloat);
+    const bool same = !bias.defined() || bias.scalar_type() == h0.scalar_type();
+    if (kernel_dtype(h0) && same) {
+        h = at::empty(h0.sizes(), f32);
+        const bool convert = bias.defined() && bias.scalar_type() != at::kFloat;
+        b = convert ? at::empty(bias.sizes(), f32) : bias;
+        check(ndc_params_prepare(dtype_code(h0), ptr(h0), h0.numel(), fptr(h), convert ? ptr(bias) : nullptr,
+                                 convert ? bias.numel() : 0, convert ? fptr(b) : nullptr, stream()),
+              ndc_proj_last_error());
+        return;
+    }
+    h = at::relu(h0).to(at::kFloat);
+    b = bias.defined() ? bias.to(at::kFloat) : bias;
+}
+
+struct Saved {
+    Tensor h, b;                       // float32 filter and bias
+    std::vector<Tensor> z, t1;         // per update that has gradients: its source and K(source)
+    int64_t first = 0;                 // index of the first such update
+};
+
+Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Tensor& bias, const Config& c,
+                   Saved* saved) {
+    Saved local;
+    Saved& sv = saved ? *saved : local;
+    prepare_params(h0, bias, sv.h, sv.b);
+    auto shape = x.sizes().vec();
+    shape[1] = c.groups * c.sc;
+    const int64_t n = x.numel() ? x.numel() / (x.size(0) * x.size(1)) : 0;
+    Tensor s = at::empty(shape, x.options());
+    channel_gemm(w, false, x, s, x.size(0), n, false);
+    sv.first = c.iters > c.grad_iters ? c.iters - c.grad_iters : 0;
+    Tensor t1;
+    for (int64_t it = 0; it < c.iters; ++it) {
+        const bool keep = saved && it >= sv.first;
+        Tensor out = at::empty(shape, x.options());
+        if (keep || !t1.defined()) t1 = at::empty(x.sizes(), x.options());
+        if (x.numel()) {
+            const NdcDesc d = make_desc(x, h0, c, it == 0);
+            Span span(0);
+            check(ndc_fwd(&d, ptr(x), ptr(s), fptr(sv.h), it == 0 ? fptr(sv.b) : nullptr, ptr(out), ptr(t1),
+                          stream()), ndc_last_error());
+        }
+        if (keep) { sv.z.push_back(s); sv.t1.push_back(t1); }
+        s = out;
+    }
+    return s;
+}
+
+struct LayerNode : public torch::autograd::Function<LayerNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& h0, const Tensor& w,
+                          const std::optional<Tensor>& bias, int64_t groups, int64_t m, int64_t sc, double eps,
+                          int64_t iters, int64_t grad_iters, int64_t flags) {
+        const Config c{groups, m, sc, eps, iters, grad_iters, flags};
+        Saved sv;
+        const Tensor b = bias ? *bias : Tensor();
+        Tensor out = run_forward(x, h0, w, b, c, &sv);
+        variable_list keep = {x, h0, w, b, sv.h, sv.b};
+        keep.insert(keep.end(), sv.z.begin(), sv.z.end());
+        keep.insert(keep.end(), sv.t1.begin(), sv.t1.end());
+        ctx->save_for_backward(keep);
+        auto& d = ctx->saved_data;
+        d["cfg"] = std::vector<int64_t>{groups, m, sc, iters, grad_iters, flags, sv.first};
+        d["eps"] = eps;
+        return out;
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        TORCH_CHECK(!at::GradMode::is_enabled(), "double backward through the fused Deconv update is not supported");
+        const variable_list kept = ctx->get_saved_variables();
+        const auto cfg = ctx->saved_data["cfg"].toIntVector();
+        const Config c{cfg[0], cfg[1], cfg[2], ctx->saved_data["eps"].toDouble(), cfg[3], cfg[4], cfg[5]};
+        const int64_t first = cfg[6], count = c.iters - first;
+        const Tensor &x = kept[0], &h0 = kept[1], &w = kept[2], &bias = kept[3], &h = kept[4], &b = kept[5];
+        const bool need_x = ctx->needs_input_grad(0), need_h = ctx->needs_input_grad(1);
+        const bool whole = first == 0;                   // gradients reach the projection
+        const bool need_w = whole && ctx->needs_input_grad(2);
+        const bool need_b = whole && bias.defined() && ctx->needs_input_grad(3);
+        c10::cuda::CUDAGuard guard(x.device());
+        const auto f32 = h.options();
+
+        Tensor g = grads[0].contiguous();
+        if (g.scalar_type() != x.scalar_type()) g = g.to(x.scalar_type());
+        Tensor gx, gh, gb, ws;
+        const int64_t n = x.numel() ? x.numel() / (x.size(0) * x.size(1)) : 0;
+        for (int64_t i = count - 1; i >= 0; --i) {
+            const Tensor &z = kept[6 + i], &t1 = kept[6 + count + i];
+            const bool it0 = first + i == 0;
+            const bool need_z = i > 0 || (it0 && (need_x || need_w || need_b));
+            Tensor gx_i, gz, gh_i;
+            if (need_x) gx_i = at::empty(x.sizes(), x.options());
+            if (need_z) gz = at::empty(z.sizes(), z.options());
+            if (need_h) gh_i = at::empty(h.sizes(), f32);
+            if (need_b && it0) gb = at::empty(bias.sizes(), f32);
+            if (x.numel()) {
+                const NdcDesc d = make_desc(x, h0, c, it0);
+                const size_t bytes = ndc_bwd_workspace_bytes(&d);
+                if (!ws.defined()) ws = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
+                Span span(1);
+                check(ndc_bwd(&d, ptr(x), ptr(z), ptr(t1), fptr(h), it0 ? fptr(b) : nullptr, ptr(g), ptr(gx_i),
+                              ptr(gz), fptr(gh_i), it0 ? fptr(gb) : nullptr, ptr(ws), bytes, stream()),
+                      ndc_last_error());
+            } else {
+                for (Tensor* t : {&gx_i, &gz, &gh_i, &gb}) if (t->defined()) t->zero_();
+            }
+            if (need_x) { if (gx.defined()) gx.add_(gx_i); else gx = gx_i; }
+            if (need_h) { if (gh.defined()) gh.add_(gh_i); else gh = gh_i; }
+            g = gz;
+        }
+        ws.reset();
+        Tensor gw, gh0, gbias;
+        if (whole) {
+            // gz of the first update: W^T gz is added to the update's own input gradient
+            if (need_x) channel_gemm(w, true, g, gx, x.size(0), n, true);
+            if (need_w) gw = weight_grad(g, x, w, x.size(0), n);
+        }
+        const bool same = !need_b || !need_h || bias.scalar_type() == h0.scalar_type();
+        if ((need_h || need_b) && kernel_dtype(need_h ? h0 : bias) && same) {
+            if (need_h) gh0 = at::empty(h0.sizes(), h0.options());
+            const bool convert = need_b && bias.scalar_type() != at::kFloat;
+            gbias = convert ? at::empty(bias.sizes(), bias.options()) : gb;
+            if (need_h || convert)
+                check(ndc_params_grad(dtype_code(need_h ? h0 : bias), need_h ? ptr(h0) : nullptr, fptr(gh),
+                                      need_h ? h0.numel() : 0, ptr(gh0), convert ? fptr(gb) : nullptr,
+                                      convert ? bias.numel() : 0, convert ? ptr(gbias) : nullptr, stream()),
+                      ndc_proj_last_error());
+        } else {
+            if (need_h) gh0 = gh.mul_(h0 > 0).to(h0.scalar_type());
+            if (need_b) gbias = gb.to(bias.scalar_type());
+        }
+        variable_list out(11);
+        out[0] = gx; out[1] = gh0; out[2] = gw; out[3] = gbias;
+        return out;
+    }
+};
+
+// s of the layer.  `h0` (C, sc, *k), `w` (groups*sc, C, 1), `bias` (groups*sc) or None.
+Tensor layer(const Tensor& x_in, const Tensor& h0_in, const Tensor& w_in, const std::optional<Tensor>& bias_in,
+             int64_t groups, int64_t m, int64_t sc, double eps, int64_t iters, int64_t grad_iters, int64_t flags) {
+    TORCH_CHECK(w_in.scalar_type() == x_in.scalar_type(), "deconver_b200: the input is ", x_in.scalar_type(),
+                " but the projection's weight is ", w_in.scalar_type());
+    for (const Tensor* t : {&h0_in, &w_in})
+        TORCH_CHECK(t->device() == x_in.device(), "deconver_b200: input on ", x_in.device(), ", parameters on ", t->device());
+    TORCH_CHECK(x_in.size(1) == groups * m && w_in.size(0) == groups * sc && w_in.size(1) == x_in.size(1) &&
+                h0_in.dim() == x_in.dim() && h0_in.size(0) == groups * m && h0_in.size(1) == sc,
+                "deconver_b200: input ", x_in.sizes(), ", filter ", h0_in.sizes(), " and projection ", w_in.sizes(),
+                " do not match groups=", groups, ", m=", m, ", sc=", sc);
+    TORCH_CHECK(!bias_in || (bias_in->device() == x_in.device() && bias_in->numel() == groups * sc),
+                "deconver_b200: the bias does not match the projection");
+    c10::cuda::CUDAGuard guard(x_in.device());
+    const Tensor x = x_in.contiguous(), h0 = h0_in.contiguous(), w = w_in.contiguous();
+    const std::optional<Tensor> bias = bias_in ? std::optional<Tensor>(bias_in->contiguous()) : std::nullopt;
+    const bool grad = at::GradMode::is_enabled() &&
+                      (x.requires_grad() || h0.requires_grad() || w.requires_grad() || (bias && bias->requires_grad()));
+    if (grad && grad_iters > 0)
+        return LayerNode::apply(x, h0, w, bias, groups, m, sc, eps, iters, grad_iters, flags);
+    at::AutoDispatchBelowADInplaceOrView below;
+    return run_forward(x, h0, w, bias ? *bias : Tensor(), Config{groups, m, sc, eps, iters, grad_iters, flags}, nullptr);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod) {
+    mod.def("layer", &layer, py::call_guard<py::gil_scoped_release>());
+    mod.def("timing_enable", &timing_enable);
+    mod.def("timing_collect", &timing_collect);
+}

@@ -3,8 +3,8 @@
 `Deconv` keeps the constructor, the methods and the state-dict keys of the reference's
 `deconver/deconvolution/deconv.py:48-295` (`init.h0`, `init.linear.linear.weight`,
 `init.linear.linear.bias`), so it can stand in for it inside `DeconvMixer` unchanged.  What
-differs is the dispatch: there is exactly one compute path, the CUDA kernels behind
-`deconv_update`.  Configurations they do not cover raise `NotImplementedError`; there is no
+differs is the dispatch: there is exactly one compute path, the CUDA kernels that
+`deconv_update` runs too.  Configurations they do not cover raise `NotImplementedError`; there is no
 Triton path, no eager path and no CPU path to fall back to.
 """
 
@@ -16,10 +16,13 @@ import torch
 import torch.nn.functional as F
 from torch import Tensor, nn
 
-from .functional import deconv_update, kernels_apply
-from .linear import Linear, conv1x1
+from ._lib import load_ext
+from .functional import current_flags, kernels_apply, warn_if_generic
+from .linear import Linear
 
 __all__ = ["Initializer", "Deconv", "NDC"]
+
+_checked = set()     # (dtype, shape, filter geometry) of inputs found to be supported
 
 _CONV = {1: F.conv1d, 2: F.conv2d, 3: F.conv3d}
 
@@ -130,33 +133,28 @@ class Deconv(nn.Module):
             return torch.no_grad()
         return nullcontext()
 
-    def _fit(self, x: Tensor) -> tuple[Tensor, Tensor]:
-        reason = self.unsupported_reason(x)
-        if reason is not None:
-            raise NotImplementedError(f"deconver_b200.Deconv: {reason}")
-        x = x.contiguous()
-        h = F.relu(self.init.h0)  # batch-invariant
-        # the source enters the update pre-ReLU and pre-bias: the kernels apply both on load
-        projection = self.init.linear.linear
-        s = conv1x1(x.flatten(2), projection.weight)
-        s = s.view(x.shape[0], -1, *x.shape[2:])
-        bias = projection.bias
-        rectify = True
-        for it in range(1, self.num_iters + 1):
-            with self.context(it):
-                s = deconv_update(
-                    x, s, h, bias,
-                    groups=self.groups, m=self.filter_channels, sc=self.source_channels,
-                    eps=self.eps, relu_input=rectify,
-                )
-            rectify = False
-            bias = None  # later iterations start from an already biased, rectified source
-        return s, h
+    def _source(self, x: Tensor) -> Tensor:
+        """The fitted source: projection and updates in one native autograd node
+        (`csrc/ndc_torch.cpp`), whose bias and ReLU the update kernels apply on load."""
+        # a geometry that has run before only needs what can change between calls looked at
+        key = (x.dtype, x.shape, self.kernel_size, self.filter_channels, self.source_channels)
+        if (key not in _checked or not x.is_cuda or self.update_filter or not self.update_source
+                or self.verbose or self._conv_kwargs or self.num_iters < 1 or torch.is_autocast_enabled("cuda")):
+            reason = self.unsupported_reason(x)
+            if reason is not None:
+                raise NotImplementedError(f"deconver_b200.Deconv: {reason}")
+            warn_if_generic(x, self.groups, self.filter_channels, self.source_channels, self.kernel_size)
+            if len(_checked) < 4096:
+                _checked.add(key)
+        init = self.init
+        projection = init.linear.linear
+        return load_ext().layer(x, init.h0, projection.weight, projection.bias, self.groups, self.filter_channels,
+                                self.source_channels, self.eps, self.num_iters, self.num_grad_iters, current_flags())
 
     # ----------------------------------------------------------------- interface
 
     def fit(self, x: Tensor) -> tuple[Tensor, Tensor]:
-        s, h = self._fit(x)
+        s, h = self._source(x), F.relu(self.init.h0)
         # the filter is reported in its batched form, as the reference does
         return s, h.expand(x.shape[0], *h.shape).contiguous()
 
@@ -182,7 +180,7 @@ class Deconv(nn.Module):
         return num / den
 
     def forward(self, x: Tensor) -> Tensor:
-        return self._fit(x)[0]
+        return self._source(x)
 
 
 NDC = Deconv

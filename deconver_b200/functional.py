@@ -66,6 +66,7 @@ class _Timing:
 
     def enable(self) -> None:
         self._events = {"ndc_fwd": [], "ndc_bwd": []}
+        _lib.load_ext().timing_enable()     # the calls the layer's native path makes
         self.enabled = True
 
     def span(self, name: str):
@@ -85,7 +86,8 @@ class _Timing:
     def disable_and_collect(self):
         self.enabled = False
         torch.cuda.synchronize()
-        return {k: [a.elapsed_time(b) for a, b in v] for k, v in self._events.items()}
+        native = dict(zip(("ndc_fwd", "ndc_bwd"), _lib.load_ext().timing_collect()))
+        return {k: [a.elapsed_time(b) for a, b in v] + native[k] for k, v in self._events.items()}
 
 
 timing = _Timing()
@@ -141,6 +143,16 @@ def _warn_if_generic(desc, flags: int) -> None:
             f"({desc.D},{desc.H},{desc.W}) runs on the generic kernels (about 20x slower per voxel); "
             "the tiled kernels cover 3x3x3 volumes up to 256 columns and 5x5 / 3x3 images up to 512",
             RuntimeWarning, stacklevel=3)
+
+
+def current_flags() -> int:
+    return _flags
+
+
+def warn_if_generic(x: Tensor, groups: int, m: int, sc: int, kernel_size: Sequence[int]) -> None:
+    """`_warn_if_generic` for an input that has not been described yet."""
+    if x.numel():
+        _warn_if_generic(_desc(x, groups, m, sc, kernel_size, 0.0, True), _flags)
 
 
 def _require(t: Optional[Tensor], name: str, like: Tensor) -> None:

@@ -233,6 +233,34 @@ int ndc_bias_gelu_bwd(int32_t batch, int32_t channels, int64_t spatial, int32_t 
                       void *workspace, size_t workspace_bytes, void *stream);
 
 /*
+ * What the layer needs around its projection GEMM (deconver/deconvolution/deconv.py:20-45, :162).
+ *     ndc_proj_wgrad      gw[o, c] = sum_{b, p} gy[b, o, p] * x[b, c, p], the weight gradient of a
+ *                         1x1 convolution; gy (batch, co, spatial), x (batch, ci, spatial) and gw
+ *                         (co, ci) of dtype `dtype`, float32 accumulation, fixed summation order.
+ *                         float32 operands: TF32 products where `tf32` is non-zero, else each
+ *                         operand is split in two TF32 terms (three products).  Needs
+ *                         ndc_proj_wgrad_workspace_bytes(...) bytes of device scratch.
+ *     ndc_proj_sum        gw[e] = sum over `slices` float32 partial products of n elements each, in a
+ *                         fixed order, converted to dtype `dtype`: the second half of a weight
+ *                         gradient whose partial products the caller computed itself
+ *     ndc_params_prepare  h = relu(h0), b = bias as float32 (nh and nb elements of dtype `dtype`;
+ *                         nb may be 0, then bias and b may be NULL)
+ *     ndc_params_grad     gh0 = h0 > 0 ? gh : 0 and gbias = gb, converted to dtype `dtype` (nh or
+ *                         nb may be 0, then the pointers of that part may be NULL)
+ * Errors: status code, message from ndc_proj_last_error().
+ */
+size_t ndc_proj_wgrad_workspace_bytes(int32_t batch, int32_t co, int32_t ci, int64_t spatial);
+const char *ndc_proj_last_error(void);
+int ndc_proj_wgrad(int32_t batch, int32_t co, int32_t ci, int64_t spatial, int32_t dtype, int32_t tf32,
+                   const void *gy, const void *x, void *gw, void *workspace, size_t workspace_bytes,
+                   void *stream);
+int ndc_proj_sum(int32_t slices, int64_t n, int32_t dtype, const float *partial, void *gw, void *stream);
+int ndc_params_prepare(int32_t dtype, const void *h0, int64_t nh, float *h, const void *bias,
+                       int64_t nb, float *b, void *stream);
+int ndc_params_grad(int32_t dtype, const void *h0, const float *gh, int64_t nh, void *gh0,
+                    const float *gb, int64_t nb, void *gbias, void *stream);
+
+/*
  * Measurement aid; no counterpart in the reference project.  Launches one kernel of
  * register-only fused multiply-add chains (4 blocks of 256 threads per multiprocessor, 8
  * independent chains per thread, iters x 64 instructions per thread) on `stream`: plain

@@ -1,0 +1,72 @@
+"""The projection's weight gradient and the native layer, against float64 and `deconv_update`."""
+
+import pytest
+import torch
+
+import deconver_b200 as dcb
+from deconver_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,tf32,tol", [(torch.float32, 1, 2e-3), (torch.float32, 0, 1e-5),
+                                            (torch.bfloat16, 0, 6e-3)], ids=["tf32", "f32", "bf16"])
+@pytest.mark.parametrize("batch,co,ci,n", [
+    (1, 1, 1, 1), (2, 4, 1, 3), (1, 128, 64, 512), (2, 129, 65, 1023), (3, 64, 16, 514),
+    (2, 200, 48, 4097), (1, 2048, 512, 256), (1, 16, 130, 40000),
+])
+def test_weight_gradient(dtype, tf32, tol, batch, co, ci, n):
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(co + n)
+    gy = torch.randn(batch, co, n, device=dev, generator=gen).to(dtype)
+    x = torch.randn(batch, ci, n, device=dev, generator=gen).to(dtype)
+    gw = torch.empty(co, ci, device=dev, dtype=dtype)
+    nbytes = lib.ndc_proj_wgrad_workspace_bytes(batch, co, ci, n)
+    ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    args = (batch, co, ci, n, _lib.NDC_BF16 if dtype == torch.bfloat16 else _lib.NDC_F32, tf32, gy.data_ptr(),
+            x.data_ptr(), gw.data_ptr(), ws.data_ptr())
+    st = torch.cuda.current_stream().cuda_stream
+    assert lib.ndc_proj_wgrad(*args, nbytes, st) == _lib.NDC_OK, lib.ndc_proj_last_error()
+    ref = torch.einsum("bon,bcn->oc", gy.double(), x.double())
+    err = ((gw.double() - ref).norm() / ref.norm()).item()
+    assert err < tol, err
+    assert lib.ndc_proj_wgrad(*args, nbytes - 4, st) == 3      # a short workspace is refused
+
+
+@pytest.mark.parametrize("num_iters,num_grad_iters", [(1, 1), (3, 3), (3, 1), (2, 0)])
+@pytest.mark.parametrize("channels,spatial,ks,groups", [(8, (5, 9, 7), (3, 3, 3), 8), (8, (12, 20), (5, 5), 8),
+                                                        (8, (9, 10), (3, 3), 2), (192, (4, 8), (3, 3), 192)])
+def test_layer_is_its_projection_followed_by_the_updates(num_iters, num_grad_iters, channels, spatial, ks, groups):
+    """The native layer against `deconv_update` on a float64-accurate projection, every gradient."""
+    dev = torch.device("cuda:0")
+    torch.manual_seed(3)
+    old = torch.backends.cudnn.allow_tf32
+    torch.backends.cudnn.allow_tf32 = False
+    try:
+        mod = dcb.Deconv(channels, ks, ratio=2 if groups == 2 else 4, groups=groups, num_iters=num_iters,
+                         num_grad_iters=num_grad_iters).to(dev)
+        with torch.no_grad():
+            mod.init.linear.linear.bias += 1.0
+        x = torch.rand(2, channels, *spatial, device=dev)
+        g = torch.randn(2, mod.groups * mod.source_channels, *spatial, device=dev)
+        params = [mod.init.h0, mod.init.linear.linear.weight, mod.init.linear.linear.bias]
+        xa = x.clone().requires_grad_(True)
+        out = mod(xa)
+        got = [out] + (list(torch.autograd.grad(out, [xa] + params, g, allow_unused=True)) if num_grad_iters else [])
+        xb = x.clone().requires_grad_(True)
+        h = torch.relu(mod.init.h0)
+        s = (params[1][:, :, 0].double() @ xb.flatten(2).double()).float().view(2, -1, *spatial)
+        bias = params[2]
+        for it in range(1, num_iters + 1):
+            with mod.context(it):
+                s = dcb.deconv_update(xb, s, h, bias, groups=mod.groups, m=mod.filter_channels,
+                                      sc=mod.source_channels, eps=mod.eps, relu_input=it == 1)
+            bias = None
+        ref = [s] + (list(torch.autograd.grad(s, [xb] + params, g, allow_unused=True)) if num_grad_iters else [])
+    finally:
+        torch.backends.cudnn.allow_tf32 = old
+    assert out.requires_grad == bool(num_grad_iters)
+    for a, b in zip(got, ref):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert ((a - b).abs().max() / b.abs().max().clamp_min(1e-30)).item() < 1e-3
