@@ -33,6 +33,7 @@ NVCC_FLAGS = [
 # (object name, source, extra defines)
 UNITS = [("abi", "ndc_abi.cu", []), ("inorm", "ndc_inorm.cu", []), ("bias", "ndc_bias.cu", []),
          ("proj", "ndc_proj.cu", [])] + [
+    ("tile_t%d" % t, "ndc_tile_inst.cu", ["-DNDC_TILE_T=%d" % t]) for t in (0, 1)] + [
     ("dw4_p%d_t%d" % (part, t), "ndc_dw4_inst.cu", ["-DNDC_DW4_PART=%d" % part, "-DNDC_DW4_T=%d" % t])
     for part in (1, 2, 0) for t in (0, 1)   # the longest units first
 ]

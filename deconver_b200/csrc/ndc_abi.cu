@@ -9,6 +9,8 @@
 #include "ndc_generic.cuh"
 #define NDC_DW4_EXTERN   // the tiled kernels are compiled in ndc_dw4_inst.cu
 #include "ndc_dw4_host.cuh"
+#define NDC_TILE_EXTERN  // compiled in ndc_tile_inst.cu
+#include "ndc_tile.cuh"
 
 namespace {
 
@@ -72,6 +74,11 @@ int path_of(const NdcDesc* d) {
     const ndc::Geo g = ndc::make_geo(*d, false);
     if (!ndc::dw4::covers(g)) return NDC_PATH_GENERIC;
     return ndc::dw4::rows_class(g) ? NDC_PATH_DEPTHWISE4_ROWS : NDC_PATH_DEPTHWISE4;
+}
+
+// Geometries outside the depthwise ratio-4 kernels: the tile kernels where they take them.
+bool tile_path(const NdcDesc* d, const ndc::Geo& g) {
+    return !(d->flags & NDC_FLAG_FORCE_GENERIC) && ndc::tile::covers(g);
 }
 
 }  // namespace
@@ -175,6 +182,14 @@ int ndc_fwd(const NdcDesc* desc, const void* x, const void* z, const float* h, c
         if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (depthwise) launch");
         if (handled) return NDC_OK;
     }
+    if (tile_path(desc, g)) {
+        if (desc->dtype == NDC_F32)
+            e = ndc::tile::forward<float>(g, (const float*)x, (const float*)z, h, bias, (float*)out, (float*)t1, st);
+        else
+            e = ndc::tile::forward<bf16>(g, (const bf16*)x, (const bf16*)z, h, bias, (bf16*)out, (bf16*)t1, st);
+        if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (tile) launch");
+        return NDC_OK;
+    }
     if (desc->dtype == NDC_F32)
         e = ndc::generic::forward<float>(g, (const float*)x, (const float*)z, h, bias, (float*)out,
                                          (float*)t1, st);
@@ -192,6 +207,7 @@ size_t ndc_bwd_workspace_bytes(const NdcDesc* desc) {
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) return p.bytes;
     }
+    if (tile_path(desc, g)) return ndc::tile::bwd_scratch(g).bytes;
     return ndc::generic::bwd_scratch(g).bytes;
 }
 
@@ -236,6 +252,17 @@ int ndc_bwd(const NdcDesc* desc, const void* x, const void* z, const void* t1, c
             if (e != cudaSuccess) return cuda_fail(e, "ndc_bwd (depthwise) launch");
             return NDC_OK;
         }
+    }
+    if (tile_path(desc, g)) {
+        typedef __nv_bfloat16 bf16;
+        if (desc->dtype == NDC_F32)
+            e = ndc::tile::backward<float>(g, (const float*)x, (const float*)z, (const float*)t1, h, bias,
+                                           (const float*)gout, (float*)gx, (float*)gz, gh, gb, workspace, st);
+        else
+            e = ndc::tile::backward<bf16>(g, (const bf16*)x, (const bf16*)z, (const bf16*)t1, h, bias,
+                                          (const bf16*)gout, (bf16*)gx, (bf16*)gz, gh, gb, workspace, st);
+        if (e != cudaSuccess) return cuda_fail(e, "ndc_bwd (tile) launch");
+        return NDC_OK;
     }
     if (desc->dtype == NDC_F32)
         e = ndc::generic::backward<float>(g, (const float*)x, (const float*)z, (const float*)t1, h,

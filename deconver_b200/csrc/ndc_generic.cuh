@@ -2,7 +2,8 @@
 //
 // One thread per output element, taps looped at run time, operands read through L1/L2.
 // These cover every filter geometry; the depthwise ratio-4 geometries of the published
-// configurations run on the tiled kernels in ndc_dw4_*.cuh instead.
+// configurations run on the tiled kernels in ndc_dw4_*.cuh instead, other groupings with 3x3x3, 5x5
+// and 3x3 filters on those in ndc_tile.cuh.
 #pragma once
 
 #include "ndc_common.cuh"

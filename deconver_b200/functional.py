@@ -140,8 +140,8 @@ def _warn_if_generic(desc, flags: int) -> None:
         _warned_generic.add(key)
         warnings.warn(
             f"deconver_b200: depthwise ratio-4 update with kernel ({desc.kD},{desc.kH},{desc.kW}) on "
-            f"({desc.D},{desc.H},{desc.W}) runs on the generic kernels (about 20x slower per voxel); "
-            "the tiled kernels cover 3x3x3 volumes up to 256 columns and 5x5 / 3x3 images up to 512",
+            f"({desc.D},{desc.H},{desc.W}) runs on the kernels for any geometry (several times slower per "
+            "voxel); the depthwise ones cover 3x3x3 volumes up to 256 columns and 5x5 / 3x3 images up to 512",
             RuntimeWarning, stacklevel=3)
 
 

@@ -55,7 +55,8 @@ enum NdcFlags {
 
 /* Which family of kernels a geometry runs on (informational; results are the same). */
 enum NdcPath {
-    NDC_PATH_GENERIC = 0, /* any m, sc <= 16, any odd kernel with <= 343 taps                */
+    NDC_PATH_GENERIC = 0, /* any m, sc <= 16, any odd kernel with <= 343 taps (3x3x3, 1x5x5 and
+                             1x3x3 kernels staged tile by tile)                              */
     NDC_PATH_DEPTHWISE4 = 1, /* m = 1, sc = 4, kernel 3x3x3, 1x5x5 or 1x3x3: tiled, fused    */
     NDC_PATH_DEPTHWISE4_ROWS = 2 /* the same kernels marching down the rows of 2-D images:
                                     5x5 or 3x3, up to 512 columns, at least 8 rows, enough
