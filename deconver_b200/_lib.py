@@ -24,6 +24,7 @@ SYMBOLS = (
     "ndc_inorm_bwd", "ndc_bias_grad_workspace_bytes", "ndc_bias_last_error", "ndc_bias_add",
     "ndc_bias_grad", "ndc_bias_gelu_fwd", "ndc_bias_gelu_bwd", "ndc_proj_wgrad_workspace_bytes",
     "ndc_proj_last_error", "ndc_proj_wgrad", "ndc_proj_sum", "ndc_params_prepare", "ndc_params_grad",
+    "ndc_row_pitch", "ndc_fwd_rows", "ndc_bwd_rows_workspace_bytes", "ndc_bwd_rows", "ndc_pad_rows", "ndc_unpad_rows",
 )
 
 
@@ -77,6 +78,18 @@ def load():
     lib.ndc_bwd.argtypes = [dp, vp, vp, vp, fp, fp, vp, vp, vp, fp, fp, vp, ctypes.c_size_t, vp]
     lib.ndc_bwd_static.restype = ctypes.c_int
     lib.ndc_bwd_static.argtypes = [dp, vp, vp, vp, fp, fp, vp, vp, vp, fp, fp, vp]
+    i32 = ctypes.c_int32
+    lib.ndc_row_pitch.restype = i32
+    lib.ndc_row_pitch.argtypes = [dp]
+    lib.ndc_fwd_rows.restype = ctypes.c_int
+    lib.ndc_fwd_rows.argtypes = [dp, i32, i32, vp, vp, fp, fp, vp, vp, vp]
+    lib.ndc_bwd_rows_workspace_bytes.restype = ctypes.c_size_t
+    lib.ndc_bwd_rows_workspace_bytes.argtypes = [dp, i32]
+    lib.ndc_bwd_rows.restype = ctypes.c_int
+    lib.ndc_bwd_rows.argtypes = [dp, i32, i32, vp, vp, vp, fp, fp, vp, vp, vp, fp, fp, vp, ctypes.c_size_t, vp]
+    for name in ("ndc_pad_rows", "ndc_unpad_rows"):
+        getattr(lib, name).restype = ctypes.c_int
+        getattr(lib, name).argtypes = [ctypes.c_int64, i32, i32, i32, vp, vp, vp]
     lib.ndc_gconv.restype = ctypes.c_int
     lib.ndc_gconv.argtypes = [dp, vp, fp, fp, ctypes.c_int32, vp, vp]
     lib.ndc_probe_fp32_fma.restype = ctypes.c_int

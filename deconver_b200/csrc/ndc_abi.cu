@@ -2,6 +2,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 
 #include "ndc_b200.h"
@@ -69,9 +70,9 @@ int check_ptr(const void* p, const char* name, int dtype) {
         if (_st != NDC_OK) return _st; \
     } while (0)
 
-int path_of(const NdcDesc* d) {
+int path_of(const NdcDesc* d, int pitch) {
     if (d->flags & NDC_FLAG_FORCE_GENERIC) return NDC_PATH_GENERIC;
-    const ndc::Geo g = ndc::make_geo(*d, false);
+    const ndc::Geo g = ndc::make_geo(*d, false, pitch, pitch);
     if (!ndc::dw4::covers(g)) return NDC_PATH_GENERIC;
     return ndc::dw4::rows_class(g) ? NDC_PATH_DEPTHWISE4_ROWS : NDC_PATH_DEPTHWISE4;
 }
@@ -79,6 +80,22 @@ int path_of(const NdcDesc* d) {
 // Geometries outside the depthwise ratio-4 kernels: the tile kernels where they take them.
 bool tile_path(const NdcDesc* d, const ndc::Geo& g) {
     return !(d->flags & NDC_FLAG_FORCE_GENERIC) && ndc::tile::covers(g);
+}
+
+// Padded rows: a multiple of 4 elements, on the depthwise kernels only.
+int check_pitch(const NdcDesc* d, int pitch, int out_pitch) {
+    if (pitch != d->W && (pitch < d->W || pitch % 4 || path_of(d, pitch) == NDC_PATH_GENERIC))
+        return fail(NDC_ERR_UNSUPPORTED, "a row pitch of %d is not supported for %d columns", pitch, d->W);
+    if (out_pitch != d->W && out_pitch != pitch)
+        return fail(NDC_ERR_INVALID, "the row pitch of out / gout must be %d or %d (got %d)", d->W, pitch, out_pitch);
+    return NDC_OK;
+}
+
+int check_padded(std::initializer_list<const void*> tensors, int dtype) {
+    for (const void* p : tensors)
+        if ((uintptr_t)p % (dtype == NDC_BF16 ? 8 : 16))
+            return fail(NDC_ERR_ALIGNMENT, "tensors with padded rows must be aligned to four elements");
+    return NDC_OK;
 }
 
 }  // namespace
@@ -154,24 +171,42 @@ uint64_t ndc_launch_count(void) {
 
 int ndc_query(const NdcDesc* desc, int32_t* path) {
     NDC_TRY(validate(desc));
-    if (path) *path = path_of(desc);
+    if (path) *path = path_of(desc, desc->W);
     return NDC_OK;
 }
 
 int ndc_fwd(const NdcDesc* desc, const void* x, const void* z, const float* h, const float* bias,
             void* out, void* t1, void* stream) {
     NDC_TRY(validate(desc));
+    return ndc_fwd_rows(desc, desc->W, desc->W, x, z, h, bias, out, t1, stream);
+}
+
+int32_t ndc_row_pitch(const NdcDesc* desc) {
+    if (validate(desc) != NDC_OK) return 0;
+    const int W = desc->W;
+    if (W % 4 == 0 || W < 5) return W;
+    int pitch = (W + 3) / 4 * 4;
+    // bfloat16: whole 16-byte vectors in a channel, so that the projection's GEMMs load them
+    if (desc->dtype == NDC_BF16 && (long long)desc->D * desc->H * pitch % 8 && W >= 16) pitch = (W + 7) / 8 * 8;
+    return path_of(desc, pitch) == NDC_PATH_GENERIC ? W : pitch;
+}
+
+int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const void* x, const void* z,
+                 const float* h, const float* bias, void* out, void* t1, void* stream) {
+    NDC_TRY(validate(desc));
+    NDC_TRY(check_pitch(desc, pitch, out_pitch));
     NDC_TRY(check_ptr(x, "x", desc->dtype));
     NDC_TRY(check_ptr(z, "z", desc->dtype));
     NDC_TRY(check_ptr(h, "h", NDC_F32));
     NDC_TRY(check_ptr(out, "out", desc->dtype));
     NDC_TRY(check_ptr(t1, "t1", desc->dtype));
     if (bias) NDC_TRY(check_ptr(bias, "bias", NDC_F32));
-    const ndc::Geo g = ndc::make_geo(*desc, bias != nullptr);
+    if (pitch != desc->W) NDC_TRY(check_padded({x, z, t1}, desc->dtype));
+    const ndc::Geo g = ndc::make_geo(*desc, bias != nullptr, pitch, out_pitch);
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
     typedef __nv_bfloat16 bf16;
-    if (path_of(desc) != NDC_PATH_GENERIC) {
+    if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
         bool handled = false;
         if (desc->dtype == NDC_F32)
             e = ndc::dw4::forward<float>(g, (const float*)x, (const float*)z, h, bias, (float*)out,
@@ -201,9 +236,13 @@ int ndc_fwd(const NdcDesc* desc, const void* x, const void* z, const float* h, c
 }
 
 size_t ndc_bwd_workspace_bytes(const NdcDesc* desc) {
-    if (validate(desc) != NDC_OK) return 0;
-    const ndc::Geo g = ndc::make_geo(*desc, false);
-    if (path_of(desc) != NDC_PATH_GENERIC) {
+    return desc ? ndc_bwd_rows_workspace_bytes(desc, desc->W) : 0;
+}
+
+size_t ndc_bwd_rows_workspace_bytes(const NdcDesc* desc, int32_t pitch) {
+    if (validate(desc) != NDC_OK || check_pitch(desc, pitch, pitch) != NDC_OK) return 0;
+    const ndc::Geo g = ndc::make_geo(*desc, false, pitch, pitch);
+    if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) return p.bytes;
     }
@@ -215,6 +254,15 @@ int ndc_bwd(const NdcDesc* desc, const void* x, const void* z, const void* t1, c
             const float* bias, const void* gout, void* gx, void* gz, float* gh, float* gb,
             void* workspace, size_t workspace_bytes, void* stream) {
     NDC_TRY(validate(desc));
+    return ndc_bwd_rows(desc, desc->W, desc->W, x, z, t1, h, bias, gout, gx, gz, gh, gb, workspace,
+                        workspace_bytes, stream);
+}
+
+int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const void* x, const void* z,
+                 const void* t1, const float* h, const float* bias, const void* gout, void* gx, void* gz,
+                 float* gh, float* gb, void* workspace, size_t workspace_bytes, void* stream) {
+    NDC_TRY(validate(desc));
+    NDC_TRY(check_pitch(desc, pitch, gout_pitch));
     NDC_TRY(check_ptr(x, "x", desc->dtype));
     NDC_TRY(check_ptr(z, "z", desc->dtype));
     NDC_TRY(check_ptr(t1, "t1", desc->dtype));
@@ -225,18 +273,19 @@ int ndc_bwd(const NdcDesc* desc, const void* x, const void* z, const void* t1, c
     if (gz) NDC_TRY(check_ptr(gz, "gz", desc->dtype));
     if (gh) NDC_TRY(check_ptr(gh, "gh", NDC_F32));
     if (gb) NDC_TRY(check_ptr(gb, "gb", NDC_F32));
+    if (pitch != desc->W) NDC_TRY(check_padded({x, z, t1, gx, gz}, desc->dtype));
     if (gb && !gz) return fail(NDC_ERR_INVALID, "gb needs gz: pass a gz buffer when gb is wanted");
     if (!gx && !gz && !gh) return NDC_OK;  // nothing wanted
-    const size_t need = ndc_bwd_workspace_bytes(desc);
+    const size_t need = ndc_bwd_rows_workspace_bytes(desc, pitch);
     if (!workspace || workspace_bytes < need)
         return fail(NDC_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need,
                     workspace ? workspace_bytes : (size_t)0);
     if ((uintptr_t)workspace % 256)
         return fail(NDC_ERR_WORKSPACE, "workspace must be 256-byte aligned");
-    const ndc::Geo g = ndc::make_geo(*desc, bias != nullptr);
+    const ndc::Geo g = ndc::make_geo(*desc, bias != nullptr, pitch, gout_pitch);
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
-    if (path_of(desc) != NDC_PATH_GENERIC) {
+    if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) {
             typedef __nv_bfloat16 bf16;

@@ -27,6 +27,11 @@ struct Geo {
     int pD, pH, pW;
     int KT;        // taps
     long long SP;  // D*H*W
+    // Rows may be padded: W is then the row pitch of every tensor but out / gout, a multiple of 4,
+    // and only the first Wv (W - Wv < 4) columns are the volume's.  x is zero in the others on entry;
+    // t1, the backward's scratch and gz are written as zero there.  Wo: row pitch of out / gout,
+    // W or Wv.  Without padding Wv = Wo = W.
+    int Wv, Wo;
     float eps;
     int relu;      // rectify the source on load
     int has_bias;
@@ -40,9 +45,19 @@ inline Geo make_geo(const NdcDesc& d, bool has_bias) {
     g.pD = d.kD / 2; g.pH = d.kH / 2; g.pW = d.kW / 2;
     g.KT = d.kD * d.kH * d.kW;
     g.SP = (long long)d.D * d.H * d.W;
+    g.Wv = g.Wo = d.W;
     g.eps = d.eps;
     g.relu = d.relu_input ? 1 : 0;
     g.has_bias = has_bias ? 1 : 0;
+    return g;
+}
+
+// The same with padded rows of `pitch` elements, and out / gout rows of `out_pitch`.
+inline Geo make_geo(const NdcDesc& d, bool has_bias, int pitch, int out_pitch) {
+    Geo g = make_geo(d, has_bias);
+    g.W = pitch;
+    g.SP = (long long)d.D * d.H * pitch;
+    g.Wo = out_pitch;
     return g;
 }
 

@@ -55,6 +55,7 @@ struct RatioParams {
     Tiling t;
     float eps;
     int relu;
+    int Wv, Wo;   // columns of the volume, row pitch of out / gout (see Geo)
 };
 
 // Deterministic per-CTA combine of per-thread accumulators: every thread writes its NACC values
@@ -82,8 +83,9 @@ __device__ __forceinline__ void cta_combine(float* scratch, const float (&acc)[N
 //                  ksrc_kernel), used where it is faster than the fused fwd_kernel.
 enum RatioMode { kRatioPlanar = 0, kRatioPairs = 1, kRatioForward = 2 };
 
-template <typename T, int KD, int KH, int KW, int NT, int MAXX, bool VEC, int WQ, int MODE = kRatioPlanar>
+template <typename T, int KD, int KH, int KW, int NT, int MAXX, int AL, int WQ, int MODE = kRatioPlanar>
 __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P) {
+    constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr bool PAIRS = MODE == kRatioPairs, FWD = MODE == kRatioForward;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     using L = RingSmem<KD, KH, KW>;
@@ -94,8 +96,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
     const int tid = threadIdx.x;
     constexpr bool ROWS = KD > 1 && KH == 1;   // images of a batch as the rows of one volume
     const int NQ = WQ ? WQ : P.t.NQ, pitch = WQ ? row_pitch(4 * WQ) : P.t.pitch,
-              W = WQ ? 4 * WQ : P.W, D = P.D;   // WQ > 0: the width is a compile-time constant
-    const SlabAddr<ROWS> addr(P.C, D, P.H, W);
+              W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, Wo = PADDED ? P.Wo : W,
+              D = P.D;   // WQ > 0: the width is a compile-time constant
+    const SlabAddr<ROWS> addr(P.C, D, P.H, W), oaddr(P.C, D, P.H, Wo);
+    const long long RWO = ROWS ? oaddr.row_z : Wo;
     const long long HW = addr.plane, SP = addr.chan;
     const long long RWX = ROWS ? addr.row_x : W, RWZ = ROWS ? addr.row_z : W;
 
@@ -116,10 +120,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
     const T* xg = reinterpret_cast<const T*>(P.x) + bx;
     const T* tg = reinterpret_cast<const T*>(P.t1) + bx;
     const T* zg = reinterpret_cast<const T*>(P.z) + bz;
-    const T* gg = FWD ? nullptr : reinterpret_cast<const T*>(P.gout) + bz;
+    const long long bo = (long long)bc * SCH * oaddr.chan + (ROWS ? h_band * RWO : 0);
+    const T* gg = FWD ? nullptr : reinterpret_cast<const T*>(P.gout) + bo;
     float* gng = FWD ? nullptr : P.gnum + (PAIRS ? 2 * bz : bz);
     float* gdg = (PAIRS || FWD) ? nullptr : P.gden + bz;
-    T* dirg = P.gz ? reinterpret_cast<T*>(P.gz) + bz : nullptr;
+    T* dirg = P.gz ? reinterpret_cast<T*>(P.gz) + (FWD ? bo : bz) : nullptr;
 
     float* wA = smem + lay.wA;
     float* xring = smem + lay.ring0;
@@ -180,12 +185,16 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
             const int a_row = item / NQ, a_q = item % NQ;
             const int hrow = h0 + a_row, w0 = VA * a_q;
             const long long off = (long long)d * HW + hrow * RWZ;
+            const long long ooff = (long long)d * oaddr.plane + hrow * RWO;
             // global strips first: their latency hides behind the tap sweep
             Raw4<T> zraw[SCH], graw[FWD ? 1 : SCH];   // converted in the epilogue
 #pragma unroll
             for (int j = 0; j < SCH; ++j) {
                 zraw[j] = load_strip_raw<T, VEC>(zg + j * SP + off, w0, W);
-                if (!FWD) graw[FWD ? 0 : j] = load_strip_raw<T, VEC>(gg + j * SP + off, w0, W);
+                if (!FWD) {
+                    const T* grow = gg + j * oaddr.chan + ooff;
+                    graw[FWD ? 0 : j] = load_strip_raw<T, VEC && !PADDED>(grow, w0, Wv);
+                }
             }
             // accumulators hold channel pairs (2jp, 2jp+1) of one voxel
             f32x2 an2[SCH / 2][VA], ad2[SCH / 2][VA];
@@ -221,7 +230,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
                         if (P.relu) s = fmaxf(s, 0.0f);
                         dv[v] = fast_div(s * lane_of(an2[j / 2][v], j & 1), lane_of(ad2[j / 2][v], j & 1));
                     }
-                    store_strip_global<T, VEC, VA>(dirg + j * SP + off, w0, W, dv);
+                    T* orow = dirg + j * oaddr.chan + ooff;
+                    if (!PADDED || Wo == W) store_strip_global<T, VEC, VA>(orow, w0, W, dv);
+                    else store_strip_global<T, false, VA>(orow, w0, Wv, dv);
                     continue;
                 }
                 raw_to_array(graw[FWD ? 0 : j], gj);
@@ -236,7 +247,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
                     dv[v] = gr * n;
                     gdv[v] = -(gn * n) * r;
                     gnv[v] = gn;
-                    if (w0 + v >= W) { gnv[v] = 0.0f; gdv[v] = 0.0f; }
+                    if (w0 + v >= Wv) { gnv[v] = 0.0f; gdv[v] = 0.0f; }
                 }
                 if (PAIRS) {
                     float* dst = gng + 2 * (j * SP + off + w0);
@@ -283,6 +294,7 @@ struct KconvParams {
     const float* h;
     int C, D, H, W;
     Tiling t;
+    int Wv;                 // columns of the volume (see Geo)
 };
 
 template <int KD, int KH, int KW>
@@ -318,8 +330,9 @@ struct KconvSmem {
 // 16-byte chunks land on 16-byte quads, and an 8-voxel strip reads a 4-quad window.
 // The KD running sums and their aux strips never move between registers: plane q lives in
 // slot q mod KD, and the step body exists in KD rotated copies.
-template <typename T, int KD, int KH, int KW, int NT, bool VEC, bool WGRAD, int WQ>
+template <typename T, int KD, int KH, int KW, int NT, int AL, bool WGRAD, int WQ>
 __global__ void __launch_bounds__(NT, 384 / NT) kconv_kernel(const KconvParams P) {
+    constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2;
     using L = KconvSmem<KD, KH, KW>;
     constexpr int WKP = L::WKP, NSB = L::NSB, KT = KD * KH * KW;
@@ -330,7 +343,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) kconv_kernel(const KconvParams P
     const int tid = threadIdx.x;
     constexpr bool ROWS = KD > 1 && KH == 1;   // images of a batch as the rows of one volume
     const int NQ = WQ ? WQ : P.t.NQ, NS8 = (NQ + 1) / 2, pitch = WQ ? row_pitch(4 * WQ) : P.t.pitch,
-              W = WQ ? 4 * WQ : P.W, D = P.D;   // WQ > 0: the width is a compile-time constant
+              W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, D = P.D;   // WQ > 0: the width is a compile-time constant
     const SlabAddr<ROWS> addr(P.C, D, P.H, W);
     const long long HW = addr.plane, SP = addr.chan;
     const long long RWX = ROWS ? addr.row_x : W, RWZ = ROWS ? addr.row_z : W;
@@ -469,6 +482,10 @@ __global__ void __launch_bounds__(NT, 384 / NT) kconv_kernel(const KconvParams P
             const int w0 = VK * strip + (hi ? 4 : 0) + (odd ? 2 : 0);
             const long long off = (long long)q * HW + (h0 + row) * RWX + w0;
             if (VEC) {
+                if (PADDED) {   // zero in the padding
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) if (w0 + i >= Wv) o2[i] = 0.0f;
+                }
                 if (w0 < W) {
                     if (outf) *reinterpret_cast<float2*>(outf + off) = make_float2(o2[0], o2[1]);
                     else if (sizeof(T) == 4) *reinterpret_cast<float2*>(outt + off) = make_float2(o2[0], o2[1]);
@@ -478,8 +495,9 @@ __global__ void __launch_bounds__(NT, 384 / NT) kconv_kernel(const KconvParams P
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     if (w0 + i < W) {
-                        if (outf) outf[off + i] = o2[i];
-                        else outt[off + i] = from_f32<T>(o2[i]);
+                        const float o = o2[i];
+                        if (outf) outf[off + i] = o;
+                        else outt[off + i] = from_f32<T>(o);
                     }
             }
         }
@@ -621,6 +639,7 @@ struct Kconv2Params {
     const float* h;
     int C, D, H, W;
     Tiling t;
+    int Wv;                 // columns of the volume (see Geo)
 };
 
 template <int KD, int KH, int KW>
@@ -658,8 +677,9 @@ template <int NT, int VK> constexpr int kconv2_min_blocks() {
                    : (NT >= 256 ? 1 : NT >= 192 ? 2 : NT >= 128 ? 3 : 4);
 }
 
-template <typename T, int KD, int KH, int KW, int NT, int VK, int MAXC, bool VEC, bool WGRAD, int WQ>
+template <typename T, int KD, int KH, int KW, int NT, int VK, int MAXC, int AL, bool WGRAD, int WQ>
 __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel(const Kconv2Params P) {
+    constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     using L = Kconv2Smem<KD, KH, KW>;
     constexpr int KWP = L::KWP, NSB = L::NSB;
@@ -672,7 +692,7 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
     const L lay(P.t, NT);
     const int tid = threadIdx.x;
     const int NQ = WQ ? WQ : P.t.NQ, pitch2 = 2 * (WQ ? row_pitch(4 * WQ) : P.t.pitch),
-              W = WQ ? 4 * WQ : P.W, D = P.D;   // WQ > 0: the width is a compile-time constant
+              W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, D = P.D;   // WQ > 0: the width is a compile-time constant
     const int NSV = (4 * NQ + VK - 1) / VK;      // strips per row
     const long long HW = (long long)P.H * W, SP = HW * D;
     const int NC2 = 2 * NQ;
@@ -826,6 +846,10 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
         if (store) {
             const int w = VK * k_strip + (hi ? VK / 2 : 0) + (odd ? VO : 0);
             const long long off = (long long)q * HW + (long long)(h0 + k_row) * W + w;
+            if (PADDED) {   // zero in the padding
+#pragma unroll
+                for (int i = 0; i < VO; ++i) if (w + i >= Wv) { o_t[i] = 0.0f; o_x[i] = 0.0f; }
+            }
             if (VEC && VO == 2) {
                 if (w < W) {
                     if (gt1g) *reinterpret_cast<float2*>(gt1g + off) = make_float2(o_t[0], o_t[VO - 1]);
@@ -953,6 +977,7 @@ struct GzParams {
     int C, D, H, W;
     Tiling t;
     int relu;
+    int Wv;                     // columns of the volume (see Geo)
 };
 
 // Floats of shared memory the end-of-kernel combine of gz_kernel needs: one row of sums (+1 pad)
@@ -966,8 +991,9 @@ __host__ __device__ constexpr int gz_combine_floats(int nthreads) {
 // whole number of pairs).  The correlation sums are per channel, so CS = 2 halves the registers
 // a thread needs (54 + 2 sums instead of 108 + 4) and twice as many warps fit on an SM; the two
 // threads sit in adjacent lanes and read the same window quads.
-template <typename T, int KD, int KH, int KW, int NT, int MAXX, bool VEC, bool WGRAD, int WQ, int CS>
+template <typename T, int KD, int KH, int KW, int NT, int MAXX, int AL, bool WGRAD, int WQ, int CS>
 __global__ void __launch_bounds__(NT, CS == 2 ? 512 / NT : 256 / NT) gz_kernel(const GzParams P) {
+    constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     using L = RingSmem<KD, KH, KW>;
     constexpr int RING = L::RING;
@@ -983,7 +1009,7 @@ __global__ void __launch_bounds__(NT, CS == 2 ? 512 / NT : 256 / NT) gz_kernel(c
     const int part = tid % CS;            // which channels: part*CH .. part*CH + CH-1
     constexpr bool ROWS = KD > 1 && KH == 1;   // images of a batch as the rows of one volume
     const int NQ = WQ ? WQ : P.t.NQ, pitch = WQ ? row_pitch(4 * WQ) : P.t.pitch,
-              W = WQ ? 4 * WQ : P.W, D = P.D;   // WQ > 0: the width is a compile-time constant
+              W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, D = P.D;   // WQ > 0: the width is a compile-time constant
     const SlabAddr<ROWS> addr(P.C, D, P.H, W);
     const long long HW = addr.plane, SP = addr.chan;
     const long long RWX = ROWS ? addr.row_x : W, RWZ = ROWS ? addr.row_z : W;
@@ -1104,7 +1130,7 @@ __global__ void __launch_bounds__(NT, CS == 2 ? 512 / NT : 256 / NT) gz_kernel(c
                 for (int v = 0; v < VA; ++v) {
                     pre[j][v] = strips[j][v] + bj[j];
                     sv[j][v] = P.relu ? fmaxf(pre[j][v], 0.0f) : pre[j][v];
-                    if (w0 + v >= W) sv[j][v] = 0.0f;
+                    if (w0 + v >= Wv) sv[j][v] = 0.0f;
                 }
             }
             // channel pairs (2jp, 2jp+1) of one voxel share a register pair; the accumulators
@@ -1165,7 +1191,7 @@ __global__ void __launch_bounds__(NT, CS == 2 ? 512 / NT : 256 / NT) gz_kernel(c
                     for (int v = 0; v < VA; ++v) {
                         float r = lane_of(ag[j / 2][v], j & 1);
                         if (P.relu && !(pre[j][v] > 0.0f)) r = 0.0f;
-                        if (w0 + v >= W) r = 0.0f;
+                        if (w0 + v >= Wv) r = 0.0f;
                         dv[v] = r;
                         // the bias gradient sums the values as stored (rounded to the storage type)
                         gbs[j] += to_f32(from_f32<T>(r));

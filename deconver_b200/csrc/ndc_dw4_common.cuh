@@ -25,6 +25,11 @@ constexpr int SCH = 4;   // source channels per group
 constexpr int VA = 4;    // voxels per strip, A-type sweeps
 constexpr int VK = 8;    // voxels per strip, K-type sweeps
 
+// How a kernel's tensors lie: rows without vector access; whole vectors; or padded rows (see Geo)
+// with out / gout possibly unpadded.  A template parameter: as a run-time choice between two ways of
+// loading gout it cost ratio_kernel 30 % (the loads of a branch are waited for where it ends).
+enum Alignment { kScalar = 0, kVector = 1, kPadded = 2 };
+
 // Host-side tiling decision for one geometry.
 struct Tiling {
     int NQ;     // quads (4 voxels) per row = ceil(W/4)

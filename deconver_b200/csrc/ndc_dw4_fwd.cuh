@@ -35,6 +35,7 @@ struct FwdParams {
     Tiling t;
     float eps;
     int relu;
+    int Wv, Wo;   // columns of the volume, row pitch of out (see Geo)
 };
 
 template <int KD, int KH, int KW>
@@ -63,8 +64,9 @@ struct FwdSmem {
     }
 };
 
-template <typename T, int KD, int KH, int KW, int NT, int MAXZ, int MAXX, int MINB, bool VEC, int WQ>
+template <typename T, int KD, int KH, int KW, int NT, int MAXZ, int MAXX, int MINB, int AL, int WQ>
 __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
+    constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2;
     using L = FwdSmem<KD, KH, KW>;
     constexpr int WKP = L::WKP, RING = L::RING, NSB = L::NSB;
@@ -74,8 +76,10 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
     const int tid = threadIdx.x;
     constexpr bool ROWS = KD > 1 && KH == 1;   // images of a batch as the rows of one volume
     const int NQ = WQ ? WQ : P.t.NQ, NS8 = (NQ + 1) / 2, pitch = WQ ? row_pitch(4 * WQ) : P.t.pitch,
-              W = WQ ? 4 * WQ : P.W, D = P.D;   // WQ > 0: the width is a compile-time constant
-    const SlabAddr<ROWS> addr(P.C, D, P.H, W);
+              W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, Wo = PADDED ? P.Wo : W,
+              D = P.D;   // WQ > 0: the width is a compile-time constant
+    const SlabAddr<ROWS> addr(P.C, D, P.H, W), oaddr(P.C, D, P.H, Wo);
+    const long long RWO = ROWS ? oaddr.row_z : Wo;
     const long long HW = addr.plane, SP = addr.chan;
     const long long RWX = ROWS ? addr.row_x : W, RWZ = ROWS ? addr.row_z : W;
 
@@ -96,7 +100,7 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
 
     const T* xg = reinterpret_cast<const T*>(P.x) + bx;
     const T* zg = reinterpret_cast<const T*>(P.z) + bz;
-    T* og = reinterpret_cast<T*>(P.out) + bz;
+    T* og = reinterpret_cast<T*>(P.out) + (long long)bc * SCH * oaddr.chan + (ROWS ? h_band * RWO : 0);
     T* tg = reinterpret_cast<T*>(P.t1) + bx;
 
     float* wA = smem + lay.wA;
@@ -148,7 +152,7 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
             const int c4 = id % NQ, t = id / NQ, r = t % RS, ch = t / RS;
             const int h = h0 - 2 * PH + r, w = 4 * c4;
             if (h >= 0 && h < H) zg_off[i] = (int)(ch * SP + h * RWZ) + w;
-            zs_off[i] = z_soff(ch, r, c4, min(4, W - w));
+            zs_off[i] = z_soff(ch, r, c4, min(4, Wv - w));
             zb[i] = ch == 0 ? bj[0] : ch == 1 ? bj[1] : ch == 2 ? bj[2] : bj[3];
         }
     }
@@ -176,7 +180,7 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
             v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f);
             v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f);
         }
-        if (!VEC && n < 4) {  // elements past the end of the row stay zero
+        if ((!VEC || PADDED) && n < 4) {  // elements past the end of the row stay zero
             if (n < 2) v.y = 0.f;
             if (n < 3) v.z = 0.f;
             v.w = 0.f;
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
         float* dst = sbuf + (plane & (NSB - 1)) * lay.plane_s;
         for (int id = tid; id < nz; id += NT) {
             const int c4 = id % NQ, t = id / NQ, r = t % RS, ch = t / RS;
-            const int h = h0 - 2 * PH + r, w = 4 * c4, n = min(4, W - w);
+            const int h = h0 - 2 * PH + r, w = 4 * c4, n = min(4, Wv - w);
             if (h < 0 || h >= H) continue;
             const int soff = z_soff(ch, r, c4, n);
             const float4 v = load4<T, VEC>(src + ch * SP + h * RWZ + w, n);
@@ -317,7 +321,7 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
             // the ring holds t1 as it is stored (rounded to the storage type), so the
             // denominator here is the one backward recomputes from the saved t1
 #pragma unroll
-            for (int v = 0; v < VA; ++v) tv[v] = (w0 + v >= W) ? 0.0f : to_f32(from_f32<T>(tv[v]));
+            for (int v = 0; v < VA; ++v) tv[v] = (w0 + v >= Wv) ? 0.0f : to_f32(from_f32<T>(tv[v]));
             store_strip<VA, PW, false>(t1ring + slot_of(qdone) * lay.plane_t + row * pitch, w0, tv);
             const int h = h0 - PH + row;
             if (qdone >= d0 && qdone < d1 && row >= PH && row < PH + TH)
@@ -399,8 +403,9 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
                     if (P.relu) s = fmaxf(s, 0.0f);
                     ov[v] = fast_div(s * lane_of(an[j / 2][v], j & 1), lane_of(ad[j / 2][v], j & 1));
                 }
-                store_strip_global<T, VEC, VA>(og + j * SP + (long long)d * HW + hrow * RWZ,
-                                               w0, W, ov);
+                T* orow = og + j * oaddr.chan + (long long)d * oaddr.plane + hrow * RWO;
+                if (!PADDED || Wo == W) store_strip_global<T, VEC, VA>(orow, w0, W, ov);
+                else store_strip_global<T, false, VA>(orow, w0, Wv, ov);
             }
         }
     }

@@ -91,9 +91,9 @@ inline bool aligned_for_vec(const void* p, int dtype) {
     return ((uintptr_t)p % (dtype == NDC_BF16 ? 8 : 16)) == 0;
 }
 
-template <typename T, int KD, int KH, int KW, typename S, bool VEC, int WQ>
+template <typename T, int KD, int KH, int KW, typename S, int AL, int WQ>
 cudaError_t launch_fwd(const FwdParams& P, size_t smem_bytes, long long BC, cudaStream_t st) {
-    auto kern = fwd_kernel<T, KD, KH, KW, S::NT, S::MAXZ, S::MAXX, S::MINB, VEC, WQ>;
+    auto kern = fwd_kernel<T, KD, KH, KW, S::NT, S::MAXZ, S::MAXX, S::MINB, AL, WQ>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem_bytes);
     if (e != cudaSuccess) return e;
@@ -114,21 +114,23 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
     if (!handled) return cudaSuccess;
     P.x = x; P.z = z; P.h = h; P.bias = bias; P.out = out; P.t1 = t1;
     P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W;
-    P.eps = g.eps; P.relu = g.relu;
+    P.eps = g.eps; P.relu = g.relu; P.Wv = g.Wv; P.Wo = g.Wo;
     const bool vec = g.W % 4 == 0 && aligned_for_vec(x, dtype) && aligned_for_vec(z, dtype) &&
-                     aligned_for_vec(out, dtype) && aligned_for_vec(t1, dtype);
+                     (g.Wo != g.W || aligned_for_vec(out, dtype)) && aligned_for_vec(t1, dtype);
+    const bool whole = vec && g.Wv == g.W && g.Wo == g.W;   // no padding: compile-time widths apply
     // widths that occur in the published configurations get kernels with a compile-time width
     if constexpr (KD > 1 && KH > 1 && S::NT == 256) {
-        if (vec && g.W == 64) return launch_fwd<T, KD, KH, KW, S, true, 16>(P, smem, BC, st);
-        if (vec && g.W == 128) return launch_fwd<T, KD, KH, KW, S, true, 32>(P, smem, BC, st);
+        if (whole && g.W == 64) return launch_fwd<T, KD, KH, KW, S, kVector, 16>(P, smem, BC, st);
+        if (whole && g.W == 128) return launch_fwd<T, KD, KH, KW, S, kVector, 32>(P, smem, BC, st);
     }
     if constexpr (KD > 1 && KH == 1) {   // rows kernels: 256, 128 and 64 columns
-        if (vec && g.W == 4 * S::NT) return launch_fwd<T, KD, KH, KW, S, true, S::NT>(P, smem, BC, st);
-        if (vec && S::NT == 64 && g.W == 128) return launch_fwd<T, KD, KH, KW, S, true, 32>(P, smem, BC, st);
-        if (vec && S::NT == 64 && g.W == 64) return launch_fwd<T, KD, KH, KW, S, true, 16>(P, smem, BC, st);
+        if (whole && g.W == 4 * S::NT) return launch_fwd<T, KD, KH, KW, S, kVector, S::NT>(P, smem, BC, st);
+        if (whole && S::NT == 64 && g.W == 128) return launch_fwd<T, KD, KH, KW, S, kVector, 32>(P, smem, BC, st);
+        if (whole && S::NT == 64 && g.W == 64) return launch_fwd<T, KD, KH, KW, S, kVector, 16>(P, smem, BC, st);
     }
-    return vec ? launch_fwd<T, KD, KH, KW, S, true, 0>(P, smem, BC, st)
-               : launch_fwd<T, KD, KH, KW, S, false, 0>(P, smem, BC, st);
+    return whole ? launch_fwd<T, KD, KH, KW, S, kVector, 0>(P, smem, BC, st)
+         : vec ? launch_fwd<T, KD, KH, KW, S, kPadded, 0>(P, smem, BC, st)
+               : launch_fwd<T, KD, KH, KW, S, kScalar, 0>(P, smem, BC, st);
 }
 
 // ---------------------------------------------------------------------------- backward
@@ -381,7 +383,7 @@ inline cudaError_t set_smem(K kern, size_t bytes) {
         if (_e != cudaSuccess) return _e;       \
     } while (0)
 
-template <typename T, int KD, int KH, int KW, typename S, bool VEC, int WQ>
+template <typename T, int KD, int KH, int KW, typename S, int AL, int WQ>
 cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T* z, const T* t1,
                             const float* h, const float* bias, const T* gout, T* gx, T* gz,
                             float* gh, float* gb, void* ws, cudaStream_t st) {
@@ -398,7 +400,8 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.x = x; P.t1 = t1; P.z = z; P.gout = gout; P.h = h; P.bias = bias;
         P.gnum = gnum; P.gden = gden; P.gz = gz;
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.ratio; P.eps = g.eps; P.relu = g.relu;
-        auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, VEC, WQ, packed_kconv<KD, KH, KW>() ? kRatioPairs : kRatioPlanar>;
+        P.Wv = g.Wv; P.Wo = g.Wo;
+        auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD, KH, KW>() ? kRatioPairs : kRatioPlanar>;
         NDC_CUDA_TRY(set_smem(kern, p.smem_ratio));
         kern<<<(unsigned)p.n_ratio, S::RatioNT, p.smem_ratio, st>>>(P);
         launched();
@@ -410,15 +413,15 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.gx = gx;
         P.t1 = t1; P.x = x;
         P.partial = gh ? pa : nullptr;
-        P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv;
+        P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv; P.Wv = g.Wv;
         auto run = [&](auto nt, auto maxc) -> cudaError_t {
             constexpr int NT = decltype(nt)::value, VK = S::Kconv2VK, MAXC = decltype(maxc)::value;
             if (gh) {
-                auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, VEC, true, WQ>;
+                auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, AL, true, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
                 kern<<<(unsigned)p.n_kconv, NT, p.smem_kconv, st>>>(P);
             } else {
-                auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, VEC, false, WQ>;
+                auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, AL, false, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
                 kern<<<(unsigned)p.n_kconv, NT, p.smem_kconv, st>>>(P);
             }
@@ -450,15 +453,15 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         for (int i = n; i < 2; ++i) {
             P.in[i] = nullptr; P.out[i] = nullptr; P.out_is_f32[i] = 0; P.aux[i] = nullptr; P.partial[i] = nullptr;
         }
-        P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv;
+        P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv; P.Wv = g.Wv;
         if (n > 0) {
             dim3 grid((unsigned)p.n_kconv, n);
             if (gh) {
-                auto kern = kconv_kernel<T, KD, KH, KW, S::KconvNT, VEC, true, WQ>;
+                auto kern = kconv_kernel<T, KD, KH, KW, S::KconvNT, AL, true, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
                 kern<<<grid, S::KconvNT, p.smem_kconv, st>>>(P);
             } else {
-                auto kern = kconv_kernel<T, KD, KH, KW, S::KconvNT, VEC, false, WQ>;
+                auto kern = kconv_kernel<T, KD, KH, KW, S::KconvNT, AL, false, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
                 kern<<<grid, S::KconvNT, p.smem_kconv, st>>>(P);
             }
@@ -468,13 +471,13 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
     if (gz || gh) {
         GzParams P;
         P.gt1 = gt1; P.z = z; P.gz = gz; P.h = h; P.bias = bias; P.partial = pb;
-        P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.gz; P.relu = g.relu;
+        P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.gz; P.relu = g.relu; P.Wv = g.Wv;
         if (gh) {
-            auto kern = gz_kernel<T, KD, KH, KW, S::GzNT, S::GzMAXX, VEC, true, WQ, kGzCS>;
+            auto kern = gz_kernel<T, KD, KH, KW, S::GzNT, S::GzMAXX, AL, true, WQ, kGzCS>;
             NDC_CUDA_TRY(set_smem(kern, p.smem_gz));
             kern<<<(unsigned)p.n_gz, S::GzNT, p.smem_gz, st>>>(P);
         } else {
-            auto kern = gz_kernel<T, KD, KH, KW, S::GzNT, S::GzMAXX, VEC, false, WQ, kGzCS>;
+            auto kern = gz_kernel<T, KD, KH, KW, S::GzNT, S::GzMAXX, AL, false, WQ, kGzCS>;
             NDC_CUDA_TRY(set_smem(kern, p.smem_gz));
             kern<<<(unsigned)p.n_gz, S::GzNT, p.smem_gz, st>>>(P);
         }
@@ -500,26 +503,28 @@ cudaError_t backward_shape(const Geo& g, const BwdPlan& p, const T* x, const T* 
                            const float* h, const float* bias, const T* gout, T* gx, T* gz,
                            float* gh, float* gb, void* ws, int dtype, cudaStream_t st) {
     bool vec = g.W % 4 == 0 && aligned_for_vec(x, dtype) && aligned_for_vec(z, dtype) &&
-               aligned_for_vec(t1, dtype) && aligned_for_vec(gout, dtype);
+               aligned_for_vec(t1, dtype) && (g.Wo != g.W || aligned_for_vec(gout, dtype));
     if (gx) vec = vec && aligned_for_vec(gx, dtype);
     if (gz) vec = vec && aligned_for_vec(gz, dtype);
+    const bool whole = vec && g.Wv == g.W && g.Wo == g.W;   // no padding: compile-time widths apply
     // widths that occur in the published configurations get kernels with a compile-time width
     if constexpr (KD > 1 && KH > 1 && S::RatioNT == 128) {
-        if (vec && g.W == 64)
-            return backward_launch<T, KD, KH, KW, S, true, 16>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
-        if (vec && g.W == 128)
-            return backward_launch<T, KD, KH, KW, S, true, 32>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
+        if (whole && g.W == 64)
+            return backward_launch<T, KD, KH, KW, S, kVector, 16>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
+        if (whole && g.W == 128)
+            return backward_launch<T, KD, KH, KW, S, kVector, 32>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
     }
     if constexpr (KD > 1 && KH == 1) {   // rows kernels: 256, 128 and 64 columns
-        if (vec && g.W == 4 * S::RatioNT)
-            return backward_launch<T, KD, KH, KW, S, true, S::RatioNT>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
-        if (vec && S::RatioNT == 64 && g.W == 128)
-            return backward_launch<T, KD, KH, KW, S, true, 32>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
-        if (vec && S::RatioNT == 64 && g.W == 64)
-            return backward_launch<T, KD, KH, KW, S, true, 16>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
+        if (whole && g.W == 4 * S::RatioNT)
+            return backward_launch<T, KD, KH, KW, S, kVector, S::RatioNT>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
+        if (whole && S::RatioNT == 64 && g.W == 128)
+            return backward_launch<T, KD, KH, KW, S, kVector, 32>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
+        if (whole && S::RatioNT == 64 && g.W == 64)
+            return backward_launch<T, KD, KH, KW, S, kVector, 16>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
     }
-    return vec ? backward_launch<T, KD, KH, KW, S, true, 0>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st)
-               : backward_launch<T, KD, KH, KW, S, false, 0>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
+    return whole ? backward_launch<T, KD, KH, KW, S, kVector, 0>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st)
+         : vec ? backward_launch<T, KD, KH, KW, S, kPadded, 0>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st)
+               : backward_launch<T, KD, KH, KW, S, kScalar, 0>(g, p, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
 }
 
 template <typename T, int K>
@@ -592,10 +597,12 @@ cudaError_t launch_ksrc(const KsrcParams& P, size_t smem_bytes, long long BC, bo
         launched();
         return cudaSuccess;
     };
-    if (vec && P.W == 64) return go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, true, 16>);
-    if (vec && P.W == 128) return go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, true, 32>);
-    return vec ? go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, true, 0>)
-               : go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, false, 0>);
+    const bool whole = vec && P.Wv == P.W;
+    if (whole && P.W == 64) return go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, kVector, 16>);
+    if (whole && P.W == 128) return go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, kVector, 32>);
+    return whole ? go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, kVector, 0>)
+         : vec ? go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, kPadded, 0>)
+               : go(ksrc_kernel<T, KD, KH, KW, S::NT, S::MAXZP, S::MINB, kScalar, 0>);
 }
 
 template <typename T, int KD, int KH, int KW, typename S>
@@ -608,10 +615,12 @@ cudaError_t launch_ratio_forward(const RatioParams& P, size_t smem_bytes, long l
         launched();
         return cudaSuccess;
     };
-    if (vec && P.W == 64) return go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, true, 16, kRatioForward>);
-    if (vec && P.W == 128) return go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, true, 32, kRatioForward>);
-    return vec ? go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, true, 0, kRatioForward>)
-               : go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, false, 0, kRatioForward>);
+    const bool whole = vec && P.Wv == P.W && P.Wo == P.W;
+    if (whole && P.W == 64) return go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, kVector, 16, kRatioForward>);
+    if (whole && P.W == 128) return go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, kVector, 32, kRatioForward>);
+    return whole ? go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, kVector, 0, kRatioForward>)
+         : vec ? go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, kPadded, 0, kRatioForward>)
+               : go(ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, kScalar, 0, kRatioForward>);
 }
 
 template <typename T>
@@ -620,12 +629,12 @@ cudaError_t forward_split(const Geo& g, const T* x, const T* z, const float* h, 
     constexpr int KD = 3, KH = 3, KW = 3;
     const long long BC = (long long)g.B * g.G;
     const bool vec = g.W % 4 == 0 && aligned_for_vec(x, dtype) && aligned_for_vec(z, dtype) &&
-                     aligned_for_vec(out, dtype) && aligned_for_vec(t1, dtype);
+                     (g.Wo != g.W || aligned_for_vec(out, dtype)) && aligned_for_vec(t1, dtype);
     handled = false;
     // ---- K: the narrowest CTA that covers the volume with as few bands as the widest
     KsrcParams K;
     K.z = z; K.h = h; K.bias = bias; K.t1 = t1;
-    K.C = g.G; K.D = g.D; K.H = g.H; K.W = g.W; K.relu = g.relu;
+    K.C = g.G; K.D = g.D; K.H = g.H; K.W = g.W; K.relu = g.relu; K.Wv = g.Wv;
     Tiling t0, tk; size_t sm0 = 0, smk = 0;
     typedef KsrcShape<128, 3> K128; typedef KsrcShape<64, 6> K64; typedef KsrcShape<32, 12> K32;
     if (!plan_ksrc<KD, KH, KW, K128>(g.D, g.H, g.W, BC, t0, sm0)) return cudaSuccess;
@@ -633,7 +642,7 @@ cudaError_t forward_split(const Geo& g, const T* x, const T* z, const float* h, 
     RatioParams R;
     R.x = x; R.t1 = t1; R.z = z; R.gout = nullptr; R.h = h; R.bias = bias;
     R.gnum = nullptr; R.gden = nullptr; R.gz = out;
-    R.C = g.G; R.D = g.D; R.H = g.H; R.W = g.W; R.eps = g.eps; R.relu = g.relu;
+    R.C = g.G; R.D = g.D; R.H = g.H; R.W = g.W; R.eps = g.eps; R.relu = g.relu; R.Wv = g.Wv; R.Wo = g.Wo;
     Tiling r0; size_t smr0 = 0;
     if (!plan_ring<KD, KH, KW>(g.D, g.H, g.W, BC, 2, BwdBands::RatioNT, BwdBands::RatioMAXX, 0, 0,
                                56 * 1024, 512 / BwdBands::RatioNT, r0, smr0))

@@ -23,6 +23,7 @@ struct KsrcParams {
     int C, D, H, W;
     Tiling t;
     int relu;
+    int Wv;      // columns of the volume (< W: padded rows)
 };
 
 template <int KD, int KH, int KW>
@@ -48,8 +49,9 @@ struct KsrcSmem {
 // lanes of a quarter-warp hit eight different 16-byte bank groups.
 __device__ __forceinline__ int swz_strip8(int chunk) { return chunk ^ ((chunk >> 3) & 3); }
 
-template <typename T, int KD, int KH, int KW, int NT, int MAXZP, int MINB, bool VEC, int WQ>
+template <typename T, int KD, int KH, int KW, int NT, int MAXZP, int MINB, int AL, int WQ>
 __global__ void __launch_bounds__(NT, MINB) ksrc_kernel(const KsrcParams P) {
+    constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     using L = KsrcSmem<KD, KH, KW>;
     constexpr int NTK = L::NTK, NSB = L::NSB;
@@ -59,7 +61,7 @@ __global__ void __launch_bounds__(NT, MINB) ksrc_kernel(const KsrcParams P) {
     const int tid = threadIdx.x;
     const int NQ = WQ ? WQ : P.t.NQ, NS8 = (NQ + 1) / 2,
               pitch2 = 2 * (WQ ? row_pitch(4 * WQ) : P.t.pitch),
-              W = WQ ? 4 * WQ : P.W, D = P.D;   // WQ > 0: the width is a compile-time constant
+              W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, D = P.D;   // WQ > 0: the width is a compile-time constant
     const long long HW = (long long)P.H * W, SP = HW * D;
 
     int blk = blockIdx.x;
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(NT, MINB) ksrc_kernel(const KsrcParams P) {
             const int row = (cp * RS + r) * pitch2;
             zs0[i] = row + (swz_strip8(2 * c4 + 2) << 2);
             zs1[i] = row + (swz_strip8(2 * c4 + 3) << 2);
-            zn[i] = min(4, W - w);
+            zn[i] = min(4, Wv - w);
             zb0[i] = cp ? bj[2] : bj[0];
             zb1[i] = cp ? bj[3] : bj[1];
         }
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(NT, MINB) ksrc_kernel(const KsrcParams P) {
             v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f);
             v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f);
         }
-        if (!VEC && n < 4) {  // elements past the end of the row stay zero
+        if ((!VEC || PADDED) && n < 4) {  // elements past the end of the row stay zero
             if (n < 2) v.y = 0.f;
             if (n < 3) v.z = 0.f;
             v.w = 0.f;
@@ -223,6 +225,7 @@ __global__ void __launch_bounds__(NT, MINB) ksrc_kernel(const KsrcParams P) {
                 const float lo = a0 + a1, up = b0 + b1;
                 const float send = cpair ? lo : up, keep = cpair ? up : lo;
                 tv[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+                if (PADDED && VK * k_strip + VA * cpair + i >= Wv) tv[i] = 0.0f;   // padding
             }
             if (k_ok)
                 store_strip_global<T, VEC, VA>(tg + (long long)qdone * HW + (long long)(h0 + k_row) * W,

@@ -316,6 +316,55 @@ __global__ void __launch_bounds__(256) params_grad_kernel(const T* __restrict__ 
     else if (i - nh < nb) gbias[i - nh] = ndc::from_f32<T>(gb[i - nh]);
 }
 
+// ---- row padding ------------------------------------------------------------------------------
+// One thread per quad of a padded row: scalar accesses to the unpadded side (neighbouring threads
+// touch neighbouring quads), one vector access to the padded one.
+template <typename T> struct Quad;
+template <> struct Quad<float> { typedef float4 type; };
+template <> struct Quad<unsigned short> { typedef ushort4 type; };
+
+template <typename T, bool PAD>
+__global__ void __launch_bounds__(256) rows_kernel(const T* __restrict__ src, T* __restrict__ dst, long long quads, int W, int nq) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= quads) return;
+    const long long row = i / nq;
+    const int w = 4 * (int)(i - row * nq);
+    typename Quad<T>::type q;
+    T* e = reinterpret_cast<T*>(&q);
+    if (PAD) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = w + k < W ? src[row * W + w + k] : T(0);
+        reinterpret_cast<typename Quad<T>::type*>(dst)[i] = q;
+    } else {
+        q = reinterpret_cast<const typename Quad<T>::type*>(src)[i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (w + k < W) dst[row * W + w + k] = e[k];
+    }
+}
+
+int launch_rows(bool pad, int64_t rows, int32_t W, int32_t pitch, int32_t dtype, const void* src, void* dst, void* stream) {
+    if (!src || !dst || rows <= 0 || W <= 0 || pitch < W || pitch % 4 || (dtype != NDC_F32 && dtype != NDC_BF16))
+        return proj_fail(NDC_ERR_INVALID, "row padding: invalid argument");
+    if ((uintptr_t)(pad ? dst : src) % (dtype == NDC_BF16 ? 8 : 16))
+        return proj_fail(NDC_ERR_ALIGNMENT, "row padding: the padded tensor is not aligned");
+    const long long quads = rows * (pitch / 4);
+    const unsigned blocks = (unsigned)((quads + 255) / 256);
+    cudaStream_t st = (cudaStream_t)stream;
+    typedef unsigned short u16;
+    if (dtype == NDC_F32) {
+        if (pad) rows_kernel<float, true><<<blocks, 256, 0, st>>>((const float*)src, (float*)dst, quads, W, pitch / 4);
+        else rows_kernel<float, false><<<blocks, 256, 0, st>>>((const float*)src, (float*)dst, quads, W, pitch / 4);
+    } else {
+        if (pad) rows_kernel<u16, true><<<blocks, 256, 0, st>>>((const u16*)src, (u16*)dst, quads, W, pitch / 4);
+        else rows_kernel<u16, false><<<blocks, 256, 0, st>>>((const u16*)src, (u16*)dst, quads, W, pitch / 4);
+    }
+    ndc::launched();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return proj_fail(NDC_ERR_CUDA, "row padding: %s", cudaGetErrorString(e));
+    return NDC_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -371,6 +420,13 @@ int ndc_proj_sum(int32_t slices, int64_t n, int32_t dtype, const float* partial,
     const cudaError_t e = launch_sum(dtype, partial, slices, n, gw, (cudaStream_t)stream);
     if (e != cudaSuccess) return proj_fail(NDC_ERR_CUDA, "projection gradient sum: %s", cudaGetErrorString(e));
     return NDC_OK;
+}
+
+int ndc_pad_rows(int64_t rows, int32_t W, int32_t pitch, int32_t dtype, const void* src, void* dst, void* stream) {
+    return launch_rows(true, rows, W, pitch, dtype, src, dst, stream);
+}
+int ndc_unpad_rows(int64_t rows, int32_t W, int32_t pitch, int32_t dtype, const void* src, void* dst, void* stream) {
+    return launch_rows(false, rows, W, pitch, dtype, src, dst, stream);
 }
 
 int ndc_params_prepare(int32_t dtype, const void* h0, int64_t nh, float* h, const void* bias, int64_t nb,

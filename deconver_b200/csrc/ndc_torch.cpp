@@ -125,7 +125,7 @@ Tensor weight_grad(const Tensor& gy, const Tensor& x, const Tensor& w, int64_t b
     // whole vectors, many samples of few channels - runs on the kernel of ndc_proj_wgrad.
     int64_t slices = 1;
     while (slices < 32 && n % (slices * 16) == 0 && n / (slices * 2) >= 2048) slices *= 2;
-    if (n % (bf16 ? 8 : 4) == 0 && (ci >= 192 || (batch <= 4 && slices > 1))) {
+    if (n % (bf16 ? 8 : 4) == 0 && (ci >= 192 || (batch <= 4 && slices >= 8))) {
         if (ci >= 192 && batch * ((co + 127) / 128) * ((ci + 127) / 128) >= 64) slices = 1;
         Tensor partial = at::empty({batch * slices, co, ci}, w.options().dtype(at::kFloat));
         const float one = 1.0f, zero = 0.0f;
@@ -192,6 +192,7 @@ void prepare_params(const Tensor& h0, const Tensor& bias, Tensor& h, Tensor& b) 
 }
 
 struct Saved {
+    Tensor x;                          // the input, rows padded where that pays
     Tensor h, b;                       // float32 filter and bias
     std::vector<Tensor> z, t1;         // per update that has gradients: its source and K(source)
     int64_t first = 0;                 // index of the first such update
@@ -202,22 +203,41 @@ Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Ten
     Saved local;
     Saved& sv = saved ? *saved : local;
     prepare_params(h0, bias, sv.h, sv.b);
-    auto shape = x.sizes().vec();
-    shape[1] = c.groups * c.sc;
-    const int64_t n = x.numel() ? x.numel() / (x.size(0) * x.size(1)) : 0;
+    auto out_shape = x.sizes().vec();
+    out_shape[1] = c.groups * c.sc;
+    // Rows that are not whole vectors: the layer owns everything between its input and its output
+    // (projection, t1, gradients), so it keeps them with padded rows.  One copy of x (a tenth of
+    // the forward's traffic) buys vector loads in every kernel and aligned GEMMs.
+    const int W = x.numel() ? (int)x.size(-1) : 0;
+    int pitch = W;
+    sv.x = x;
+    if (x.numel()) {
+        const NdcDesc d = make_desc(x, h0, c, true);
+        pitch = ndc_row_pitch(&d);
+        if (pitch != W) {
+            auto xs = x.sizes().vec();
+            xs.back() = pitch;
+            sv.x = at::empty(xs, x.options());
+            check(ndc_pad_rows(x.numel() / W, W, pitch, d.dtype, ptr(x), ptr(sv.x), stream()), ndc_proj_last_error());
+        }
+    }
+    auto shape = out_shape;
+    if (W) shape.back() = pitch;
+    const int64_t n = sv.x.numel() ? sv.x.numel() / (x.size(0) * x.size(1)) : 0;
     Tensor s = at::empty(shape, x.options());
-    channel_gemm(w, false, x, s, x.size(0), n, false);
+    channel_gemm(w, false, sv.x, s, x.size(0), n, false);
     sv.first = c.iters > c.grad_iters ? c.iters - c.grad_iters : 0;
     Tensor t1;
     for (int64_t it = 0; it < c.iters; ++it) {
         const bool keep = saved && it >= sv.first;
-        Tensor out = at::empty(shape, x.options());
-        if (keep || !t1.defined()) t1 = at::empty(x.sizes(), x.options());
+        const bool last = it + 1 == c.iters;
+        Tensor out = at::empty(last ? out_shape : shape, x.options());
+        if (keep || !t1.defined()) t1 = at::empty(sv.x.sizes(), x.options());
         if (x.numel()) {
             const NdcDesc d = make_desc(x, h0, c, it == 0);
             Span span(0);
-            check(ndc_fwd(&d, ptr(x), ptr(s), fptr(sv.h), it == 0 ? fptr(sv.b) : nullptr, ptr(out), ptr(t1),
-                          stream()), ndc_last_error());
+            check(ndc_fwd_rows(&d, pitch, last ? W : pitch, ptr(sv.x), ptr(s), fptr(sv.h), it == 0 ? fptr(sv.b) : nullptr,
+                               ptr(out), ptr(t1), stream()), ndc_last_error());
         }
         if (keep) { sv.z.push_back(s); sv.t1.push_back(t1); }
         s = out;
@@ -233,12 +253,12 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
         Saved sv;
         const Tensor b = bias ? *bias : Tensor();
         Tensor out = run_forward(x, h0, w, b, c, &sv);
-        variable_list keep = {x, h0, w, b, sv.h, sv.b};
+        variable_list keep = {sv.x, h0, w, b, sv.h, sv.b};
         keep.insert(keep.end(), sv.z.begin(), sv.z.end());
         keep.insert(keep.end(), sv.t1.begin(), sv.t1.end());
         ctx->save_for_backward(keep);
         auto& d = ctx->saved_data;
-        d["cfg"] = std::vector<int64_t>{groups, m, sc, iters, grad_iters, flags, sv.first};
+        d["cfg"] = std::vector<int64_t>{groups, m, sc, iters, grad_iters, flags, sv.first, x.size(-1)};
         d["eps"] = eps;
         return out;
     }
@@ -248,7 +268,7 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
         const variable_list kept = ctx->get_saved_variables();
         const auto cfg = ctx->saved_data["cfg"].toIntVector();
         const Config c{cfg[0], cfg[1], cfg[2], ctx->saved_data["eps"].toDouble(), cfg[3], cfg[4], cfg[5]};
-        const int64_t first = cfg[6], count = c.iters - first;
+        const int64_t first = cfg[6], count = c.iters - first, W = cfg[7];
         const Tensor &x = kept[0], &h0 = kept[1], &w = kept[2], &bias = kept[3], &h = kept[4], &b = kept[5];
         const bool need_x = ctx->needs_input_grad(0), need_h = ctx->needs_input_grad(1);
         const bool whole = first == 0;                   // gradients reach the projection
@@ -271,13 +291,15 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
             if (need_h) gh_i = at::empty(h.sizes(), f32);
             if (need_b && it0) gb = at::empty(bias.sizes(), f32);
             if (x.numel()) {
-                const NdcDesc d = make_desc(x, h0, c, it0);
-                const size_t bytes = ndc_bwd_workspace_bytes(&d);
+                NdcDesc d = make_desc(x, h0, c, it0);
+                const int pitch = d.W;
+                d.W = (int)W;
+                const size_t bytes = ndc_bwd_rows_workspace_bytes(&d, pitch);
                 if (!ws.defined()) ws = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
                 Span span(1);
-                check(ndc_bwd(&d, ptr(x), ptr(z), ptr(t1), fptr(h), it0 ? fptr(b) : nullptr, ptr(g), ptr(gx_i),
-                              ptr(gz), fptr(gh_i), it0 ? fptr(gb) : nullptr, ptr(ws), bytes, stream()),
-                      ndc_last_error());
+                check(ndc_bwd_rows(&d, pitch, i == count - 1 ? (int)W : pitch, ptr(x), ptr(z), ptr(t1), fptr(h),
+                                   it0 ? fptr(b) : nullptr, ptr(g), ptr(gx_i), ptr(gz), fptr(gh_i),
+                                   it0 ? fptr(gb) : nullptr, ptr(ws), bytes, stream()), ndc_last_error());
             } else {
                 for (Tensor* t : {&gx_i, &gz, &gh_i, &gb}) if (t->defined()) t->zero_();
             }
@@ -291,6 +313,14 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
             // gz of the first update: W^T gz is added to the update's own input gradient
             if (need_x) channel_gemm(w, true, g, gx, x.size(0), n, true);
             if (need_w) gw = weight_grad(g, x, w, x.size(0), n);
+        }
+        if (need_x && x.numel() && x.size(-1) != W) {
+            auto xs = x.sizes().vec();
+            xs.back() = W;
+            Tensor plain = at::empty(xs, x.options());
+            check(ndc_unpad_rows(plain.numel() / W, (int)W, (int)x.size(-1), dtype_code(x), ptr(gx), ptr(plain), stream()),
+                  ndc_proj_last_error());
+            gx = plain;
         }
         const bool same = !need_b || !need_h || bias.scalar_type() == h0.scalar_type();
         if ((need_h || need_b) && kernel_dtype(need_h ? h0 : bias) && same) {

@@ -138,6 +138,25 @@ int ndc_bwd(const NdcDesc *desc, const void *x, const void *z, const void *t1, c
             void *workspace, size_t workspace_bytes, void *stream);
 
 /*
+ * The same two calls for tensors whose rows are padded: x, z, t1, gx and gz have rows of `pitch`
+ * elements of which the first W are the problem's, out / gout rows of W or of `pitch`.  Row lengths
+ * that are not a multiple of four cost the kernels their vector loads and stores (and the 1x1
+ * projections around them theirs); a caller that owns the inner tensors pads them instead.
+ * ndc_row_pitch says what pitch is worth it (W itself: none).  x must be zero in the padding, gout
+ * (if padded) finite; t1, gx and gz are written as zero there, a padded out is not defined there.
+ * ndc_pad_rows / ndc_unpad_rows copy `rows` rows of W elements from or to a tensor without padding.
+ */
+int32_t ndc_row_pitch(const NdcDesc *desc);
+int ndc_fwd_rows(const NdcDesc *desc, int32_t pitch, int32_t out_pitch, const void *x, const void *z,
+                 const float *h, const float *bias, void *out, void *t1, void *stream);
+size_t ndc_bwd_rows_workspace_bytes(const NdcDesc *desc, int32_t pitch);
+int ndc_bwd_rows(const NdcDesc *desc, int32_t pitch, int32_t gout_pitch, const void *x, const void *z,
+                 const void *t1, const float *h, const float *bias, const void *gout, void *gx, void *gz,
+                 float *gh, float *gb, void *workspace, size_t workspace_bytes, void *stream);
+int ndc_pad_rows(int64_t rows, int32_t W, int32_t pitch, int32_t dtype, const void *src, void *dst, void *stream);
+int ndc_unpad_rows(int64_t rows, int32_t W, int32_t pitch, int32_t dtype, const void *src, void *dst, void *stream);
+
+/*
  * Size of the library-owned scratch array used by ndc_bwd_static.  Every GPU that uses this
  * library holds these bytes until the process exits.  When they are reserved depends on the
  * CUDA module-loading mode: with lazy loading (the default) it can be as late as the first

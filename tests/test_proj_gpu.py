@@ -34,8 +34,11 @@ def test_weight_gradient(dtype, tf32, tol, batch, co, ci, n):
 
 
 @pytest.mark.parametrize("num_iters,num_grad_iters", [(1, 1), (3, 3), (3, 1), (2, 0)])
+# among the sizes: rows that are padded inside the layer (one to three columns), on every kernel class
 @pytest.mark.parametrize("channels,spatial,ks,groups", [(8, (5, 9, 7), (3, 3, 3), 8), (8, (12, 20), (5, 5), 8),
-                                                        (8, (9, 10), (3, 3), 2), (192, (4, 8), (3, 3), 192)])
+                                                        (8, (9, 10), (3, 3), 2), (192, (4, 8), (3, 3), 192),
+                                                        (8, (4, 6, 5), (3, 3, 3), 8), (8, (30, 101), (3, 3), 8),
+                                                        (6, (14, 45, 66), (3, 3, 3), 6), (4, (23, 17), (5, 5), 4)])
 def test_layer_is_its_projection_followed_by_the_updates(num_iters, num_grad_iters, channels, spatial, ks, groups):
     """The native layer against `deconv_update` on a float64-accurate projection, every gradient."""
     dev = torch.device("cuda:0")
@@ -70,3 +73,17 @@ def test_layer_is_its_projection_followed_by_the_updates(num_iters, num_grad_ite
         assert (a is None) == (b is None)
         if a is not None:
             assert ((a - b).abs().max() / b.abs().max().clamp_min(1e-30)).item() < 1e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("rows,W,pitch", [(1, 5, 8), (7, 13, 16), (1000, 171, 176), (3, 8, 8)])
+def test_row_padding(rows, W, pitch, dtype):
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    x = torch.randn(rows, W, device=dev).to(dtype)
+    p = torch.full((rows, pitch), 7.0, device=dev, dtype=dtype)
+    y = torch.empty_like(x)
+    st, code = torch.cuda.current_stream().cuda_stream, _lib.NDC_BF16 if dtype == torch.bfloat16 else _lib.NDC_F32
+    assert lib.ndc_pad_rows(rows, W, pitch, code, x.data_ptr(), p.data_ptr(), st) == 0
+    assert lib.ndc_unpad_rows(rows, W, pitch, code, p.data_ptr(), y.data_ptr(), st) == 0
+    assert torch.equal(p[:, :W], x) and torch.equal(y, x) and not p[:, W:].any()
+    assert lib.ndc_pad_rows(rows, W, W - 1, code, x.data_ptr(), p.data_ptr(), st) == 1
