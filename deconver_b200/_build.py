@@ -32,7 +32,7 @@ NVCC_FLAGS = [
 
 # (object name, source, extra defines)
 UNITS = [("abi", "ndc_abi.cu", []), ("inorm", "ndc_inorm.cu", []), ("bias", "ndc_bias.cu", []),
-         ("proj", "ndc_proj.cu", [])] + [
+         ("proj", "ndc_proj.cu", []), ("tc", "ndc_tc.cu", [])] + [
     ("tile_t%d" % t, "ndc_tile_inst.cu", ["-DNDC_TILE_T=%d" % t]) for t in (0, 1)] + [
     ("dw4_p%d_t%d" % (part, t), "ndc_dw4_inst.cu", ["-DNDC_DW4_PART=%d" % part, "-DNDC_DW4_T=%d" % t])
     for part in (1, 2, 0) for t in (0, 1)   # the longest units first
@@ -41,7 +41,7 @@ UNITS = [("abi", "ndc_abi.cu", []), ("inorm", "ndc_inorm.cu", []), ("bias", "ndc
 
 def sources():
     deps = [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC))
-            if f.endswith((".cu", ".cuh"))]
+            if f.endswith((".cu", ".cuh", ".h"))]
     deps.append(os.path.join(INCLUDE, "ndc_b200.h"))
     return deps
 

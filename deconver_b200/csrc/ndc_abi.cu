@@ -8,6 +8,7 @@
 #include "ndc_b200.h"
 #include "ndc_common.cuh"
 #include "ndc_generic.cuh"
+#include "ndc_tc_host.h"
 #define NDC_DW4_EXTERN   // the tiled kernels are compiled in ndc_dw4_inst.cu
 #include "ndc_dw4_host.cuh"
 #define NDC_TILE_EXTERN  // compiled in ndc_tile_inst.cu
@@ -34,7 +35,7 @@ constexpr int kMaxTaps = 343;
 
 int validate(const NdcDesc* d) {
     if (!d) return fail(NDC_ERR_INVALID, "descriptor is NULL");
-    if (d->flags & ~NDC_FLAG_FORCE_GENERIC)
+    if (d->flags & ~(NDC_FLAG_FORCE_GENERIC | NDC_FLAG_BF16_PARAMS))
         return fail(NDC_ERR_INVALID, "descriptor.flags has unknown bits set (0x%x)", d->flags);
     if (d->batch <= 0 || d->groups <= 0 || d->m <= 0 || d->sc <= 0)
         return fail(NDC_ERR_INVALID, "batch, groups, m and sc must be positive (got %d, %d, %d, %d)",
@@ -165,6 +166,8 @@ const char* ndc_status_string(int status) {
     }
 }
 
+uint32_t ndc_wait_expired(void) { return ndc::tc::wait_expired(); }
+
 uint64_t ndc_launch_count(void) {
     return (uint64_t)ndc::launch_counter().load(std::memory_order_relaxed);
 }
@@ -207,6 +210,13 @@ int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const vo
     cudaError_t e;
     typedef __nv_bfloat16 bf16;
     if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
+        // bfloat16 tensors with bfloat16 parameters: exact products on the tensor cores
+        if (desc->dtype == NDC_BF16 && (desc->flags & NDC_FLAG_BF16_PARAMS) && ndc::tc::covers(g) &&
+            (((uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0)) & 7) == 0) {
+            e = ndc::tc::forward(g, (const bf16*)x, (const bf16*)z, h, bias, (bf16*)out, (bf16*)t1, st);
+            if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (tensor core) launch");
+            return NDC_OK;
+        }
         bool handled = false;
         if (desc->dtype == NDC_F32)
             e = ndc::dw4::forward<float>(g, (const float*)x, (const float*)z, h, bias, (float*)out,

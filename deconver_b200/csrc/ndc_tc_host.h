@@ -1,0 +1,17 @@
+// Entry points of the tensor-core forward (ndc_tc.cu) for the ABI unit.
+#pragma once
+
+#include "ndc_common.cuh"
+
+namespace ndc {
+namespace tc {
+
+// Whether the tensor-core kernels take this geometry and are the faster ones for it.
+bool covers(const Geo& g);
+cudaError_t forward(const Geo& g, const __nv_bfloat16* x, const __nv_bfloat16* z, const float* h, const float* bias,
+                    __nv_bfloat16* out, __nv_bfloat16* t1, cudaStream_t st);
+// Non-zero once a kernel's bounded wait has run out on the current device (synchronises; for tests).
+unsigned wait_expired();
+
+}  // namespace tc
+}  // namespace ndc

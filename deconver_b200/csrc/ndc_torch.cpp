@@ -160,6 +160,7 @@ struct Config {
     int64_t groups, m, sc;
     double eps;
     int64_t iters, grad_iters, flags;
+    bool bf16_params = false;          // filter and bias are bfloat16 values
 };
 
 NdcDesc make_desc(const Tensor& x, const Tensor& h0, const Config& c, bool relu) {
@@ -171,6 +172,7 @@ NdcDesc make_desc(const Tensor& x, const Tensor& h0, const Config& c, bool relu)
     d.D = (int)sp[0]; d.H = (int)sp[1]; d.W = (int)sp[2];
     d.kD = (int)k[0]; d.kH = (int)k[1]; d.kW = (int)k[2];
     d.eps = (float)c.eps; d.relu_input = relu ? 1 : 0; d.dtype = dtype_code(x); d.flags = (int)c.flags;
+    if (c.bf16_params) d.flags |= NDC_FLAG_BF16_PARAMS;
     return d;
 }
 
@@ -198,10 +200,12 @@ struct Saved {
     int64_t first = 0;                 // index of the first such update
 };
 
-Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Tensor& bias, const Config& c,
+Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Tensor& bias, const Config& config,
                    Saved* saved) {
     Saved local;
     Saved& sv = saved ? *saved : local;
+    Config c = config;
+    c.bf16_params = h0.scalar_type() == at::kBFloat16 && (!bias.defined() || bias.scalar_type() == at::kBFloat16);
     prepare_params(h0, bias, sv.h, sv.b);
     auto out_shape = x.sizes().vec();
     out_shape[1] = c.groups * c.sc;

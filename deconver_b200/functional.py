@@ -218,6 +218,8 @@ class DeconvUpdate(torch.autograd.Function):
         z = z.contiguous()
         ks = tuple(h.shape[2:])
         flags = _flags   # read once: backward runs later, on an autograd thread
+        if h.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16):
+            flags |= _lib.FLAG_BF16_PARAMS
         desc = _desc(x, groups, m, sc, ks, eps, relu_input, flags)
         _warn_if_generic(desc, flags)
         hf, bf = _f32(h), _f32(bias)

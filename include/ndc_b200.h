@@ -50,7 +50,10 @@ enum NdcStatus {
 };
 
 enum NdcFlags {
-    NDC_FLAG_FORCE_GENERIC = 1 /* run the generic kernels even where the tiled ones apply    */
+    NDC_FLAG_FORCE_GENERIC = 1, /* run the generic kernels even where the tiled ones apply   */
+    NDC_FLAG_BF16_PARAMS = 2    /* the caller knows every value of h and bias to be a bfloat16
+                                   value (as in a bfloat16 module): with NDC_BF16 tensors the
+                                   forward then runs on the tensor cores                     */
 };
 
 /* Which family of kernels a geometry runs on (informational; results are the same). */
@@ -95,6 +98,10 @@ const char *ndc_status_string(int status);
 /* Number of kernel launches this library has issued in this process (all threads).  Lets a
  * caller verify that the CUDA path, and not some other path, did the work. */
 uint64_t ndc_launch_count(void);
+
+/* Non-zero once a bounded wait inside a kernel has run out on the current device (a kernel bug:
+ * the outputs of that launch are undefined).  Synchronises with the device; for tests. */
+uint32_t ndc_wait_expired(void);
 
 /*
  * Whether a geometry is covered, and by which kernel family.  Returns NDC_OK and writes an
