@@ -135,13 +135,12 @@ struct At {
     }
 };
 
-// Eight places of a shared row: columns 8 q - PW .. 8 q + 7 - PW of a global row, from the words
-// around them.  `negb`: two copies of -bias; SOURCE: max(value, -bias) inside the volume (RELU).
-template <int PW, bool SOURCE, bool WIDE>
-__device__ __forceinline__ uint4 load_places(const bf16* row, int q, const Band& b, unsigned negb, bool relu) {
-    const int w = 8 * q;
-    unsigned a[5] = {0u, 0u, 0u, 0u, 0u};          // columns w-2 .. w+7
-    if (q > 0 && w - 4 < b.W) a[0] = __ldg(reinterpret_cast<const unsigned*>(row + w - 2));
+// Columns w-2 .. w+7 of a global row as five words, w = 8 q; zero outside the row.
+template <bool WIDE>
+__device__ __forceinline__ void load_words(const bf16* row, int w, const Band& b, unsigned (&a)[5]) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) a[i] = 0u;
+    if (w > 0 && w - 4 < b.W) a[0] = __ldg(reinterpret_cast<const unsigned*>(row + w - 2));
     if (WIDE) {
         if (w < b.W) {
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + w));
@@ -151,22 +150,27 @@ __device__ __forceinline__ uint4 load_places(const bf16* row, int q, const Band&
         if (w < b.W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + w)); a[1] = v.x; a[2] = v.y; }
         if (w + 4 < b.W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + w + 4)); a[3] = v.x; a[4] = v.y; }
     }
-    if (SOURCE && relu) {
+}
+// The eight places of block q of a shared row (columns 8 q - PW .. 8 q + 7 - PW) from those words.
+// SOURCE: max(value, -bias) inside the volume (`negb`: two copies of -bias), zero in the padding.
+template <int PW, bool SOURCE>
+__device__ __forceinline__ uint4 to_places(unsigned (&a)[5], int w, const Band& b, unsigned negb, bool relu) {
+    if (SOURCE) {
+        if (relu) {
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
-            const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a[i]), *reinterpret_cast<const __nv_bfloat162*>(&negb));
-            unsigned m = *reinterpret_cast<const unsigned*>(&v);
-            const int c = w - 2 + 2 * i;           // outside the volume: zero
-            if (c < 0 || c >= b.Wv) m = 0u;
-            else if (c + 1 >= b.Wv) m &= 0xffffu;
-            a[i] = m;
+            for (int i = 0; i < 5; ++i) {
+                const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a[i]), *reinterpret_cast<const __nv_bfloat162*>(&negb));
+                a[i] = *reinterpret_cast<const unsigned*>(&v);
+            }
+            if (w == 0) a[0] = 0u;
         }
-    } else if (SOURCE) {                           // the padding of a source is not defined
+        if (w + 7 >= b.Wv) {                       // the row ends here
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
-            const int c = w - 2 + 2 * i;
-            if (c >= b.Wv) a[i] = 0u;
-            else if (c + 1 >= b.Wv) a[i] &= 0xffffu;
+            for (int i = 0; i < 5; ++i) {
+                const int c = w - 2 + 2 * i;
+                if (c >= b.Wv) a[i] = 0u;
+                else if (c + 1 >= b.Wv) a[i] &= 0xffffu;
+            }
         }
     }
     if (PW == 2) return make_uint4(a[0], a[1], a[2], a[3]);
@@ -174,18 +178,68 @@ __device__ __forceinline__ uint4 load_places(const bf16* row, int q, const Band&
                       __funnelshift_l(a[3], a[4], 16));
 }
 
-// One channel's band, halo included, into shared memory; rows outside the volume are zero.
-template <int KD, int KH, int KW, bool SOURCE, bool WIDE>
-__device__ __forceinline__ void stage(uint4* dst, const bf16* src, const Band& b, const At& at, unsigned negb, bool relu,
-                                      int first, int step) {
-    const int rows = b.TH + KH - 1, total = (at.DC + KD - 1) * rows * b.PB;
-    for (int i = first; i < total; i += step) {
-        const int q = i % b.PB, r = i / b.PB, pl = r / rows, row = r - pl * rows;
-        const int d = at.d0 - KD / 2 + pl, h = at.h0 - KH / 2 + row;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (d >= 0 && d < b.D && h >= 0 && h < b.H)
-            v = load_places<KW / 2, SOURCE, WIDE>(src + ((long long)d * b.H + h) * b.W, q, b, negb, relu);
-        dst[i] = v;
+constexpr int kStagers = 256;     // threads that stage (and then run the epilogue)
+
+// Bands of NCH channels (`src + ch * stride`, `dst + ch * blocks`), halo included, into shared memory;
+// rows outside the volume are zero.  Four blocks per thread are in flight at a time: one at a time, the
+// staging of a CTA took 20 us of latency.
+template <int KD, int KH, int KW, int NCH, bool SOURCE, bool WIDE>
+__device__ __forceinline__ void stage(uint4* dst, int blocks, const bf16* src, long long stride, const Band& b, const At& at,
+                                      const unsigned (&negb)[NCH], bool relu) {
+    constexpr int U = 2;                           // times NCH channels in flight
+    const int rows = b.TH + KH - 1, planes = at.DC + KD - 1;
+    const int dq = kStagers % b.PB, dr = kStagers / b.PB;
+    int q = threadIdx.x % b.PB, row = threadIdx.x / b.PB, pl = 0, i = threadIdx.x;
+    while (row >= rows) { row -= rows; ++pl; }
+    while (pl < planes) {
+        unsigned a[U][NCH][5];
+        int w[U], at_i[U];
+        bool in[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int d = at.d0 - KD / 2 + pl, h = at.h0 - KH / 2 + row;
+            at_i[u] = pl < planes ? i : -1;
+            w[u] = 8 * q;
+            in[u] = pl < planes && d >= 0 && d < b.D && h >= 0 && h < b.H;
+            if (in[u]) {
+                const bf16* p = src + ((long long)d * b.H + h) * b.W;
+#pragma unroll
+                for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride, w[u], b, a[u][ch]);
+            }
+            i += kStagers; q += dq; row += dr;
+            if (q >= b.PB) { q -= b.PB; ++row; }
+            while (row >= rows) { row -= rows; ++pl; }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (at_i[u] < 0) continue;
+#pragma unroll
+            for (int ch = 0; ch < NCH; ++ch)
+                dst[ch * blocks + at_i[u]] = in[u] ? to_places<KW / 2, SOURCE>(a[u][ch], w[u], b, negb[ch], relu)
+                                                   : make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+}
+
+// The banded matrices of a kernel by one warp: `value(t, n, kw)` is the filter tap of matrix t, column n.
+// Layout of one matrix: groups of eight columns, then the two halves of K, eight 16-byte rows each.
+template <int NCOL, int KW, bool ADJ, typename F>
+__device__ __forceinline__ void build_bands(bf16* bmat, int mats, int lane, F value) {
+    for (int e = lane; e < mats * NCOL * 2; e += 32) {
+        const int n = e % 8, half = (e / 8) % 2, g = (e / 16) % (NCOL / 8), t = e / (2 * NCOL);
+        unsigned words[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k = 8 * half + 2 * i + u, kw = ADJ ? n + KW - 1 - k : k - n;
+                v[u] = kw >= 0 && kw < KW ? value(t, 8 * g + n, kw) : 0.0f;
+            }
+            const __nv_bfloat162 p = __floats2bfloat162_rn(v[0], v[1]);
+            words[i] = *reinterpret_cast<const unsigned*>(&p);
+        }
+        reinterpret_cast<uint4*>(bmat)[e] = make_uint4(words[0], words[1], words[2], words[3]);
     }
 }
 
@@ -196,7 +250,7 @@ __host__ __device__ inline int band_blocks(const Band& b) { return (b.DC + KD - 
 __host__ __device__ inline int slack_blocks(const Band& b) { return b.MT * MB + 1 - b.TH * b.PB > 1 ? b.MT * MB + 1 - b.TH * b.PB : 1; }
 
 constexpr int kThreads = 288;     // eight staging / epilogue warps and the MMA warp
-constexpr int kHeader = 256;      // bytes: barriers, TMEM address
+constexpr int kHeader = 1024;     // bytes: barriers, TMEM address (256), the filter as float32
 
 enum Access { kWide = 0, kQuad = 1, kPaddedOut = 2 };   // 16-byte rows; 8-byte rows; 8-byte rows, out unpadded
 
@@ -254,14 +308,17 @@ __global__ void __launch_bounds__(kThreads, 2) tc_adjoint_kernel(const AdjointAr
         for (int i = 0; i < BUFS; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int e = tid; e < ROWT * NCOL * 16; e += kThreads) {       // [filter row][n][k]
-        const int k = e % 16, n = (e / 16) % NCOL, t = e / (16 * NCOL);
-        const int j = n / 8, kw = n % 8 + KW - 1 - k;
-        const float v = kw >= 0 && kw < KW ? P.h[((long long)at.c * SC + j) * ROWT * KW + t * KW + kw] : 0.0f;
-        bmat[t * NCOL * 16 + (n / 8) * 128 + (k / 8) * 64 + (n % 8) * 8 + k % 8] = __float2bfloat16_rn(v);
+    if (warp == 8) {
+        float* const hs = reinterpret_cast<float*>(smem_tc + 256);
+        for (int e = lane; e < SC * ROWT * KW; e += 32) hs[e] = P.h[(long long)at.c * SC * ROWT * KW + e];
+        __syncwarp();
+        build_bands<NCOL, KW, true>(bmat, ROWT, lane, [&](int t, int n, int kw) { return hs[(n / 8) * ROWT * KW + t * KW + kw]; });
+    } else {
+        // x and t1 as two channels: the distance between the tensors takes the place of the stride
+        const unsigned none[2] = {0u, 0u};
+        const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
+        stage<KD, KH, KW, 2, false, AL == kWide>(xs, blocks, P.x + (long long)at.bc * b.SP, apart, b, at, none, false);
     }
-    stage<KD, KH, KW, false, AL == kWide>(xs, P.x + (long long)at.bc * b.SP, b, at, 0u, false, tid, kThreads);
-    stage<KD, KH, KW, false, AL == kWide>(ts, P.t1 + (long long)at.bc * b.SP, b, at, 0u, false, tid, kThreads);
     // what the windows of valid blocks may touch past the staged planes has to be a number
     for (int i = tid; i < slack; i += kThreads) ts[blocks + i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0 && at.DC < b.DC) {
@@ -394,39 +451,45 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
         for (int i = 0; i < steps; ++i) mbar_init(base + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const float* hc = P.h + (long long)at.c * SC * KT;
-    for (int e = tid; e < NMAT * NCOL * 16; e += kThreads) {       // [channel, kh][n][k]
-        const int k = e % 16, n = (e / 16) % NCOL, t = e / (16 * NCOL);
-        const int j = t / KH, kh = t % KH, g = n / 8, kw = k - n % 8;
-        const int kd = KD - 1 - g;                                 // column group g: output plane p - kd
-        const float v = kd >= 0 && kw >= 0 && kw < KW ? hc[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
-        bmat[t * NCOL * 16 + (n / 8) * 128 + (k / 8) * 64 + (n % 8) * 8 + k % 8] = __float2bfloat16_rn(v);
-    }
-    // sum over channels and the taps inside the volume of bias * filter, by how many taps are cut off
-    // at either end of each axis
-    for (int e = tid; e < TABLE; e += kThreads) {
-        int q = e;
-        const int wh = q % (PW + 1); q /= PW + 1;
-        const int wl = q % (PW + 1); q /= PW + 1;
-        const int hh = q % (PH + 1); q /= PH + 1;
-        const int hl = q % (PH + 1); q /= PH + 1;
-        const int dh = q % (PD + 1), dl = q / (PD + 1);
-        float s = 0.0f;
-        if (P.bias)
-            for (int j = 0; j < SC; ++j) {
-                float r = 0.0f;
-                for (int kd = dl; kd < KD - dh; ++kd)
-                    for (int kh = hl; kh < KH - hh; ++kh)
-                        for (int kw = wl; kw < KW - wh; ++kw) r += hc[j * KT + (kd * KH + kh) * KW + kw];
-                s = fmaf(P.bias[at.c * SC + j], r, s);
-            }
-        table[e] = s;
-    }
-    for (int j = 0; j < SC; ++j) {
-        const __nv_bfloat16 nb = __float2bfloat16_rn(P.bias ? -P.bias[at.c * SC + j] : 0.0f);
-        const unsigned short u = *reinterpret_cast<const unsigned short*>(&nb);
-        stage<KD, KH, KW, true, AL == kWide>(zs + j * blocks, P.z + ((long long)at.bc * SC + j) * b.SP, b, at,
-                                             (unsigned)u << 16 | u, b.relu, tid, kThreads);
+    if (warp == 8) {
+        float* const hs = reinterpret_cast<float*>(smem_tc + 256);
+        for (int e = lane; e < SC * KT; e += 32) hs[e] = P.h[(long long)at.c * SC * KT + e];
+        float bj[SC];
+#pragma unroll
+        for (int j = 0; j < SC; ++j) bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
+        __syncwarp();
+        // column group g: output plane p - kd, kd = KD - 1 - g
+        build_bands<NCOL, KW, false>(bmat, NMAT, lane, [&](int t, int n, int kw) {
+            const int j = t / KH, kh = t % KH, kd = KD - 1 - n / 8;
+            return kd >= 0 ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
+        });
+        // sum over channels and the taps inside the volume of bias * filter, by how many taps are cut
+        // off at either end of each axis
+        for (int e = lane; e < TABLE; e += 32) {
+            int q = e;
+            const int wh = q % (PW + 1); q /= PW + 1;
+            const int wl = q % (PW + 1); q /= PW + 1;
+            const int hh = q % (PH + 1); q /= PH + 1;
+            const int hl = q % (PH + 1); q /= PH + 1;
+            const int dh = q % (PD + 1), dl = q / (PD + 1);
+            float s = 0.0f;
+            for (int kd = dl; kd < KD - dh; ++kd)
+                for (int kh = hl; kh < KH - hh; ++kh)
+                    for (int kw = wl; kw < KW - wh; ++kw) {
+                        const int tau = (kd * KH + kh) * KW + kw;
+#pragma unroll
+                        for (int j = 0; j < SC; ++j) s = fmaf(bj[j], hs[j * KT + tau], s);
+                    }
+            table[e] = s;
+        }
+    } else {
+        unsigned negb[SC];
+#pragma unroll
+        for (int j = 0; j < SC; ++j) {
+            const __nv_bfloat162 nb = __float2bfloat162_rn(P.bias ? -P.bias[at.c * SC + j] : 0.0f);
+            negb[j] = *reinterpret_cast<const unsigned*>(&nb);
+        }
+        stage<KD, KH, KW, SC, true, AL == kWide>(zs, blocks, P.z + (long long)at.bc * SC * b.SP, b.SP, b, at, negb, b.relu);
     }
     for (int i = tid; i < slack; i += kThreads) zs[SC * blocks + i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < SC && at.DC < b.DC) zs[tid * blocks + used] = make_uint4(0u, 0u, 0u, 0u);
