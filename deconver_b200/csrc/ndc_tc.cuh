@@ -7,16 +7,19 @@
 // number PB of 8-column blocks.  The MMA's A operand is not a copy of that: its row r is the window
 // of 16 places that starts at block r, and in the K-major layout without swizzle (8-row groups of
 // 16-byte rows) this is the memory as it lies, with 16 bytes between the two halves of the window
-// and 128 bytes between groups of eight blocks.  A filter row (kd, kh) is a shift of the start
-// address.  The B operand is a banded matrix of one filter row: window place k, output column o of
-// the block, one copy per output channel,
+// and 128 bytes between groups of eight blocks.  A filter row kh is a shift of the start address.  The
+// B operand is a banded matrix: window place k, output column o of the block,
 //
 //     A: B[k][8 j + o] = h[j][kd][kh][o + 2 PW - k]        K: B[k][o] = h[j][kd][kh][k - o]
 //
-// so one M = 128, K = 16 MMA computes 1024 voxels of one filter row.  With KW = 3 a third of the
-// products meet a zero of the band; the tensor cores do them 30 times faster than the FMA pipe does
-// the useful ones.  What bounds an MMA of so few columns is reading its A operand (4 KB of shared
-// memory, 32 cycles).
+// with the matrices of the KD depth taps side by side: one M = 128, K = 16 MMA multiplies 1024 voxels
+// of a source plane by one filter row of every depth tap, onto the accumulators of KD output
+// planes, which lie next to each other in TMEM.  So a source plane is read once, when the CTA's march
+// through the depth comes to it.  Batches of images march down their rows the same way (planes = image
+// rows, plane rows = images, KH = 1: see SlabAddr).  An MMA of up to 128 columns takes 64 cycles here,
+// whatever its width (reading 4 KB of A operand), hence the wide ones.  With KW = 3 a third of the products
+// meet a zero of the band; the tensor cores do them 30 times faster than the FMA pipe does the useful
+// ones.
 //
 // Precision: every product is one of two bfloat16 values, exact in float32, accumulated in float32:
 // what the FMA kernels compute, in another order.  The source relu(z + b) is not a bfloat16 value, but
@@ -40,8 +43,7 @@ struct Band {
     int C, D, H, W;               // W: row pitch (a multiple of 4)
     int Wv, Wo;                   // columns of the volume, row pitch of out (see Geo)
     int NB, PB;                   // blocks that hold columns, blocks per row in shared memory
-    int TH, nth, DC, ndc, MT;     // rows and bands, planes and chunks, MMA tiles per band and plane
-    long long SP;
+    int TH, nth, DC, ndc;         // rows and bands, planes and chunks
     float eps;
     int relu;
 };
@@ -102,8 +104,9 @@ __device__ __forceinline__ void tmem_load8x2(unsigned addr_a, unsigned addr_b, f
 #pragma unroll
     for (int i = 0; i < 8; ++i) { a[i] = __uint_as_float(r[i]); b[i] = __uint_as_float(r[8 + i]); }
 }
-__device__ __forceinline__ void tmem_zero8(unsigned addr) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(addr), "r"(0u) : "memory");
+__device__ __forceinline__ void tmem_zero32(unsigned addr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+                 "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(addr), "r"(0u) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -123,7 +126,17 @@ __device__ __forceinline__ unsigned instr_desc(int n) { return 1u << 4 | 1u << 7
 // Set where a wait ran out; the results of that launch are then undefined.
 static __device__ unsigned g_wait_expired;
 
-// Place of a band in the volume, and of the shared-memory planes in it.
+// Roles of a CTA's warps: two groups of four for the epilogue (they take turns, output plane by output
+// plane; TMEM lane 32 i + l belongs to lane l of the warps i of a group), four that stage source
+// planes, one that builds the banded matrices and issues the MMAs.
+constexpr int kEpilogueWarps = 8, kStageWarps = 4, kMmaWarp = kEpilogueWarps + kStageWarps;
+constexpr int kThreads = 32 * (kMmaWarp + 1), kStagers = 32 * kStageWarps;
+constexpr int kSlots = 4;         // staged planes
+constexpr int kHeader = 1024;     // bytes: barriers and the TMEM address (512), the filter as float32
+constexpr int kMaxBlocks = 2 * kStagers;   // blocks of a staged plane (and channel), at most
+
+// Place of a CTA: (sample, channel), band of rows, chunk of planes; all addresses in elements.
+template <bool ROWS>
 struct At {
     int bc, c, h0, TH, d0, DC;
     __device__ __forceinline__ At(const Band& b, int blk) {
@@ -178,48 +191,105 @@ __device__ __forceinline__ uint4 to_places(unsigned (&a)[5], int w, const Band& 
                       __funnelshift_l(a[3], a[4], 16));
 }
 
-constexpr int kStagers = 256;     // threads that stage (and then run the epilogue)
+// Stages planes of NCH channels (`src + ch * stride`), halo rows included; rows outside the volume are
+// zero.  A thread has up to two blocks of a plane; their loads are issued a plane ahead of the stores
+// and the lines of the plane after that are asked for from L2.
+template <int KH, int KW, int NCH, bool SOURCE, bool WIDE>
+struct Stager {
+    const Band& b;
+    const bf16* src;
+    long long stride, plane;
+    int blocks;                    // per channel of a slot
+    long long off[2];              // this thread's blocks: row offset, or -1 outside the volume
+    int w[2], at[2];               // column; block, or -1
+    unsigned a[2][NCH][5];
 
-// Bands of NCH channels (`src + ch * stride`, `dst + ch * blocks`), halo included, into shared memory;
-// rows outside the volume are zero.  Four blocks per thread are in flight at a time: one at a time, the
-// staging of a CTA took 20 us of latency.
-template <int KD, int KH, int KW, int NCH, bool SOURCE, bool WIDE>
-__device__ __forceinline__ void stage(uint4* dst, int blocks, const bf16* src, long long stride, const Band& b, const At& at,
-                                      const unsigned (&negb)[NCH], bool relu) {
-    constexpr int U = 2;                           // times NCH channels in flight
-    const int rows = b.TH + KH - 1, planes = at.DC + KD - 1;
-    const int dq = kStagers % b.PB, dr = kStagers / b.PB;
-    int q = threadIdx.x % b.PB, row = threadIdx.x / b.PB, pl = 0, i = threadIdx.x;
-    while (row >= rows) { row -= rows; ++pl; }
-    while (pl < planes) {
-        unsigned a[U][NCH][5];
-        int w[U], at_i[U];
-        bool in[U];
+    __device__ __forceinline__ Stager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, int h0,
+                                      int tid)
+        : b(b_), src(src_), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int d = at.d0 - KD / 2 + pl, h = at.h0 - KH / 2 + row;
-            at_i[u] = pl < planes ? i : -1;
+        for (int u = 0; u < 2; ++u) {
+            const int i = tid + u * kStagers, row = i / b.PB, q = i - row * b.PB, h = h0 - KH / 2 + row;
+            at[u] = i < blocks ? i : -1;
             w[u] = 8 * q;
-            in[u] = pl < planes && d >= 0 && d < b.D && h >= 0 && h < b.H;
-            if (in[u]) {
-                const bf16* p = src + ((long long)d * b.H + h) * b.W;
-#pragma unroll
-                for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride, w[u], b, a[u][ch]);
-            }
-            i += kStagers; q += dq; row += dr;
-            if (q >= b.PB) { q -= b.PB; ++row; }
-            while (row >= rows) { row -= rows; ++pl; }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (at_i[u] < 0) continue;
-#pragma unroll
-            for (int ch = 0; ch < NCH; ++ch)
-                dst[ch * blocks + at_i[u]] = in[u] ? to_places<KW / 2, SOURCE>(a[u][ch], w[u], b, negb[ch], relu)
-                                                   : make_uint4(0u, 0u, 0u, 0u);
+            off[u] = i < blocks && h >= 0 && h < b.H ? h * row_stride : -1;
         }
     }
+    __device__ __forceinline__ void load(int d) {
+        const bf16* p = src + d * plane;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (off[u] >= 0) {
+#pragma unroll
+                for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride + off[u], w[u], b, a[u][ch]);
+            }
+    }
+    __device__ __forceinline__ void prefetch(int d) const {
+        const bf16* p = src + d * plane;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (off[u] >= 0 && (w[u] & 63) == 0 && w[u] < b.W) {
+#pragma unroll
+                for (int ch = 0; ch < NCH; ++ch)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off[u] + w[u]));
+            }
+    }
+    __device__ __forceinline__ void store(uint4* dst, const unsigned (&negb)[NCH], bool relu) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (at[u] < 0) continue;
+#pragma unroll
+            for (int ch = 0; ch < NCH; ++ch)
+                dst[ch * blocks + at[u]] = off[u] >= 0 ? to_places<KW / 2, SOURCE>(a[u][ch], w[u], b, negb[ch], relu)
+                                                       : make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    // All planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are passed
+    // on without data.
+    __device__ __forceinline__ bool run(uint4* slots, int slot_blocks, int d0, int PD, int planes, unsigned full, unsigned empty,
+                                        const unsigned (&negb)[NCH], bool relu, int lane) {
+        const int first = max(0, PD - d0), last = min(planes - 1, b.D - 1 + PD - d0);   // those inside
+        load(d0 - PD + first);
+        for (int p = 0; p < planes; ++p) {
+            const int s = p % kSlots;
+            if (p >= kSlots && !mbar_wait(empty + 8 * s, (p / kSlots - 1) & 1)) return false;
+            if (p >= first && p <= last) {
+                store(slots + s * slot_blocks, negb, relu);
+                if (p + 1 <= last) load(d0 - PD + p + 1);
+                if (p + 2 <= last) prefetch(d0 - PD + p + 2);
+                fence_async_proxy();
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + 8 * s);
+        }
+        return true;
+    }
+};
+
+// Blocks an MMA may read past the last staged row of a slot's last channel: 128 windows of two blocks
+// from the band's first row on.
+__host__ __device__ inline int slack_blocks(const Band& b) { return MB + 1 - b.TH * b.PB > 1 ? MB + 1 - b.TH * b.PB : 1; }
+
+// ---- two-lane float32 -------------------------------------------------------------------------
+using dw4::f32x2;
+using dw4::pack2;
+using dw4::unpack2;
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float rcp(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }  // i static
 
 // The banded matrices of a kernel by one warp: `value(t, n, kw)` is the filter tap of matrix t, column n.
 // Layout of one matrix: groups of eight columns, then the two halves of K, eight 16-byte rows each.
@@ -242,15 +312,6 @@ __device__ __forceinline__ void build_bands(bf16* bmat, int mats, int lane, F va
         reinterpret_cast<uint4*>(bmat)[e] = make_uint4(words[0], words[1], words[2], words[3]);
     }
 }
-
-// blocks of one channel's band in shared memory
-template <int KD, int KH>
-__host__ __device__ inline int band_blocks(const Band& b) { return (b.DC + KD - 1) * (b.TH + KH - 1) * b.PB; }
-// blocks the last MMA tile of a band may read past it
-__host__ __device__ inline int slack_blocks(const Band& b) { return b.MT * MB + 1 - b.TH * b.PB > 1 ? b.MT * MB + 1 - b.TH * b.PB : 1; }
-
-constexpr int kThreads = 288;     // eight staging / epilogue warps and the MMA warp
-constexpr int kHeader = 1024;     // bytes: barriers, TMEM address (256), the filter as float32
 
 enum Access { kWide = 0, kQuad = 1, kPaddedOut = 2 };   // 16-byte rows; 8-byte rows; 8-byte rows, out unpadded
 
@@ -286,122 +347,155 @@ struct AdjointArgs {
     const float* h; const float* bias;
 };
 
-// Work of a CTA: a band of TH rows of a chunk of DC planes.  x and t1 are staged whole, then the MMA
-// warp runs ahead of the epilogue by up to four (plane, MMA tile) items of 64 accumulator columns (A(x)
-// and A(t1), four channels of eight voxels each).
+// Accumulators: per output plane 32 columns of A(x) and 32 of A(t1) (four channels of eight voxels),
+// RING of them in turn; the epilogue leaves them zero.  Three depth taps: a ring of four planes, 256
+// columns, two CTAs per multiprocessor; five: eight planes, all 512.
+template <int KD> __host__ __device__ constexpr int adjoint_ring() { return KD > 3 ? 8 : 4; }
+
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kThreads, 2) tc_adjoint_kernel(const AdjointArgs P) {
-    constexpr int ROWT = KD * KH, NCOL = SC * 8, BUFS = 4, TCOLS = 256;
+__global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(const AdjointArgs P) {
+    constexpr bool ROWS = KH == 1;
+    constexpr int PD = KD / 2, NC = SC * 8, RING = adjoint_ring<KD>(), TCOLS = RING * 2 * NC, KT = KD * KH * KW;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     const Band& b = P.b;
-    const At at(b, blockIdx.x);
+    const At<ROWS> at(b, blockIdx.x);
+    const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W), oaddr(b.C, b.D, b.H, b.Wo);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned base = smem_u32(smem_tc);
-    const unsigned full = base, empty = base + 8 * BUFS, slot = base + 16 * BUFS;
+    const unsigned sfull = base, sempty = base + 8 * kSlots, afull = base + 16 * kSlots, aempty = afull + 8 * RING;
+    constexpr int kTmemAt = 16 * kSlots + 16 * RING;
     bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader);
-    uint4* const xs = reinterpret_cast<uint4*>(smem_tc + kHeader + ROWT * NCOL * 32);
-    const int blocks = band_blocks<KD, KH>(b), slack = slack_blocks(b);
-    uint4* const ts = xs + blocks;
+    uint4* const slots = reinterpret_cast<uint4*>(smem_tc + kHeader + KH * KD * NC * 32);
+    const int blocks = (b.TH + KH - 1) * b.PB, slot_blocks = 2 * blocks;
+    const int planes = at.DC + KD - 1;
 
-    if (warp == 8) tmem_alloc(slot, TCOLS);
+    if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, TCOLS);
     if (tid == 0) {
-        for (int i = 0; i < BUFS; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 4); }
+        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, kStageWarps); mbar_init(sempty + 8 * i, 1); }
+        for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 8) {
-        float* const hs = reinterpret_cast<float*>(smem_tc + 256);
-        for (int e = lane; e < SC * ROWT * KW; e += 32) hs[e] = P.h[(long long)at.c * SC * ROWT * KW + e];
+    // windows of valid blocks may touch blocks that no plane has been staged to: those have to be numbers
+    for (int i = tid; i < kSlots * slot_blocks + slack_blocks(b); i += kThreads) slots[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (warp == kMmaWarp) {
+        float* const hs = reinterpret_cast<float*>(smem_tc + 512);
+        for (int e = lane; e < SC * KT; e += 32) hs[e] = P.h[(long long)at.c * SC * KT + e];
         __syncwarp();
-        build_bands<NCOL, KW, true>(bmat, ROWT, lane, [&](int t, int n, int kw) { return hs[(n / 8) * ROWT * KW + t * KW + kw]; });
-    } else {
-        // x and t1 as two channels: the distance between the tensors takes the place of the stride
-        const unsigned none[2] = {0u, 0u};
-        const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
-        stage<KD, KH, KW, 2, false, AL == kWide>(xs, blocks, P.x + (long long)at.bc * b.SP, apart, b, at, none, false);
-    }
-    // what the windows of valid blocks may touch past the staged planes has to be a number
-    for (int i = tid; i < slack; i += kThreads) ts[blocks + i] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0 && at.DC < b.DC) {
-        const int end = (at.DC + KD - 1) * (b.TH + KH - 1) * b.PB;
-        xs[end] = make_uint4(0u, 0u, 0u, 0u);
-        ts[end] = make_uint4(0u, 0u, 0u, 0u);
+        // [kh][output plane p - (KD - 1) + kd: groups of 32 columns][channel, column]
+        build_bands<KD * NC, KW, true>(bmat, KH, lane, [&](int kh, int n, int kw) {
+            const int kd = n / NC, j = n % NC / 8;
+            return hs[j * KT + (kd * KH + kh) * KW + kw];
+        });
     }
     fence_async_proxy();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + 16 * BUFS);
-    const int items = at.DC * b.MT, plane = (b.TH + KH - 1) * b.PB;
+    const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + kTmemAt);
+    if (warp < kEpilogueWarps) {
+        for (int c = 32 * (warp >> 2); c < TCOLS; c += 64) tmem_zero32(tmem + ((unsigned)(warp & 3) << 21) + c);
+        tmem_wait_st();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
     bool ok = true;
-    if (warp == 8) {
-        const unsigned idesc = instr_desc(NCOL);
-        const unsigned xa = smem_u32(xs), ta = smem_u32(ts), ba = smem_u32(bmat);
-        for (int it = 0; it < items && ok; ++it) {
-            const int buf = it % BUFS, pl = it / b.MT, mt = it - pl * b.MT;
-            if (it >= BUFS) ok = mbar_wait(empty + 8 * buf, ((it / BUFS) - 1) & 1);
+    if (warp == kMmaWarp) {
+        const unsigned xa = smem_u32(slots), ba = smem_u32(bmat);
+        for (int p = 0; p < planes && ok; ++p) {
+            const int s = p % kSlots, d = at.d0 - PD + p;
+            ok = mbar_wait(sfull + 8 * s, (p / kSlots) & 1);
+            // a new output plane begins: its accumulators have been read and zeroed
+            if (p >= RING && p < at.DC) ok = mbar_wait(aempty + 8 * (p % RING), (p / RING - 1) & 1) && ok;
             tc_fence_after();
             if (lane == 0 && ok) {
-                const unsigned d = tmem + buf * 2 * NCOL;
-                for (int t = 0; t < ROWT; ++t) {
-                    const int kd = t / KH, kh = t - kd * KH;
-                    const unsigned off = 16 * ((pl + KD - 1 - kd) * plane + (KH - 1 - kh) * b.PB + mt * MB);
-                    const unsigned long long bd = mat_desc(ba + t * NCOL * 32, 128, 256);
-                    mma(d, mat_desc(xa + off, 16, 128), bd, idesc, t > 0);
-                    mma(d + NCOL, mat_desc(ta + off, 16, 128), bd, idesc, t > 0);
+                if (d >= 0 && d < b.D) {
+                    // groups g of output planes o = p - (KD - 1) + g inside the chunk
+                    const int g0 = max(0, KD - 1 - p), g1 = min(KD - 1, at.DC - 1 + KD - 1 - p), o0 = p - (KD - 1) + g0;
+                    const int r0 = o0 % RING, n = g1 - g0 + 1, n0 = min(n, RING - r0);
+                    for (int kh = 0; kh < KH; ++kh) {
+                        const unsigned off = 16 * (s * slot_blocks + (KH - 1 - kh) * b.PB);
+                        const unsigned bm = ba + (kh * KD + g0) * NC * 32;
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) {                            // x, t1
+                            const unsigned long long ad = mat_desc(xa + off + a * 16 * blocks, 16, 128);
+                            const unsigned acc = tmem + a * RING * NC;
+                            mma(acc + r0 * NC, ad, mat_desc(bm, 128, 256), instr_desc(n0 * NC), 1);
+                            if (n > n0) mma(acc, ad, mat_desc(bm + n0 * NC * 32, 128, 256), instr_desc((n - n0) * NC), 1);
+                        }
+                    }
                 }
-                mma_commit(full + 8 * buf);
+                mma_commit(sempty + 8 * s);
+                const int o = p - (KD - 1);
+                if (o >= 0) mma_commit(afull + 8 * (o % RING));
             }
             __syncwarp();
         }
+    } else if (warp >= kEpilogueWarps) {
+        const unsigned none[2] = {0u, 0u};
+        // x and t1 as two channels: the distance between the tensors takes the place of the stride
+        const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
+        Stager<KH, KW, 2, false, AL == kWide> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at.h0,
+                                                 tid - 32 * kEpilogueWarps);
+        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, none, false, lane);
     } else {
-        const int grp = warp >> 2, m = (warp & 3) * 32 + lane;
-        float bj[SC];
+        const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q;
+        const bool valid = r < at.TH && q < b.NB;
+        const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
+        const f32x2 eps2 = pack2(b.eps, b.eps);
+        f32x2 b2[SC];
 #pragma unroll
-        for (int j = 0; j < SC; ++j) bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
-        const bf16* const zb = P.z + (long long)at.bc * SC * b.SP;
-        const long long osp = (long long)b.D * b.H * b.Wo;
-        bf16* const ob = P.out + (long long)at.bc * SC * osp;
-        for (int it = grp; it < items && ok; it += 2) {
-            const int buf = it % BUFS, pl = it / b.MT, mt = it - pl * b.MT;
-            const int blk = mt * MB + m, r = blk / b.PB, q = blk - r * b.PB, w = 8 * q;
-            const bool valid = r < at.TH && q < b.NB;
-            const long long line = (long long)(at.d0 + pl) * b.H + at.h0 + r;
+        for (int j = 0; j < SC; ++j) {
+            const float v = P.bias ? P.bias[at.c * SC + j] : 0.0f;
+            b2[j] = pack2(v, v);
+        }
+        const bf16* const zb = P.z + (long long)at.bc * SC * addr.chan + (at.h0 + r) * addr.row_z;
+        bf16* const ob = P.out + (long long)at.bc * SC * oaddr.chan + (at.h0 + r) * oaddr.row_z;
+        for (int o = warp >> 2; o < at.DC && ok; o += 2) {
+            const int slot = o % RING;
+            const long long d = at.d0 + o;
             uint4 zr[SC];
 #pragma unroll
             for (int j = 0; j < SC; ++j) {
                 zr[j] = make_uint4(0u, 0u, 0u, 0u);
-                if (valid) zr[j] = load8<AL>(zb + j * b.SP + line * b.W, w, b.W);
+                if (valid) zr[j] = load8<AL>(zb + j * addr.chan + d * addr.plane, w, b.W);
             }
-            ok = mbar_wait(full + 8 * buf, (it / BUFS) & 1);
+            ok = mbar_wait(afull + 8 * slot, (o / RING) & 1);
             tc_fence_after();
-            const unsigned d = tmem + ((unsigned)(warp & 3) << 21) + buf * 2 * NCOL;   // lane in bits 16+: 32 lanes per warp
+            const unsigned acc = lanes + slot * NC;
 #pragma unroll
             for (int j = 0; j < SC; ++j) {
-                float n[8], dn[8], o[8];
+                float n[8], dn[8];
                 __syncwarp();
-                tmem_load8x2(d + 8 * j, d + NCOL + 8 * j, n, dn);
-                if (j == SC - 1) {                       // the accumulators are free again
+                tmem_load8x2(acc + 8 * j, acc + RING * NC + 8 * j, n, dn);
+                if (j == SC - 1) {                       // read: zero for the plane that takes the place
+                    tmem_zero32(acc);
+                    tmem_zero32(acc + RING * NC);
+                    tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(empty + 8 * buf);
+                    if (lane == 0) mbar_arrive(aempty + 8 * slot);
                 }
+                unsigned v[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    float s = word_lane(zr[j], i) + bj[j];
-                    if (b.relu) s = fmaxf(s, 0.0f);
-                    o[i] = dw4::fast_div(s * (n[i] + b.eps), dn[i] + b.eps);
+                for (int i = 0; i < 4; ++i) {
+                    const unsigned u = word_of(zr[j], i);
+                    f32x2 s2 = add2(pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)), b2[j]);
+                    float lo, hi, dl, dh;
+                    unpack2(s2, lo, hi);
+                    if (b.relu) { lo = fmaxf(lo, 0.0f); hi = fmaxf(hi, 0.0f); }
+                    const f32x2 num = mul2(pack2(lo, hi), add2(pack2(n[2 * i], n[2 * i + 1]), eps2));
+                    unpack2(add2(pack2(dn[2 * i], dn[2 * i + 1]), eps2), dl, dh);
+                    unpack2(mul2(num, pack2(rcp(dl), rcp(dh))), lo, hi);
+                    v[i] = pack_bf16(lo, hi);
                 }
                 if (valid) {
-                    const uint4 v = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
-                    bf16* orow = ob + j * osp + line * b.Wo;
-                    if (AL != kPaddedOut || b.Wo == b.W) store8<AL>(orow, w, b.W, v);
+                    bf16* orow = ob + j * oaddr.chan + d * oaddr.plane;
+                    if (AL != kPaddedOut || b.Wo == b.W) store8<AL>(orow, w, b.W, make_uint4(v[0], v[1], v[2], v[3]));
                     else {
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
-                            if (w + i < b.Wv) {
-                                const unsigned u = i < 2 ? v.x : i < 4 ? v.y : i < 6 ? v.z : v.w;
-                                reinterpret_cast<unsigned short*>(orow)[w + i] = (unsigned short)(i & 1 ? u >> 16 : u);
-                            }
+                            if (w + i < b.Wv) reinterpret_cast<unsigned short*>(orow)[w + i] = (unsigned short)(i & 1 ? v[i / 2] >> 16 : v[i / 2]);
                     }
                 }
             }
@@ -410,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_adjoint_kernel(const AdjointAr
     if (!ok && lane == 0) atomicExch(&g_wait_expired, 1u);
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) tmem_free(tmem, TCOLS);
+    if (warp == kMmaWarp) tmem_free(tmem, TCOLS);
 }
 
 // ---- t1 = K(relu(z + b)) ------------------------------------------------------------------------
@@ -420,45 +514,50 @@ struct SourceArgs {
     const float* h; const float* bias;
 };
 
-// Accumulator columns.  Volumes: a source plane p is multiplied once per (channel, kh) by the banded
-// matrices of its KD = 3 depth taps side by side (24 columns, 8 of zeros: N is a multiple of 16), onto
-// the accumulators of output planes p, p - 1, p - 2 of the chunk, which lie 8 columns apart: 12 MMAs a
-// plane where one per tap would be 36.  All accumulators start at zero.  Images: N = 16 with 8
-// columns of zeros, one MMA per (channel, kh).
-template <int KD> __host__ __device__ constexpr int source_cols(int DC) { return KD > 1 ? 8 * (DC + KD + 2) : 16; }
-inline int tmem_cols(int n) { int c = 32; while (c < n) c *= 2; return c; }
+// Accumulators: 8 columns per output plane of the chunk.  A source plane is multiplied once per
+// (channel, kh), by the matrices of all depth taps at once: 12 MMAs of a 3x3x3 filter, 4 of an image
+// filter.  N is a multiple of 16, so an odd number of taps is padded by columns of zeros.
+template <int KD> __host__ __device__ constexpr int source_groups() { return (KD + 1) / 2 * 2; }
+constexpr int kSourceCols = 256;
+// planes of a chunk whose accumulators (and those of the taps that fall outside it) fit
+template <int KD> __host__ __device__ constexpr int source_planes() { return kSourceCols / 8 - KD + 2 - source_groups<KD>(); }
 
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs P, int tcols) {
+__global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs P) {
+    constexpr bool ROWS = KH == 1;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
-    constexpr int NCOL = KD > 1 ? 32 : 16, NMAT = SC * KH, MAXSTEP = 24;
+    constexpr int NCOL = 8 * source_groups<KD>(), NMAT = SC * KH;
     constexpr int TABLE = (PD + 1) * (PD + 1) * (PH + 1) * (PH + 1) * (PW + 1) * (PW + 1);
+    static_assert(2 * kSlots + source_planes<KD>() + 1 <= 64, "barriers");
     extern __shared__ __align__(128) unsigned char smem_tc[];
     const Band& b = P.b;
-    const At at(b, blockIdx.x);
+    const At<ROWS> at(b, blockIdx.x);
+    const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const unsigned base = smem_u32(smem_tc), slot = base + 8 * MAXSTEP;
+    const unsigned base = smem_u32(smem_tc);
+    const unsigned sfull = base, sempty = base + 8 * kSlots, afull = base + 16 * kSlots;
+    constexpr int kTmemAt = 504;
     float* const table = reinterpret_cast<float*>(smem_tc + kHeader);
     bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader + (TABLE * 4 + 127) / 128 * 128);
-    uint4* const zs = reinterpret_cast<uint4*>(bmat + NMAT * NCOL * 16);
-    const int blocks = band_blocks<KD, KH>(b), slack = slack_blocks(b);
-    const int plane = (b.TH + KH - 1) * b.PB, used = (at.DC + KD - 1) * plane;
-    const int steps = KD > 1 ? at.DC + KD - 1 : b.MT;
-    const int mcols = source_cols<KD>(b.DC);
+    uint4* const slots = reinterpret_cast<uint4*>(bmat + NMAT * NCOL * 16);
+    const int blocks = (b.TH + KH - 1) * b.PB, slot_blocks = SC * blocks;
+    const int planes = at.DC + KD - 1;
 
-    if (warp == 8) tmem_alloc(slot, tcols);
+    if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, kSourceCols);
     if (tid == 0) {
-        for (int i = 0; i < steps; ++i) mbar_init(base + 8 * i, 1);
+        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, kStageWarps); mbar_init(sempty + 8 * i, 1); }
+        for (int i = 0; i < at.DC; ++i) mbar_init(afull + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 8) {
-        float* const hs = reinterpret_cast<float*>(smem_tc + 256);
+    for (int i = tid; i < kSlots * slot_blocks + slack_blocks(b); i += kThreads) slots[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (warp == kMmaWarp) {
+        float* const hs = reinterpret_cast<float*>(smem_tc + 512);
         for (int e = lane; e < SC * KT; e += 32) hs[e] = P.h[(long long)at.c * SC * KT + e];
         float bj[SC];
 #pragma unroll
         for (int j = 0; j < SC; ++j) bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
         __syncwarp();
-        // column group g: output plane p - kd, kd = KD - 1 - g
+        // [channel, kh][output plane p - kd, kd = KD - 1 - g: groups of 8 columns]
         build_bands<NCOL, KW, false>(bmat, NMAT, lane, [&](int t, int n, int kw) {
             const int j = t / KH, kh = t % KH, kd = KD - 1 - n / 8;
             return kd >= 0 ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
@@ -482,83 +581,81 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
                     }
             table[e] = s;
         }
-    } else {
+    }
+    fence_async_proxy();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + kTmemAt);
+    if (warp < kEpilogueWarps) {
+        for (int c = 32 * (warp >> 2); c < kSourceCols; c += 64) tmem_zero32(tmem + ((unsigned)(warp & 3) << 21) + c);
+        tmem_wait_st();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    bool ok = true;
+    if (warp == kMmaWarp) {
+        const unsigned za = smem_u32(slots), ba = smem_u32(bmat), idesc = instr_desc(NCOL);
+        for (int p = 0; p < planes && ok; ++p) {
+            const int s = p % kSlots, d = at.d0 - PD + p;
+            ok = mbar_wait(sfull + 8 * s, (p / kSlots) & 1);
+            tc_fence_after();
+            if (lane == 0 && ok) {
+                if (d >= 0 && d < b.D)
+                    for (int t = 0; t < NMAT; ++t) {
+                        const int j = t / KH, kh = t - j * KH;
+                        mma(tmem + 8 * p, mat_desc(za + 16 * (s * slot_blocks + j * blocks + kh * b.PB), 16, 128),
+                            mat_desc(ba + t * NCOL * 32, 128, 256), idesc, 1);
+                    }
+                mma_commit(sempty + 8 * s);
+                const int o = p - (KD - 1);
+                if (o >= 0) mma_commit(afull + 8 * o);
+            }
+            __syncwarp();
+        }
+    } else if (warp >= kEpilogueWarps) {
         unsigned negb[SC];
 #pragma unroll
         for (int j = 0; j < SC; ++j) {
             const __nv_bfloat162 nb = __float2bfloat162_rn(P.bias ? -P.bias[at.c * SC + j] : 0.0f);
             negb[j] = *reinterpret_cast<const unsigned*>(&nb);
         }
-        stage<KD, KH, KW, SC, true, AL == kWide>(zs, blocks, P.z + (long long)at.bc * SC * b.SP, b.SP, b, at, negb, b.relu);
-    }
-    for (int i = tid; i < slack; i += kThreads) zs[SC * blocks + i] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid < SC && at.DC < b.DC) zs[tid * blocks + used] = make_uint4(0u, 0u, 0u, 0u);
-    fence_async_proxy();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + 8 * MAXSTEP);
-    const unsigned lanes = (unsigned)(warp & 3) << 21;
-    if (KD > 1) {
-        if (warp < 8) {
-            for (int c = 8 * (warp >> 2); c < b.MT * mcols; c += 16) tmem_zero8(tmem + lanes + c);
-            tmem_wait_st();
-            tc_fence_before();
-        }
-        __syncthreads();
-        tc_fence_after();
-    }
-    bool ok = true;
-    if (warp == 8) {
-        if (lane == 0) {
-            const unsigned idesc = instr_desc(NCOL);
-            const unsigned za = smem_u32(zs), ba = smem_u32(bmat);
-            for (int step = 0; step < steps; ++step) {
-                const int mt0 = KD > 1 ? 0 : step, mt1 = KD > 1 ? b.MT : step + 1, p = KD > 1 ? step : 0;
-                for (int mt = mt0; mt < mt1; ++mt)
-                    for (int t = 0; t < NMAT; ++t) {
-                        const int j = t / KH, kh = t - j * KH;
-                        mma(tmem + mt * mcols + 8 * p, mat_desc(za + 16 * (j * blocks + p * plane + kh * b.PB + mt * MB), 16, 128),
-                            mat_desc(ba + t * NCOL * 32, 128, 256), idesc, KD > 1 || t > 0);
-                    }
-                mma_commit(base + 8 * step);
-            }
-        }
+        Stager<KH, KW, SC, true, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at.h0,
+                                                 tid - 32 * kEpilogueWarps);
+        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, negb, b.relu, lane);
     } else {
-        const int grp = warp >> 2, m = (warp & 3) * 32 + lane;
-        bf16* const tb = P.t1 + (long long)at.bc * b.SP;
-        const int items = at.DC * b.MT;
-        // item: output plane pl of MMA tile mt; complete after source plane pl + KD - 1 (volumes)
-        for (int it = grp; it < items && ok; it += 2) {
-            const int pl = it / b.MT, mt = it - pl * b.MT;
-            const int blk = mt * MB + m, r = blk / b.PB, q = blk - r * b.PB, w = 8 * q;
-            const bool valid = r < at.TH && q < b.NB;
-            const int d = at.d0 + pl, h = at.h0 + r;
-            const int dl = max(0, PD - d), dh = max(0, d + PD - (b.D - 1)), hl = max(0, PH - h), hh = min(PH, max(0, h + PH - (b.H - 1)));
+        const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q, h = at.h0 + r;
+        const bool valid = r < at.TH && q < b.NB, inner = w >= PW && w + 7 + PW < b.Wv;
+        const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
+        bf16* const tb = P.t1 + (long long)at.bc * addr.chan + h * addr.row_x;
+        // images: every row of a plane is an image of its own, KH = 1
+        const int hl = max(0, PH - h), hh = min(PH, max(0, h + PH - (b.H - 1)));
+        for (int o = warp >> 2; o < at.DC && ok; o += 2) {
+            const int d = at.d0 + o, dl = max(0, PD - d), dh = max(0, d + PD - (b.D - 1));
             const float* tab = table + (((dl * (PD + 1) + dh) * (PH + 1) + hl) * (PH + 1) + hh) * (PW + 1) * (PW + 1);
-            ok = mbar_wait(base + 8 * (KD > 1 ? pl + KD - 1 : mt), 0);
+            ok = mbar_wait(afull + 8 * o, 0);
             tc_fence_after();
             __syncwarp();
-            float o[8];
-            tmem_load8(tmem + lanes + mt * mcols + 8 * (KD > 1 ? pl + KD - 1 : 0), o);
+            float v[8];
+            tmem_load8(lanes + 8 * (o + KD - 1), v);
             if (valid) {
-                const bool inner = w >= PW && w + 7 + PW < b.Wv;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     int cut = 0;
                     if (!inner) cut = max(0, PW - w - i) * (PW + 1) + min(PW, max(0, w + i + PW - (b.Wv - 1)));
-                    o[i] += tab[cut];
-                    if (!inner && w + i >= b.Wv) o[i] = 0.0f;
+                    v[i] += tab[cut];
+                    if (!inner && w + i >= b.Wv) v[i] = 0.0f;
                 }
-                store8<AL>(tb + ((long long)d * b.H + h) * b.W, w, b.W,
-                           make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7])));
+                store8<AL>(tb + (long long)d * addr.plane, w, b.W,
+                           make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])));
             }
         }
     }
     if (!ok && lane == 0) atomicExch(&g_wait_expired, 1u);
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) tmem_free(tmem, tcols);
+    if (warp == kMmaWarp) tmem_free(tmem, kSourceCols);
 }
 
 }  // namespace tc

@@ -20,10 +20,11 @@ CASES = [
     (4, (3, 3, 3), 1, (1, 16, 20)),
     (300, (3, 3, 3), 1, (18, 16, 16)),
     (6, (5, 5), 3, (130, 128)),
-    (5, (5, 5), 2, (37, 68)),
+    (5, (5, 5), 5, (37, 68)),
     (3, (5, 5), 1, (40, 512)),
-    (40, (5, 5), 1, (16, 16)),
+    (40, (5, 5), 9, (16, 28)),
     (3, (3, 3), 4, (45, 256)),
+    (7, (3, 3), 20, (9, 36)),
 ]
 
 
@@ -57,7 +58,7 @@ def test_matches_the_fma_kernels(case, relu):
 
 
 @pytest.mark.parametrize("spatial,ks", [((9, 31, 45), (3, 3, 3)), ((5, 20, 27), (3, 3, 3)), ((33, 29, 62), (3, 3, 3)),
-                                        ((41, 171), (5, 5)), ((30, 53), (3, 3))])
+                                        ((41, 171), (5, 5)), ((30, 253), (3, 3))])
 def test_layer_with_padded_rows(spatial, ks):
     """Row lengths of every remainder modulo eight, two updates, against the generic kernels."""
     dev = torch.device("cuda:0")
