@@ -15,12 +15,14 @@ bool plan(const Geo& g, int most, Band& b) {
     b.C = g.G; b.D = g.D; b.H = g.H; b.W = g.W; b.Wv = g.Wv; b.Wo = g.Wo; b.eps = g.eps; b.relu = g.relu;
     b.NB = (g.Wv + 7) / 8;
     b.PB = (g.Wv + KW / 2 + 7) / 8;
-    b.TH = std::min(g.H, MB / b.PB);
+    b.TH = std::min(g.H, std::min(MB / b.PB, kSourceStagers / b.PB - (KH - 1)));
     if (b.TH < 1) return false;
     b.nth = (g.H + b.TH - 1) / b.TH;
     b.TH = (g.H + b.nth - 1) / b.nth;
     b.nth = (g.H + b.TH - 1) / b.TH;
-    if ((b.TH + KH - 1) * b.PB > kMaxBlocks) return false;
+    // 32-bit offsets inside a band
+    const long long row = KH == 1 ? (long long)g.D * g.W * g.G * SC : g.W;
+    if ((b.TH + KH - 1) * row >= (1LL << 31)) return false;
     const long long per = (long long)g.B * g.G * b.nth;
     long long ndc = (g.D + most - 1) / most;
     const long long want = (4 * 148 + per - 1) / per, finest = std::max(1, g.D / (6 * (KD / 2)));
@@ -44,12 +46,12 @@ template <int KD, int KH, int KW> size_t source_smem(const Band& b) {
 }
 
 template <typename K, typename P>
-cudaError_t launch(K kern, const Band& b, const Geo& g, size_t smem, cudaStream_t st, const P& p) {
+cudaError_t launch(K kern, int threads, const Band& b, const Geo& g, size_t smem, cudaStream_t st, const P& p) {
     const long long grid = (long long)g.B * g.G * b.nth * b.ndc;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)grid, kThreads, smem, st>>>(p);
+    kern<<<(unsigned)grid, threads, smem, st>>>(p);
     launched();
     return cudaGetLastError();
 }
@@ -63,13 +65,13 @@ cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, cons
     S.z = z; S.t1 = t1; S.h = h; S.bias = bias;
     const size_t sa = adjoint_smem<KD, KH, KW>(A.b), ss = source_smem<KD, KH, KW>(S.b);
     auto on16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-    const bool wide = g.W % 8 == 0 && on16(x) && on16(z) && on16(t1);
-    cudaError_t e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, S.b, g, ss, st, S)
-                         : launch(tc_source_kernel<KD, KH, KW, kQuad>, S.b, g, ss, st, S);
+    const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1);
+    cudaError_t e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, g, ss, st, S)
+                         : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, g, ss, st, S);
     if (e != cudaSuccess) return e;
-    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut>, A.b, g, sa, st, A);
-    return wide && on16(out) ? launch(tc_adjoint_kernel<KD, KH, KW, kWide>, A.b, g, sa, st, A)
-                             : launch(tc_adjoint_kernel<KD, KH, KW, kQuad>, A.b, g, sa, st, A);
+    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut>, kAdjointThreads, A.b, g, sa, st, A);
+    return wide && on16(out) ? launch(tc_adjoint_kernel<KD, KH, KW, kWide>, kAdjointThreads, A.b, g, sa, st, A)
+                             : launch(tc_adjoint_kernel<KD, KH, KW, kQuad>, kAdjointThreads, A.b, g, sa, st, A);
 }
 
 template <int KD, int KH, int KW>

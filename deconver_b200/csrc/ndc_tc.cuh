@@ -61,8 +61,8 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase) {
     unsigned long long start = 0;
     for (;;) {
         unsigned done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(bar), "r"(phase) : "memory");
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(bar), "r"(phase), "r"(1000000u) : "memory");   // asleep for up to 1 ms
         if (done) return true;
         unsigned long long now;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
@@ -104,9 +104,11 @@ __device__ __forceinline__ void tmem_load8x2(unsigned addr_a, unsigned addr_b, f
 #pragma unroll
     for (int i = 0; i < 8; ++i) { a[i] = __uint_as_float(r[i]); b[i] = __uint_as_float(r[8 + i]); }
 }
-__device__ __forceinline__ void tmem_zero32(unsigned addr) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
-                 "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(addr), "r"(0u) : "memory");
+// `n` columns (a multiple of 8) of this thread's lane; eight at a time, since every column takes a register
+__device__ __forceinline__ void tmem_fill(unsigned addr, float v, int n) {
+#pragma unroll 4
+    for (int i = 0; i < n; i += 8)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(addr + i), "r"(__float_as_uint(v)) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -126,14 +128,15 @@ __device__ __forceinline__ unsigned instr_desc(int n) { return 1u << 4 | 1u << 7
 // Set where a wait ran out; the results of that launch are then undefined.
 static __device__ unsigned g_wait_expired;
 
-// Roles of a CTA's warps: two groups of four for the epilogue (they take turns, output plane by output
-// plane; TMEM lane 32 i + l belongs to lane l of the warps i of a group), four that stage source
-// planes, one that builds the banded matrices and issues the MMAs.
-constexpr int kEpilogueWarps = 8, kStageWarps = 4, kMmaWarp = kEpilogueWarps + kStageWarps;
-constexpr int kThreads = 32 * (kMmaWarp + 1), kStagers = 32 * kStageWarps;
+// Roles of a CTA's warps: groups of four for the epilogue (they take turns, output plane by output
+// plane; TMEM lane 32 i + l belongs to lane l of warp i of a group), groups that stage source planes (in
+// turns as well), one warp that issues the MMAs.  The adjoint kernel has two epilogue groups and one group
+// of four warps that stages; the source kernel, whose epilogue is short and whose source planes have four
+// channels, has one and two groups of five.
+constexpr int kAdjointThreads = 32 * (8 + 4 + 1), kSourceThreads = 32 * (4 + 10 + 1);
+constexpr int kSourceStagers = 160;
 constexpr int kSlots = 4;         // staged planes
 constexpr int kHeader = 1024;     // bytes: barriers and the TMEM address (512), the filter as float32
-constexpr int kMaxBlocks = 2 * kStagers;   // blocks of a staged plane (and channel), at most
 
 // Place of a CTA: (sample, channel), band of rows, chunk of planes; all addresses in elements.
 template <bool ROWS>
@@ -148,41 +151,45 @@ struct At {
     }
 };
 
-// Columns w-2 .. w+7 of a global row as five words, w = 8 q; zero outside the row.
+// Columns w-2 .. w+7 of a global row as five words, w = 8 q at `p[off]`; zero outside the row of W.
 template <bool WIDE>
-__device__ __forceinline__ void load_words(const bf16* row, int w, const Band& b, unsigned (&a)[5]) {
+__device__ __forceinline__ void load_words(const bf16* p, unsigned off, int w, int W, unsigned (&a)[5]) {
 #pragma unroll
     for (int i = 0; i < 5; ++i) a[i] = 0u;
-    if (w > 0 && w - 4 < b.W) a[0] = __ldg(reinterpret_cast<const unsigned*>(row + w - 2));
+    if (w > 0 && w - 4 < W) a[0] = __ldg(reinterpret_cast<const unsigned*>(p + (off - 2u)));
     if (WIDE) {
-        if (w < b.W) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + w));
+        if (w < W) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + off));
             a[1] = v.x; a[2] = v.y; a[3] = v.z; a[4] = v.w;
         }
     } else {
-        if (w < b.W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + w)); a[1] = v.x; a[2] = v.y; }
-        if (w + 4 < b.W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + w + 4)); a[3] = v.x; a[4] = v.y; }
+        if (w < W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + off)); a[1] = v.x; a[2] = v.y; }
+        if (w + 4 < W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (off + 4u))); a[3] = v.x; a[4] = v.y; }
     }
 }
 // The eight places of block q of a shared row (columns 8 q - PW .. 8 q + 7 - PW) from those words.
-// SOURCE: max(value, -bias) inside the volume (`negb`: two copies of -bias), zero in the padding.
-template <int PW, bool SOURCE>
-__device__ __forceinline__ uint4 to_places(unsigned (&a)[5], int w, const Band& b, unsigned negb, bool relu) {
+// SOURCE: max(value, -bias) inside the volume (`negb`: two copies of -bias), zero outside: with RELU, z is
+// zero there, and so is max(0, 0).  `inside`: with whole blocks (WIDE) bits 0 and 1 for the first word and the
+// others, else two bits per word, one per column.
+template <int PW, bool SOURCE, bool WIDE>
+__device__ __forceinline__ uint4 to_places(unsigned (&a)[5], unsigned inside, unsigned negb, bool relu) {
     if (SOURCE) {
-        if (relu) {
 #pragma unroll
-            for (int i = 0; i < 5; ++i) {
-                const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a[i]), *reinterpret_cast<const __nv_bfloat162*>(&negb));
-                a[i] = *reinterpret_cast<const unsigned*>(&v);
+        for (int i = 0; i < 5; ++i) {
+            unsigned m;
+            if (WIDE) {
+                m = inside & (i ? 2u : 1u) ? 0xffffffffu : 0u;
+            } else {
+                // byte 0 or 1 of 0xff00, twice per column
+                const unsigned two = inside >> (2 * i);
+                m = __byte_perm(0xff00u, 0u, (two & 1u) * 0x0011u + (two & 2u) * 0x0880u);
             }
-            if (w == 0) a[0] = 0u;
-        }
-        if (w + 7 >= b.Wv) {                       // the row ends here
-#pragma unroll
-            for (int i = 0; i < 5; ++i) {
-                const int c = w - 2 + 2 * i;
-                if (c >= b.Wv) a[i] = 0u;
-                else if (c + 1 >= b.Wv) a[i] &= 0xffffu;
+            if (relu) {
+                const unsigned nb = negb & m;
+                const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a[i]), *reinterpret_cast<const __nv_bfloat162*>(&nb));
+                a[i] = *reinterpret_cast<const unsigned*>(&v);
+            } else {
+                a[i] &= m;
             }
         }
     }
@@ -192,75 +199,89 @@ __device__ __forceinline__ uint4 to_places(unsigned (&a)[5], int w, const Band& 
 }
 
 // Stages planes of NCH channels (`src + ch * stride`), halo rows included; rows outside the volume are
-// zero.  A thread has up to two blocks of a plane; their loads are issued a plane ahead of the stores
-// and the lines of the plane after that are asked for from L2.
-template <int KH, int KW, int NCH, bool SOURCE, bool WIDE>
+// zero.  A thread of a group of NTHR has up to U blocks of a plane, and the loads of its group's next plane
+// are on their way in registers while it waits for a slot; the lines of the one after are asked for
+// from L2.  Addresses are a base that is the same for the whole CTA and a 32-bit offset.
+template <int KH, int KW, int NCH, bool SOURCE, bool WIDE, int NTHR, int U, int GROUPS>
 struct Stager {
     const Band& b;
-    const bf16* src;
+    const bf16* src;               // row h0 - KH / 2 of plane 0
     long long stride, plane;
     int blocks;                    // per channel of a slot
-    long long off[2];              // this thread's blocks: row offset, or -1 outside the volume
-    int w[2], at[2];               // column; block, or -1
-    unsigned a[2][NCH][5];
+    unsigned off[U];               // this thread's blocks: offset of the first column
+    bool in[U];                    // inside the volume (else zero)
+    int w[U], at[U];               // column; block, or -1
+    unsigned inside[U];
+    unsigned a[U][NCH][5];
 
     __device__ __forceinline__ Stager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, int h0,
                                       int tid)
-        : b(b_), src(src_), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB) {
+        : b(b_), src(src_ + (h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int i = tid + u * kStagers, row = i / b.PB, q = i - row * b.PB, h = h0 - KH / 2 + row;
+        for (int u = 0; u < U; ++u) {
+            const int i = tid + u * NTHR, row = i / b.PB, q = i - row * b.PB, h = h0 - KH / 2 + row;
             at[u] = i < blocks ? i : -1;
             w[u] = 8 * q;
-            off[u] = i < blocks && h >= 0 && h < b.H ? h * row_stride : -1;
+            off[u] = (unsigned)(row * row_stride) + w[u];
+            in[u] = i < blocks && h >= 0 && h < b.H;
+            inside[u] = 0u;
+            if (WIDE) {
+                inside[u] = (w[u] > 0 ? 1u : 0u) | (w[u] < b.Wv ? 2u : 0u);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 10; ++k) {
+                    const int c = w[u] - 2 + k;
+                    if (c >= 0 && c < b.Wv) inside[u] |= 1u << k;
+                }
+            }
         }
     }
     __device__ __forceinline__ void load(int d) {
         const bf16* p = src + d * plane;
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
-            if (off[u] >= 0) {
+        for (int u = 0; u < U; ++u)
+            if (in[u]) {
 #pragma unroll
-                for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride + off[u], w[u], b, a[u][ch]);
+                for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride, off[u], w[u], b.W, a[u][ch]);
             }
     }
     __device__ __forceinline__ void prefetch(int d) const {
         const bf16* p = src + d * plane;
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
-            if (off[u] >= 0 && (w[u] & 63) == 0 && w[u] < b.W) {
+        for (int u = 0; u < U; ++u)
+            if (in[u] && (w[u] & 63) == 0 && w[u] < b.W) {
 #pragma unroll
                 for (int ch = 0; ch < NCH; ++ch)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off[u] + w[u]));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off[u]));
             }
     }
     __device__ __forceinline__ void store(uint4* dst, const unsigned (&negb)[NCH], bool relu) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < U; ++u) {
             if (at[u] < 0) continue;
 #pragma unroll
             for (int ch = 0; ch < NCH; ++ch)
-                dst[ch * blocks + at[u]] = off[u] >= 0 ? to_places<KW / 2, SOURCE>(a[u][ch], w[u], b, negb[ch], relu)
-                                                       : make_uint4(0u, 0u, 0u, 0u);
+                dst[ch * blocks + at[u]] = in[u] ? to_places<KW / 2, SOURCE, WIDE>(a[u][ch], inside[u], negb[ch], relu)
+                                                 : make_uint4(0u, 0u, 0u, 0u);
         }
     }
-    // All planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are passed
-    // on without data.
+    // This group's planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are
+    // passed on without data.
     __device__ __forceinline__ bool run(uint4* slots, int slot_blocks, int d0, int PD, int planes, unsigned full, unsigned empty,
-                                        const unsigned (&negb)[NCH], bool relu, int lane) {
+                                        const unsigned (&negb)[NCH], bool relu, int group, int lane) {
         const int first = max(0, PD - d0), last = min(planes - 1, b.D - 1 + PD - d0);   // those inside
-        load(d0 - PD + first);
-        for (int p = 0; p < planes; ++p) {
+        if (group >= first && group <= last) load(d0 - PD + group);
+        for (int p = group; p < planes; p += GROUPS) {
             const int s = p % kSlots;
             if (p >= kSlots && !mbar_wait(empty + 8 * s, (p / kSlots - 1) & 1)) return false;
             if (p >= first && p <= last) {
                 store(slots + s * slot_blocks, negb, relu);
-                if (p + 1 <= last) load(d0 - PD + p + 1);
-                if (p + 2 <= last) prefetch(d0 - PD + p + 2);
                 fence_async_proxy();
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * s);
+            if (p + GROUPS >= first && p + GROUPS <= last) load(d0 - PD + p + GROUPS);
+            if (p + 2 * GROUPS <= last) prefetch(d0 - PD + p + 2 * GROUPS);
         }
         return true;
     }
@@ -291,11 +312,11 @@ __device__ __forceinline__ float rcp(float v) {
 }
 __device__ __forceinline__ unsigned word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }  // i static
 
-// The banded matrices of a kernel by one warp: `value(t, n, kw)` is the filter tap of matrix t, column n.
+// The banded matrices of a kernel: `value(t, n, kw)` is the filter tap of matrix t, column n.
 // Layout of one matrix: groups of eight columns, then the two halves of K, eight 16-byte rows each.
 template <int NCOL, int KW, bool ADJ, typename F>
-__device__ __forceinline__ void build_bands(bf16* bmat, int mats, int lane, F value) {
-    for (int e = lane; e < mats * NCOL * 2; e += 32) {
+__device__ __forceinline__ void build_bands(bf16* bmat, int mats, F value) {
+    for (int e = threadIdx.x; e < mats * NCOL * 2; e += blockDim.x) {
         const int n = e % 8, half = (e / 8) % 2, g = (e / 16) % (NCOL / 8), t = e / (2 * NCOL);
         unsigned words[4];
 #pragma unroll
@@ -313,7 +334,8 @@ __device__ __forceinline__ void build_bands(bf16* bmat, int mats, int lane, F va
     }
 }
 
-enum Access { kWide = 0, kQuad = 1, kPaddedOut = 2 };   // 16-byte rows; 8-byte rows; 8-byte rows, out unpadded
+// whole blocks of 16 bytes (no padding); 8-byte rows; 8-byte rows, out unpadded
+enum Access { kWide = 0, kQuad = 1, kPaddedOut = 2 };
 
 // eight voxels of a row from column w (8-aligned), zero past the pitch
 template <int AL>
@@ -348,13 +370,14 @@ struct AdjointArgs {
 };
 
 // Accumulators: per output plane 32 columns of A(x) and 32 of A(t1) (four channels of eight voxels),
-// RING of them in turn; the epilogue leaves them zero.  Three depth taps: a ring of four planes, 256
+// RING of them in turn, which start at eps: the epilogue leaves them so.  Three depth taps: a ring of four planes, 256
 // columns, two CTAs per multiprocessor; five: eight planes, all 512.
 template <int KD> __host__ __device__ constexpr int adjoint_ring() { return KD > 3 ? 8 : 4; }
 
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(const AdjointArgs P) {
+__global__ void __launch_bounds__(kAdjointThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(const AdjointArgs P) {
     constexpr bool ROWS = KH == 1;
+    constexpr int kThreads = kAdjointThreads, kEpilogueWarps = 8, kMmaWarp = 12;
     constexpr int PD = KD / 2, NC = SC * 8, RING = adjoint_ring<KD>(), TCOLS = RING * 2 * NC, KT = KD * KH * KW;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     const Band& b = P.b;
@@ -371,29 +394,27 @@ __global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(co
 
     if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, TCOLS);
     if (tid == 0) {
-        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, kStageWarps); mbar_init(sempty + 8 * i, 1); }
+        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, 4); mbar_init(sempty + 8 * i, 1); }
         for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // windows of valid blocks may touch blocks that no plane has been staged to: those have to be numbers
     for (int i = tid; i < kSlots * slot_blocks + slack_blocks(b); i += kThreads) slots[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (warp == kMmaWarp) {
-        float* const hs = reinterpret_cast<float*>(smem_tc + 512);
-        for (int e = lane; e < SC * KT; e += 32) hs[e] = P.h[(long long)at.c * SC * KT + e];
-        __syncwarp();
-        // [kh][output plane p - (KD - 1) + kd: groups of 32 columns][channel, column]
-        build_bands<KD * NC, KW, true>(bmat, KH, lane, [&](int kh, int n, int kw) {
-            const int kd = n / NC, j = n % NC / 8;
-            return hs[j * KT + (kd * KH + kh) * KW + kw];
-        });
-    }
+    float* const hs = reinterpret_cast<float*>(smem_tc + 512);
+    for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)at.c * SC * KT + e];
+    __syncthreads();
+    // [kh][output plane p - (KD - 1) + kd: groups of 32 columns][channel, column]
+    build_bands<KD * NC, KW, true>(bmat, KH, [&](int kh, int n, int kw) {
+        const int kd = n / NC, j = n % NC / 8;
+        return hs[j * KT + (kd * KH + kh) * KW + kw];
+    });
     fence_async_proxy();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + kTmemAt);
     if (warp < kEpilogueWarps) {
-        for (int c = 32 * (warp >> 2); c < TCOLS; c += 64) tmem_zero32(tmem + ((unsigned)(warp & 3) << 21) + c);
+        for (int c = 32 * (warp >> 2); c < TCOLS; c += 64) tmem_fill(tmem + ((unsigned)(warp & 3) << 21) + c, b.eps, 32);
         tmem_wait_st();
         tc_fence_before();
     }
@@ -401,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(co
     tc_fence_after();
     bool ok = true;
     if (warp == kMmaWarp) {
-        const unsigned xa = smem_u32(slots), ba = smem_u32(bmat);
+        const unsigned long long ad = mat_desc(smem_u32(slots), 16, 128), md = mat_desc(smem_u32(bmat), 128, 256);
         for (int p = 0; p < planes && ok; ++p) {
             const int s = p % kSlots, d = at.d0 - PD + p;
             ok = mbar_wait(sfull + 8 * s, (p / kSlots) & 1);
@@ -413,17 +434,17 @@ __global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(co
                     // groups g of output planes o = p - (KD - 1) + g inside the chunk
                     const int g0 = max(0, KD - 1 - p), g1 = min(KD - 1, at.DC - 1 + KD - 1 - p), o0 = p - (KD - 1) + g0;
                     const int r0 = o0 % RING, n = g1 - g0 + 1, n0 = min(n, RING - r0);
-                    for (int kh = 0; kh < KH; ++kh) {
-                        const unsigned off = 16 * (s * slot_blocks + (KH - 1 - kh) * b.PB);
-                        const unsigned bm = ba + (kh * KD + g0) * NC * 32;
+                    // descriptors differ in their start address alone, in units of 16 bytes
+                    const unsigned long long a0 = ad + s * slot_blocks, m0 = md + g0 * NC * 2;
+                    const unsigned i0 = instr_desc(n0 * NC), i1 = instr_desc((n - n0) * NC);
+#pragma unroll
+                    for (int kh = 0; kh < KH; ++kh)
 #pragma unroll
                         for (int a = 0; a < 2; ++a) {                            // x, t1
-                            const unsigned long long ad = mat_desc(xa + off + a * 16 * blocks, 16, 128);
-                            const unsigned acc = tmem + a * RING * NC;
-                            mma(acc + r0 * NC, ad, mat_desc(bm, 128, 256), instr_desc(n0 * NC), 1);
-                            if (n > n0) mma(acc, ad, mat_desc(bm + n0 * NC * 32, 128, 256), instr_desc((n - n0) * NC), 1);
+                            const unsigned long long ak = a0 + (KH - 1 - kh) * b.PB + a * blocks, mk = m0 + kh * KD * NC * 2;
+                            mma(tmem + a * RING * NC + r0 * NC, ak, mk, i0, 1);
+                            if (n > n0) mma(tmem + a * RING * NC, ak, mk + n0 * NC * 2, i1, 1);
                         }
-                    }
                 }
                 mma_commit(sempty + 8 * s);
                 const int o = p - (KD - 1);
@@ -435,14 +456,13 @@ __global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(co
         const unsigned none[2] = {0u, 0u};
         // x and t1 as two channels: the distance between the tensors takes the place of the stride
         const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
-        Stager<KH, KW, 2, false, AL == kWide> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at.h0,
+        Stager<KH, KW, 2, false, AL == kWide, 128, 2, 1> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at.h0,
                                                  tid - 32 * kEpilogueWarps);
-        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, none, false, lane);
+        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, none, false, 0, lane);
     } else {
         const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q;
         const bool valid = r < at.TH && q < b.NB;
         const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
-        const f32x2 eps2 = pack2(b.eps, b.eps);
         f32x2 b2[SC];
 #pragma unroll
         for (int j = 0; j < SC; ++j) {
@@ -468,9 +488,9 @@ __global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(co
                 float n[8], dn[8];
                 __syncwarp();
                 tmem_load8x2(acc + 8 * j, acc + RING * NC + 8 * j, n, dn);
-                if (j == SC - 1) {                       // read: zero for the plane that takes the place
-                    tmem_zero32(acc);
-                    tmem_zero32(acc + RING * NC);
+                if (j == SC - 1) {                       // read: eps again for the plane that takes the place
+                    tmem_fill(acc, b.eps, NC);
+                    tmem_fill(acc + RING * NC, b.eps, NC);
                     tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
@@ -481,12 +501,11 @@ __global__ void __launch_bounds__(kThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(co
                 for (int i = 0; i < 4; ++i) {
                     const unsigned u = word_of(zr[j], i);
                     f32x2 s2 = add2(pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)), b2[j]);
-                    float lo, hi, dl, dh;
+                    float lo, hi;
                     unpack2(s2, lo, hi);
                     if (b.relu) { lo = fmaxf(lo, 0.0f); hi = fmaxf(hi, 0.0f); }
-                    const f32x2 num = mul2(pack2(lo, hi), add2(pack2(n[2 * i], n[2 * i + 1]), eps2));
-                    unpack2(add2(pack2(dn[2 * i], dn[2 * i + 1]), eps2), dl, dh);
-                    unpack2(mul2(num, pack2(rcp(dl), rcp(dh))), lo, hi);
+                    const f32x2 num = mul2(pack2(lo, hi), pack2(n[2 * i], n[2 * i + 1]));
+                    unpack2(mul2(num, pack2(rcp(dn[2 * i]), rcp(dn[2 * i + 1]))), lo, hi);
                     v[i] = pack_bf16(lo, hi);
                 }
                 if (valid) {
@@ -523,8 +542,9 @@ constexpr int kSourceCols = 256;
 template <int KD> __host__ __device__ constexpr int source_planes() { return kSourceCols / 8 - KD + 2 - source_groups<KD>(); }
 
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs P) {
+__global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const SourceArgs P) {
     constexpr bool ROWS = KH == 1;
+    constexpr int kThreads = kSourceThreads, kEpilogueWarps = 4, kMmaWarp = 14;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     constexpr int NCOL = 8 * source_groups<KD>(), NMAT = SC * KH;
     constexpr int TABLE = (PD + 1) * (PD + 1) * (PH + 1) * (PH + 1) * (PW + 1) * (PW + 1);
@@ -545,42 +565,37 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
 
     if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, kSourceCols);
     if (tid == 0) {
-        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, kStageWarps); mbar_init(sempty + 8 * i, 1); }
+        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, kSourceStagers / 32); mbar_init(sempty + 8 * i, 1); }
         for (int i = 0; i < at.DC; ++i) mbar_init(afull + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < kSlots * slot_blocks + slack_blocks(b); i += kThreads) slots[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (warp == kMmaWarp) {
-        float* const hs = reinterpret_cast<float*>(smem_tc + 512);
-        for (int e = lane; e < SC * KT; e += 32) hs[e] = P.h[(long long)at.c * SC * KT + e];
-        float bj[SC];
+    float* const hs = reinterpret_cast<float*>(smem_tc + 512);
+    for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)at.c * SC * KT + e];
+    __syncthreads();
+    // [channel, kh][output plane p - kd, kd = KD - 1 - g: groups of 8 columns]
+    build_bands<NCOL, KW, false>(bmat, NMAT, [&](int t, int n, int kw) {
+        const int j = t / KH, kh = t % KH, kd = KD - 1 - n / 8;
+        return kd >= 0 ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
+    });
+    // sum over channels and the taps inside the volume of bias * filter, by how many taps are cut off at
+    // either end of each axis
+    for (int e = tid; e < TABLE; e += kThreads) {
+        int q = e;
+        const int wh = q % (PW + 1); q /= PW + 1;
+        const int wl = q % (PW + 1); q /= PW + 1;
+        const int hh = q % (PH + 1); q /= PH + 1;
+        const int hl = q % (PH + 1); q /= PH + 1;
+        const int dh = q % (PD + 1), dl = q / (PD + 1);
+        float s = 0.0f;
+        for (int kd = dl; kd < KD - dh; ++kd)
+            for (int kh = hl; kh < KH - hh; ++kh)
+                for (int kw = wl; kw < KW - wh; ++kw) {
+                    const int tau = (kd * KH + kh) * KW + kw;
 #pragma unroll
-        for (int j = 0; j < SC; ++j) bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
-        __syncwarp();
-        // [channel, kh][output plane p - kd, kd = KD - 1 - g: groups of 8 columns]
-        build_bands<NCOL, KW, false>(bmat, NMAT, lane, [&](int t, int n, int kw) {
-            const int j = t / KH, kh = t % KH, kd = KD - 1 - n / 8;
-            return kd >= 0 ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
-        });
-        // sum over channels and the taps inside the volume of bias * filter, by how many taps are cut
-        // off at either end of each axis
-        for (int e = lane; e < TABLE; e += 32) {
-            int q = e;
-            const int wh = q % (PW + 1); q /= PW + 1;
-            const int wl = q % (PW + 1); q /= PW + 1;
-            const int hh = q % (PH + 1); q /= PH + 1;
-            const int hl = q % (PH + 1); q /= PH + 1;
-            const int dh = q % (PD + 1), dl = q / (PD + 1);
-            float s = 0.0f;
-            for (int kd = dl; kd < KD - dh; ++kd)
-                for (int kh = hl; kh < KH - hh; ++kh)
-                    for (int kw = wl; kw < KW - wh; ++kw) {
-                        const int tau = (kd * KH + kh) * KW + kw;
-#pragma unroll
-                        for (int j = 0; j < SC; ++j) s = fmaf(bj[j], hs[j * KT + tau], s);
-                    }
-            table[e] = s;
-        }
+                    for (int j = 0; j < SC; ++j) s = fmaf(P.bias ? P.bias[at.c * SC + j] : 0.0f, hs[j * KT + tau], s);
+                }
+        table[e] = s;
     }
     fence_async_proxy();
     tc_fence_before();
@@ -588,7 +603,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
     tc_fence_after();
     const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + kTmemAt);
     if (warp < kEpilogueWarps) {
-        for (int c = 32 * (warp >> 2); c < kSourceCols; c += 64) tmem_zero32(tmem + ((unsigned)(warp & 3) << 21) + c);
+        for (int c = 0; c < kSourceCols; c += 32) tmem_fill(tmem + ((unsigned)(warp & 3) << 21) + c, 0.0f, 32);
         tmem_wait_st();
         tc_fence_before();
     }
@@ -596,18 +611,19 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
     tc_fence_after();
     bool ok = true;
     if (warp == kMmaWarp) {
-        const unsigned za = smem_u32(slots), ba = smem_u32(bmat), idesc = instr_desc(NCOL);
+        const unsigned long long ad = mat_desc(smem_u32(slots), 16, 128), md = mat_desc(smem_u32(bmat), 128, 256);
+        const unsigned idesc = instr_desc(NCOL);
         for (int p = 0; p < planes && ok; ++p) {
             const int s = p % kSlots, d = at.d0 - PD + p;
             ok = mbar_wait(sfull + 8 * s, (p / kSlots) & 1);
             tc_fence_after();
             if (lane == 0 && ok) {
-                if (d >= 0 && d < b.D)
-                    for (int t = 0; t < NMAT; ++t) {
-                        const int j = t / KH, kh = t - j * KH;
-                        mma(tmem + 8 * p, mat_desc(za + 16 * (s * slot_blocks + j * blocks + kh * b.PB), 16, 128),
-                            mat_desc(ba + t * NCOL * 32, 128, 256), idesc, 1);
-                    }
+                if (d >= 0 && d < b.D) {
+                    const unsigned long long a0 = ad + s * slot_blocks;
+#pragma unroll
+                    for (int t = 0; t < NMAT; ++t)
+                        mma(tmem + 8 * p, a0 + (t / KH) * blocks + (t % KH) * b.PB, md + t * NCOL * 2, idesc, 1);
+                }
                 mma_commit(sempty + 8 * s);
                 const int o = p - (KD - 1);
                 if (o >= 0) mma_commit(afull + 8 * o);
@@ -621,9 +637,9 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
             const __nv_bfloat162 nb = __float2bfloat162_rn(P.bias ? -P.bias[at.c * SC + j] : 0.0f);
             negb[j] = *reinterpret_cast<const unsigned*>(&nb);
         }
-        Stager<KH, KW, SC, true, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at.h0,
-                                                 tid - 32 * kEpilogueWarps);
-        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, negb, b.relu, lane);
+        Stager<KH, KW, SC, true, AL == kWide, kSourceStagers, 1, 2> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at.h0,
+                                                 (tid - 32 * kEpilogueWarps) % kSourceStagers);
+        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, negb, b.relu, (warp - kEpilogueWarps) / 5, lane);
     } else {
         const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q, h = at.h0 + r;
         const bool valid = r < at.TH && q < b.NB, inner = w >= PW && w + 7 + PW < b.Wv;
@@ -631,7 +647,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_source_kernel(const SourceArgs
         bf16* const tb = P.t1 + (long long)at.bc * addr.chan + h * addr.row_x;
         // images: every row of a plane is an image of its own, KH = 1
         const int hl = max(0, PH - h), hh = min(PH, max(0, h + PH - (b.H - 1)));
-        for (int o = warp >> 2; o < at.DC && ok; o += 2) {
+        for (int o = 0; o < at.DC && ok; ++o) {
             const int d = at.d0 + o, dl = max(0, PD - d), dh = max(0, d + PD - (b.D - 1));
             const float* tab = table + (((dl * (PD + 1) + dh) * (PH + 1) + hl) * (PH + 1) + hh) * (PW + 1) * (PW + 1);
             ok = mbar_wait(afull + 8 * o, 0);
