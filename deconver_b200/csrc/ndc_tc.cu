@@ -69,9 +69,9 @@ cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, cons
     cudaError_t e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, g, ss, st, S)
                          : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, g, ss, st, S);
     if (e != cudaSuccess) return e;
-    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut>, kAdjointThreads, A.b, g, sa, st, A);
-    return wide && on16(out) ? launch(tc_adjoint_kernel<KD, KH, KW, kWide>, kAdjointThreads, A.b, g, sa, st, A)
-                             : launch(tc_adjoint_kernel<KD, KH, KW, kQuad>, kAdjointThreads, A.b, g, sa, st, A);
+    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut>, AdjointShape<KD>::THREADS, A.b, g, sa, st, A);
+    return wide && on16(out) ? launch(tc_adjoint_kernel<KD, KH, KW, kWide>, AdjointShape<KD>::THREADS, A.b, g, sa, st, A)
+                             : launch(tc_adjoint_kernel<KD, KH, KW, kQuad>, AdjointShape<KD>::THREADS, A.b, g, sa, st, A);
 }
 
 template <int KD, int KH, int KW>

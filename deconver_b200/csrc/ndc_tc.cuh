@@ -130,12 +130,16 @@ static __device__ unsigned g_wait_expired;
 
 // Roles of a CTA's warps: groups of four for the epilogue (they take turns, output plane by output
 // plane; TMEM lane 32 i + l belongs to lane l of warp i of a group), groups that stage source planes (in
-// turns as well), one warp that issues the MMAs.  The adjoint kernel has two epilogue groups and one group
-// of four warps that stages; the source kernel, whose epilogue is short and whose source planes have four
-// channels, has one and two groups of five.
-constexpr int kAdjointThreads = 32 * (8 + 4 + 1), kSourceThreads = 32 * (4 + 10 + 1);
-constexpr int kSourceStagers = 160;
-constexpr int kSlots = 4;         // staged planes
+// turns as well), one warp that issues the MMAs.  The source kernel, whose epilogue is short and whose
+// source planes have four channels, has one epilogue group and stages with two groups of five warps.  The
+// adjoint kernel: two and two groups of two warps, two CTAs per multiprocessor; with five depth taps, whose
+// accumulators leave room for one, four and four.
+constexpr int kSourceThreads = 32 * (4 + 10 + 1), kSourceStagers = 160;
+template <int KD> struct AdjointShape {
+    static constexpr int EPI = KD > 3 ? 4 : 2, GROUPS = KD > 3 ? 4 : 2, STAGERS = 64, BLOCKS = KD > 3 ? 2 : 3;
+    static constexpr int THREADS = 32 * (4 * EPI + 2 * GROUPS + 1), CTAS = KD > 3 ? 1 : 2;
+};
+constexpr int kSlots = 8;         // staged planes
 constexpr int kHeader = 1024;     // bytes: barriers and the TMEM address (512), the filter as float32
 
 // Place of a CTA: (sample, channel), band of rows, chunk of planes; all addresses in elements.
@@ -375,9 +379,10 @@ struct AdjointArgs {
 template <int KD> __host__ __device__ constexpr int adjoint_ring() { return KD > 3 ? 8 : 4; }
 
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kAdjointThreads, KD > 3 ? 1 : 2) tc_adjoint_kernel(const AdjointArgs P) {
+__global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::CTAS) tc_adjoint_kernel(const AdjointArgs P) {
     constexpr bool ROWS = KH == 1;
-    constexpr int kThreads = kAdjointThreads, kEpilogueWarps = 8, kMmaWarp = 12;
+    typedef AdjointShape<KD> Shape;
+    constexpr int kThreads = Shape::THREADS, kEpilogueWarps = 4 * Shape::EPI, kMmaWarp = kThreads / 32 - 1;
     constexpr int PD = KD / 2, NC = SC * 8, RING = adjoint_ring<KD>(), TCOLS = RING * 2 * NC, KT = KD * KH * KW;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     const Band& b = P.b;
@@ -394,7 +399,7 @@ __global__ void __launch_bounds__(kAdjointThreads, KD > 3 ? 1 : 2) tc_adjoint_ke
 
     if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, TCOLS);
     if (tid == 0) {
-        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, 4); mbar_init(sempty + 8 * i, 1); }
+        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, Shape::STAGERS / 32); mbar_init(sempty + 8 * i, 1); }
         for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(kAdjointThreads, KD > 3 ? 1 : 2) tc_adjoint_ke
     tc_fence_after();
     const unsigned tmem = *reinterpret_cast<volatile unsigned*>(smem_tc + kTmemAt);
     if (warp < kEpilogueWarps) {
-        for (int c = 32 * (warp >> 2); c < TCOLS; c += 64) tmem_fill(tmem + ((unsigned)(warp & 3) << 21) + c, b.eps, 32);
+        for (int c = 32 * (warp >> 2); c < TCOLS; c += 32 * Shape::EPI) tmem_fill(tmem + ((unsigned)(warp & 3) << 21) + c, b.eps, 32);
         tmem_wait_st();
         tc_fence_before();
     }
@@ -456,9 +461,9 @@ __global__ void __launch_bounds__(kAdjointThreads, KD > 3 ? 1 : 2) tc_adjoint_ke
         const unsigned none[2] = {0u, 0u};
         // x and t1 as two channels: the distance between the tensors takes the place of the stride
         const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
-        Stager<KH, KW, 2, false, AL == kWide, 128, 2, 1> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at.h0,
-                                                 tid - 32 * kEpilogueWarps);
-        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, none, false, 0, lane);
+        Stager<KH, KW, 2, false, AL == kWide, Shape::STAGERS, Shape::BLOCKS, Shape::GROUPS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at.h0,
+                                                 (tid - 32 * kEpilogueWarps) % Shape::STAGERS);
+        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, none, false, (tid - 32 * kEpilogueWarps) / Shape::STAGERS, lane);
     } else {
         const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q;
         const bool valid = r < at.TH && q < b.NB;
@@ -471,7 +476,7 @@ __global__ void __launch_bounds__(kAdjointThreads, KD > 3 ? 1 : 2) tc_adjoint_ke
         }
         const bf16* const zb = P.z + (long long)at.bc * SC * addr.chan + (at.h0 + r) * addr.row_z;
         bf16* const ob = P.out + (long long)at.bc * SC * oaddr.chan + (at.h0 + r) * oaddr.row_z;
-        for (int o = warp >> 2; o < at.DC && ok; o += 2) {
+        for (int o = warp >> 2; o < at.DC && ok; o += Shape::EPI) {
             const int slot = o % RING;
             const long long d = at.d0 + o;
             uint4 zr[SC];
