@@ -92,6 +92,10 @@ int check_pitch(const NdcDesc* d, int pitch, int out_pitch) {
     return NDC_OK;
 }
 
+bool tensor_cores(const NdcDesc* d, const ndc::Geo& g) {
+    return d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && ndc::tc::covers(g);
+}
+
 int check_padded(std::initializer_list<const void*> tensors, int dtype) {
     for (const void* p : tensors)
         if ((uintptr_t)p % (dtype == NDC_BF16 ? 8 : 16))
@@ -211,8 +215,7 @@ int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const vo
     typedef __nv_bfloat16 bf16;
     if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
         // bfloat16 tensors with bfloat16 parameters: exact products on the tensor cores
-        if (desc->dtype == NDC_BF16 && (desc->flags & NDC_FLAG_BF16_PARAMS) && ndc::tc::covers(g) &&
-            (((uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0)) & 7) == 0) {
+        if (tensor_cores(desc, g) && (((uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0)) & 7) == 0) {
             e = ndc::tc::forward(g, (const bf16*)x, (const bf16*)z, h, bias, (bf16*)out, (bf16*)t1, st);
             if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (tensor core) launch");
             return NDC_OK;
@@ -299,6 +302,14 @@ int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const v
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) {
             typedef __nv_bfloat16 bf16;
+            if (tensor_cores(desc, g) && (((uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (uintptr_t)gz |
+                                           (gout_pitch == pitch ? (uintptr_t)gout : 0)) & 7) == 0) {
+                e = ndc::tc::backward_ratio(g, (const bf16*)x, (const bf16*)z, (const bf16*)t1, h, bias, (const bf16*)gout,
+                                            (float*)((char*)workspace + p.off_gnum), (float*)((char*)workspace + p.off_gden),
+                                            (bf16*)gz, st);
+                if (e != cudaSuccess) return cuda_fail(e, "ndc_bwd (tensor core) launch");
+                p.ratio_done = true;
+            }
             if (desc->dtype == NDC_F32)
                 e = ndc::dw4::backward<float>(g, p, (const float*)x, (const float*)z,
                                               (const float*)t1, h, bias, (const float*)gout,

@@ -268,6 +268,7 @@ struct BwdPlan {
     int kconv_wide;                     // packed K kernel: the wide CTA was planned
     int rows;                           // 0: band kernels; else the rows class planned
     int small;                          // 0, or the small-volume class planned (16 or 8)
+    bool ratio_done = false;            // gnum, gden and the direct term are there already
 };
 
 template <int KD, int KH, int KW, typename S>
@@ -395,7 +396,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
     float* pb = (float*)((char*)ws + p.off_pb);
     if (p.n_ratio > 0x7fffffffLL || p.n_kconv > 0x7fffffffLL || p.n_gz > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    {
+    if (!p.ratio_done) {
         RatioParams P;
         P.x = x; P.t1 = t1; P.z = z; P.gout = gout; P.h = h; P.bias = bias;
         P.gnum = gnum; P.gden = gden; P.gz = gz;
@@ -492,7 +493,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.ctas_per_bc_b = (long long)p.gz.ndc * p.gz.nth;
         P.b_has_w = gh ? 1 : 0;
         P.B = g.B; P.C = g.G; P.KT = g.KT; P.gh = gh; P.gb = gb;
-        reduce_kernel<kPartialStride><<<g.G, kPartialStride, 0, st>>>(P);
+        reduce_kernel<<<g.G, kPartialStride * kReduceWays, 0, st>>>(P);
         launched();
     }
     return cudaGetLastError();

@@ -56,28 +56,55 @@ cudaError_t launch(K kern, int threads, const Band& b, const Geo& g, size_t smem
     return cudaGetLastError();
 }
 
+bool on16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+template <int KD, int KH, int KW, int MODE>
+cudaError_t launch_adjoint(const Geo& g, const AdjointArgs& A, bool wide, cudaStream_t st) {
+    const size_t smem = adjoint_smem<KD, KH, KW>(A.b);
+    constexpr int NT = AdjointShape<KD>::THREADS;
+    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut, MODE>, NT, A.b, g, smem, st, A);
+    return wide ? launch(tc_adjoint_kernel<KD, KH, KW, kWide, MODE>, NT, A.b, g, smem, st, A)
+                : launch(tc_adjoint_kernel<KD, KH, KW, kQuad, MODE>, NT, A.b, g, smem, st, A);
+}
+
 template <int KD, int KH, int KW>
 cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, const float* bias, bf16* out, bf16* t1, cudaStream_t st) {
-    AdjointArgs A;
-    SourceArgs S;
+    AdjointArgs A{};
+    SourceArgs S{};
     if (!plan<KD, KH, KW>(g, g.D, A.b) || !plan<KD, KH, KW>(g, source_planes<KD>(), S.b)) return cudaErrorInvalidConfiguration;
     A.x = x; A.t1 = t1; A.z = z; A.out = out; A.h = h; A.bias = bias;
     S.z = z; S.t1 = t1; S.h = h; S.bias = bias;
-    const size_t sa = adjoint_smem<KD, KH, KW>(A.b), ss = source_smem<KD, KH, KW>(S.b);
-    auto on16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+    const size_t ss = source_smem<KD, KH, KW>(S.b);
     const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1);
     cudaError_t e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, g, ss, st, S)
                          : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, g, ss, st, S);
     if (e != cudaSuccess) return e;
-    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut>, AdjointShape<KD>::THREADS, A.b, g, sa, st, A);
-    return wide && on16(out) ? launch(tc_adjoint_kernel<KD, KH, KW, kWide>, AdjointShape<KD>::THREADS, A.b, g, sa, st, A)
-                             : launch(tc_adjoint_kernel<KD, KH, KW, kQuad>, AdjointShape<KD>::THREADS, A.b, g, sa, st, A);
+    return launch_adjoint<KD, KH, KW, kOut>(g, A, wide && on16(out), st);
 }
 
 template <int KD, int KH, int KW>
+cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1, const float* h, const float* bias, const bf16* gout,
+                      float* gnum, float* gden, bf16* direct, cudaStream_t st) {
+    AdjointArgs A{};
+    if (!plan<KD, KH, KW>(g, g.D, A.b)) return cudaErrorInvalidConfiguration;
+    A.x = x; A.t1 = t1; A.z = z; A.out = direct; A.gout = gout; A.gnum = gnum; A.gden = gden; A.h = h; A.bias = bias;
+    const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1) && on16(gout) && (!direct || on16(direct));
+    return launch_adjoint<KD, KH, KW, KH == 1 ? kPlanar : kPairs>(g, A, wide, st);
+}
+
+// How large a problem has to be, and how much of the MMAs' rows it has to fill, for the tensor cores to be the
+// faster way (measured on 46 shapes of either kind): volumes from 0.8 M group-voxels on, rows of 128 at
+// least 30 % full (16^3 fills 25 % and takes 0.90x the FMA kernels' speed, 20^3 39 % and 1.22x); images from 3 M on
+// and 45 % (8 images of 64 columns; 4 take 0.58x), 80 % for 3x3 filters at the widths the FMA kernels
+// have compile-time instances for (0.88x at 50 %, 1.06x - 1.11x at 89 %).
+template <int KD, int KH, int KW>
 bool worth(const Geo& g) {
     Band a, s;
-    return plan<KD, KH, KW>(g, g.D, a) && plan<KD, KH, KW>(g, source_planes<KD>(), s) && useful(a) >= 0.2;
+    if (!plan<KD, KH, KW>(g, g.D, a) || !plan<KD, KH, KW>(g, source_planes<KD>(), s)) return false;
+    const double voxels = (double)g.B * g.G * g.D * g.H * g.Wv, use = std::min(useful(a), useful(s));
+    if (KH > 1) return voxels >= 0.8e6 && use >= 0.3;
+    const bool tuned = KW == 3 && (g.W == 64 || g.W == 128 || g.W == 256);
+    return voxels >= 3e6 && use >= (tuned ? 0.8 : 0.45);
 }
 
 // Image batches as volumes whose planes are the image rows and whose plane rows are the images.
@@ -104,6 +131,13 @@ cudaError_t forward(const Geo& g, const bf16* x, const bf16* z, const float* h, 
     if (g.kD == 3) return run<3, 3, 3>(g, x, z, h, bias, out, t1, st);
     if (g.kH == 5) return run<5, 1, 5>(as_rows(g), x, z, h, bias, out, t1, st);
     return run<3, 1, 3>(as_rows(g), x, z, h, bias, out, t1, st);
+}
+
+cudaError_t backward_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1, const float* h, const float* bias,
+                           const bf16* gout, float* gnum, float* gden, bf16* direct, cudaStream_t st) {
+    if (g.kD == 3) return run_ratio<3, 3, 3>(g, x, z, t1, h, bias, gout, gnum, gden, direct, st);
+    if (g.kH == 5) return run_ratio<5, 1, 5>(as_rows(g), x, z, t1, h, bias, gout, gnum, gden, direct, st);
+    return run_ratio<3, 1, 3>(as_rows(g), x, z, t1, h, bias, gout, gnum, gden, direct, st);
 }
 
 unsigned wait_expired() {

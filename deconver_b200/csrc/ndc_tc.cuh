@@ -366,10 +366,24 @@ __device__ __forceinline__ float word_lane(const uint4& v, int i) {      // i st
     return __uint_as_float(i & 1 ? w & 0xffff0000u : w << 16);
 }
 
-// ---- out = s (A(x) + eps) / (A(t1) + eps) -------------------------------------------------------
+// 32 bytes of consecutive float32 values, on a 32-byte boundary
+__device__ __forceinline__ void store_f32x8(float* p, const float (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])),
+                 "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+                 "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])) : "memory");
+}
+
+// ---- A(x) and A(t1), and what follows from them -------------------------------------------------
+//   kOut       out = s (A(x) + eps) / (A(t1) + eps)                          (the forward)
+//   kPairs     (gden, gnum) pairs and the direct term of the backward of volumes, see ratio_kernel
+//   kPlanar    the same as two tensors, for images
+enum AdjointMode { kOut = 0, kPairs = 1, kPlanar = 2 };
+
 struct AdjointArgs {
     Band b;
-    const bf16* x; const bf16* t1; const bf16* z; bf16* out;
+    const bf16* x; const bf16* t1; const bf16* z;
+    bf16* out;                        // kOut: out; else the direct term (rows of W), or NULL
+    const bf16* gout; float* gnum; float* gden;
     const float* h; const float* bias;
 };
 
@@ -378,7 +392,7 @@ struct AdjointArgs {
 // columns, two CTAs per multiprocessor; five: eight planes, all 512.
 template <int KD> __host__ __device__ constexpr int adjoint_ring() { return KD > 3 ? 8 : 4; }
 
-template <int KD, int KH, int KW, int AL>
+template <int KD, int KH, int KW, int AL, int MODE>
 __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::CTAS) tc_adjoint_kernel(const AdjointArgs P) {
     constexpr bool ROWS = KH == 1;
     typedef AdjointShape<KD> Shape;
@@ -474,22 +488,37 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
             const float v = P.bias ? P.bias[at.c * SC + j] : 0.0f;
             b2[j] = pack2(v, v);
         }
-        const bf16* const zb = P.z + (long long)at.bc * SC * addr.chan + (at.h0 + r) * addr.row_z;
-        bf16* const ob = P.out + (long long)at.bc * SC * oaddr.chan + (at.h0 + r) * oaddr.row_z;
+        const long long zrow = (long long)at.bc * SC * addr.chan + (at.h0 + r) * addr.row_z;
+        const long long orow = (long long)at.bc * SC * oaddr.chan + (at.h0 + r) * oaddr.row_z;
+        const bf16* const zb = P.z + zrow;
+        const bf16* const gb = MODE == kOut ? nullptr : P.gout + orow;
         for (int o = warp >> 2; o < at.DC && ok; o += Shape::EPI) {
             const int slot = o % RING;
             const long long d = at.d0 + o;
-            uint4 zr[SC];
+            // z (and gout) of a channel are on their way while the one before is worked on
+            uint4 zr[2], gr[2];
+            auto fetch = [&](int j) {
+                zr[j & 1] = make_uint4(0u, 0u, 0u, 0u);
+                gr[j & 1] = make_uint4(0u, 0u, 0u, 0u);
+                if (!valid) return;
+                zr[j & 1] = load8<AL>(zb + j * addr.chan + d * addr.plane, w, b.W);
+                if (MODE == kOut) return;
+                const bf16* row = gb + j * oaddr.chan + d * oaddr.plane;
+                if (AL != kPaddedOut || b.Wo == b.W) gr[j & 1] = load8<AL>(row, w, b.W);
+                else {
+                    unsigned e[8];
 #pragma unroll
-            for (int j = 0; j < SC; ++j) {
-                zr[j] = make_uint4(0u, 0u, 0u, 0u);
-                if (valid) zr[j] = load8<AL>(zb + j * addr.chan + d * addr.plane, w, b.W);
-            }
+                    for (int i = 0; i < 8; ++i) e[i] = w + i < b.Wv ? reinterpret_cast<const unsigned short*>(row)[w + i] : 0u;
+                    gr[j & 1] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+                }
+            };
+            fetch(0);
             ok = mbar_wait(afull + 8 * slot, (o / RING) & 1);
             tc_fence_after();
             const unsigned acc = lanes + slot * NC;
 #pragma unroll
             for (int j = 0; j < SC; ++j) {
+                if (j + 1 < SC) fetch(j + 1);
                 float n[8], dn[8];
                 __syncwarp();
                 tmem_load8x2(acc + 8 * j, acc + RING * NC + 8 * j, n, dn);
@@ -502,24 +531,60 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                     if (lane == 0) mbar_arrive(aempty + 8 * slot);
                 }
                 unsigned v[4];
+                float gd[8];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const unsigned u = word_of(zr[j], i);
+                    const unsigned u = word_of(zr[j & 1], i);
                     f32x2 s2 = add2(pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)), b2[j]);
                     float lo, hi;
                     unpack2(s2, lo, hi);
                     if (b.relu) { lo = fmaxf(lo, 0.0f); hi = fmaxf(hi, 0.0f); }
-                    const f32x2 num = mul2(pack2(lo, hi), pack2(n[2 * i], n[2 * i + 1]));
-                    unpack2(mul2(num, pack2(rcp(dn[2 * i]), rcp(dn[2 * i + 1]))), lo, hi);
+                    const f32x2 n2 = pack2(n[2 * i], n[2 * i + 1]), r2 = pack2(rcp(dn[2 * i]), rcp(dn[2 * i + 1]));
+                    if (MODE == kOut) {
+                        unpack2(mul2(mul2(pack2(lo, hi), n2), r2), lo, hi);
+                    } else {
+                        const unsigned q2 = word_of(gr[j & 1], i);
+                        const f32x2 g2 = mul2(pack2(__uint_as_float(q2 << 16), __uint_as_float(q2 & 0xffff0000u)), r2);
+                        const f32x2 gn2 = mul2(g2, pack2(lo, hi));
+                        float a, c;
+                        unpack2(mul2(mul2(gn2, n2), r2), a, c);
+                        gd[2 * i] = -a; gd[2 * i + 1] = -c;
+                        unpack2(mul2(g2, n2), lo, hi);           // the direct term
+                        unpack2(gn2, n[2 * i], n[2 * i + 1]);
+                    }
                     v[i] = pack_bf16(lo, hi);
                 }
-                if (valid) {
-                    bf16* orow = ob + j * oaddr.chan + d * oaddr.plane;
-                    if (AL != kPaddedOut || b.Wo == b.W) store8<AL>(orow, w, b.W, make_uint4(v[0], v[1], v[2], v[3]));
+                if (MODE != kOut && w + 8 > b.Wv) {              // zero in the padding
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) if (w + i >= b.Wv) { n[i] = 0.0f; gd[i] = 0.0f; }
+                }
+                if (valid && MODE == kOut) {
+                    bf16* row = P.out + orow + j * oaddr.chan + d * oaddr.plane;
+                    if (AL != kPaddedOut || b.Wo == b.W) store8<AL>(row, w, b.W, make_uint4(v[0], v[1], v[2], v[3]));
                     else {
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
-                            if (w + i < b.Wv) reinterpret_cast<unsigned short*>(orow)[w + i] = (unsigned short)(i & 1 ? v[i / 2] >> 16 : v[i / 2]);
+                            if (w + i < b.Wv) reinterpret_cast<unsigned short*>(row)[w + i] = (unsigned short)(i & 1 ? v[i / 2] >> 16 : v[i / 2]);
+                    }
+                } else if (valid) {
+                    const long long e = zrow + j * addr.chan + d * addr.plane + w;
+                    if (P.out) store8<AL>(P.out + e - w, w, b.W, make_uint4(v[0], v[1], v[2], v[3]));
+                    const bool both = AL == kWide || w + 4 < b.W;
+                    if (MODE == kPairs) {
+                        const float lo8[8] = {gd[0], n[0], gd[1], n[1], gd[2], n[2], gd[3], n[3]};
+                        const float hi8[8] = {gd[4], n[4], gd[5], n[5], gd[6], n[6], gd[7], n[7]};
+                        store_f32x8(P.gnum + 2 * e, lo8);
+                        if (both) store_f32x8(P.gnum + 2 * e + 8, hi8);
+                    } else if (AL == kWide) {
+                        store_f32x8(P.gnum + e, n);
+                        store_f32x8(P.gden + e, gd);
+                    } else {
+                        *reinterpret_cast<float4*>(P.gnum + e) = make_float4(n[0], n[1], n[2], n[3]);
+                        *reinterpret_cast<float4*>(P.gden + e) = make_float4(gd[0], gd[1], gd[2], gd[3]);
+                        if (both) {
+                            *reinterpret_cast<float4*>(P.gnum + e + 4) = make_float4(n[4], n[5], n[6], n[7]);
+                            *reinterpret_cast<float4*>(P.gden + e + 4) = make_float4(gd[4], gd[5], gd[6], gd[7]);
+                        }
                     }
                 }
             }

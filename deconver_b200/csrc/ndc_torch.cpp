@@ -163,6 +163,10 @@ struct Config {
     bool bf16_params = false;          // filter and bias are bfloat16 values
 };
 
+bool bf16_params(const Tensor& h0, const Tensor& bias) {
+    return h0.scalar_type() == at::kBFloat16 && (!bias.defined() || bias.scalar_type() == at::kBFloat16);
+}
+
 NdcDesc make_desc(const Tensor& x, const Tensor& h0, const Config& c, bool relu) {
     NdcDesc d;
     int64_t sp[3] = {1, 1, 1}, k[3] = {1, 1, 1};
@@ -205,7 +209,7 @@ Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Ten
     Saved local;
     Saved& sv = saved ? *saved : local;
     Config c = config;
-    c.bf16_params = h0.scalar_type() == at::kBFloat16 && (!bias.defined() || bias.scalar_type() == at::kBFloat16);
+    c.bf16_params = bf16_params(h0, bias);
     prepare_params(h0, bias, sv.h, sv.b);
     auto out_shape = x.sizes().vec();
     out_shape[1] = c.groups * c.sc;
@@ -271,9 +275,10 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
         TORCH_CHECK(!at::GradMode::is_enabled(), "double backward through the fused Deconv update is not supported");
         const variable_list kept = ctx->get_saved_variables();
         const auto cfg = ctx->saved_data["cfg"].toIntVector();
-        const Config c{cfg[0], cfg[1], cfg[2], ctx->saved_data["eps"].toDouble(), cfg[3], cfg[4], cfg[5]};
+        Config c{cfg[0], cfg[1], cfg[2], ctx->saved_data["eps"].toDouble(), cfg[3], cfg[4], cfg[5]};
         const int64_t first = cfg[6], count = c.iters - first, W = cfg[7];
         const Tensor &x = kept[0], &h0 = kept[1], &w = kept[2], &bias = kept[3], &h = kept[4], &b = kept[5];
+        c.bf16_params = bf16_params(h0, bias);
         const bool need_x = ctx->needs_input_grad(0), need_h = ctx->needs_input_grad(1);
         const bool whole = first == 0;                   // gradients reach the projection
         const bool need_w = whole && ctx->needs_input_grad(2);

@@ -11,20 +11,20 @@ from deconver_b200 import functional as Fn
 pytestmark = pytest.mark.gpu
 
 CASES = [
-    # channels, kernel, batch, spatial
-    (3, (3, 3, 3), 1, (7, 9, 64)),
-    (2, (3, 3, 3), 2, (33, 31, 32)),
-    (50, (3, 3, 3), 2, (9, 20, 24)),
-    (2, (3, 3, 3), 1, (5, 40, 128)),
-    (2, (3, 3, 3), 1, (3, 17, 256)),
-    (4, (3, 3, 3), 1, (1, 16, 20)),
-    (300, (3, 3, 3), 1, (18, 16, 16)),
-    (6, (5, 5), 3, (130, 128)),
-    (5, (5, 5), 5, (37, 68)),
-    (3, (5, 5), 1, (40, 512)),
-    (40, (5, 5), 9, (16, 28)),
-    (3, (3, 3), 4, (45, 256)),
-    (7, (3, 3), 20, (9, 36)),
+    # channels, kernel, batch, spatial (large enough for the dispatch to take the tensor cores)
+    (200, (3, 3, 3), 1, (7, 9, 64)),
+    (13, (3, 3, 3), 2, (33, 31, 32)),
+    (100, (3, 3, 3), 2, (9, 20, 24)),
+    (32, (3, 3, 3), 1, (5, 40, 128)),
+    (62, (3, 3, 3), 1, (3, 17, 256)),
+    (2600, (3, 3, 3), 1, (1, 16, 20)),
+    (150, (3, 3, 3), 1, (18, 17, 20)),
+    (50, (5, 5), 4, (130, 128)),
+    (45, (5, 5), 14, (77, 68)),
+    (37, (5, 5), 1, (180, 512)),
+    (280, (5, 5), 27, (16, 28)),
+    (70, (3, 3), 3, (60, 252)),
+    (420, (3, 3), 24, (9, 36)),
 ]
 
 
@@ -57,17 +57,40 @@ def test_matches_the_fma_kernels(case, relu):
     assert diff.norm().item() < 2e-3 * ref.float().norm().item()
 
 
-@pytest.mark.parametrize("spatial,ks", [((9, 31, 45), (3, 3, 3)), ((5, 20, 27), (3, 3, 3)), ((33, 29, 62), (3, 3, 3)),
-                                        ((41, 171), (5, 5)), ((30, 253), (3, 3))])
-def test_layer_with_padded_rows(spatial, ks):
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "C%d_k%d_b%d_%s" % (c[0], c[1][0], c[2], "x".join(map(str, c[3]))))
+def test_gradients_match_the_fma_kernels(case):
+    C, ks, B, spatial = case
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(C)
+    x = torch.rand(B, C, *spatial, device=dev, generator=gen).bfloat16()
+    z = (torch.randn(B, 4 * C, *spatial, device=dev, generator=gen) * 0.5 + 0.8).bfloat16()
+    h = (torch.rand(C, 4, *ks, device=dev, generator=gen) / 27).bfloat16()
+    bias = (torch.randn(4 * C, device=dev, generator=gen) * 0.1).bfloat16()
+    g = torch.randn(B, 4 * C, *spatial, device=dev, generator=gen).bfloat16()
+    res = []
+    for dtype in (torch.bfloat16, torch.float32):      # of the parameters: the same values
+        t = [v.clone().requires_grad_(True) for v in (x, z, h.to(dtype), bias.to(dtype))]
+        out = dcb.deconv_update(*t, groups=C, m=1, sc=4, eps=1e-16, relu_input=True)
+        out.backward(g)
+        res.append([v.grad.float() for v in t])
+    torch.cuda.synchronize()
+    assert _lib.load().ndc_wait_expired() == 0
+    for name, a, r in zip(("gx", "gz", "gh", "gb"), *res):
+        assert ((a - r).norm() / r.norm()).item() < 5e-3, name
+
+
+@pytest.mark.parametrize("channels,batch,spatial,ks", [(34, 2, (9, 31, 45), (3, 3, 3)), (150, 2, (5, 20, 27), (3, 3, 3)),
+                                                       (8, 2, (33, 29, 62), (3, 3, 3)), (75, 6, (41, 171), (5, 5)),
+                                                       (70, 6, (30, 253), (3, 3))])
+def test_layer_with_padded_rows(channels, batch, spatial, ks):
     """Row lengths of every remainder modulo eight, two updates, against the generic kernels."""
     dev = torch.device("cuda:0")
     torch.manual_seed(1)
-    mod = dcb.Deconv(8, ks, ratio=4, num_iters=2).to(device=dev, dtype=torch.bfloat16)
+    mod = dcb.Deconv(channels, ks, ratio=4, num_iters=2).to(device=dev, dtype=torch.bfloat16)
     with torch.no_grad():
         mod.init.linear.linear.bias += 1.0
-    x = torch.rand(2, 8, *spatial, device=dev).bfloat16()
-    g = torch.randn(2, 32, *spatial, device=dev).bfloat16()
+    x = torch.rand(batch, channels, *spatial, device=dev).bfloat16()
+    g = torch.randn(batch, 4 * channels, *spatial, device=dev).bfloat16()
     res = []
     for generic in (False, True):
         xi = x.clone().requires_grad_(True)
