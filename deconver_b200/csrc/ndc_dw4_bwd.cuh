@@ -674,7 +674,7 @@ template <int VK> __device__ __forceinline__ int swz2(int chunk) {
 // Threads per SM the packed K kernel is built for, by CTA size and strip length.
 template <int NT, int VK> constexpr int kconv2_min_blocks() {
     return VK == 8 ? (NT >= 256 ? 1 : NT >= 128 ? 2 : NT >= 64 ? 4 : 8)
-                   : (NT >= 256 ? 1 : NT >= 192 ? 2 : NT >= 128 ? 3 : 4);
+                   : (NT >= 256 ? 1 : NT >= 128 ? 2 : 4);
 }
 
 template <typename T, int KD, int KH, int KW, int NT, int VK, int MAXC, int AL, bool WGRAD, int WQ>
@@ -694,7 +694,10 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
     const int NQ = WQ ? WQ : P.t.NQ, pitch2 = 2 * (WQ ? row_pitch(4 * WQ) : P.t.pitch),
               W = WQ ? 4 * WQ : P.W, Wv = PADDED ? P.Wv : W, D = P.D;   // WQ > 0: the width is a compile-time constant
     const int NSV = (4 * NQ + VK - 1) / VK;      // strips per row
-    const long long HW = (long long)P.H * W, SP = HW * D;
+    constexpr bool ROWS = KH == 1;               // images of a batch as the rows of one volume
+    const SlabAddr<ROWS> addr(P.C, D, P.H, W);
+    const long long HW = addr.plane, SP = addr.chan;
+    const long long RWX = ROWS ? addr.row_x : W, RWZ = ROWS ? addr.row_z : W;
     const int NC2 = 2 * NQ;
 
     int blk = blockIdx.x;
@@ -702,13 +705,15 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
     const int dch = blk % P.t.ndc; blk /= P.t.ndc;
     const int bc = blk;
     const int c = bc % P.C;
-    const int h0 = th * P.t.TH, H = P.H;
-    const int TH = min(P.t.TH, H - h0);
+    const int h_band = th * P.t.TH;
+    const int TH = min(P.t.TH, P.H - h_band);
+    // rows mode: the band is folded into the base pointers and rows are counted from it
+    const int h0 = ROWS ? 0 : h_band, H = ROWS ? P.H - h_band : P.H;
     const int d0 = dch * P.t.DC, d1 = min(D, d0 + P.t.DC);
     const int RS = lay.RS;
-    const long long bx = (long long)bc * SP;
+    const long long bx = (long long)bc * SP + (ROWS ? h_band * RWX : 0);
 
-    const float* ing = P.in + 2 * (long long)bc * SCH * SP;
+    const float* ing = P.in + 2 * ((long long)bc * SCH * SP + (ROWS ? h_band * RWZ : 0));
     float* gt1g = P.gt1 ? P.gt1 + bx : nullptr;
     T* gxg = P.gx ? reinterpret_cast<T*>(P.gx) + bx : nullptr;
     const T* t1g = reinterpret_cast<const T*>(P.t1) + bx;
@@ -736,7 +741,7 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
         if (id < nz) {
             const int c2 = id % NC2, t = id / NC2, r = t % RS, ch = t / RS;
             const int h = h0 - PH + r, w = 2 * c2, n = min(2, W - w);
-            if (h >= 0 && h < H && n > 0) cg_off[i] = (int)(ch * SP + (long long)h * W) + w;
+            if (h >= 0 && h < H && n > 0) cg_off[i] = (int)(ch * SP + h * RWZ) + w;
             cs_off[i] = ((ch * RS + r) * pitch2 + (swz2<VK>(c2 + 2) << 2)) | (max(n, 0) << 26);
         }
     }
@@ -845,7 +850,7 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
         }
         if (store) {
             const int w = VK * k_strip + (hi ? VK / 2 : 0) + (odd ? VO : 0);
-            const long long off = (long long)q * HW + (long long)(h0 + k_row) * W + w;
+            const long long off = (long long)q * HW + (h0 + k_row) * RWX + w;
             if (PADDED) {   // zero in the padding
 #pragma unroll
                 for (int i = 0; i < VO; ++i) if (w + i >= Wv) { o_t[i] = 0.0f; o_x[i] = 0.0f; }
@@ -869,8 +874,8 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
         }
     };
     // (t1, x) strips of plane q, raw; zero outside the chunk
-    const T* t1_row = t1g + (long long)(h0 + k_row) * W;
-    const T* x_row = xg + (long long)(h0 + k_row) * W;
+    const T* t1_row = t1g + (h0 + k_row) * RWX;
+    const T* x_row = xg + (h0 + k_row) * RWX;
     auto aux_raw = [&](int q, Raw4<T> (&dst)[2 * VO]) {
         if (WGRAD && k_ok && q >= d0 && q < d1) {
 #pragma unroll

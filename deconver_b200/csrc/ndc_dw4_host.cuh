@@ -148,8 +148,8 @@ struct BwdBands {
 // Rows: one-row planes of NQ 4-voxel strips (2-D images run as volumes, see FwdRows).
 template <int NQ_> struct BwdRows {
     static constexpr int RatioNT = NQ_, RatioMAXX = 1, KconvNT = 2 * NQ_, GzNT = NQ_, GzMAXX = 1;
-    // (not used: the row kernels keep two K passes)
-    static constexpr int Kconv2NT = 4 * NQ_, Kconv2VK = 4, Kconv2MAXC = 4, Kconv2WideNT = 0, Kconv2WideMAXC = 0;
+    // packed K: a strip per group of four channel lanes.  kconv_threads / kconv_strip below.
+    static constexpr int Kconv2WideNT = 0, Kconv2WideMAXC = 0, Kconv2MAXC = 4;
 };
 // Small volumes (3x3x3): narrower CTAs where they cover the same bands as the default ones
 // (a wide CTA would mostly idle on a band of 16 or 8 short rows).
@@ -230,14 +230,21 @@ inline bool plan_kconv(int D, int H, int W, long long BC, Tiling& t, size_t& sme
     return true;
 }
 
-// The packed K kernel (both scratch tensors in one pass) serves the 3x3x3 volumes.
-template <int KD, int KH, int KW>
-constexpr bool packed_kconv() { return KD == 3 && KH == 3 && KW == 3; }
+// The packed K kernel (both scratch tensors in one pass) serves the 3x3x3 volumes and the row-marching
+// images, except 5x5 rows of more than 256 columns, whose 512 threads of 200 registers fit no CTA.
+template <int KD, int KH, int KW, typename S>
+constexpr bool packed_kconv() { return KD == 3 ? KH != 1 || KW == 3 : KD == 5 && KH == 1 && S::RatioNT <= 64; }
+// Its strips: eight voxels; four for 5x5 images, whose five running sums and aux strips of eight
+// pairs would not fit the registers.
+template <int KD, int KH, typename S>
+constexpr int kconv2_strip() { if constexpr (KH == 1) return KD == 3 ? 8 : 4; else return S::Kconv2VK; }
+template <int KD, int KH, typename S>
+constexpr int kconv2_threads() { if constexpr (KH == 1) return KD == 3 ? 2 * S::RatioNT : 4 * S::RatioNT; else return S::Kconv2NT; }
 
 template <int KD, int KH, int KW, int NT, int VK, int MAXC>
 inline bool plan_kconv2(int D, int H, int W, long long BC, Tiling& t, size_t& smem_bytes) {
     constexpr int PH = KH / 2;
-    if ((long long)D * H * W >= (1LL << 29) || W > 256) return false;
+    if ((long long)D * H * W >= (1LL << 29) || W > (KH == 1 ? 512 : 256)) return false;
     t.NQ = (W + 3) / 4;
     t.pitch = row_pitch(W);
     const int NSV = (4 * t.NQ + VK - 1) / VK;
@@ -269,6 +276,8 @@ struct BwdPlan {
     int rows;                           // 0: band kernels; else the rows class planned
     int small;                          // 0, or the small-volume class planned (16 or 8)
     bool ratio_done = false;            // gnum, gden and the direct term are there already
+    bool pairs() const { return pairs_; }   // (gden, gnum) pairs in the scratch, or two tensors
+    bool pairs_;
 };
 
 template <int KD, int KH, int KW, typename S>
@@ -278,7 +287,8 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
                                512 / S::RatioNT, p.ratio, p.smem_ratio))
         return false;
     p.kconv_wide = 0;
-    if constexpr (packed_kconv<KD, KH, KW>()) {
+    p.pairs_ = packed_kconv<KD, KH, KW, S>();
+    if constexpr (packed_kconv<KD, KH, KW, S>()) {
         bool ok = false;
         if constexpr (S::Kconv2WideNT > 0) {
             if (g.W > 64) {
@@ -286,7 +296,7 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
                 p.kconv_wide = ok ? 1 : 0;
             }
         }
-        if (!ok && !plan_kconv2<KD, KH, KW, S::Kconv2NT, S::Kconv2VK, S::Kconv2MAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv))
+        if (!ok && !plan_kconv2<KD, KH, KW, kconv2_threads<KD, KH, S>(), kconv2_strip<KD, KH, S>(), S::Kconv2MAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv))
             return false;
     } else {
         if (!plan_kconv<KD, KH, KW, S::KconvNT>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv)) return false;
@@ -402,12 +412,12 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.gnum = gnum; P.gden = gden; P.gz = gz;
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.ratio; P.eps = g.eps; P.relu = g.relu;
         P.Wv = g.Wv; P.Wo = g.Wo;
-        auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD, KH, KW>() ? kRatioPairs : kRatioPlanar>;
+        auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD, KH, KW, S>() ? kRatioPairs : kRatioPlanar>;
         NDC_CUDA_TRY(set_smem(kern, p.smem_ratio));
         kern<<<(unsigned)p.n_ratio, S::RatioNT, p.smem_ratio, st>>>(P);
         launched();
     }
-    if constexpr (packed_kconv<KD, KH, KW>()) {
+    if constexpr (packed_kconv<KD, KH, KW, S>()) {
         Kconv2Params P;
         P.in = gnum;                          // (gden, gnum) pairs fill the gnum | gden area
         P.gt1 = (gz || gh) ? gt1 : nullptr;
@@ -416,7 +426,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.partial = gh ? pa : nullptr;
         P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv; P.Wv = g.Wv;
         auto run = [&](auto nt, auto maxc) -> cudaError_t {
-            constexpr int NT = decltype(nt)::value, VK = S::Kconv2VK, MAXC = decltype(maxc)::value;
+            constexpr int NT = decltype(nt)::value, VK = kconv2_strip<KD, KH, S>(), MAXC = decltype(maxc)::value;
             if (gh) {
                 auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, AL, true, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
@@ -432,9 +442,9 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
             if (p.kconv_wide)
                 NDC_CUDA_TRY(run(std::integral_constant<int, S::Kconv2WideNT>{}, std::integral_constant<int, S::Kconv2WideMAXC>{}));
             else
-                NDC_CUDA_TRY(run(std::integral_constant<int, S::Kconv2NT>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
+                NDC_CUDA_TRY(run(std::integral_constant<int, kconv2_threads<KD, KH, S>()>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
         } else {
-            NDC_CUDA_TRY(run(std::integral_constant<int, S::Kconv2NT>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
+            NDC_CUDA_TRY(run(std::integral_constant<int, kconv2_threads<KD, KH, S>()>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
         }
         launched();
     } else {
@@ -487,7 +497,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
     if (gh || gb) {
         ReduceParams P;
         P.partial_a = gh ? pa : nullptr;
-        P.partial_a2 = (gh && !packed_kconv<KD, KH, KW>()) ? pa2 : nullptr;   // packed: one record set
+        P.partial_a2 = (gh && !packed_kconv<KD, KH, KW, S>()) ? pa2 : nullptr;   // packed: one record set
         P.partial_b = pb;
         P.ctas_per_bc_a = (long long)p.kconv.ndc * p.kconv.nth;
         P.ctas_per_bc_b = (long long)p.gz.ndc * p.gz.nth;

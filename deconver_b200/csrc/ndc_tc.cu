@@ -84,12 +84,15 @@ cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, cons
 
 template <int KD, int KH, int KW>
 cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1, const float* h, const float* bias, const bf16* gout,
-                      float* gnum, float* gden, bf16* direct, cudaStream_t st) {
+                      float* gnum, float* gden, bf16* direct, bool pairs, cudaStream_t st) {
     AdjointArgs A{};
     if (!plan<KD, KH, KW>(g, g.D, A.b)) return cudaErrorInvalidConfiguration;
     A.x = x; A.t1 = t1; A.z = z; A.out = direct; A.gout = gout; A.gnum = gnum; A.gden = gden; A.h = h; A.bias = bias;
     const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1) && on16(gout) && (!direct || on16(direct));
-    return launch_adjoint<KD, KH, KW, KH == 1 ? kPlanar : kPairs>(g, A, wide, st);
+    if constexpr (KH == 1) {
+        if (!pairs) return launch_adjoint<KD, KH, KW, kPlanar>(g, A, wide, st);
+    }
+    return launch_adjoint<KD, KH, KW, kPairs>(g, A, wide, st);
 }
 
 // How large a problem has to be, and how much of the MMAs' rows it has to fill, for the tensor cores to be the
@@ -134,10 +137,10 @@ cudaError_t forward(const Geo& g, const bf16* x, const bf16* z, const float* h, 
 }
 
 cudaError_t backward_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1, const float* h, const float* bias,
-                           const bf16* gout, float* gnum, float* gden, bf16* direct, cudaStream_t st) {
-    if (g.kD == 3) return run_ratio<3, 3, 3>(g, x, z, t1, h, bias, gout, gnum, gden, direct, st);
-    if (g.kH == 5) return run_ratio<5, 1, 5>(as_rows(g), x, z, t1, h, bias, gout, gnum, gden, direct, st);
-    return run_ratio<3, 1, 3>(as_rows(g), x, z, t1, h, bias, gout, gnum, gden, direct, st);
+                           const bf16* gout, float* gnum, float* gden, bf16* direct, bool pairs, cudaStream_t st) {
+    if (g.kD == 3) return run_ratio<3, 3, 3>(g, x, z, t1, h, bias, gout, gnum, gden, direct, pairs, st);
+    if (g.kH == 5) return run_ratio<5, 1, 5>(as_rows(g), x, z, t1, h, bias, gout, gnum, gden, direct, pairs, st);
+    return run_ratio<3, 1, 3>(as_rows(g), x, z, t1, h, bias, gout, gnum, gden, direct, pairs, st);
 }
 
 unsigned wait_expired() {

@@ -495,30 +495,36 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         for (int o = warp >> 2; o < at.DC && ok; o += Shape::EPI) {
             const int slot = o % RING;
             const long long d = at.d0 + o;
-            // z (and gout) of a channel are on their way while the one before is worked on
-            uint4 zr[2], gr[2];
+            // z of all channels, or z and gout of two (the registers do not hold more), are on their way
+            // while the accumulators are waited for; their lines of this group's next plane come to L2
+            constexpr int AHEAD = MODE == kOut ? SC : 2;
+            uint4 zr[AHEAD], gr[AHEAD];
             auto fetch = [&](int j) {
-                zr[j & 1] = make_uint4(0u, 0u, 0u, 0u);
-                gr[j & 1] = make_uint4(0u, 0u, 0u, 0u);
+                zr[j % AHEAD] = make_uint4(0u, 0u, 0u, 0u);
+                gr[j % AHEAD] = make_uint4(0u, 0u, 0u, 0u);
                 if (!valid) return;
-                zr[j & 1] = load8<AL>(zb + j * addr.chan + d * addr.plane, w, b.W);
+                const bf16* zp = zb + j * addr.chan + d * addr.plane;
+                const bool more = (q & 7) == 0 && o + Shape::EPI < at.DC;
+                zr[j % AHEAD] = load8<AL>(zp, w, b.W);
+                if (more) asm volatile("prefetch.global.L2 [%0];" ::"l"(zp + Shape::EPI * addr.plane + w));
                 if (MODE == kOut) return;
+                if (more) asm volatile("prefetch.global.L2 [%0];" ::"l"(gb + j * oaddr.chan + (d + Shape::EPI) * oaddr.plane + w));
                 const bf16* row = gb + j * oaddr.chan + d * oaddr.plane;
-                if (AL != kPaddedOut || b.Wo == b.W) gr[j & 1] = load8<AL>(row, w, b.W);
+                if (AL != kPaddedOut || b.Wo == b.W) gr[j % AHEAD] = load8<AL>(row, w, b.W);
                 else {
                     unsigned e[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) e[i] = w + i < b.Wv ? reinterpret_cast<const unsigned short*>(row)[w + i] : 0u;
-                    gr[j & 1] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+                    gr[j % AHEAD] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
                 }
             };
-            fetch(0);
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j) fetch(j);
             ok = mbar_wait(afull + 8 * slot, (o / RING) & 1);
             tc_fence_after();
             const unsigned acc = lanes + slot * NC;
 #pragma unroll
             for (int j = 0; j < SC; ++j) {
-                if (j + 1 < SC) fetch(j + 1);
                 float n[8], dn[8];
                 __syncwarp();
                 tmem_load8x2(acc + 8 * j, acc + RING * NC + 8 * j, n, dn);
@@ -534,7 +540,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                 float gd[8];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const unsigned u = word_of(zr[j & 1], i);
+                    const unsigned u = word_of(zr[j % AHEAD], i);
                     f32x2 s2 = add2(pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)), b2[j]);
                     float lo, hi;
                     unpack2(s2, lo, hi);
@@ -543,7 +549,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                     if (MODE == kOut) {
                         unpack2(mul2(mul2(pack2(lo, hi), n2), r2), lo, hi);
                     } else {
-                        const unsigned q2 = word_of(gr[j & 1], i);
+                        const unsigned q2 = word_of(gr[j % AHEAD], i);
                         const f32x2 g2 = mul2(pack2(__uint_as_float(q2 << 16), __uint_as_float(q2 & 0xffff0000u)), r2);
                         const f32x2 gn2 = mul2(g2, pack2(lo, hi));
                         float a, c;
@@ -554,6 +560,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                     }
                     v[i] = pack_bf16(lo, hi);
                 }
+                if (j + AHEAD < SC) fetch(j + AHEAD);
                 if (MODE != kOut && w + 8 > b.Wv) {              // zero in the padding
 #pragma unroll
                     for (int i = 0; i < 8; ++i) if (w + i >= b.Wv) { n[i] = 0.0f; gd[i] = 0.0f; }

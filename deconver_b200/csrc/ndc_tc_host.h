@@ -10,11 +10,11 @@ namespace tc {
 bool covers(const Geo& g);
 cudaError_t forward(const Geo& g, const __nv_bfloat16* x, const __nv_bfloat16* z, const float* h, const float* bias,
                     __nv_bfloat16* out, __nv_bfloat16* t1, cudaStream_t st);
-// First step of the backward: gnum, gden (volumes: (gden, gnum) pairs at `gnum`; images: two tensors) and the
-// direct term, as ratio_kernel writes them.
+// First step of the backward: gnum, gden (two tensors, or (gden, gnum) pairs at `gnum`) and the direct term,
+// as ratio_kernel writes them.
 cudaError_t backward_ratio(const Geo& g, const __nv_bfloat16* x, const __nv_bfloat16* z, const __nv_bfloat16* t1, const float* h,
                            const float* bias, const __nv_bfloat16* gout, float* gnum, float* gden, __nv_bfloat16* direct,
-                           cudaStream_t st);
+                           bool pairs, cudaStream_t st);
 // Non-zero once a kernel's bounded wait has run out on the current device (synchronises; for tests).
 unsigned wait_expired();
 
