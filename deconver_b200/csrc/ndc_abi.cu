@@ -306,7 +306,7 @@ int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const v
                                            (gout_pitch == pitch ? (uintptr_t)gout : 0)) & 7) == 0) {
                 e = ndc::tc::backward_ratio(g, (const bf16*)x, (const bf16*)z, (const bf16*)t1, h, bias, (const bf16*)gout,
                                             (float*)((char*)workspace + p.off_gnum), (float*)((char*)workspace + p.off_gden),
-                                            (bf16*)gz, p.pairs(), st);
+                                            (bf16*)gz, p.pairs, st);
                 if (e != cudaSuccess) return cuda_fail(e, "ndc_bwd (tensor core) launch");
                 p.ratio_done = true;
             }

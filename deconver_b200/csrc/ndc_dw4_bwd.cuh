@@ -667,18 +667,15 @@ struct Kconv2Smem {
 // 16-byte chunk c of a row of pairs -> its place in shared memory.  The eight lanes of a
 // quarter-warp read chunks VK/2 apart (strips of VK voxels); folding bits 3.. of the chunk index
 // into the low bits sends them to eight different 16-byte bank groups.
-template <int VK> __device__ __forceinline__ int swz2(int chunk) {
-    return chunk ^ ((chunk >> 3) & (VK == 8 ? 3 : 1));
+__device__ __forceinline__ int swz2(int chunk) {
+    return chunk ^ ((chunk >> 3) & 3);
 }
 
-// Threads per SM the packed K kernel is built for, by CTA size and strip length.
-template <int NT, int VK> constexpr int kconv2_min_blocks() {
-    return VK == 8 ? (NT >= 256 ? 1 : NT >= 128 ? 2 : NT >= 64 ? 4 : 8)
-                   : (NT >= 256 ? 1 : NT >= 128 ? 2 : 4);
-}
+// CTAs per SM the packed K kernel is built for: 256 threads in all.
+template <int NT> constexpr int kconv2_min_blocks() { return NT >= 256 ? 1 : NT >= 128 ? 2 : NT >= 64 ? 4 : 8; }
 
 template <typename T, int KD, int KH, int KW, int NT, int VK, int MAXC, int AL, bool WGRAD, int WQ>
-__global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel(const Kconv2Params P) {
+__global__ void __launch_bounds__(NT, kconv2_min_blocks<NT>()) kconv2_kernel(const Kconv2Params P) {
     constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     using L = Kconv2Smem<KD, KH, KW>;
@@ -687,7 +684,7 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
     constexpr int NW = WGRAD ? KT : 1;           // correlation accumulators (pairs) per thread
     constexpr int NWIN = VK + 4;                 // window pairs held: voxels w0-2 .. w0+VK+1
     constexpr int VO = VK / 4;                   // voxels a lane owns after the channel lanes add up
-    static_assert(KD > 1 && PW <= 2 && (VK == 4 || VK == 8), "packed K kernel: marching kernels with up to 5 columns");
+    static_assert(KD > 1 && PW <= 2 && VK == 8, "packed K kernel: marching kernels, strips of 8");
     extern __shared__ __align__(16) float smem[];
     const L lay(P.t, NT);
     const int tid = threadIdx.x;
@@ -742,7 +739,7 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
             const int c2 = id % NC2, t = id / NC2, r = t % RS, ch = t / RS;
             const int h = h0 - PH + r, w = 2 * c2, n = min(2, W - w);
             if (h >= 0 && h < H && n > 0) cg_off[i] = (int)(ch * SP + h * RWZ) + w;
-            cs_off[i] = ((ch * RS + r) * pitch2 + (swz2<VK>(c2 + 2) << 2)) | (max(n, 0) << 26);
+            cs_off[i] = ((ch * RS + r) * pitch2 + (swz2(c2 + 2) << 2)) | (max(n, 0) << 26);
         }
     }
     const int lane = tid & 31;
@@ -782,7 +779,7 @@ __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT, VK>()) kconv2_kernel
     // (VK/2)*strip + 1 .. + VK/2 + 2 of a row hold voxels w0-2 .. w0+VK+1
     int qo[NWIN / 2];
 #pragma unroll
-    for (int q = 0; q < NWIN / 2; ++q) qo[q] = swz2<VK>((VK / 2) * k_strip + 1 + q) << 2;
+    for (int q = 0; q < NWIN / 2; ++q) qo[q] = swz2((VK / 2) * k_strip + 1 + q) << 2;
 
     f32x2 kacc[KD][VK], auxs[WGRAD ? KD : 1][VK];
 #pragma unroll

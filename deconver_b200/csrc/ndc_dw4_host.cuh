@@ -31,6 +31,9 @@ constexpr size_t kSmemMax = 227 * 1024;
 template <int KD, int KH, int KW> struct FwdShape;
 template <> struct FwdShape<1, 5, 5> { static constexpr int NT = 256, MAXZ = 1, MAXX = 1, MINB = 2; };
 template <> struct FwdShape<1, 3, 3> { static constexpr int NT = 256, MAXZ = 1, MAXX = 1, MINB = 2; };
+// Images whose strips fill 128 threads at most (16 x 16): half the CTA, and twice as many of them on a
+// multiprocessor.
+struct FwdBandSmall { static constexpr int NT = 128, MAXZ = 1, MAXX = 1, MINB = 4; };
 // 2-D image batches run as volumes of one-row planes: rows become the marching axis,
 // so nothing is recomputed between row bands and the loads of the next row overlap the work
 // on this one.  A CTA is as wide as one row has 4-voxel strips.
@@ -148,8 +151,7 @@ struct BwdBands {
 // Rows: one-row planes of NQ 4-voxel strips (2-D images run as volumes, see FwdRows).
 template <int NQ_> struct BwdRows {
     static constexpr int RatioNT = NQ_, RatioMAXX = 1, KconvNT = 2 * NQ_, GzNT = NQ_, GzMAXX = 1;
-    // packed K: a strip per group of four channel lanes.  kconv_threads / kconv_strip below.
-    static constexpr int Kconv2WideNT = 0, Kconv2WideMAXC = 0, Kconv2MAXC = 4;
+    static constexpr int Kconv2VK = 8, Kconv2MAXC = 4, Kconv2WideNT = 0, Kconv2WideMAXC = 0;   // 3x3: kconv2_threads
 };
 // Small volumes (3x3x3): narrower CTAs where they cover the same bands as the default ones
 // (a wide CTA would mostly idle on a band of 16 or 8 short rows).
@@ -231,15 +233,12 @@ inline bool plan_kconv(int D, int H, int W, long long BC, Tiling& t, size_t& sme
 }
 
 // The packed K kernel (both scratch tensors in one pass) serves the 3x3x3 volumes and the row-marching
-// images, except 5x5 rows of more than 256 columns, whose 512 threads of 200 registers fit no CTA.
-template <int KD, int KH, int KW, typename S>
-constexpr bool packed_kconv() { return KD == 3 ? KH != 1 || KW == 3 : KD == 5 && KH == 1 && S::RatioNT <= 64; }
-// Its strips: eight voxels; four for 5x5 images, whose five running sums and aux strips of eight
-// pairs would not fit the registers.
-template <int KD, int KH, typename S>
-constexpr int kconv2_strip() { if constexpr (KH == 1) return KD == 3 ? 8 : 4; else return S::Kconv2VK; }
-template <int KD, int KH, typename S>
-constexpr int kconv2_threads() { if constexpr (KH == 1) return KD == 3 ? 2 * S::RatioNT : 4 * S::RatioNT; else return S::Kconv2NT; }
+// 3x3 images (three updates on 5 x 24 x 203x171: 368 -> 289 us).  For 5x5 images its five running sums
+// and aux strips leave one CTA of 256 threads to a multiprocessor, and it is no faster than two scalar
+// passes (948 against 916 us at 16 x 32 x 256^2).
+template <int KD> constexpr bool packed_kconv() { return KD == 3; }
+template <int KH, typename S>
+constexpr int kconv2_threads() { if constexpr (KH == 1) return 2 * S::RatioNT; else return S::Kconv2NT; }
 
 template <int KD, int KH, int KW, int NT, int VK, int MAXC>
 inline bool plan_kconv2(int D, int H, int W, long long BC, Tiling& t, size_t& smem_bytes) {
@@ -254,7 +253,7 @@ inline bool plan_kconv2(int D, int H, int W, long long BC, Tiling& t, size_t& sm
         return (size_t)Kconv2Smem<KD, KH, KW>(q, NT).total_floats * sizeof(float);
     };
     auto chunks = [&](int th) { return SCH * (th + 2 * PH) * 2 * t.NQ; };
-    constexpr int per_sm = kconv2_min_blocks<NT, VK>();
+    constexpr int per_sm = kconv2_min_blocks<NT>();
     const size_t target = (kSmemMax - 8 * 1024) / per_sm;
     while (TH > 1 && (bytes(TH) > target || chunks(TH) > MAXC * NT ||
                       SCH * (TH + 2 * PH) * 2 * t.pitch >= (1 << 26)))
@@ -276,8 +275,7 @@ struct BwdPlan {
     int rows;                           // 0: band kernels; else the rows class planned
     int small;                          // 0, or the small-volume class planned (16 or 8)
     bool ratio_done = false;            // gnum, gden and the direct term are there already
-    bool pairs() const { return pairs_; }   // (gden, gnum) pairs in the scratch, or two tensors
-    bool pairs_;
+    bool pairs;                         // (gden, gnum) pairs in the scratch, or two tensors
 };
 
 template <int KD, int KH, int KW, typename S>
@@ -287,8 +285,8 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
                                512 / S::RatioNT, p.ratio, p.smem_ratio))
         return false;
     p.kconv_wide = 0;
-    p.pairs_ = packed_kconv<KD, KH, KW, S>();
-    if constexpr (packed_kconv<KD, KH, KW, S>()) {
+    p.pairs = packed_kconv<KD>();
+    if constexpr (packed_kconv<KD>()) {
         bool ok = false;
         if constexpr (S::Kconv2WideNT > 0) {
             if (g.W > 64) {
@@ -296,7 +294,7 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
                 p.kconv_wide = ok ? 1 : 0;
             }
         }
-        if (!ok && !plan_kconv2<KD, KH, KW, kconv2_threads<KD, KH, S>(), kconv2_strip<KD, KH, S>(), S::Kconv2MAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv))
+        if (!ok && !plan_kconv2<KD, KH, KW, kconv2_threads<KH, S>(), S::Kconv2VK, S::Kconv2MAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv))
             return false;
     } else {
         if (!plan_kconv<KD, KH, KW, S::KconvNT>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv)) return false;
@@ -329,8 +327,14 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
 // group whose planes are the image rows and whose plane rows are the images of the batch (the
 // same memory and the same filter layout; kernel K x 1 x K, so images never mix).  A CTA takes
 // as many images as fill its threads (one image of 129..512 columns, four of 64, ...).  Returns
-// the CTA size class (strips of 4 per CTA), or 0 where the band kernels stay: a batch too small
-// to fill even the small CTA, or a band whose 32-bit offsets would overflow.
+// the CTA size class (strips of 4 per CTA), or 0 where the band kernels stay:
+//  - a batch too small to fill even the small CTA, or a band whose 32-bit offsets would overflow;
+//  - fewer than 32 rows and fewer CTAs than SMs: so short a march is not cut, and the band
+//    kernels have more blocks (bf16 8 x 40 groups of 28x30, 5x5: 213 -> 181 us for a training
+//    update of which ~100 us are launches; 16 x 512 of 16x16 stays, 403 against 671 us);
+//  - 5x5 on images of 129..192 columns, where one image leaves a quarter or more of the 64 lanes
+//    idle and a second does not fit (5 x 24 of 203x171: 878 -> 708 us; 3x3 there is 563 against
+//    580 us for the bands and keeps its rows).
 inline int rows_class(const Geo& g) {
     if (g.D != 1 || g.kD != 1 || g.kH != g.kW || (g.kH != 5 && g.kH != 3) || g.H < 8) return 0;
     const int NQ = (g.W + 3) / 4;
@@ -338,7 +342,9 @@ inline int rows_class(const Geo& g) {
     const int images = NQ > 64 ? 1 : std::min(g.B, 64 / NQ);   // per CTA
     const long long image = (long long)g.H * g.W;       // elements of one channel
     if ((images * (long long)g.G + 1) * SCH * image >= (1LL << 31)) return 0;
+    if (g.H < 32 && (long long)g.G * ((g.B + images - 1) / images) < 148) return 0;
     const int strips = images * NQ;
+    if (g.kH == 5 && images == 1 && strips > 32 && strips <= 48) return 0;
     return strips > 64 ? 128 : strips > 32 ? 64 : strips >= 24 ? 32 : 0;
 }
 inline Geo as_rows(const Geo& g) {
@@ -412,12 +418,12 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.gnum = gnum; P.gden = gden; P.gz = gz;
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.ratio; P.eps = g.eps; P.relu = g.relu;
         P.Wv = g.Wv; P.Wo = g.Wo;
-        auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD, KH, KW, S>() ? kRatioPairs : kRatioPlanar>;
+        auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD>() ? kRatioPairs : kRatioPlanar>;
         NDC_CUDA_TRY(set_smem(kern, p.smem_ratio));
         kern<<<(unsigned)p.n_ratio, S::RatioNT, p.smem_ratio, st>>>(P);
         launched();
     }
-    if constexpr (packed_kconv<KD, KH, KW, S>()) {
+    if constexpr (packed_kconv<KD>()) {
         Kconv2Params P;
         P.in = gnum;                          // (gden, gnum) pairs fill the gnum | gden area
         P.gt1 = (gz || gh) ? gt1 : nullptr;
@@ -426,7 +432,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.partial = gh ? pa : nullptr;
         P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv; P.Wv = g.Wv;
         auto run = [&](auto nt, auto maxc) -> cudaError_t {
-            constexpr int NT = decltype(nt)::value, VK = kconv2_strip<KD, KH, S>(), MAXC = decltype(maxc)::value;
+            constexpr int NT = decltype(nt)::value, VK = S::Kconv2VK, MAXC = decltype(maxc)::value;
             if (gh) {
                 auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, AL, true, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
@@ -442,9 +448,9 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
             if (p.kconv_wide)
                 NDC_CUDA_TRY(run(std::integral_constant<int, S::Kconv2WideNT>{}, std::integral_constant<int, S::Kconv2WideMAXC>{}));
             else
-                NDC_CUDA_TRY(run(std::integral_constant<int, kconv2_threads<KD, KH, S>()>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
+                NDC_CUDA_TRY(run(std::integral_constant<int, kconv2_threads<KH, S>()>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
         } else {
-            NDC_CUDA_TRY(run(std::integral_constant<int, kconv2_threads<KD, KH, S>()>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
+            NDC_CUDA_TRY(run(std::integral_constant<int, kconv2_threads<KH, S>()>{}, std::integral_constant<int, S::Kconv2MAXC>{}));
         }
         launched();
     } else {
@@ -497,7 +503,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
     if (gh || gb) {
         ReduceParams P;
         P.partial_a = gh ? pa : nullptr;
-        P.partial_a2 = (gh && !packed_kconv<KD, KH, KW, S>()) ? pa2 : nullptr;   // packed: one record set
+        P.partial_a2 = (gh && !packed_kconv<KD>()) ? pa2 : nullptr;   // packed: one record set
         P.partial_b = pb;
         P.ctas_per_bc_a = (long long)p.kconv.ndc * p.kconv.nth;
         P.ctas_per_bc_b = (long long)p.gz.ndc * p.gz.nth;
@@ -722,6 +728,9 @@ cudaError_t forward_image(const Geo& g, const T* x, const T* z, const float* h, 
             : forward_shape<T, K, 1, K, FwdRows<32>>(v, x, z, h, bias, out, t1, dtype, st, handled);
         if (handled || e != cudaSuccess) return e;
     }
+    const int NQ = (g.W + 3) / 4;
+    if (g.D == 1 && g.H * NQ <= FwdBandSmall::NT && (g.H + K - 1) * ((NQ + 1) / 2) * 2 <= FwdBandSmall::NT)
+        return forward_shape<T, 1, K, K, FwdBandSmall>(g, x, z, h, bias, out, t1, dtype, st, handled);
     return forward_shape<T, 1, K, K>(g, x, z, h, bias, out, t1, dtype, st, handled);
 }
 
