@@ -3,9 +3,10 @@ layer's native host path (`csrc/ndc_torch.cpp`, on that library and PyTorch's C+
 `deconver_b200/_ndc_torch.so` with the host compiler.
 
 Both are built in-tree (next to this file) so that they travel with the source tree.
-nvcc cross-compiles without a GPU.  The tiled kernels are compiled as six translation units
-(forward / backward of volumes / backward of images, each for float32 and bfloat16) next to the
-ABI unit and the instance-norm and bias units, in parallel, then linked.  Run as `python -m deconver_b200._build [--force]`.
+nvcc cross-compiles without a GPU.  The marching kernels are compiled as six translation units
+(forward / backward of volumes / backward of images, each for float32 and bfloat16) and the tile
+kernels as two, next to the ABI unit and those of the instance norm, the bias passes, the projection
+and the tensor-core kernels, in parallel, then linked.  Run as `python -m deconver_b200._build [--force]`.
 """
 
 import os

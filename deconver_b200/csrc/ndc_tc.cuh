@@ -1,6 +1,7 @@
 // The forward update of bfloat16 tensors on the 5th-generation tensor cores (m = 1, sc = 4; 3x3x3,
 // 5x5 and 3x3 kernels), where the filter and the bias are bfloat16 values too, as in a bfloat16
-// module.  Two launches: tc_source_kernel (t1 = K(relu(z + b))) and tc_adjoint_kernel (out).
+// module.  Two launches: tc_source_kernel (t1 = K(relu(z + b))) and tc_adjoint_kernel (out).  The latter is
+// the ratio step of the backward too (gnum, gden and the direct term, see AdjointMode).
 //
 // A depthwise convolution as a matrix product.  Rows of a plane lie in shared memory one after the
 // other as bfloat16, column w at place w + PW of its row, zeros between the rows; a row takes a whole
