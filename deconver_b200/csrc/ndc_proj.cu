@@ -431,7 +431,7 @@ int ndc_unpad_rows(int64_t rows, int32_t W, int32_t pitch, int32_t dtype, const 
 
 int ndc_params_prepare(int32_t dtype, const void* h0, int64_t nh, float* h, const void* bias, int64_t nb,
                        float* b, void* stream) {
-    if (!h0 || !h || nh <= 0 || nb < 0 || (nb && (!bias || !b)) || (dtype != NDC_F32 && dtype != NDC_BF16))
+    if (nh < 0 || nb < 0 || nh + nb == 0 || (nh && (!h0 || !h)) || (nb && (!bias || !b)) || (dtype != NDC_F32 && dtype != NDC_BF16))
         return proj_fail(NDC_ERR_INVALID, "parameter preparation: invalid argument");
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)((nh + nb + 255) / 256);

@@ -1,17 +1,19 @@
-// The layer's host path in native code: one autograd node for the whole `Deconv` layer
-// (parameters -> float32, 1x1 projection, multiplicative updates), on the C ABI of
-// libndc_b200.so and cuBLAS.
+// The host path in native code: one autograd node for the whole `Deconv` layer (parameters ->
+// float32, 1x1 projection, multiplicative updates), and one each for its neighbours in a block
+// (1x1 projection with bias, bias + GELU, instance norm), on the C ABI of libndc_b200.so and cuBLAS.
 //
 // What bounds the layer at the deep stages and on single images is not the GPU: at 512 channels
 // x 8^3 a forward and backward are 0.16 ms of kernels, and issuing them from Python through
 // separate autograd nodes took 0.60 ms.  One node, one pass over the parameters in each
-// direction, and no intermediate tensor that the update kernels do not read.
+// direction, and no intermediate tensor that the update kernels do not read.  The neighbours the same:
+// see the figures at their section.
 #include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/relu.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cublas_v2.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/extension.h>
 
 #include <mutex>
@@ -375,10 +377,267 @@ Tensor layer(const Tensor& x_in, const Tensor& h0_in, const Tensor& w_in, const 
     return run_forward(x, h0, w, bias ? *bias : Tensor(), Config{groups, m, sc, eps, iters, grad_iters, flags}, nullptr);
 }
 
+// ---- the layer's neighbours in a block ---------------------------------------------------------
+// Small blocks are bound by the host here too: with one Python autograd node each and their parameters
+// converted one by one, a training step of a bf16 block of 32 channels x 16^3 took 1.44 - 2.16 ms for
+// 0.22 ms of kernels; from here it takes 0.72.  float32 projections lose the convolution route's copies
+// to channels-last as well (8 x 32 x 40^3: 11.4 -> 3.4 ms).
+
+// A vector of parameters as float32, and a float32 gradient in the parameters' type: one launch.
+Tensor as_f32(const Tensor& t) {
+    if (!t.defined() || t.scalar_type() == at::kFloat) return t.defined() ? t.contiguous() : t;
+    if (t.scalar_type() != at::kBFloat16 || !t.numel()) return t.to(at::kFloat).contiguous();
+    const Tensor in = t.contiguous();
+    Tensor out = at::empty(in.sizes(), in.options().dtype(at::kFloat));
+    check(ndc_params_prepare(NDC_BF16, nullptr, 0, nullptr, ptr(in), in.numel(), fptr(out), stream()), ndc_proj_last_error());
+    return out;
+}
+Tensor from_f32(const Tensor& g, at::ScalarType type) {
+    if (!g.defined() || type == at::kFloat) return g;
+    if (type != at::kBFloat16 || !g.numel()) return g.to(type);
+    Tensor out = at::empty(g.sizes(), g.options().dtype(type));
+    check(ndc_params_grad(NDC_BF16, nullptr, nullptr, 0, nullptr, fptr(g), g.numel(), ptr(out), stream()), ndc_proj_last_error());
+    return out;
+}
+
+// The gradients of a node whose backward is not itself differentiable: they are computed without a
+// graph, and differentiating them raises an error.
+variable_list once(const variable_list& grads, variable_list out) {
+    bool any = false;
+    for (const Tensor& g : grads) any = any || (g.defined() && g.requires_grad());
+    if (!at::GradMode::is_enabled() || !any) return out;
+    auto error = std::make_shared<torch::autograd::DelayedError>(
+        "trying to differentiate twice a function that was marked with @once_differentiable", (int64_t)out.size());
+    for (Tensor& t : out)
+        if (t.defined()) t = t.detach().requires_grad_();
+    return (*error)(std::move(out));
+}
+
+struct Slabs { int batch, channels; int64_t n; };
+Slabs slabs(const Tensor& x) {
+    const int64_t bc = x.size(0) * x.size(1);
+    int64_t n = 1;
+    for (int64_t i = 2; i < x.dim(); ++i) n *= x.size(i);
+    return {(int)x.size(0), (int)x.size(1), bc ? n : 0};
+}
+Tensor like(const Tensor& g, const Tensor& x) {
+    Tensor c = g.contiguous();
+    return c.scalar_type() == x.scalar_type() ? c : c.to(x.scalar_type());
+}
+Tensor bias_scratch(const Slabs& s, const Tensor& x) {
+    return at::empty({(int64_t)ndc_bias_grad_workspace_bytes(s.batch, s.channels)}, x.options().dtype(at::kByte));
+}
+
+// y = w x (+ bias) over the channel axis; `w` (Co, Ci, 1)
+struct LinearNode : public torch::autograd::Function<LinearNode> {
+    static Tensor run(const Tensor& x, const Tensor& w, const Tensor& bias) {
+        auto shape = x.sizes().vec();
+        shape[1] = w.size(0);
+        Tensor y = at::empty(shape, x.options());
+        const Slabs s = slabs(y), in = slabs(x);
+        if (!y.numel()) return y;
+        if (!in.channels) y.zero_();
+        else channel_gemm(w, false, x, y, s.batch, s.n, false);
+        if (bias.defined()) {
+            const Tensor b = as_f32(bias);
+            check(ndc_bias_add(s.batch, s.channels, s.n, dtype_code(y), ptr(y), fptr(b), stream()), ndc_bias_last_error());
+        }
+        return y;
+    }
+
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const std::optional<Tensor>& bias) {
+        const Tensor b = bias ? *bias : Tensor();
+        ctx->save_for_backward({x, w});
+        ctx->saved_data["bias"] = b.defined();
+        ctx->saved_data["type"] = (int64_t)(b.defined() ? b.scalar_type() : at::kFloat);
+        return run(x, w, b);
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list out(3);
+        {
+            at::AutoGradMode off(false);
+            const variable_list kept = ctx->get_saved_variables();
+            const Tensor &x = kept[0], &w = kept[1];
+            c10::cuda::CUDAGuard guard(x.device());
+            const Tensor g = like(grads[0], x);
+            const Slabs s = slabs(g);
+            if (ctx->needs_input_grad(0)) {
+                out[0] = at::empty(x.sizes(), x.options());
+                if (s.n) channel_gemm(w, true, g, out[0], s.batch, s.n, false);
+                else out[0].zero_();
+            }
+            if (ctx->needs_input_grad(1)) out[1] = weight_grad(g, x, w, s.batch, s.n);
+            if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) {
+                Tensor gb = at::empty({s.channels}, x.options().dtype(at::kFloat));
+                if (s.n) {
+                    Tensor ws = bias_scratch(s, x);
+                    check(ndc_bias_grad(s.batch, s.channels, s.n, dtype_code(g), ptr(g), fptr(gb), ptr(ws), ws.numel(), stream()),
+                          ndc_bias_last_error());
+                } else {
+                    gb.zero_();
+                }
+                out[2] = from_f32(gb, (at::ScalarType)ctx->saved_data["type"].toInt());
+            }
+        }
+        return once(grads, out);
+    }
+};
+
+bool wants_grad(std::initializer_list<const Tensor*> tensors) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor* t : tensors)
+        if (t->defined() && t->requires_grad()) return true;
+    return false;
+}
+
+Tensor linear(const Tensor& x_in, const Tensor& w_in, const std::optional<Tensor>& bias_in) {
+    TORCH_CHECK(kernel_dtype(x_in) && w_in.scalar_type() == x_in.scalar_type() && w_in.device() == x_in.device() &&
+                x_in.dim() >= 3 && w_in.dim() == 3 && w_in.size(2) == 1 && w_in.size(1) == x_in.size(1),
+                "deconver_b200: input ", x_in.sizes(), " (", x_in.scalar_type(), ", ", x_in.device(), ") and 1x1 weight ",
+                w_in.sizes(), " (", w_in.scalar_type(), ", ", w_in.device(), ") do not match");
+    TORCH_CHECK(!bias_in || (bias_in->device() == x_in.device() && bias_in->numel() == w_in.size(0)),
+                "deconver_b200: the bias does not match the projection");
+    c10::cuda::CUDAGuard guard(x_in.device());
+    const Tensor x = x_in.contiguous(), w = w_in.contiguous(), b = bias_in ? *bias_in : Tensor();
+    if (wants_grad({&x, &w, &b})) return LinearNode::apply(x, w, bias_in);
+    at::AutoDispatchBelowADInplaceOrView below;
+    return LinearNode::run(x, w, b);
+}
+
+// gelu(h + bias[c]), erf form
+struct BiasGeluNode : public torch::autograd::Function<BiasGeluNode> {
+    static Tensor run(const Tensor& h, const Tensor& b) {
+        Tensor out = at::empty(h.sizes(), h.options());
+        const Slabs s = slabs(h);
+        if (h.numel())
+            check(ndc_bias_gelu_fwd(s.batch, s.channels, s.n, dtype_code(h), ptr(h), fptr(b), ptr(out), stream()), ndc_bias_last_error());
+        return out;
+    }
+
+    static Tensor forward(AutogradContext* ctx, const Tensor& h, const std::optional<Tensor>& bias) {
+        const Tensor b = as_f32(bias ? *bias : Tensor());
+        ctx->save_for_backward({h, b});
+        ctx->saved_data["bias"] = (int64_t)(bias ? bias->scalar_type() : at::kFloat);
+        return run(h, b);
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list out(2);
+        {
+            at::AutoGradMode off(false);
+            const variable_list kept = ctx->get_saved_variables();
+            const Tensor &h = kept[0], &b = kept[1];
+            c10::cuda::CUDAGuard guard(h.device());
+            const Tensor g = like(grads[0], h);
+            const Slabs s = slabs(h);
+            const bool want_bias = b.defined() && ctx->needs_input_grad(1);
+            out[0] = at::empty(h.sizes(), h.options());
+            Tensor gb, ws;
+            if (want_bias) {
+                gb = at::empty({s.channels}, h.options().dtype(at::kFloat));
+                ws = bias_scratch(s, h);
+            }
+            if (s.n)
+                check(ndc_bias_gelu_bwd(s.batch, s.channels, s.n, dtype_code(h), ptr(g), ptr(h), fptr(b), ptr(out[0]), fptr(gb),
+                                        ptr(ws), want_bias ? ws.numel() : 0, stream()), ndc_bias_last_error());
+            else if (want_bias)
+                gb.zero_();
+            if (want_bias) out[1] = from_f32(gb, (at::ScalarType)ctx->saved_data["bias"].toInt());
+        }
+        return once(grads, out);
+    }
+};
+
+Tensor bias_gelu(const Tensor& h_in, const std::optional<Tensor>& bias) {
+    TORCH_CHECK(kernel_dtype(h_in) && h_in.is_cuda() && h_in.dim() >= 2 &&
+                (!bias || (bias->device() == h_in.device() && bias->numel() == h_in.size(1))),
+                "deconver_b200: the bias does not match the tensor");
+    c10::cuda::CUDAGuard guard(h_in.device());
+    const Tensor h = h_in.contiguous(), b = bias ? *bias : Tensor();
+    if (wants_grad({&h, &b})) return BiasGeluNode::apply(h, bias);
+    at::AutoDispatchBelowADInplaceOrView below;
+    return BiasGeluNode::run(h, as_f32(b));
+}
+
+// (x - mean) / sqrt(var + eps) [* weight + bias] per (sample, channel)
+struct NormNode : public torch::autograd::Function<NormNode> {
+    static Tensor run(const Tensor& x, const Tensor& w, const Tensor& b, double eps, Tensor& stats) {
+        Tensor y = at::empty(x.sizes(), x.options());
+        const Slabs s = slabs(x);
+        stats = at::empty({(int64_t)s.batch * s.channels * 2}, x.options().dtype(at::kFloat));
+        if (x.numel()) {
+            const size_t bytes = ndc_inorm_workspace_bytes(s.batch, s.channels);
+            Tensor ws = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
+            check(ndc_inorm_fwd(s.batch, s.channels, s.n, dtype_code(x), ptr(x), fptr(w), fptr(b), (float)eps, ptr(y), fptr(stats),
+                                ptr(ws), bytes, stream()), ndc_inorm_last_error());
+        }
+        return y;
+    }
+
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& weight,
+                          const std::optional<Tensor>& bias, double eps) {
+        const Tensor w = weight ? *weight : Tensor();
+        Tensor stats;
+        Tensor y = run(x, as_f32(w), as_f32(bias ? *bias : Tensor()), eps, stats);
+        ctx->save_for_backward({x, w, stats});
+        // a bias without a weight keeps its gradient in float32
+        ctx->saved_data["type"] = (int64_t)(w.defined() ? w.scalar_type() : at::kFloat);
+        ctx->saved_data["bias"] = bias.has_value();
+        return y;
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list out(4);
+        {
+            at::AutoGradMode off(false);
+            const variable_list kept = ctx->get_saved_variables();
+            const Tensor &x = kept[0], &w = kept[1], &stats = kept[2];
+            c10::cuda::CUDAGuard guard(x.device());
+            const Tensor g = like(grads[0], x);
+            const Slabs s = slabs(x);
+            const auto f32 = x.options().dtype(at::kFloat);
+            Tensor gx = at::empty(x.sizes(), x.options()), gw, gb;
+            if (w.defined() && ctx->needs_input_grad(1)) gw = at::empty({s.channels}, f32);
+            // (gradients are counted over the tensors that are there)
+            if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(w.defined() ? 2 : 1)) gb = at::empty({s.channels}, f32);
+            if (x.numel()) {
+                const Tensor wf = as_f32(w);
+                const size_t bytes = ndc_inorm_workspace_bytes(s.batch, s.channels);
+                Tensor ws = at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
+                check(ndc_inorm_bwd(s.batch, s.channels, s.n, dtype_code(x), ptr(x), ptr(g), fptr(wf), fptr(stats), ptr(gx), fptr(gw),
+                                    fptr(gb), ptr(ws), bytes, stream()), ndc_inorm_last_error());
+            } else {
+                for (Tensor* t : {&gw, &gb}) if (t->defined()) t->zero_();
+            }
+            const auto type = (at::ScalarType)ctx->saved_data["type"].toInt();
+            if (ctx->needs_input_grad(0)) out[0] = gx;
+            out[1] = from_f32(gw, type);
+            out[2] = from_f32(gb, type);
+        }
+        return once(grads, out);
+    }
+};
+
+Tensor instance_norm(const Tensor& x_in, const std::optional<Tensor>& weight, const std::optional<Tensor>& bias, double eps) {
+    for (const auto* t : {&weight, &bias})
+        TORCH_CHECK(!*t || ((*t)->device() == x_in.device() && (*t)->numel() == x_in.size(1)),
+                    "deconver_b200: instance norm parameters do not match the input ", x_in.sizes());
+    c10::cuda::CUDAGuard guard(x_in.device());
+    const Tensor x = x_in.contiguous(), w = weight ? *weight : Tensor(), b = bias ? *bias : Tensor();
+    if (wants_grad({&x, &w, &b})) return NormNode::apply(x, weight, bias, eps);
+    at::AutoDispatchBelowADInplaceOrView below;
+    Tensor stats;
+    return NormNode::run(x, as_f32(w), as_f32(b), eps, stats);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod) {
     mod.def("layer", &layer, py::call_guard<py::gil_scoped_release>());
+    mod.def("linear", &linear, py::call_guard<py::gil_scoped_release>());
+    mod.def("bias_gelu", &bias_gelu, py::call_guard<py::gil_scoped_release>());
+    mod.def("instance_norm", &instance_norm, py::call_guard<py::gil_scoped_release>());
     mod.def("timing_enable", &timing_enable);
     mod.def("timing_collect", &timing_collect);
 }

@@ -15,60 +15,17 @@ from typing import Optional
 
 import torch
 from torch import nn
-from torch.autograd.function import once_differentiable
 from torch.nn.modules.utils import _pair
 
-from . import _lib
-from .linear import _DTYPES, Linear, _check, conv1x1
-
-
-class _BiasGelu(torch.autograd.Function):
-    """``gelu(h + bias[c])`` (erf form, erf to an absolute error below 1e-6) of a contiguous
-    ``(B, C, L)`` tensor."""
-
-    @staticmethod
-    def forward(ctx, h, bias):
-        h = h.contiguous()
-        B, C, L = h.shape
-        bf = None if bias is None else bias.detach().to(torch.float32).contiguous()
-        out = torch.empty_like(h)
-        if h.numel():
-            with torch.cuda.device(h.device):
-                _check(_lib.load().ndc_bias_gelu_fwd(
-                    B, C, L, _DTYPES[h.dtype], h.data_ptr(), 0 if bf is None else bf.data_ptr(),
-                    out.data_ptr(), torch.cuda.current_stream().cuda_stream))
-        ctx.save_for_backward(h, bf)
-        ctx.bias_dtype = None if bias is None else bias.dtype
-        return out
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, ga):
-        h, bf = ctx.saved_tensors
-        ga = ga.contiguous()
-        B, C, L = h.shape
-        want_bias = bf is not None and ctx.needs_input_grad[1]
-        gh = torch.empty_like(h)
-        gbias = torch.zeros(C, device=h.device, dtype=torch.float32) if want_bias else None
-        if h.numel():
-            lib = _lib.load()
-            with torch.cuda.device(h.device):
-                nbytes = lib.ndc_bias_grad_workspace_bytes(B, C) if want_bias else 0
-                ws = torch.empty(nbytes, device=h.device, dtype=torch.uint8) if want_bias else None
-                _check(lib.ndc_bias_gelu_bwd(
-                    B, C, L, _DTYPES[h.dtype], ga.data_ptr(), h.data_ptr(),
-                    0 if bf is None else bf.data_ptr(), gh.data_ptr(),
-                    gbias.data_ptr() if want_bias else 0, ws.data_ptr() if want_bias else 0, nbytes,
-                    torch.cuda.current_stream().cuda_stream))
-        return gh, (gbias.to(ctx.bias_dtype) if want_bias else None)
+from ._lib import load_ext
+from .linear import _DTYPES, Linear, native_operands
 
 
 def bias_gelu(h: torch.Tensor, bias: Optional[torch.Tensor]) -> torch.Tensor:
     """``gelu(h + bias)`` over the channel axis (dim 1) of a CUDA float32 / bfloat16 tensor."""
     if not h.is_cuda or h.dtype not in _DTYPES:
         raise RuntimeError("bias_gelu runs on CUDA float32 / bfloat16 tensors only")
-    shape = h.shape
-    return _BiasGelu.apply(h.reshape(shape[0], shape[1], -1), bias).view(shape)
+    return load_ext().bias_gelu(h, bias)
 
 
 class MLP(nn.Module):
@@ -89,12 +46,9 @@ class MLP(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         first, act, drop1, second, drop2 = self.block
-        fused = (x.is_cuda and x.dtype in _DTYPES and x.dim() >= 3 and isinstance(act, nn.GELU)
-                 and act.approximate == "none" and type(first) is Linear)
-        if not fused:
+        operands = native_operands(x, first.linear.weight) if type(first) is Linear else None
+        if operands is None or not isinstance(act, nn.GELU) or act.approximate != "none":
             return self.block(x)
-        shape = x.shape
-        h = conv1x1(x.flatten(2), first.linear.weight)
-        a = _BiasGelu.apply(h, first.linear.bias)
-        a = drop1(a)
-        return drop2(second(a.view(shape[0], -1, *shape[2:])))
+        ext = load_ext()
+        a = ext.bias_gelu(ext.linear(*operands, None), first.linear.bias)
+        return drop2(second(drop1(a)))

@@ -271,7 +271,7 @@ int ndc_bias_gelu_bwd(int32_t batch, int32_t channels, int64_t spatial, int32_t 
  *                         fixed order, converted to dtype `dtype`: the second half of a weight
  *                         gradient whose partial products the caller computed itself
  *     ndc_params_prepare  h = relu(h0), b = bias as float32 (nh and nb elements of dtype `dtype`;
- *                         nb may be 0, then bias and b may be NULL)
+ *                         nh or nb may be 0, then the pointers of that part may be NULL)
  *     ndc_params_grad     gh0 = h0 > 0 ? gh : 0 and gbias = gb, converted to dtype `dtype` (nh or
  *                         nb may be 0, then the pointers of that part may be NULL)
  * Errors: status code, message from ndc_proj_last_error().
