@@ -43,21 +43,36 @@ inline bool shape_supported(int kD, int kH, int kW) {
            (kD == 1 && kH == 3 && kW == 3);
 }
 
-// Chunks along depth: enough CTAs for about `waves` rounds of `ctas_per_sm` CTAs per SM, but
-// chunks of at least 16*PD planes (every chunk recomputes 2*PD planes of its neighbours); only
-// a grid that would not even fill the GPU once is cut finer, down to 4*PD planes.
-inline void plan_depth(int KD, int D, long long ctas_per_chunk, int waves, Tiling& t,
-                       int ctas_per_sm = 2) {
+// Chunks along depth.  The starting point: enough CTAs for about `waves` rounds of `ctas_per_sm` CTAs
+// per SM, but chunks of at least 16*PD planes; only a grid that would not even fill the GPU once is
+// cut finer, down to 4*PD planes.  From there, the cut of least expected time, if that is 6 % less:
+// a CTA takes DC planes and `halo` planes' worth of work on its neighbours' (measured: 1.5 for the
+// adjoint sweeps, whose halo comes from L2; 3*PD for K; 2*PD for the fused forward), and SMs take CTAs
+// in rounds of `ctas_per_sm`, where k of them together need 0.4 + 0.6 k/ctas_per_sm of a full round
+// (a CTA alone waits for its own loads and barriers most of the time).  Measured against the starting
+// point, on sweeps of DC: ratio_kernel on 2 x 48 x 37x53x45 213 -> 180 us, on 5 x 24 images of 203x171
+// 121 -> 98; kconv_kernel on 3 x 32 of 128x120, 5x5, 119 -> 90; fwd_kernel on 4 x 72 of 128x120
+// 157 -> 113.
+inline void plan_depth(int KD, int D, long long ctas_per_chunk, int waves, Tiling& t, int ctas_per_sm, float halo) {
     if (KD == 1) {
         t.DC = 1;
     } else {
-        const int PD = KD / 2;
+        const int PD = KD / 2, sms = num_sms();
         const long long per = std::max(1LL, ctas_per_chunk);
-        const long long one_wave = (long long)ctas_per_sm * num_sms();
+        const long long one_wave = (long long)ctas_per_sm * sms;
         long long ndc = std::min(waves * one_wave / per, (long long)std::max(1, D / (16 * PD)));
         if (ndc * per < one_wave)
             ndc = std::min((one_wave + per - 1) / per, (long long)std::max(1, D / (4 * PD)));
         ndc = std::max(1LL, ndc);
+        auto time = [&](long long n) {
+            const long long planes = (D + n - 1) / n, ctas = (per * ((D + planes - 1) / planes) + sms - 1) / sms;
+            const long long rest = ctas % ctas_per_sm;
+            return ((float)planes + halo) * ((float)(ctas / ctas_per_sm) + (rest ? 0.4f + 0.6f * (float)rest / (float)ctas_per_sm : 0.0f));
+        };
+        float least = 0.94f * time(ndc);
+        const long long most = std::min(2 * ndc + 2, (long long)std::max(1, D / (2 * PD)));
+        for (long long n = std::max(1LL, ndc / 3), from = ndc; n <= most; ++n)
+            if (n != from && time(n) < least) { least = time(n); ndc = n; }
         t.DC = (int)((D + ndc - 1) / ndc);
     }
     t.ndc = (D + t.DC - 1) / t.DC;
@@ -85,7 +100,7 @@ inline bool plan_fwd(int D, int H, int W, long long BC, Tiling& t, size_t& smem_
     if (TH < 1 || bytes(TH) > kSmemMax || SCH * (TH + 4 * PH) * t.pitch > 65535) return false;
     t.nth = (H + TH - 1) / TH;
     t.TH = (H + t.nth - 1) / t.nth;
-    plan_depth(KD, D, BC * t.nth, 5, t, S::MINB);
+    plan_depth(KD, D, BC * t.nth, 5, t, S::MINB, 2.0f * (KD / 2));
     smem_bytes = bytes(t.TH);
     return true;
 }
@@ -203,7 +218,7 @@ inline bool plan_ring(int D, int H, int W, long long BC, int ntensors, int nt, i
         t.nth = best_nth;
     }
     t.TH = (H + t.nth - 1) / t.nth;
-    plan_depth(KD, D, BC * t.nth, 4, t, ctas_per_sm);
+    plan_depth(KD, D, BC * t.nth, 4, t, ctas_per_sm, 1.5f);
     smem_bytes = bytes(t.TH);
     return true;
 }
@@ -227,7 +242,7 @@ inline bool plan_kconv(int D, int H, int W, long long BC, Tiling& t, size_t& sme
     if (TH < 1 || bytes(TH) > kSmemMax) return false;
     t.nth = (H + TH - 1) / TH;
     t.TH = (H + t.nth - 1) / t.nth;
-    plan_depth(KD, D, 2 * BC * t.nth, 6, t, 384 / NT);
+    plan_depth(KD, D, 2 * BC * t.nth, 6, t, 384 / NT, 3.0f * (KD / 2));
     smem_bytes = bytes(t.TH);
     return true;
 }
@@ -261,7 +276,7 @@ inline bool plan_kconv2(int D, int H, int W, long long BC, Tiling& t, size_t& sm
     if (TH < 1 || bytes(TH) > target || chunks(TH) > MAXC * NT) return false;
     t.nth = (H + TH - 1) / TH;
     t.TH = (H + t.nth - 1) / t.nth;
-    plan_depth(KD, D, BC * t.nth, 6, t, per_sm);
+    plan_depth(KD, D, BC * t.nth, 6, t, per_sm, 3.0f * (KD / 2));
     smem_bytes = bytes(t.TH);
     return true;
 }
@@ -599,7 +614,7 @@ inline bool plan_ksrc(int D, int H, int W, long long BC, Tiling& t, size_t& smem
     if (TH < 1 || bytes(TH) > target) return false;
     t.nth = (H + TH - 1) / TH;
     t.TH = (H + t.nth - 1) / t.nth;
-    plan_depth(KD, D, BC * t.nth, 6, t, S::MINB);
+    plan_depth(KD, D, BC * t.nth, 6, t, S::MINB, 3.0f * (KD / 2));
     smem_bytes = bytes(t.TH);
     return true;
 }
