@@ -8,10 +8,17 @@ namespace tc {
 namespace {
 
 // Bands: as many rows as fill the 128 blocks of an MMA.  Chunks of planes: all of them, but for what
-// the accumulators hold (`most`) and for a grid that would leave multiprocessors idle; a chunk
-// stages KD - 1 planes of its neighbours.
+// the accumulators hold (`most`) and for a grid that would leave multiprocessors idle; from there,
+// the cut of least expected time, if that is 2 % less: the CTAs of the fullest multiprocessor times
+// a chunk's planes and `halo` more (its filling of the pipeline and its neighbours' planes).  The
+// adjoint's CTAs take turns on the tensor core, so two together need twice the time (halo 4 planes of
+// volumes, 12 of image rows; not for rows that are not whole 8-column blocks, which wait for their loads);
+// of the source's two, one alone needs 0.65 of their time (halo 7).  These figures fit sweeps of DC within
+// 10 %; against the starting point they took the adjoint of 16 x 64 images of 128^2 from 147 to 126 us, of
+// 12 x 128 of 60x64 from 68 to 41, and of 2 x 64 volumes of 64^3 from 201 to 188 (its ratio step 428 to 394).
 template <int KD, int KH, int KW>
-bool plan(const Geo& g, int most, Band& b) {
+bool plan(const Geo& g, bool source, Band& b) {
+    const int most = source ? source_planes<KD>() : g.D;
     b.C = g.G; b.D = g.D; b.H = g.H; b.W = g.W; b.Wv = g.Wv; b.Wo = g.Wo; b.eps = g.eps; b.relu = g.relu;
     b.NB = (g.Wv + 7) / 8;
     b.PB = (g.Wv + KW / 2 + 7) / 8;
@@ -26,7 +33,19 @@ bool plan(const Geo& g, int most, Band& b) {
     const long long per = (long long)g.B * g.G * b.nth;
     long long ndc = (g.D + most - 1) / most;
     const long long want = (4 * 148 + per - 1) / per, finest = std::max(1, g.D / (6 * (KD / 2)));
+    const long long fewest = ndc;
     ndc = std::max(ndc, std::min(want, finest));
+    if (source || (g.W % 8 == 0 && g.Wv == g.W)) {
+        const float halo = source ? 7.0f : KD > 3 ? 12.0f : 4.0f;
+        auto time = [&](long long n) {
+            const long long planes = (g.D + n - 1) / n, ctas = (per * ((g.D + planes - 1) / planes) + 147) / 148;
+            return ((float)planes + halo) * (source ? (float)(ctas / 2) + (ctas % 2 ? 0.65f : 0.0f) : (float)ctas);
+        };
+        float least = 0.98f * time(ndc);
+        const long long last = std::min(2 * ndc + 2, (long long)finest);
+        for (long long n = std::max(fewest, ndc / 6), from = ndc; n <= last; ++n)
+            if (n != from && time(n) < least) { least = time(n); ndc = n; }
+    }
     b.DC = (int)((g.D + ndc - 1) / ndc);
     b.ndc = (g.D + b.DC - 1) / b.DC;
     return true;
@@ -71,7 +90,7 @@ template <int KD, int KH, int KW>
 cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, const float* bias, bf16* out, bf16* t1, cudaStream_t st) {
     AdjointArgs A{};
     SourceArgs S{};
-    if (!plan<KD, KH, KW>(g, g.D, A.b) || !plan<KD, KH, KW>(g, source_planes<KD>(), S.b)) return cudaErrorInvalidConfiguration;
+    if (!plan<KD, KH, KW>(g, false, A.b) || !plan<KD, KH, KW>(g, true, S.b)) return cudaErrorInvalidConfiguration;
     A.x = x; A.t1 = t1; A.z = z; A.out = out; A.h = h; A.bias = bias;
     S.z = z; S.t1 = t1; S.h = h; S.bias = bias;
     const size_t ss = source_smem<KD, KH, KW>(S.b);
@@ -86,7 +105,7 @@ template <int KD, int KH, int KW>
 cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1, const float* h, const float* bias, const bf16* gout,
                       float* gnum, float* gden, bf16* direct, bool pairs, cudaStream_t st) {
     AdjointArgs A{};
-    if (!plan<KD, KH, KW>(g, g.D, A.b)) return cudaErrorInvalidConfiguration;
+    if (!plan<KD, KH, KW>(g, false, A.b)) return cudaErrorInvalidConfiguration;
     A.x = x; A.t1 = t1; A.z = z; A.out = direct; A.gout = gout; A.gnum = gnum; A.gden = gden; A.h = h; A.bias = bias;
     const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1) && on16(gout) && (!direct || on16(direct));
     if constexpr (KH == 1) {
@@ -103,7 +122,7 @@ cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1
 template <int KD, int KH, int KW>
 bool worth(const Geo& g) {
     Band a, s;
-    if (!plan<KD, KH, KW>(g, g.D, a) || !plan<KD, KH, KW>(g, source_planes<KD>(), s)) return false;
+    if (!plan<KD, KH, KW>(g, false, a) || !plan<KD, KH, KW>(g, true, s)) return false;
     const double voxels = (double)g.B * g.G * g.D * g.H * g.Wv, use = std::min(useful(a), useful(s));
     if (KH > 1) return voxels >= 0.8e6 && use >= 0.3;
     const bool tuned = KW == 3 && (g.W == 64 || g.W == 128 || g.W == 256);
