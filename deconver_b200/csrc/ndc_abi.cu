@@ -35,7 +35,7 @@ constexpr int kMaxTaps = 343;
 
 int validate(const NdcDesc* d) {
     if (!d) return fail(NDC_ERR_INVALID, "descriptor is NULL");
-    if (d->flags & ~(NDC_FLAG_FORCE_GENERIC | NDC_FLAG_BF16_PARAMS))
+    if (d->flags & ~(NDC_FLAG_FORCE_GENERIC | NDC_FLAG_BF16_PARAMS | NDC_FLAG_RELU_FILTER))
         return fail(NDC_ERR_INVALID, "descriptor.flags has unknown bits set (0x%x)", d->flags);
     if (d->batch <= 0 || d->groups <= 0 || d->m <= 0 || d->sc <= 0)
         return fail(NDC_ERR_INVALID, "batch, groups, m and sc must be positive (got %d, %d, %d, %d)",
@@ -93,7 +93,13 @@ int check_pitch(const NdcDesc* d, int pitch, int out_pitch) {
 }
 
 bool tensor_cores(const NdcDesc* d, const ndc::Geo& g) {
-    return d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && ndc::tc::covers(g);
+    return d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && !(d->flags & NDC_FLAG_RELU_FILTER) && ndc::tc::covers(g);
+}
+
+int raw_filter_refused(const NdcDesc* d) {
+    if (d->flags & NDC_FLAG_RELU_FILTER)
+        return fail(NDC_ERR_UNSUPPORTED, "NDC_FLAG_RELU_FILTER is for the depthwise forward only");
+    return NDC_OK;
 }
 
 int check_padded(std::initializer_list<const void*> tensors, int dtype) {
@@ -230,6 +236,7 @@ int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const vo
         if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (depthwise) launch");
         if (handled) return NDC_OK;
     }
+    NDC_TRY(raw_filter_refused(desc));
     if (tile_path(desc, g)) {
         if (desc->dtype == NDC_F32)
             e = ndc::tile::forward<float>(g, (const float*)x, (const float*)z, h, bias, (float*)out, (float*)t1, st);
@@ -275,6 +282,7 @@ int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const v
                  const void* t1, const float* h, const float* bias, const void* gout, void* gx, void* gz,
                  float* gh, float* gb, void* workspace, size_t workspace_bytes, void* stream) {
     NDC_TRY(validate(desc));
+    NDC_TRY(raw_filter_refused(desc));
     NDC_TRY(check_pitch(desc, pitch, gout_pitch));
     NDC_TRY(check_ptr(x, "x", desc->dtype));
     NDC_TRY(check_ptr(z, "z", desc->dtype));
@@ -412,6 +420,7 @@ int ndc_probe_fp32_fma(int32_t packed, int32_t iters, float* out, size_t out_ele
 int ndc_gconv(const NdcDesc* desc, const void* in, const float* h, const float* bias,
               int32_t adjoint, void* out, void* stream) {
     NDC_TRY(validate(desc));
+    NDC_TRY(raw_filter_refused(desc));
     NDC_TRY(check_ptr(in, "in", desc->dtype));
     NDC_TRY(check_ptr(h, "h", NDC_F32));
     NDC_TRY(check_ptr(out, "out", desc->dtype));

@@ -1,6 +1,8 @@
 // Shared device/host helpers of the NDC kernels (sm_100a).
 #pragma once
 
+#include <cmath>
+
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -35,7 +37,11 @@ struct Geo {
     float eps;
     int relu;      // rectify the source on load
     int has_bias;
+    float h_min;   // the filter's lower bound on load: 0 rectifies it, -infinity leaves it
 };
+
+// A filter value on load (NaN stays).
+__device__ __forceinline__ float filter_value(float h, float h_min) { return h < h_min ? h_min : h; }
 
 inline Geo make_geo(const NdcDesc& d, bool has_bias) {
     Geo g;
@@ -49,6 +55,7 @@ inline Geo make_geo(const NdcDesc& d, bool has_bias) {
     g.eps = d.eps;
     g.relu = d.relu_input ? 1 : 0;
     g.has_bias = has_bias ? 1 : 0;
+    g.h_min = d.flags & NDC_FLAG_RELU_FILTER ? 0.0f : -INFINITY;
     return g;
 }
 

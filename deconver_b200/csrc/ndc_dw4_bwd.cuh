@@ -56,6 +56,7 @@ struct RatioParams {
     float eps;
     int relu;
     int Wv, Wo;   // columns of the volume, row pitch of out / gout (see Geo)
+    float h_min;
 };
 
 // Deterministic per-CTA combine of per-thread accumulators: every thread writes its NACC values
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
     for (int i = tid; i < 2 * RING * lay.plane_t; i += NT) xring[i] = 0.0f;
     {
         const float* hc = P.h + (long long)c * SCH * KT;
-        for (int i = tid; i < KT * SCH; i += NT) wA[i] = hc[(i % SCH) * KT + i / SCH];  // [tau][j]
+        for (int i = tid; i < KT * SCH; i += NT) wA[i] = filter_value(hc[(i % SCH) * KT + i / SCH], P.h_min);  // [tau][j]
     }
     const int nx = RT * NQ;
     if (KD > 1) build_descs(desc, 1, RT, NQ, pitch, h0 - PH, H, W, SP, RWX, NT);

@@ -36,6 +36,7 @@ struct FwdParams {
     float eps;
     int relu;
     int Wv, Wo;   // columns of the volume, row pitch of out (see Geo)
+    float h_min;
 };
 
 template <int KD, int KH, int KW>
@@ -117,14 +118,14 @@ __global__ void __launch_bounds__(NT, MINB) fwd_kernel(const FwdParams P) {
         const float* hc = P.h + (long long)c * SCH * (KD * KH * KW);
         for (int i = tid; i < KD * KH * KW * SCH; i += NT) {
             const int j = i % SCH, tau = i / SCH;           // wA[tau][j]
-            wA[i] = hc[j * (KD * KH * KW) + tau];
+            wA[i] = filter_value(hc[j * (KD * KH * KW) + tau], P.h_min);
         }
         for (int i = tid; i < KH * SCH * WKP; i += NT) {    // wK[kh][j][kd*KW + kw]
             const int e = i % WKP, j = (i / WKP) % SCH, kh = i / (WKP * SCH);
             float v = 0.0f;
             if (e < KD * KW) {
                 const int kd = e / KW, kw = e % KW;
-                v = hc[j * (KD * KH * KW) + (kd * KH + kh) * KW + kw];
+                v = filter_value(hc[j * (KD * KH * KW) + (kd * KH + kh) * KW + kw], P.h_min);
             }
             wK[i] = v;
         }

@@ -132,7 +132,7 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
     if (!handled) return cudaSuccess;
     P.x = x; P.z = z; P.h = h; P.bias = bias; P.out = out; P.t1 = t1;
     P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W;
-    P.eps = g.eps; P.relu = g.relu; P.Wv = g.Wv; P.Wo = g.Wo;
+    P.eps = g.eps; P.relu = g.relu; P.Wv = g.Wv; P.Wo = g.Wo; P.h_min = g.h_min;
     const bool vec = g.W % 4 == 0 && aligned_for_vec(x, dtype) && aligned_for_vec(z, dtype) &&
                      (g.Wo != g.W || aligned_for_vec(out, dtype)) && aligned_for_vec(t1, dtype);
     const bool whole = vec && g.Wv == g.W && g.Wo == g.W;   // no padding: compile-time widths apply
@@ -432,7 +432,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.x = x; P.t1 = t1; P.z = z; P.gout = gout; P.h = h; P.bias = bias;
         P.gnum = gnum; P.gden = gden; P.gz = gz;
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.ratio; P.eps = g.eps; P.relu = g.relu;
-        P.Wv = g.Wv; P.Wo = g.Wo;
+        P.Wv = g.Wv; P.Wo = g.Wo; P.h_min = g.h_min;
         auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD>() ? kRatioPairs : kRatioPlanar>;
         NDC_CUDA_TRY(set_smem(kern, p.smem_ratio));
         kern<<<(unsigned)p.n_ratio, S::RatioNT, p.smem_ratio, st>>>(P);
@@ -666,7 +666,7 @@ cudaError_t forward_split(const Geo& g, const T* x, const T* z, const float* h, 
     // ---- K: the narrowest CTA that covers the volume with as few bands as the widest
     KsrcParams K;
     K.z = z; K.h = h; K.bias = bias; K.t1 = t1;
-    K.C = g.G; K.D = g.D; K.H = g.H; K.W = g.W; K.relu = g.relu; K.Wv = g.Wv;
+    K.C = g.G; K.D = g.D; K.H = g.H; K.W = g.W; K.relu = g.relu; K.Wv = g.Wv; K.h_min = g.h_min;
     Tiling t0, tk; size_t sm0 = 0, smk = 0;
     typedef KsrcShape<128, 3> K128; typedef KsrcShape<64, 6> K64; typedef KsrcShape<32, 12> K32;
     if (!plan_ksrc<KD, KH, KW, K128>(g.D, g.H, g.W, BC, t0, sm0)) return cudaSuccess;
@@ -674,7 +674,7 @@ cudaError_t forward_split(const Geo& g, const T* x, const T* z, const float* h, 
     RatioParams R;
     R.x = x; R.t1 = t1; R.z = z; R.gout = nullptr; R.h = h; R.bias = bias;
     R.gnum = nullptr; R.gden = nullptr; R.gz = out;
-    R.C = g.G; R.D = g.D; R.H = g.H; R.W = g.W; R.eps = g.eps; R.relu = g.relu; R.Wv = g.Wv; R.Wo = g.Wo;
+    R.C = g.G; R.D = g.D; R.H = g.H; R.W = g.W; R.eps = g.eps; R.relu = g.relu; R.Wv = g.Wv; R.Wo = g.Wo; R.h_min = g.h_min;
     Tiling r0; size_t smr0 = 0;
     if (!plan_ring<KD, KH, KW>(g.D, g.H, g.W, BC, 2, BwdBands::RatioNT, BwdBands::RatioMAXX, 0, 0,
                                56 * 1024, 512 / BwdBands::RatioNT, r0, smr0))

@@ -24,6 +24,7 @@ struct KsrcParams {
     Tiling t;
     int relu;
     int Wv;      // columns of the volume (< W: padded rows)
+    float h_min;
 };
 
 template <int KD, int KH, int KW>
@@ -88,8 +89,8 @@ __global__ void __launch_bounds__(NT, MINB) ksrc_kernel(const KsrcParams P) {
             float a = 0.0f, b = 0.0f;
             if (e < KD * KW) {
                 const int tap = ((e / KW) * KH + kh) * KW + e % KW;
-                a = hc[(2 * cp) * KT + tap];
-                b = hc[(2 * cp + 1) * KT + tap];
+                a = filter_value(hc[(2 * cp) * KT + tap], P.h_min);
+                b = filter_value(hc[(2 * cp + 1) * KT + tap], P.h_min);
             }
             wK[2 * i] = a; wK[2 * i + 1] = b;
         }

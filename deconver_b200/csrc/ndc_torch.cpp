@@ -212,7 +212,12 @@ Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Ten
     Saved& sv = saved ? *saved : local;
     Config c = config;
     c.bf16_params = bf16_params(h0, bias);
-    prepare_params(h0, bias, sv.h, sv.b);
+    // Without gradients float32 parameters need no pass of their own: the depthwise kernels rectify the
+    // filter on load (one launch of three less on a single small image).
+    bool raw = !saved && c.m == 1 && c.sc == 4 && h0.scalar_type() == at::kFloat &&
+               (!bias.defined() || bias.scalar_type() == at::kFloat) && !(c.flags & NDC_FLAG_FORCE_GENERIC);
+    if (raw) { sv.h = h0; sv.b = bias; }
+    else prepare_params(h0, bias, sv.h, sv.b);
     auto out_shape = x.sizes().vec();
     out_shape[1] = c.groups * c.sc;
     // Rows that are not whole vectors: the layer owns everything between its input and its output
@@ -244,10 +249,20 @@ Tensor run_forward(const Tensor& x, const Tensor& h0, const Tensor& w, const Ten
         Tensor out = at::empty(last ? out_shape : shape, x.options());
         if (keep || !t1.defined()) t1 = at::empty(sv.x.sizes(), x.options());
         if (x.numel()) {
-            const NdcDesc d = make_desc(x, h0, c, it == 0);
+            NdcDesc d = make_desc(x, h0, c, it == 0);
             Span span(0);
-            check(ndc_fwd_rows(&d, pitch, last ? W : pitch, ptr(sv.x), ptr(s), fptr(sv.h), it == 0 ? fptr(sv.b) : nullptr,
-                               ptr(out), ptr(t1), stream()), ndc_last_error());
+            auto update = [&](int flag) {
+                d.flags = (int)c.flags | (c.bf16_params ? NDC_FLAG_BF16_PARAMS : 0) | flag;
+                return ndc_fwd_rows(&d, pitch, last ? W : pitch, ptr(sv.x), ptr(s), fptr(sv.h), it == 0 ? fptr(sv.b) : nullptr,
+                                    ptr(out), ptr(t1), stream());
+            };
+            int status = update(raw ? NDC_FLAG_RELU_FILTER : 0);
+            if (raw && status == NDC_ERR_UNSUPPORTED) {   // not the depthwise kernels
+                raw = false;
+                prepare_params(h0, bias, sv.h, sv.b);
+                status = update(0);
+            }
+            check(status, ndc_last_error());
         }
         if (keep) { sv.z.push_back(s); sv.t1.push_back(t1); }
         s = out;

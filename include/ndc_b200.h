@@ -51,9 +51,12 @@ enum NdcStatus {
 
 enum NdcFlags {
     NDC_FLAG_FORCE_GENERIC = 1, /* run the generic kernels even where the tiled ones apply   */
-    NDC_FLAG_BF16_PARAMS = 2    /* the caller knows every value of h and bias to be a bfloat16
+    NDC_FLAG_BF16_PARAMS = 2,   /* the caller knows every value of h and bias to be a bfloat16
                                    value (as in a bfloat16 module): with NDC_BF16 tensors the
                                    forward then runs on the tensor cores                     */
+    NDC_FLAG_RELU_FILTER = 4    /* forward only: the kernels rectify h on load, so a layer can
+                                   hand in its raw filter.  NDC_ERR_UNSUPPORTED, and nothing is
+                                   launched, where the depthwise kernels do not apply        */
 };
 
 /* Which family of kernels a geometry runs on (informational; results are the same). */

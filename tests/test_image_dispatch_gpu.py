@@ -39,3 +39,15 @@ def test_image_kernels_match_the_generic_ones(case, dtype, tol):
         res.append([out.detach()] + [v.grad for v in t])
     for name, a, r in zip(("out", "gx", "gz", "gh", "gb"), res[1], res[0]):
         assert max_norm_error(a.float().cpu().numpy(), r.float().cpu().numpy()) < tol, name
+
+
+@pytest.mark.parametrize("k,spatial", [(5, (16, 16)), (5, (40, 128)), (3, (40, 171)), (3, (8, 8, 8)), (3, (9, 20, 33)), (7, (12, 12))])
+def test_inference_rectifies_the_filter_as_training_does(k, spatial):
+    torch.manual_seed(0)
+    net = dcb.Deconv(6, kernel_size=(k,) * len(spatial), ratio=4, groups=-1, num_iters=2).to("cuda:0")
+    with torch.no_grad():
+        net.init.h0.copy_(torch.randn_like(net.init.h0) / k)     # a filter of both signs
+    x = torch.rand(2, 6, *spatial, device="cuda:0")
+    with torch.no_grad():
+        y = net(x)
+    assert torch.equal(y, net(x).detach())
