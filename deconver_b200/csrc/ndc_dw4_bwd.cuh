@@ -18,6 +18,8 @@
 
 #include <type_traits>
 
+#include <type_traits>
+
 #include "ndc_dw4_common.cuh"
 
 namespace ndc {
@@ -56,8 +58,9 @@ struct RatioParams {
     float eps;
     int relu;
     int Wv, Wo;   // columns of the volume, row pitch of out / gout (see Geo)
-    float h_min;
 };
+// The forward's: one member more, apart because it cost the backward's kernel its last registers.
+struct RatioForwardParams : RatioParams { float h_min; };
 
 // Deterministic per-CTA combine of per-thread accumulators: every thread writes its NACC values
 // to a padded row of shared memory, then thread k sums column k over the threads in order.
@@ -85,7 +88,7 @@ __device__ __forceinline__ void cta_combine(float* scratch, const float (&acc)[N
 enum RatioMode { kRatioPlanar = 0, kRatioPairs = 1, kRatioForward = 2 };
 
 template <typename T, int KD, int KH, int KW, int NT, int MAXX, int AL, int WQ, int MODE = kRatioPlanar>
-__global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P) {
+__global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const std::conditional_t<MODE == kRatioForward, RatioForwardParams, RatioParams> P) {
     constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr bool PAIRS = MODE == kRatioPairs, FWD = MODE == kRatioForward;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
@@ -135,7 +138,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) ratio_kernel(const RatioParams P
     for (int i = tid; i < 2 * RING * lay.plane_t; i += NT) xring[i] = 0.0f;
     {
         const float* hc = P.h + (long long)c * SCH * KT;
-        for (int i = tid; i < KT * SCH; i += NT) wA[i] = filter_value(hc[(i % SCH) * KT + i / SCH], P.h_min);  // [tau][j]
+        for (int i = tid; i < KT * SCH; i += NT) {                                       // [tau][j]
+            const float v = hc[(i % SCH) * KT + i / SCH];
+            if constexpr (FWD) wA[i] = filter_value(v, P.h_min);
+            else wA[i] = v;
+        }
     }
     const int nx = RT * NQ;
     if (KD > 1) build_descs(desc, 1, RT, NQ, pitch, h0 - PH, H, W, SP, RWX, NT);

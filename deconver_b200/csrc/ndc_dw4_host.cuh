@@ -432,7 +432,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.x = x; P.t1 = t1; P.z = z; P.gout = gout; P.h = h; P.bias = bias;
         P.gnum = gnum; P.gden = gden; P.gz = gz;
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.ratio; P.eps = g.eps; P.relu = g.relu;
-        P.Wv = g.Wv; P.Wo = g.Wo; P.h_min = g.h_min;
+        P.Wv = g.Wv; P.Wo = g.Wo;
         auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD>() ? kRatioPairs : kRatioPlanar>;
         NDC_CUDA_TRY(set_smem(kern, p.smem_ratio));
         kern<<<(unsigned)p.n_ratio, S::RatioNT, p.smem_ratio, st>>>(P);
@@ -638,7 +638,7 @@ cudaError_t launch_ksrc(const KsrcParams& P, size_t smem_bytes, long long BC, bo
 }
 
 template <typename T, int KD, int KH, int KW, typename S>
-cudaError_t launch_ratio_forward(const RatioParams& P, size_t smem_bytes, long long n_ctas, bool vec,
+cudaError_t launch_ratio_forward(const RatioForwardParams& P, size_t smem_bytes, long long n_ctas, bool vec,
                                  cudaStream_t st) {
     if (n_ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     auto go = [&](auto kern) -> cudaError_t {
@@ -671,7 +671,7 @@ cudaError_t forward_split(const Geo& g, const T* x, const T* z, const float* h, 
     typedef KsrcShape<128, 3> K128; typedef KsrcShape<64, 6> K64; typedef KsrcShape<32, 12> K32;
     if (!plan_ksrc<KD, KH, KW, K128>(g.D, g.H, g.W, BC, t0, sm0)) return cudaSuccess;
     // ---- A: the same classes as the backward's ratio kernel
-    RatioParams R;
+    RatioForwardParams R;
     R.x = x; R.t1 = t1; R.z = z; R.gout = nullptr; R.h = h; R.bias = bias;
     R.gnum = nullptr; R.gden = nullptr; R.gz = out;
     R.C = g.G; R.D = g.D; R.H = g.H; R.W = g.W; R.eps = g.eps; R.relu = g.relu; R.Wv = g.Wv; R.Wo = g.Wo; R.h_min = g.h_min;
