@@ -9,6 +9,7 @@ kernels as two, next to the ABI unit and those of the instance norm, the bias pa
 and the tensor-core kernels, in parallel, then linked.  Run as `python -m deconver_b200._build [--force]`.
 """
 
+import importlib.metadata
 import os
 import subprocess
 import sys
@@ -22,6 +23,7 @@ INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(PKG, "libndc_b200.so")
 EXT = os.path.join(PKG, "_ndc_torch.so")
 EXT_SRC = os.path.join(CSRC, "ndc_torch.cpp")
+EXT_KEY = os.path.join(PKG, "_ndc_torch.key")     # what the extension was built for; travels with it
 OBJ = os.path.join(PKG, "_obj")
 
 NVCC_FLAGS = [
@@ -58,8 +60,23 @@ def is_stale():
     return _older(LIB, sources())
 
 
+def ext_target():
+    """The PyTorch and Python that an extension built now is for: it uses their C++ interfaces, which
+    hold for one version only."""
+    return "torch %s, %s" % (importlib.metadata.version("torch"), sys.implementation.cache_tag)
+
+
+def ext_built_for():
+    """The same of the extension that is there; None where that was not written down."""
+    try:
+        with open(EXT_KEY) as f:
+            return f.read().strip()
+    except FileNotFoundError:
+        return None
+
+
 def ext_is_stale():
-    return _older(EXT, [EXT_SRC, os.path.join(INCLUDE, "ndc_b200.h")])
+    return _older(EXT, [EXT_SRC, os.path.join(INCLUDE, "ndc_b200.h")]) or ext_built_for() != ext_target()
 
 
 def _compile_ext():
@@ -80,7 +97,8 @@ def _compile_ext():
 
 
 def build_library(force=False, verbose=False, extra_flags=()):
-    """Build the shared library and the host extension if missing or older than a source file."""
+    """Build the shared library and the host extension if missing or older than a source file; the
+    extension also where it was built for another PyTorch or Python."""
     if not (force or is_stale() or ext_is_stale()):
         return LIB
     os.makedirs(OBJ, exist_ok=True)
@@ -97,6 +115,8 @@ def build_library(force=False, verbose=False, extra_flags=()):
             if verbose:
                 print(" ".join(link), flush=True)
             subprocess.check_call(link, cwd=ROOT)
+            with open(EXT_KEY, "w") as f:
+                f.write(ext_target() + "\n")
     return LIB
 
 

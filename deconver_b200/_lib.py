@@ -8,7 +8,7 @@ import ctypes
 import importlib.util
 import os
 
-from ._build import EXT, LIB
+from ._build import EXT, LIB, ext_built_for, ext_target
 
 NDC_F32, NDC_BF16 = 0, 1
 NDC_OK = 0
@@ -144,6 +144,9 @@ def load_ext():
     if _ext is None:
         if not os.path.exists(EXT):
             raise RuntimeError(f"{EXT} has not been built; run `python -m deconver_b200._build`.")
+        if ext_built_for() not in (None, ext_target()):
+            raise RuntimeError(f"{EXT} was built for {ext_built_for()}, this is {ext_target()}; "
+                               "run `python -m deconver_b200._build`.")
         load()
         spec = importlib.util.spec_from_file_location("_ndc_torch", EXT)
         module = importlib.util.module_from_spec(spec)

@@ -9,6 +9,7 @@ import torch
 
 import deconver_b200 as dcb
 from conftest import load_golden
+from deconver_b200 import _build, _lib
 from deconver_b200._build import build_library
 
 
@@ -169,3 +170,12 @@ def test_linear_and_mlp_keep_the_reference_state_dict_layout():
         ref.load_state_dict(mine.state_dict(), strict=True)
         inp = x[next(iter(ref_sd.values())).shape[1]]
         assert torch.allclose(ref(inp), mine(inp), atol=1e-6)     # CPU tensors: the plain sequence
+
+
+def test_the_extension_is_rebuilt_for_another_pytorch(monkeypatch):
+    assert not _build.ext_is_stale() and _build.ext_built_for() == _build.ext_target()
+    monkeypatch.setattr(_build.importlib.metadata, "version", lambda name: "0.0.0")
+    assert _build.ext_is_stale()
+    monkeypatch.setattr(_lib, "_ext", None)
+    with pytest.raises(RuntimeError, match="was built for"):      # and not a failure of the dynamic linker
+        _lib.load_ext()
