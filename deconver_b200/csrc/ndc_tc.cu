@@ -7,21 +7,20 @@ namespace ndc {
 namespace tc {
 namespace {
 
-// Bands: as many rows as fill the 128 blocks of an MMA.  Chunks of planes: all of them, but for what
-// the accumulators hold (`most`) and for a grid that would leave multiprocessors idle; from there,
-// the cut of least expected time, if that is 2 % less: the CTAs of the fullest multiprocessor times
-// a chunk's planes and `halo` more (its filling of the pipeline and its neighbours' planes).  The
-// adjoint's CTAs take turns on the tensor core, so two together need twice the time (halo 4 planes of
-// volumes, 12 of image rows; not for rows that are not whole 8-column blocks, which wait for their loads);
-// of the source's two, one alone needs 0.65 of their time (halo 7).  These figures fit sweeps of DC within
-// 10 %; against the starting point they took the adjoint of 16 x 64 images of 128^2 from 147 to 126 us, of
-// 12 x 128 of 60x64 from 68 to 41, and of 2 x 64 volumes of 64^3 from 201 to 188 (its ratio step 428 to 394).
+// Bands: as many rows as fill the 128 blocks of an MMA.  Chunks of planes: all of them, but for a grid that
+// would leave multiprocessors idle; from there, the cut of least expected time, if that is 2 % less: the
+// CTAs of the fullest multiprocessor times a chunk's planes and `halo` more (its filling of the pipeline and
+// its neighbours' planes).  The adjoint's CTAs take turns on the tensor core, so two together need twice the
+// time (halo 4 planes of volumes, 12 of image rows; not for rows that are not whole 8-column blocks, which
+// wait for their loads); of the source's two, one alone needs 0.65 of their time (halo 7).  The adjoint's figures
+// fit sweeps of DC within 10 %; against the starting point they took the adjoint of 16 x 64 images of 128^2
+// from 147 to 126 us, of 12 x 128 of 60x64 from 68 to 41, and of 2 x 64 volumes of 64^3 from 201 to 188 (its
+// ratio step 428 to 394).  The source's choose a cut within 2 % of the best of ten on each of twelve shapes.
 template <int KD, int KH, int KW>
 bool plan(const Geo& g, bool source, Band& b) {
-    const int most = source ? source_planes<KD>() : g.D;
     b.C = g.G; b.D = g.D; b.H = g.H; b.W = g.W; b.Wv = g.Wv; b.Wo = g.Wo; b.eps = g.eps; b.relu = g.relu;
     b.NB = (g.Wv + 7) / 8;
-    b.PB = (g.Wv + KW / 2 + 7) / 8;
+    b.PB = source ? b.NB : (g.Wv + KW / 2 + 7) / 8;
     b.TH = std::min(g.H, std::min(MB / b.PB, kSourceStagers / b.PB - (KH - 1)));
     if (b.TH < 1) return false;
     b.nth = (g.H + b.TH - 1) / b.TH;
@@ -31,9 +30,8 @@ bool plan(const Geo& g, bool source, Band& b) {
     const long long row = KH == 1 ? (long long)g.D * g.W * g.G * SC : g.W;
     if ((b.TH + KH - 1) * row >= (1LL << 31)) return false;
     const long long per = (long long)g.B * g.G * b.nth;
-    long long ndc = (g.D + most - 1) / most;
+    long long ndc = 1;
     const long long want = (4 * 148 + per - 1) / per, finest = std::max(1, g.D / (6 * (KD / 2)));
-    const long long fewest = ndc;
     ndc = std::max(ndc, std::min(want, finest));
     if (source || (g.W % 8 == 0 && g.Wv == g.W)) {
         const float halo = source ? 7.0f : KD > 3 ? 12.0f : 4.0f;
@@ -43,7 +41,7 @@ bool plan(const Geo& g, bool source, Band& b) {
         };
         float least = 0.98f * time(ndc);
         const long long last = std::min(2 * ndc + 2, (long long)finest);
-        for (long long n = std::max(fewest, ndc / 6), from = ndc; n <= last; ++n)
+        for (long long n = std::max(1LL, ndc / 6), from = ndc; n <= last; ++n)
             if (n != from && time(n) < least) { least = time(n); ndc = n; }
     }
     b.DC = (int)((g.D + ndc - 1) / ndc);
@@ -58,10 +56,7 @@ template <int KD, int KH, int KW> size_t adjoint_smem(const Band& b) {
     return kHeader + (size_t)KH * KD * SC * 8 * 32 + 16 * ((size_t)kSlots * 2 * (b.TH + KH - 1) * b.PB + slack_blocks(b));
 }
 template <int KD, int KH, int KW> size_t source_smem(const Band& b) {
-    constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2;
-    return kHeader + ((PD + 1) * (PD + 1) * (PH + 1) * (PH + 1) * (PW + 1) * (PW + 1) * 4 + 127) / 128 * 128 +
-           (size_t)SC * KH * 8 * source_groups<KD>() * 32 +
-           16 * ((size_t)kSlots * SC * (b.TH + KH - 1) * b.PB + slack_blocks(b));
+    return kHeader + (size_t)SC * KH * KD * kGroup * 32 + 16 * ((size_t)kSourceSlots * 2 * SC * (b.TH + KH - 1) * b.NB + slack_blocks(b));
 }
 
 template <typename K, typename P>

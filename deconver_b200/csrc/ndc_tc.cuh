@@ -4,28 +4,35 @@
 // the ratio step of the backward too (gnum, gden and the direct term, see AdjointMode).
 //
 // A depthwise convolution as a matrix product.  Rows of a plane lie in shared memory one after the
-// other as bfloat16, column w at place w + PW of its row, zeros between the rows; a row takes a whole
-// number PB of 8-column blocks.  The MMA's A operand is not a copy of that: its row r is the window
-// of 16 places that starts at block r, and in the K-major layout without swizzle (8-row groups of
-// 16-byte rows) this is the memory as it lies, with 16 bytes between the two halves of the window
-// and 128 bytes between groups of eight blocks.  A filter row kh is a shift of the start address.  The
-// B operand is a banded matrix: window place k, output column o of the block,
+// other as bfloat16, in blocks of 8 columns; one M = 128, K = 16 MMA multiplies 128 blocks of a source plane
+// (1024 voxels) by one filter row of every depth tap, laid out as banded matrices side by side, onto the
+// accumulators of KD output planes, which lie next to each other in TMEM.  So a source plane is read
+// once, when the CTA's march through the depth comes to it, and a filter row kh is a shift of the start
+// address.  Batches of images march down their rows the same way (planes = image rows, plane rows =
+// images, KH = 1: see SlabAddr).  An MMA of up to 128 columns takes 64 cycles here, whatever its width
+// (reading 4 KB of A operand), hence the wide ones.  With KW = 3 most of the products meet a zero of the
+// band; the tensor cores do them 30 times faster than the FMA pipe does the useful ones.  What K = 16
+// holds differs:
 //
-//     A: B[k][8 j + o] = h[j][kd][kh][o + 2 PW - k]        K: B[k][o] = h[j][kd][kh][k - o]
+//   A (tc_adjoint_kernel): the window of 16 places that starts at a block, column w at place w + PW of
+//     its row, zeros between the rows.  No copy of that is made: in the K-major layout without
+//     swizzle (8-row groups of 16-byte rows) it is the memory as it lies, with 16 bytes between the two halves
+//     of the window and 128 bytes between groups of eight blocks; a row takes a whole number PB of blocks.
+//     Window place k, output column o of the block:     B[k][8 j + o] = h[j][kd][kh][o + 2 PW - k]
 //
-// with the matrices of the KD depth taps side by side: one M = 128, K = 16 MMA multiplies 1024 voxels
-// of a source plane by one filter row of every depth tap, onto the accumulators of KD output
-// planes, which lie next to each other in TMEM.  So a source plane is read once, when the CTA's march
-// through the depth comes to it.  Batches of images march down their rows the same way (planes = image
-// rows, plane rows = images, KH = 1: see SlabAddr).  An MMA of up to 128 columns takes 64 cycles here,
-// whatever its width (reading 4 KB of A operand), hence the wide ones.  With KW = 3 a third of the products
-// meet a zero of the band; the tensor cores do them 30 times faster than the FMA pipe does the useful
-// ones.
+//   K (tc_source_kernel): the source of a block as the sum of two bfloat16 terms, eight places each (next
+//     paragraph).  There is no room for the neighbouring columns, so the band is wider instead: a
+//     block gives 8 columns of its own and PW of either neighbour's, which the epilogue adds.
+//     Place k of either term, output column o = -PW .. 7 + PW:      B[k][o] = h[j][kd][kh][k - o + PW]
 //
 // Precision: every product is one of two bfloat16 values, exact in float32, accumulated in float32:
-// what the FMA kernels compute, in another order.  The source relu(z + b) is not a bfloat16 value, but
-// relu(z + b) = max(z, -b) + b and max(z, -b) is one; b K(1) is added in float32 afterwards, from a
-// table over which filter taps lie inside the volume.
+// what the FMA kernels compute, in another order.  The source s = relu(z + b) is not a bfloat16 value, but
+// with L = 1 where z + b > 0, else 0, s = L z + L b, two of them; where everything is rectified away
+// both are zero and t1 is zero, as it is with the FMA kernels, and of nearly equal z and -b the
+// products meet in one MMA.  (max(z, -b) and a table of b K(1) would be one term, but leave the rounding of
+// sums that cancel: with 2 % of the sources positive t1 was off by up to 6.6 times its value, and where
+// everything is rectified away it was a residue of either sign.  As it is, t1 is off by 2^-8 of itself at
+// most, its rounding to bfloat16, like the FMA kernels'.)
 #pragma once
 
 #include <algorithm>
@@ -86,15 +93,8 @@ __device__ __forceinline__ void mma(unsigned d, unsigned long long a, unsigned l
 __device__ __forceinline__ void mma_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Eight columns of this thread's lane; the wait is part of the statement, so that nothing that uses
-// the values can move in between.
-__device__ __forceinline__ void tmem_load8(unsigned addr, float (&v)[8]) {
-    unsigned r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr) : "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
+// Eight columns each of two accumulators of this thread's lane; the wait is part of the statement, so that
+// nothing that uses the values can move in between.
 __device__ __forceinline__ void tmem_load8x2(unsigned addr_a, unsigned addr_b, float (&a)[8], float (&b)[8]) {
     unsigned r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
@@ -104,6 +104,27 @@ __device__ __forceinline__ void tmem_load8x2(unsigned addr_a, unsigned addr_b, f
                  : "r"(addr_a), "r"(addr_b) : "memory");
 #pragma unroll
     for (int i = 0; i < 8; ++i) { a[i] = __uint_as_float(r[i]); b[i] = __uint_as_float(r[8 + i]); }
+}
+// Eight columns, and the N that follow them.
+template <int N>
+__device__ __forceinline__ void tmem_load_group(unsigned addr, float (&v)[8], float (&n)[N]) {
+    static_assert(N == 2 || N == 4, "columns");
+    unsigned r[8], e[4];
+    if (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%10];\n\t"
+                     "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%8,%9}, [%11];\n\ttcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(e[0]), "=r"(e[1])
+                     : "r"(addr), "r"(addr + 8) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%12];\n\t"
+                     "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%13];\n\ttcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(e[0]), "=r"(e[1]),
+                       "=r"(e[2]), "=r"(e[3])
+                     : "r"(addr), "r"(addr + 8) : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) n[i] = __uint_as_float(e[i]);
 }
 // `n` columns (a multiple of 8) of this thread's lane; eight at a time, since every column takes a register
 __device__ __forceinline__ void tmem_fill(unsigned addr, float v, int n) {
@@ -141,6 +162,7 @@ template <int KD> struct AdjointShape {
     static constexpr int THREADS = 32 * (4 * EPI + 2 * GROUPS + 1), CTAS = KD > 3 ? 1 : 2;
 };
 constexpr int kSlots = 8;         // staged planes
+constexpr int kSourceSlots = 4;   // of the source kernel, which stages two terms of four channels
 constexpr int kHeader = 1024;     // bytes: barriers and the TMEM address (512), the filter as float32
 
 // Place of a CTA: (sample, channel), band of rows, chunk of planes; all addresses in elements.
@@ -173,41 +195,40 @@ __device__ __forceinline__ void load_words(const bf16* p, unsigned off, int w, i
     }
 }
 // The eight places of block q of a shared row (columns 8 q - PW .. 8 q + 7 - PW) from those words.
-// SOURCE: max(value, -bias) inside the volume (`negb`: two copies of -bias), zero outside: with RELU, z is
-// zero there, and so is max(0, 0).  `inside`: with whole blocks (WIDE) bits 0 and 1 for the first word and the
-// others, else two bits per word, one per column.
-template <int PW, bool SOURCE, bool WIDE>
-__device__ __forceinline__ uint4 to_places(unsigned (&a)[5], unsigned inside, unsigned negb, bool relu) {
-    if (SOURCE) {
-#pragma unroll
-        for (int i = 0; i < 5; ++i) {
-            unsigned m;
-            if (WIDE) {
-                m = inside & (i ? 2u : 1u) ? 0xffffffffu : 0u;
-            } else {
-                // byte 0 or 1 of 0xff00, twice per column
-                const unsigned two = inside >> (2 * i);
-                m = __byte_perm(0xff00u, 0u, (two & 1u) * 0x0011u + (two & 2u) * 0x0880u);
-            }
-            if (relu) {
-                const unsigned nb = negb & m;
-                const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a[i]), *reinterpret_cast<const __nv_bfloat162*>(&nb));
-                a[i] = *reinterpret_cast<const unsigned*>(&v);
-            } else {
-                a[i] &= m;
-            }
-        }
-    }
+template <int PW>
+__device__ __forceinline__ uint4 to_places(const unsigned (&a)[5]) {
     if (PW == 2) return make_uint4(a[0], a[1], a[2], a[3]);
     return make_uint4(__funnelshift_l(a[0], a[1], 16), __funnelshift_l(a[1], a[2], 16), __funnelshift_l(a[2], a[3], 16),
                       __funnelshift_l(a[3], a[4], 16));
+}
+
+// A group's planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are passed
+// on without data.  `S`: load, prefetch and store a plane.
+template <int SLOTS, int GROUPS, typename S, typename F>
+__device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int PD, int planes, unsigned full, unsigned empty, int group,
+                                             int lane) {
+    const int first = max(0, PD - d0), last = min(planes - 1, D - 1 + PD - d0);   // those inside
+    if (group >= first && group <= last) st.load(d0 - PD + group);
+    for (int p = group; p < planes; p += GROUPS) {
+        const int s = p % SLOTS;
+        if (p >= SLOTS && !mbar_wait(empty + 8 * s, (p / SLOTS - 1) & 1)) return false;
+        if (p >= first && p <= last) {
+            store(s);
+            fence_async_proxy();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8 * s);
+        if (p + GROUPS >= first && p + GROUPS <= last) st.load(d0 - PD + p + GROUPS);
+        if (p + 2 * GROUPS <= last) st.prefetch(d0 - PD + p + 2 * GROUPS);
+    }
+    return true;
 }
 
 // Stages planes of NCH channels (`src + ch * stride`), halo rows included; rows outside the volume are
 // zero.  A thread of a group of NTHR has up to U blocks of a plane, and the loads of its group's next plane
 // are on their way in registers while it waits for a slot; the lines of the one after are asked for
 // from L2.  Addresses are a base that is the same for the whole CTA and a 32-bit offset.
-template <int KH, int KW, int NCH, bool SOURCE, bool WIDE, int NTHR, int U, int GROUPS>
+template <int KH, int KW, int NCH, bool WIDE, int NTHR, int U>
 struct Stager {
     const Band& b;
     const bf16* src;               // row h0 - KH / 2 of plane 0
@@ -216,7 +237,6 @@ struct Stager {
     unsigned off[U];               // this thread's blocks: offset of the first column
     bool in[U];                    // inside the volume (else zero)
     int w[U], at[U];               // column; block, or -1
-    unsigned inside[U];
     unsigned a[U][NCH][5];
 
     __device__ __forceinline__ Stager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, int h0,
@@ -229,16 +249,6 @@ struct Stager {
             w[u] = 8 * q;
             off[u] = (unsigned)(row * row_stride) + w[u];
             in[u] = i < blocks && h >= 0 && h < b.H;
-            inside[u] = 0u;
-            if (WIDE) {
-                inside[u] = (w[u] > 0 ? 1u : 0u) | (w[u] < b.Wv ? 2u : 0u);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 10; ++k) {
-                    const int c = w[u] - 2 + k;
-                    if (c >= 0 && c < b.Wv) inside[u] |= 1u << k;
-                }
-            }
         }
     }
     __device__ __forceinline__ void load(int d) {
@@ -260,40 +270,19 @@ struct Stager {
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off[u]));
             }
     }
-    __device__ __forceinline__ void store(uint4* dst, const unsigned (&negb)[NCH], bool relu) {
+    __device__ __forceinline__ void store(uint4* dst) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (at[u] < 0) continue;
 #pragma unroll
             for (int ch = 0; ch < NCH; ++ch)
-                dst[ch * blocks + at[u]] = in[u] ? to_places<KW / 2, SOURCE, WIDE>(a[u][ch], inside[u], negb[ch], relu)
-                                                 : make_uint4(0u, 0u, 0u, 0u);
+                dst[ch * blocks + at[u]] = in[u] ? to_places<KW / 2>(a[u][ch]) : make_uint4(0u, 0u, 0u, 0u);
         }
-    }
-    // This group's planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are
-    // passed on without data.
-    __device__ __forceinline__ bool run(uint4* slots, int slot_blocks, int d0, int PD, int planes, unsigned full, unsigned empty,
-                                        const unsigned (&negb)[NCH], bool relu, int group, int lane) {
-        const int first = max(0, PD - d0), last = min(planes - 1, b.D - 1 + PD - d0);   // those inside
-        if (group >= first && group <= last) load(d0 - PD + group);
-        for (int p = group; p < planes; p += GROUPS) {
-            const int s = p % kSlots;
-            if (p >= kSlots && !mbar_wait(empty + 8 * s, (p / kSlots - 1) & 1)) return false;
-            if (p >= first && p <= last) {
-                store(slots + s * slot_blocks, negb, relu);
-                fence_async_proxy();
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(full + 8 * s);
-            if (p + GROUPS >= first && p + GROUPS <= last) load(d0 - PD + p + GROUPS);
-            if (p + 2 * GROUPS <= last) prefetch(d0 - PD + p + 2 * GROUPS);
-        }
-        return true;
     }
 };
 
 // Blocks an MMA may read past the last staged row of a slot's last channel: 128 windows of two blocks
-// from the band's first row on.
+// from the band's first row on (the source kernel: of one).
 __host__ __device__ inline int slack_blocks(const Band& b) { return MB + 1 - b.TH * b.PB > 1 ? MB + 1 - b.TH * b.PB : 1; }
 
 // ---- two-lane float32 -------------------------------------------------------------------------
@@ -317,22 +306,16 @@ __device__ __forceinline__ float rcp(float v) {
 }
 __device__ __forceinline__ unsigned word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }  // i static
 
-// The banded matrices of a kernel: `value(t, n, kw)` is the filter tap of matrix t, column n.
+// The banded matrices of a kernel: `value(t, n, k)` is what place k of matrix t, column n is multiplied by.
 // Layout of one matrix: groups of eight columns, then the two halves of K, eight 16-byte rows each.
-template <int NCOL, int KW, bool ADJ, typename F>
+template <int NCOL, typename F>
 __device__ __forceinline__ void build_bands(bf16* bmat, int mats, F value) {
     for (int e = threadIdx.x; e < mats * NCOL * 2; e += blockDim.x) {
         const int n = e % 8, half = (e / 8) % 2, g = (e / 16) % (NCOL / 8), t = e / (2 * NCOL);
         unsigned words[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            float v[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int k = 8 * half + 2 * i + u, kw = ADJ ? n + KW - 1 - k : k - n;
-                v[u] = kw >= 0 && kw < KW ? value(t, 8 * g + n, kw) : 0.0f;
-            }
-            const __nv_bfloat162 p = __floats2bfloat162_rn(v[0], v[1]);
+            const __nv_bfloat162 p = __floats2bfloat162_rn(value(t, 8 * g + n, 8 * half + 2 * i), value(t, 8 * g + n, 8 * half + 2 * i + 1));
             words[i] = *reinterpret_cast<const unsigned*>(&p);
         }
         reinterpret_cast<uint4*>(bmat)[e] = make_uint4(words[0], words[1], words[2], words[3]);
@@ -424,9 +407,9 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
     for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)at.c * SC * KT + e];
     __syncthreads();
     // [kh][output plane p - (KD - 1) + kd: groups of 32 columns][channel, column]
-    build_bands<KD * NC, KW, true>(bmat, KH, [&](int kh, int n, int kw) {
-        const int kd = n / NC, j = n % NC / 8;
-        return hs[j * KT + (kd * KH + kh) * KW + kw];
+    build_bands<KD * NC>(bmat, KH, [&](int kh, int n, int k) {
+        const int kd = n / NC, j = n % NC / 8, kw = n % 8 + KW - 1 - k;
+        return kw >= 0 && kw < KW ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
     });
     fence_async_proxy();
     tc_fence_before();
@@ -473,12 +456,12 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
             __syncwarp();
         }
     } else if (warp >= kEpilogueWarps) {
-        const unsigned none[2] = {0u, 0u};
         // x and t1 as two channels: the distance between the tensors takes the place of the stride
         const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
-        Stager<KH, KW, 2, false, AL == kWide, Shape::STAGERS, Shape::BLOCKS, Shape::GROUPS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at.h0,
-                                                 (tid - 32 * kEpilogueWarps) % Shape::STAGERS);
-        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, none, false, (tid - 32 * kEpilogueWarps) / Shape::STAGERS, lane);
+        Stager<KH, KW, 2, AL == kWide, Shape::STAGERS, Shape::BLOCKS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x,
+                                                                         at.h0, (tid - 32 * kEpilogueWarps) % Shape::STAGERS);
+        ok = stage_planes<kSlots, Shape::GROUPS>(st, [&](int s) { st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, planes, sfull, sempty,
+                                                 (tid - 32 * kEpilogueWarps) / Shape::STAGERS, lane);
     } else {
         const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q;
         const bool valid = r < at.TH && q < b.NB;
@@ -611,70 +594,118 @@ struct SourceArgs {
     const float* h; const float* bias;
 };
 
-// Accumulators: 8 columns per output plane of the chunk.  A source plane is multiplied once per
-// (channel, kh), by the matrices of all depth taps at once: 12 MMAs of a 3x3x3 filter, 4 of an image
-// filter.  N is a multiple of 16, so an odd number of taps is padded by columns of zeros.
-template <int KD> __host__ __device__ constexpr int source_groups() { return (KD + 1) / 2 * 2; }
-constexpr int kSourceCols = 256;
-// planes of a chunk whose accumulators (and those of the taps that fall outside it) fit
-template <int KD> __host__ __device__ constexpr int source_planes() { return kSourceCols / 8 - KD + 2 - source_groups<KD>(); }
+// Accumulators: 16 columns per output plane, of which the block's own eight, PW of the left and PW of the
+// right neighbour's; all 256 make a ring of P planes and KD - 1 more.  A source plane is multiplied once
+// per (channel, kh), by the matrices of all depth taps at once: 12 MMAs of 48 columns for a 3x3x3 filter, 4 of
+// 48 or 80 for an image filter.  Plane p of the march starts at ring place p % P and runs on over the
+// ring's end, so that no MMA is split there: the sums of an output plane at one of the first KD - 1 places
+// are then in two parts, P places apart, which the epilogue adds.
+//
+// What bounds the kernel is the issue of these MMAs: 12 x 64 cycles a plane and band, 1.38 ms at
+// 4 x 64 x 128^3.  A block of places for each of two terms takes as many of them as a window of one
+// term, and rows without zeros between them fill the 128 blocks better (16 rows of 64 columns, not 14), so
+// that the exact form is the faster one too: the forward 4.66 -> 3.95 ms there, 368 -> 316 us at 2 x 64 x 64^3,
+// 228 -> 181 on 16 x 64 images of 128^2, 5x5 (one term, chunks of up to 27 planes: before).
+constexpr int kSourceCols = 256, kGroup = 16;
+template <int KD> __host__ __device__ constexpr int source_ring() { return kSourceCols / kGroup - (KD - 1); }
+
+// Stages the two terms of the source: per channel the blocks of L z, then those of L b.  A thread has one
+// block of a plane; see Stager.
+template <int KH, bool WIDE>
+struct SourceStager {
+    const Band& b;
+    const bf16* src;
+    long long stride, plane;
+    int blocks;
+    unsigned off;
+    bool in;
+    int w, at;
+    uint4 a[SC];
+
+    __device__ __forceinline__ SourceStager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, int h0,
+                                            int i)
+        : b(b_), src(src_ + (h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.NB) {
+        const int row = i / b.NB, h = h0 - KH / 2 + row;
+        at = i < blocks ? i : -1;
+        w = 8 * (i - row * b.NB);
+        off = (unsigned)(row * row_stride) + w;
+        in = i < blocks && h >= 0 && h < b.H;
+    }
+    __device__ __forceinline__ void load(int d) {
+        if (!in) return;
+        const bf16* p = src + d * plane;
+#pragma unroll
+        for (int ch = 0; ch < SC; ++ch) a[ch] = load8<WIDE ? kWide : kQuad>(p + ch * stride + (off - w), w, b.W);
+    }
+    __device__ __forceinline__ void prefetch(int d) const {
+        if (!in || (w & 63)) return;
+        const bf16* p = src + d * plane;
+#pragma unroll
+        for (int ch = 0; ch < SC; ++ch) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off));
+    }
+    // `bias`: two copies of b per channel
+    __device__ __forceinline__ void store(uint4* dst, const unsigned (&bias)[SC], bool relu) {
+        if (at < 0) return;
+#pragma unroll
+        for (int ch = 0; ch < SC; ++ch) {
+            unsigned z[4], c[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                z[i] = i == 0 ? a[ch].x : i == 1 ? a[ch].y : i == 2 ? a[ch].z : a[ch].w;
+                const unsigned nb = bias[ch] ^ 0x80008000u;
+                unsigned m = in ? 0xffffffffu : 0u;
+                if (!WIDE) {
+                    if (w + 2 * i >= b.Wv) m &= 0xffff0000u;
+                    if (w + 2 * i + 1 >= b.Wv) m &= 0x0000ffffu;
+                }
+                if (relu) m &= __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&z[i]), *reinterpret_cast<const __nv_bfloat162*>(&nb));
+                z[i] &= m;
+                c[i] = bias[ch] & m;
+            }
+            dst[2 * ch * blocks + at] = make_uint4(z[0], z[1], z[2], z[3]);
+            dst[(2 * ch + 1) * blocks + at] = make_uint4(c[0], c[1], c[2], c[3]);
+        }
+    }
+};
 
 template <int KD, int KH, int KW, int AL>
 __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const SourceArgs P) {
     constexpr bool ROWS = KH == 1;
     constexpr int kThreads = kSourceThreads, kEpilogueWarps = 4, kMmaWarp = 14;
-    constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
-    constexpr int NCOL = 8 * source_groups<KD>(), NMAT = SC * KH;
-    constexpr int TABLE = (PD + 1) * (PD + 1) * (PH + 1) * (PH + 1) * (PW + 1) * (PW + 1);
-    static_assert(2 * kSlots + source_planes<KD>() + 1 <= 64, "barriers");
+    constexpr int PD = KD / 2, PW = KW / 2, KT = KD * KH * KW, RING = source_ring<KD>();
+    constexpr int NCOL = kGroup * KD, NMAT = SC * KH;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     const Band& b = P.b;
     const At<ROWS> at(b, blockIdx.x);
     const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned base = smem_u32(smem_tc);
-    const unsigned sfull = base, sempty = base + 8 * kSlots, afull = base + 16 * kSlots;
-    constexpr int kTmemAt = 504;
-    float* const table = reinterpret_cast<float*>(smem_tc + kHeader);
-    bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader + (TABLE * 4 + 127) / 128 * 128);
+    const unsigned sfull = base, sempty = sfull + 8 * kSourceSlots, afull = sempty + 8 * kSourceSlots, aempty = afull + 8 * RING,
+                   edges = aempty + 8 * RING;
+    constexpr int kEdgesAt = 320, kTmemAt = 504;
+    static_assert(8 * (2 * kSourceSlots + 2 * RING + 1) <= kEdgesAt && kEdgesAt + 64 * PW <= kTmemAt, "header");
+    float* const edge = reinterpret_cast<float*>(smem_tc + kEdgesAt);      // [parity][warp][side][PW]
+    bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader);
     uint4* const slots = reinterpret_cast<uint4*>(bmat + NMAT * NCOL * 16);
-    const int blocks = (b.TH + KH - 1) * b.PB, slot_blocks = SC * blocks;
+    const int blocks = (b.TH + KH - 1) * b.NB, slot_blocks = 2 * SC * blocks;
     const int planes = at.DC + KD - 1;
 
     if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, kSourceCols);
     if (tid == 0) {
-        for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, kSourceStagers / 32); mbar_init(sempty + 8 * i, 1); }
-        for (int i = 0; i < at.DC; ++i) mbar_init(afull + 8 * i, 1);
+        for (int i = 0; i < kSourceSlots; ++i) { mbar_init(sfull + 8 * i, kSourceStagers / 32); mbar_init(sempty + 8 * i, 1); }
+        for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, kEpilogueWarps); }
+        mbar_init(edges, kEpilogueWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < kSlots * slot_blocks + slack_blocks(b); i += kThreads) slots[i] = make_uint4(0u, 0u, 0u, 0u);
     float* const hs = reinterpret_cast<float*>(smem_tc + 512);
     for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)at.c * SC * KT + e];
     __syncthreads();
-    // [channel, kh][output plane p - kd, kd = KD - 1 - g: groups of 8 columns]
-    build_bands<NCOL, KW, false>(bmat, NMAT, [&](int t, int n, int kw) {
-        const int j = t / KH, kh = t % KH, kd = KD - 1 - n / 8;
-        return kd >= 0 ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
+    // [channel, kh][output plane p - kd, kd = KD - 1 - g: groups of 16 columns][own eight columns, left, right]
+    build_bands<NCOL>(bmat, NMAT, [&](int t, int n, int k) {
+        const int j = t / KH, kh = t % KH, kd = KD - 1 - n / kGroup, i = n % kGroup;
+        const int o = i < 8 ? i : i < 8 + PW ? i - 8 - PW : i - PW, kw = k % 8 - o + PW;
+        return i < 8 + 2 * PW && kw >= 0 && kw < KW ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
     });
-    // sum over channels and the taps inside the volume of bias * filter, by how many taps are cut off at
-    // either end of each axis
-    for (int e = tid; e < TABLE; e += kThreads) {
-        int q = e;
-        const int wh = q % (PW + 1); q /= PW + 1;
-        const int wl = q % (PW + 1); q /= PW + 1;
-        const int hh = q % (PH + 1); q /= PH + 1;
-        const int hl = q % (PH + 1); q /= PH + 1;
-        const int dh = q % (PD + 1), dl = q / (PD + 1);
-        float s = 0.0f;
-        for (int kd = dl; kd < KD - dh; ++kd)
-            for (int kh = hl; kh < KH - hh; ++kh)
-                for (int kw = wl; kw < KW - wh; ++kw) {
-                    const int tau = (kd * KH + kh) * KW + kw;
-#pragma unroll
-                    for (int j = 0; j < SC; ++j) s = fmaf(P.bias ? P.bias[at.c * SC + j] : 0.0f, hs[j * KT + tau], s);
-                }
-        table[e] = s;
-    }
     fence_async_proxy();
     tc_fence_before();
     __syncthreads();
@@ -689,59 +720,97 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
     tc_fence_after();
     bool ok = true;
     if (warp == kMmaWarp) {
-        const unsigned long long ad = mat_desc(smem_u32(slots), 16, 128), md = mat_desc(smem_u32(bmat), 128, 256);
-        const unsigned idesc = instr_desc(NCOL);
+        const unsigned long long ad = mat_desc(smem_u32(slots), 16 * blocks, 128), md = mat_desc(smem_u32(bmat), 128, 256);
         for (int p = 0; p < planes && ok; ++p) {
-            const int s = p % kSlots, d = at.d0 - PD + p;
-            ok = mbar_wait(sfull + 8 * s, (p / kSlots) & 1);
+            const int s = p % kSourceSlots, d = at.d0 - PD + p;
+            ok = mbar_wait(sfull + 8 * s, (p / kSourceSlots) & 1);
+            // the ring place that this plane's last group begins anew has been read and zeroed
+            if (p >= RING) ok = mbar_wait(aempty + 8 * (p % RING), (p / RING - 1) & 1) && ok;
             tc_fence_after();
             if (lane == 0 && ok) {
                 if (d >= 0 && d < b.D) {
-                    const unsigned long long a0 = ad + s * slot_blocks;
+                    const int g0 = max(0, KD - 1 - p);       // output planes of the chunk only
+                    const unsigned long long a0 = ad + s * slot_blocks, m0 = md + g0 * kGroup * 2;
+                    const unsigned idesc = instr_desc(NCOL - g0 * kGroup), acc = tmem + kGroup * (p % RING + g0);
 #pragma unroll
                     for (int t = 0; t < NMAT; ++t)
-                        mma(tmem + 8 * p, a0 + (t / KH) * blocks + (t % KH) * b.PB, md + t * NCOL * 2, idesc, 1);
+                        mma(acc, a0 + 2 * (t / KH) * blocks + (t % KH) * b.NB, m0 + t * NCOL * 2, idesc, 1);
                 }
                 mma_commit(sempty + 8 * s);
                 const int o = p - (KD - 1);
-                if (o >= 0) mma_commit(afull + 8 * o);
+                if (o >= 0) mma_commit(afull + 8 * (o % RING));
             }
             __syncwarp();
         }
     } else if (warp >= kEpilogueWarps) {
-        unsigned negb[SC];
+        unsigned bias[SC];
 #pragma unroll
         for (int j = 0; j < SC; ++j) {
-            const __nv_bfloat162 nb = __float2bfloat162_rn(P.bias ? -P.bias[at.c * SC + j] : 0.0f);
-            negb[j] = *reinterpret_cast<const unsigned*>(&nb);
+            const __nv_bfloat162 v = __float2bfloat162_rn(P.bias ? P.bias[at.c * SC + j] : 0.0f);
+            bias[j] = *reinterpret_cast<const unsigned*>(&v);
         }
-        Stager<KH, KW, SC, true, AL == kWide, kSourceStagers, 1, 2> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at.h0,
-                                                 (tid - 32 * kEpilogueWarps) % kSourceStagers);
-        ok = st.run(slots, slot_blocks, at.d0, PD, planes, sfull, sempty, negb, b.relu, (warp - kEpilogueWarps) / 5, lane);
+        SourceStager<KH, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at.h0,
+                                         (tid - 32 * kEpilogueWarps) % kSourceStagers);
+        ok = stage_planes<kSourceSlots, 2>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, sfull,
+                                           sempty, (warp - kEpilogueWarps) / 5, lane);
     } else {
-        const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q, h = at.h0 + r;
-        const bool valid = r < at.TH && q < b.NB, inner = w >= PW && w + 7 + PW < b.Wv;
-        const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
+        const int m = warp * 32 + lane, r = m / b.NB, q = m - r * b.NB, w = 8 * q, h = at.h0 + r;
+        const bool valid = r < at.TH, left = q > 0, right = q + 1 < b.NB;
+        const bool split = 32 % b.NB != 0;              // rows go on in another warp's lanes
+        const unsigned lanes = tmem + ((unsigned)warp << 21);
         bf16* const tb = P.t1 + (long long)at.bc * addr.chan + h * addr.row_x;
-        // images: every row of a plane is an image of its own, KH = 1
-        const int hl = max(0, PH - h), hh = min(PH, max(0, h + PH - (b.H - 1)));
         for (int o = 0; o < at.DC && ok; ++o) {
-            const int d = at.d0 + o, dl = max(0, PD - d), dh = max(0, d + PD - (b.D - 1));
-            const float* tab = table + (((dl * (PD + 1) + dh) * (PH + 1) + hl) * (PH + 1) + hh) * (PW + 1) * (PW + 1);
-            ok = mbar_wait(afull + 8 * o, 0);
+            const int place = (o + KD - 1) % RING;
+            ok = mbar_wait(afull + 8 * (o % RING), (o / RING) & 1);
             tc_fence_after();
             __syncwarp();
-            float v[8];
-            tmem_load8(lanes + 8 * (o + KD - 1), v);
+            float v[8], n[2 * PW];                       // its own columns; the left and the right neighbour's
+            tmem_load_group<2 * PW>(lanes + kGroup * place, v, n);
+            tmem_fill(lanes + kGroup * place, 0.0f, kGroup);
+            if (place < KD - 1 && o + KD - 1 >= RING) {
+                float v2[8], n2[2 * PW];
+                tmem_load_group<2 * PW>(lanes + kGroup * (place + RING), v2, n2);
+                tmem_fill(lanes + kGroup * (place + RING), 0.0f, kGroup);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] += v2[i];
+#pragma unroll
+                for (int i = 0; i < 2 * PW; ++i) n[i] += n2[i];
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(aempty + 8 * (o % RING));
+            float from_right[PW], from_left[PW];
+#pragma unroll
+            for (int i = 0; i < PW; ++i) {
+                from_right[i] = __shfl_down_sync(0xffffffffu, n[i], 1);
+                from_left[i] = __shfl_up_sync(0xffffffffu, n[PW + i], 1);
+            }
+            if (split) {
+                float* const e = edge + (o & 1) * 8 * PW;
+                if (lane == 0 || lane == 31)
+#pragma unroll
+                    for (int i = 0; i < PW; ++i) e[(2 * warp + (lane ? 1 : 0)) * PW + i] = lane ? n[PW + i] : n[i];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(edges);
+                ok = mbar_wait(edges, o & 1) && ok;
+                if (lane == 31 && warp < 3)
+#pragma unroll
+                    for (int i = 0; i < PW; ++i) from_right[i] = e[2 * (warp + 1) * PW + i];
+                if (lane == 0 && warp > 0)
+#pragma unroll
+                    for (int i = 0; i < PW; ++i) from_left[i] = e[(2 * (warp - 1) + 1) * PW + i];
+            }
+#pragma unroll
+            for (int i = 0; i < PW; ++i) {
+                v[8 - PW + i] += right ? from_right[i] : 0.0f;
+                v[i] += left ? from_left[i] : 0.0f;
+            }
             if (valid) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    int cut = 0;
-                    if (!inner) cut = max(0, PW - w - i) * (PW + 1) + min(PW, max(0, w + i + PW - (b.Wv - 1)));
-                    v[i] += tab[cut];
-                    if (!inner && w + i >= b.Wv) v[i] = 0.0f;
-                }
-                store8<AL>(tb + (long long)d * addr.plane, w, b.W,
+                for (int i = 0; i < 8; ++i)
+                    if (AL != kWide && w + i >= b.Wv) v[i] = 0.0f;
+                store8<AL>(tb + (at.d0 + o) * addr.plane, w, b.W,
                            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])));
             }
         }

@@ -7,6 +7,7 @@ import torch
 import deconver_b200 as dcb
 from deconver_b200 import _lib
 from deconver_b200 import functional as Fn
+from oracle import ndc_oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -77,6 +78,66 @@ def test_gradients_match_the_fma_kernels(case):
     assert _lib.load().ndc_wait_expired() == 0
     for name, a, r in zip(("gx", "gz", "gh", "gb"), *res):
         assert ((a - r).norm() / r.norm()).item() < 5e-3, name
+
+
+# volumes and images, rows of whole blocks of eight columns and not, several bands and chunks of planes
+CANCELLING = [(150, (3, 3, 3), 1, (18, 17, 20)), (200, (3, 3, 3), 1, (7, 9, 64)), (50, (5, 5), 4, (130, 128)),
+              (45, (5, 5), 14, (77, 68)), (70, (3, 3), 3, (60, 252))]
+
+
+@pytest.mark.parametrize("live", [0.0, 0.002, 0.05, 0.6])
+@pytest.mark.parametrize("mixed", [False, True], ids=["even", "mixed"])
+@pytest.mark.parametrize("case", CANCELLING, ids=lambda c: "C%d_k%d_b%d_%s" % (c[0], c[1][0], c[2], "x".join(map(str, c[3]))))
+def test_rectified_sources_leave_no_rounding_behind(case, mixed, live):
+    """A source that is rectified away all but for a share `live`, down to one unit of the bias's last
+    place above it, against the oracle in 64 bits, element by element: zeros are zeros, and no value is
+    further off than its roundings to bfloat16 (2^-8 each) and a float32 sum's share of one.  `mixed`: the
+    channels' biases differ by factors of ten, so that what is left is small beside what cancelled."""
+    C, ks, B, spatial = case
+    gen = torch.Generator().manual_seed(C)
+    x = torch.rand(B, C, *spatial, generator=gen).bfloat16()
+    bias = torch.rand(4 * C, generator=gen) * 0.2 + 0.9
+    if mixed:
+        bias = bias * 10.0 ** -(torch.arange(4 * C) % 4).float()
+    bias = bias.bfloat16()
+    b = bias.view(1, -1, *[1] * len(ks)).float()
+    on = torch.rand(B, 4 * C, *spatial, generator=gen) < live
+    share = torch.where(torch.rand(on.shape, generator=gen) < 0.5, 0.01, 1.0)
+    z = torch.where(on, (torch.rand(on.shape, generator=gen) * share - 1.0) * b, -b - torch.rand(on.shape, generator=gen) * b).bfloat16()
+    h = (torch.rand(C, 4, *ks, generator=gen) / 27).bfloat16()
+    xd, zd, hd, bd = (t.to("cuda:0") for t in (x, z, h.float(), bias.float()))
+    out, t1 = torch.empty_like(zd), torch.empty_like(xd)
+    desc = _lib.make_desc(B, C, 1, 4, spatial, ks, 1e-16, True, _lib.NDC_BF16, _lib.FLAG_BF16_PARAMS)
+    _lib.check(_lib.load().ndc_fwd(desc, xd.data_ptr(), zd.data_ptr(), hd.data_ptr(), bd.data_ptr(), out.data_ptr(), t1.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream))
+    s = torch.relu(z.double() + b.double())
+    ref_t1 = O.K(s, h.double(), C)
+    got = t1.double().cpu()
+    assert not got[ref_t1 == 0].any()
+    assert ((got - ref_t1).abs() <= (2.0 ** -8 + 2.0 ** -10) * ref_t1).all()
+    ref = s * (O.A(x.double(), h.double(), C) + 1e-16) / (O.A(ref_t1, h.double(), C) + 1e-16)
+    assert ((out.double().cpu() - ref).abs() <= (2.0 ** -7 + 2.0 ** -9) * ref).all()
+
+
+@pytest.mark.parametrize("relu", [True, False])
+@pytest.mark.parametrize("ks,B,spatial,pitch", [((3, 3, 3), 2, (9, 31, 45), 48), ((5, 5), 6, (41, 171), 172)])
+def test_padding_of_the_source_is_not_read(ks, B, spatial, pitch, relu):
+    """Only x has to be zero in the padding of the rows; z may hold anything there."""
+    C, (*lead, W), lib, dev = 75, spatial, _lib.load(), "cuda:0"
+    gen = torch.Generator(device=dev).manual_seed(3)
+    x, z = (torch.zeros(B, n, *lead, pitch, device=dev, dtype=torch.bfloat16) for n in (C, 4 * C))
+    x[..., :W] = torch.rand(B, C, *lead, W, device=dev, generator=gen)
+    z[..., :W] = torch.rand(B, 4 * C, *lead, W, device=dev, generator=gen)
+    h = (torch.rand(C, 4, *ks, device=dev, generator=gen) / 27).bfloat16().float()
+    desc = _lib.make_desc(B, C, 1, 4, spatial, ks, 1e-16, relu, _lib.NDC_BF16, _lib.FLAG_BF16_PARAMS)
+    res = []
+    for garbage in (0.0, 1000.0):
+        z[..., W:] = garbage
+        out, t1 = torch.zeros_like(z), torch.empty_like(x)
+        _lib.check(lib.ndc_fwd_rows(desc, pitch, pitch, x.data_ptr(), z.data_ptr(), h.data_ptr(), None, out.data_ptr(), t1.data_ptr(),
+                                    torch.cuda.current_stream().cuda_stream))
+        res.append((out[..., :W].clone(), t1))
+    assert all(torch.equal(a, b) for a, b in zip(*res)) and not t1[..., W:].any()
 
 
 @pytest.mark.parametrize("channels,batch,spatial,ks", [(34, 2, (9, 31, 45), (3, 3, 3)), (150, 2, (5, 20, 27), (3, 3, 3)),
