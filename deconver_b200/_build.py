@@ -76,7 +76,7 @@ def ext_built_for():
 
 
 def ext_is_stale():
-    return _older(EXT, [EXT_SRC, os.path.join(INCLUDE, "ndc_b200.h")]) or ext_built_for() != ext_target()
+    return _older(EXT, [EXT_SRC, os.path.join(INCLUDE, "ndc_b200.h"), os.path.abspath(__file__)]) or ext_built_for() != ext_target()
 
 
 def _compile_ext():
@@ -92,7 +92,10 @@ def _compile_ext():
            "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
            "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"], "-c", EXT_SRC, "-o", obj]
     link = [cmd[0], "-shared", obj, "-o", EXT, "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
-            "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L", PKG, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+            "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L", PKG, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN",
+            # The C++ runtime that PyTorch uses.  A compiler that comes with the archive alone would put a second
+            # one into the extension, and the first exception thrown there would crash the process.
+            "-l:libstdc++.so.6"]
     return subprocess.run(cmd, cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True), link
 
 

@@ -3,12 +3,14 @@ Modelled on the reference's `tests/test_deconv_equivalence.py:244-254` (state-di
 trip) and `tests/test_deconver.py` (shape/smoke), minus anything that needs a GPU."""
 
 import contextlib
+import subprocess
+import sys
 
 import pytest
 import torch
 
 import deconver_b200 as dcb
-from conftest import load_golden
+from conftest import ROOT, load_golden
 from deconver_b200 import _build, _lib
 from deconver_b200._build import build_library
 
@@ -179,3 +181,20 @@ def test_the_extension_is_rebuilt_for_another_pytorch(monkeypatch):
     monkeypatch.setattr(_lib, "_ext", None)
     with pytest.raises(RuntimeError, match="was built for"):      # and not a failure of the dynamic linker
         _lib.load_ext()
+
+
+def test_errors_of_the_extension_are_python_exceptions():
+    """Not crashes: in a process of its own."""
+    program = """if True:
+        import torch
+        from deconver_b200 import _lib
+        x, h, w, ext = torch.rand(2, 4, 8), torch.rand(4, 4, 3), torch.rand(16, 5, 1), _lib.load_ext()
+        for call in (lambda: ext.linear(x, w, None), lambda: ext.bias_gelu(x, None), lambda: ext.instance_norm(x, x, None, 1e-5),
+                     lambda: ext.layer(x, h, w, None, 4, 1, 4, 1e-16, 1, 1, 0)):
+            try:
+                call()
+                raise SystemExit("no error")
+            except RuntimeError as e:
+                assert "deconver_b200" in str(e), e
+        """
+    subprocess.run([sys.executable, "-c", program], check=True, timeout=300, cwd=ROOT)
