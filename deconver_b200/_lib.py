@@ -24,7 +24,7 @@ SYMBOLS = (
     "ndc_inorm_bwd", "ndc_bias_grad_workspace_bytes", "ndc_bias_last_error", "ndc_bias_add",
     "ndc_bias_grad", "ndc_bias_gelu_fwd", "ndc_bias_gelu_bwd", "ndc_proj_wgrad_workspace_bytes",
     "ndc_proj_last_error", "ndc_proj_wgrad", "ndc_proj_sum", "ndc_params_prepare", "ndc_params_grad",
-    "ndc_wait_expired", "ndc_row_pitch", "ndc_fwd_rows", "ndc_bwd_rows_workspace_bytes", "ndc_bwd_rows", "ndc_pad_rows", "ndc_unpad_rows",
+    "ndc_wait_expired", "ndc_probe_wait", "ndc_row_pitch", "ndc_fwd_rows", "ndc_bwd_rows_workspace_bytes", "ndc_bwd_rows", "ndc_pad_rows", "ndc_unpad_rows",
 )
 
 
@@ -80,6 +80,8 @@ def load():
     lib.ndc_bwd_static.argtypes = [dp, vp, vp, vp, fp, fp, vp, vp, vp, fp, fp, vp]
     i32 = ctypes.c_int32
     lib.ndc_wait_expired.restype = ctypes.c_uint32
+    lib.ndc_probe_wait.restype = ctypes.c_int
+    lib.ndc_probe_wait.argtypes = [ctypes.c_uint32, vp]
     lib.ndc_row_pitch.restype = i32
     lib.ndc_row_pitch.argtypes = [dp]
     lib.ndc_fwd_rows.restype = ctypes.c_int

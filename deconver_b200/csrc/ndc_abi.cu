@@ -96,6 +96,14 @@ bool tensor_cores(const NdcDesc* d, const ndc::Geo& g) {
     return d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && !(d->flags & NDC_FLAG_RELU_FILTER) && ndc::tc::covers(g);
 }
 
+// Launches return long before their kernels run, so that a wait that ran out in one of them is
+// reported by the next call.
+int check_expired() {
+    if (!ndc::tc::take_expired()) return NDC_OK;
+    return fail(NDC_ERR_TIMEOUT, "a wait inside a kernel of an earlier call ran out after one second (a kernel bug, or a GPU "
+                                 "that was taken away for that long): the results of that call are undefined; this one was not run");
+}
+
 int raw_filter_refused(const NdcDesc* d) {
     if (d->flags & NDC_FLAG_RELU_FILTER)
         return fail(NDC_ERR_UNSUPPORTED, "NDC_FLAG_RELU_FILTER is for the depthwise forward only");
@@ -172,6 +180,7 @@ const char* ndc_status_string(int status) {
         case NDC_ERR_WORKSPACE: return "workspace missing, too small or misaligned";
         case NDC_ERR_CUDA: return "CUDA error";
         case NDC_ERR_ALIGNMENT: return "misaligned pointer";
+        case NDC_ERR_TIMEOUT: return "a wait inside an earlier launch ran out";
         default: return "unknown status";
     }
 }
@@ -207,6 +216,7 @@ int32_t ndc_row_pitch(const NdcDesc* desc) {
 int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const void* x, const void* z,
                  const float* h, const float* bias, void* out, void* t1, void* stream) {
     NDC_TRY(validate(desc));
+    NDC_TRY(check_expired());
     NDC_TRY(check_pitch(desc, pitch, out_pitch));
     NDC_TRY(check_ptr(x, "x", desc->dtype));
     NDC_TRY(check_ptr(z, "z", desc->dtype));
@@ -283,6 +293,7 @@ int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const v
                  float* gh, float* gb, void* workspace, size_t workspace_bytes, void* stream) {
     NDC_TRY(validate(desc));
     NDC_TRY(raw_filter_refused(desc));
+    NDC_TRY(check_expired());
     NDC_TRY(check_pitch(desc, pitch, gout_pitch));
     NDC_TRY(check_ptr(x, "x", desc->dtype));
     NDC_TRY(check_ptr(z, "z", desc->dtype));
@@ -414,6 +425,13 @@ int ndc_probe_fp32_fma(int32_t packed, int32_t iters, float* out, size_t out_ele
     // per thread: iters x 8 rounds x 8 chains, two lanes per packed instruction
     if (fma_count)
         *fma_count = (uint64_t)threads * blocks * (uint64_t)iters * 64u * (packed ? 2u : 1u);
+    return NDC_OK;
+}
+
+int ndc_probe_wait(uint32_t limit_us, void* stream) {
+    if (limit_us == 0 || limit_us > 1000000u) return fail(NDC_ERR_INVALID, "ndc_probe_wait: a limit of 1 to 1000000 microseconds");
+    const cudaError_t e = ndc::tc::probe_wait(limit_us, (cudaStream_t)stream);
+    if (e != cudaSuccess) return cuda_fail(e, "ndc_probe_wait launch");
     return NDC_OK;
 }
 

@@ -1,11 +1,59 @@
 // Host side of the tensor-core forward (ndc_tc.cuh): tiling and launches.
 #include "ndc_tc.cuh"
 
+#include <atomic>
+#include <mutex>
+
 #include "ndc_tc_host.h"
 
 namespace ndc {
 namespace tc {
 namespace {
+
+// One word per device in host memory, where a kernel whose wait ran out writes 1: a call after it reads the
+// word without synchronising, reports it and writes 2.  Allocated once; a launch may be the first one under
+// stream capture, which forbids allocations unless the thread says that it knows what it does.
+constexpr int kMaxDevices = 64;
+std::atomic<unsigned*> g_expired{nullptr};
+
+cudaError_t expired_word(unsigned*& word) {
+    static std::mutex mu;
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    unsigned* all = g_expired.load(std::memory_order_acquire);
+    if (!all) {
+        std::lock_guard<std::mutex> lock(mu);
+        all = g_expired.load(std::memory_order_acquire);
+        if (!all) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            if ((e = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return e;
+            void* p = nullptr;
+            e = cudaHostAlloc(&p, kMaxDevices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+            const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) return e;
+            if (back != cudaSuccess) return back;
+            all = static_cast<unsigned*>(p);
+            for (int i = 0; i < kMaxDevices; ++i) all[i] = 0u;
+            g_expired.store(all, std::memory_order_release);
+        }
+    }
+    word = all + dev;
+    return cudaSuccess;
+}
+
+// A wait for what never comes, to see that one that runs out is reported.
+__global__ void probe_wait_kernel(unsigned limit, unsigned* expired) {
+    __shared__ unsigned long long bar;
+    const unsigned at = smem_u32(&bar);
+    if (threadIdx.x == 0) {
+        mbar_init(at, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (!mbar_wait(at, 0, limit) && threadIdx.x == 0) report_expired(expired);
+}
 
 // Bands: as many rows as fill the 128 blocks of an MMA.  Chunks of planes: all of them, but for a grid that
 // would leave multiprocessors idle; from there, the cut of least expected time, if that is 2 % less: the
@@ -89,9 +137,12 @@ cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, cons
     A.x = x; A.t1 = t1; A.z = z; A.out = out; A.h = h; A.bias = bias;
     S.z = z; S.t1 = t1; S.h = h; S.bias = bias;
     const size_t ss = source_smem<KD, KH, KW>(S.b);
+    cudaError_t e = expired_word(S.expired);
+    if (e != cudaSuccess) return e;
+    A.expired = S.expired;
     const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1);
-    cudaError_t e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, g, ss, st, S)
-                         : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, g, ss, st, S);
+    e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, g, ss, st, S)
+             : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, g, ss, st, S);
     if (e != cudaSuccess) return e;
     return launch_adjoint<KD, KH, KW, kOut>(g, A, wide && on16(out), st);
 }
@@ -101,6 +152,8 @@ cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1
                       float* gnum, float* gden, bf16* direct, bool pairs, cudaStream_t st) {
     AdjointArgs A{};
     if (!plan<KD, KH, KW>(g, false, A.b)) return cudaErrorInvalidConfiguration;
+    const cudaError_t e = expired_word(A.expired);
+    if (e != cudaSuccess) return e;
     A.x = x; A.t1 = t1; A.z = z; A.out = direct; A.gout = gout; A.gnum = gnum; A.gden = gden; A.h = h; A.bias = bias;
     const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1) && on16(gout) && (!direct || on16(direct));
     if constexpr (KH == 1) {
@@ -158,9 +211,28 @@ cudaError_t backward_ratio(const Geo& g, const bf16* x, const bf16* z, const bf1
 }
 
 unsigned wait_expired() {
-    unsigned v = 0;
-    (void)cudaMemcpyFromSymbol(&v, g_wait_expired, sizeof(v));
-    return v;
+    int dev = -1;
+    unsigned* all = g_expired.load(std::memory_order_acquire);
+    if (!all || cudaDeviceSynchronize() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    return __atomic_load_n(all + dev, __ATOMIC_ACQUIRE);
+}
+
+bool take_expired() {
+    int dev = -1;
+    unsigned* all = g_expired.load(std::memory_order_acquire);
+    if (!all || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+    unsigned one = 1u;
+    return __atomic_load_n(all + dev, __ATOMIC_ACQUIRE) == 1u &&
+           __atomic_compare_exchange_n(all + dev, &one, 2u, false, __ATOMIC_ACQ_REL, __ATOMIC_ACQUIRE);
+}
+
+cudaError_t probe_wait(unsigned limit_us, cudaStream_t st) {
+    unsigned* word = nullptr;
+    const cudaError_t e = expired_word(word);
+    if (e != cudaSuccess) return e;
+    probe_wait_kernel<<<1, 32, 0, st>>>(limit_us * 1000u, word);
+    launched();
+    return cudaGetLastError();
 }
 
 }  // namespace tc

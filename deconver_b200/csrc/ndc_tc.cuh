@@ -64,8 +64,10 @@ __device__ __forceinline__ void mbar_init(unsigned bar, int count) {
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Waits for the phase to complete; gives up (false) after a second, far above any MMA's time.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase) {
+// Waits for the phase to complete, one thread or all of a warp; gives up (false, in all of them) after
+// `limit` nanoseconds.  A second is far above any MMA's time.
+constexpr unsigned kWaitLimit = 1000000000u;
+__device__ __forceinline__ bool mbar_wait_thread(unsigned bar, unsigned phase, unsigned limit) {
     unsigned long long start = 0;
     for (;;) {
         unsigned done;
@@ -75,8 +77,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase) {
         unsigned long long now;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
         if (!start) start = now;
-        if (now - start > 1000000000ull) return false;
+        if (now - start > limit) return false;
     }
+}
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase, unsigned limit = kWaitLimit) {
+    return __all_sync(0xffffffffu, mbar_wait_thread(bar, phase, limit));
+}
+// A wait ran out: the launch's results are undefined.  `flag` is host memory that the host looks at before
+// the next call (see ndc_tc.cu).
+__device__ __forceinline__ void report_expired(unsigned* flag) {
+    asm volatile("st.release.sys.global.u32 [%0], 1;" ::"l"(flag) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(unsigned slot, int cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
@@ -147,9 +157,6 @@ __device__ __forceinline__ unsigned long long mat_desc(unsigned addr, int kstep,
 __device__ __forceinline__ unsigned instr_desc(int n) { return 1u << 4 | 1u << 7 | 1u << 10 | (unsigned)(n >> 3) << 17 | (unsigned)(MB >> 4) << 24; }
 
 // ---- staging ----------------------------------------------------------------------------------
-// Set where a wait ran out; the results of that launch are then undefined.
-static __device__ unsigned g_wait_expired;
-
 // Roles of a CTA's warps: groups of four for the epilogue (they take turns, output plane by output
 // plane; TMEM lane 32 i + l belongs to lane l of warp i of a group), groups that stage source planes (in
 // turns as well), one warp that issues the MMAs.  The source kernel, whose epilogue is short and whose
@@ -369,6 +376,7 @@ struct AdjointArgs {
     bf16* out;                        // kOut: out; else the direct term (rows of W), or NULL
     const bf16* gout; float* gnum; float* gden;
     const float* h; const float* bias;
+    unsigned* expired;                // see report_expired
 };
 
 // Accumulators: per output plane 32 columns of A(x) and 32 of A(t1) (four channels of eight voxels),
@@ -426,13 +434,13 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
     bool ok = true;
     if (warp == kMmaWarp) {
         const unsigned long long ad = mat_desc(smem_u32(slots), 16, 128), md = mat_desc(smem_u32(bmat), 128, 256);
-        for (int p = 0; p < planes && ok; ++p) {
+        for (int p = 0; p < planes && ok && lane == 0; ++p) {
             const int s = p % kSlots, d = at.d0 - PD + p;
-            ok = mbar_wait(sfull + 8 * s, (p / kSlots) & 1);
+            ok = mbar_wait_thread(sfull + 8 * s, (p / kSlots) & 1, kWaitLimit);
             // a new output plane begins: its accumulators have been read and zeroed
-            if (p >= RING && p < at.DC) ok = mbar_wait(aempty + 8 * (p % RING), (p / RING - 1) & 1) && ok;
+            if (p >= RING && p < at.DC) ok = mbar_wait_thread(aempty + 8 * (p % RING), (p / RING - 1) & 1, kWaitLimit) && ok;
             tc_fence_after();
-            if (lane == 0 && ok) {
+            if (ok) {
                 if (d >= 0 && d < b.D) {
                     // groups g of output planes o = p - (KD - 1) + g inside the chunk
                     const int g0 = max(0, KD - 1 - p), g1 = min(KD - 1, at.DC - 1 + KD - 1 - p), o0 = p - (KD - 1) + g0;
@@ -453,7 +461,6 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                 const int o = p - (KD - 1);
                 if (o >= 0) mma_commit(afull + 8 * (o % RING));
             }
-            __syncwarp();
         }
     } else if (warp >= kEpilogueWarps) {
         // x and t1 as two channels: the distance between the tensors takes the place of the stride
@@ -581,9 +588,10 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
             }
         }
     }
-    if (!ok && lane == 0) atomicExch(&g_wait_expired, 1u);
+    if (!ok && lane == 0) report_expired(P.expired);
     tc_fence_before();
     __syncthreads();
+    __syncwarp();
     if (warp == kMmaWarp) tmem_free(tmem, TCOLS);
 }
 
@@ -592,6 +600,7 @@ struct SourceArgs {
     Band b;
     const bf16* z; bf16* t1;
     const float* h; const float* bias;
+    unsigned* expired;
 };
 
 // Accumulators: 16 columns per output plane, of which the block's own eight, PW of the left and PW of the
@@ -721,13 +730,13 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
     bool ok = true;
     if (warp == kMmaWarp) {
         const unsigned long long ad = mat_desc(smem_u32(slots), 16 * blocks, 128), md = mat_desc(smem_u32(bmat), 128, 256);
-        for (int p = 0; p < planes && ok; ++p) {
+        for (int p = 0; p < planes && ok && lane == 0; ++p) {
             const int s = p % kSourceSlots, d = at.d0 - PD + p;
-            ok = mbar_wait(sfull + 8 * s, (p / kSourceSlots) & 1);
+            ok = mbar_wait_thread(sfull + 8 * s, (p / kSourceSlots) & 1, kWaitLimit);
             // the ring place that this plane's last group begins anew has been read and zeroed
-            if (p >= RING) ok = mbar_wait(aempty + 8 * (p % RING), (p / RING - 1) & 1) && ok;
+            if (p >= RING) ok = mbar_wait_thread(aempty + 8 * (p % RING), (p / RING - 1) & 1, kWaitLimit) && ok;
             tc_fence_after();
-            if (lane == 0 && ok) {
+            if (ok) {
                 if (d >= 0 && d < b.D) {
                     const int g0 = max(0, KD - 1 - p);       // output planes of the chunk only
                     const unsigned long long a0 = ad + s * slot_blocks, m0 = md + g0 * kGroup * 2;
@@ -740,7 +749,6 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
                 const int o = p - (KD - 1);
                 if (o >= 0) mma_commit(afull + 8 * (o % RING));
             }
-            __syncwarp();
         }
     } else if (warp >= kEpilogueWarps) {
         unsigned bias[SC];
@@ -815,9 +823,10 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
             }
         }
     }
-    if (!ok && lane == 0) atomicExch(&g_wait_expired, 1u);
+    if (!ok && lane == 0) report_expired(P.expired);
     tc_fence_before();
     __syncthreads();
+    __syncwarp();
     if (warp == kMmaWarp) tmem_free(tmem, kSourceCols);
 }
 

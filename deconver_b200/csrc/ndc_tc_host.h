@@ -15,8 +15,12 @@ cudaError_t forward(const Geo& g, const __nv_bfloat16* x, const __nv_bfloat16* z
 cudaError_t backward_ratio(const Geo& g, const __nv_bfloat16* x, const __nv_bfloat16* z, const __nv_bfloat16* t1, const float* h,
                            const float* bias, const __nv_bfloat16* gout, float* gnum, float* gden, __nv_bfloat16* direct,
                            bool pairs, cudaStream_t st);
-// Non-zero once a kernel's bounded wait has run out on the current device (synchronises; for tests).
+// Non-zero once a kernel's bounded wait has run out on the current device (synchronises).
 unsigned wait_expired();
+// The same for launches that are known to have run by now, without synchronising; true once for each.
+bool take_expired();
+// Launches one wait that runs out after `limit_us` (up to a second).
+cudaError_t probe_wait(unsigned limit_us, cudaStream_t st);
 
 }  // namespace tc
 }  // namespace ndc

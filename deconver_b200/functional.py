@@ -86,6 +86,8 @@ class _Timing:
     def disable_and_collect(self):
         self.enabled = False
         torch.cuda.synchronize()
+        if _lib.load().ndc_wait_expired():
+            raise RuntimeError("deconver_b200: a wait inside a kernel ran out; the results of that call are undefined")
         native = dict(zip(("ndc_fwd", "ndc_bwd"), _lib.load_ext().timing_collect()))
         return {k: [a.elapsed_time(b) for a, b in v] + native[k] for k, v in self._events.items()}
 

@@ -46,7 +46,8 @@ enum NdcStatus {
     NDC_ERR_UNSUPPORTED = 2, /* geometry outside what the kernels cover                     */
     NDC_ERR_WORKSPACE = 3,   /* workspace missing, too small or misaligned                  */
     NDC_ERR_CUDA = 4,        /* a CUDA runtime call or a launch failed                      */
-    NDC_ERR_ALIGNMENT = 5    /* a tensor pointer is not aligned to its element size         */
+    NDC_ERR_ALIGNMENT = 5,   /* a tensor pointer is not aligned to its element size         */
+    NDC_ERR_TIMEOUT = 6      /* a wait inside a kernel of an EARLIER call ran out           */
 };
 
 enum NdcFlags {
@@ -102,9 +103,14 @@ const char *ndc_status_string(int status);
  * caller verify that the CUDA path, and not some other path, did the work. */
 uint64_t ndc_launch_count(void);
 
-/* Non-zero once a bounded wait inside a kernel has run out on the current device (a kernel bug:
- * the outputs of that launch are undefined).  Synchronises with the device; for tests. */
+/* Every wait inside a kernel is bounded (one second).  Where one runs out - a kernel bug, or a GPU
+ * that another process held for so long - the outputs of that launch are undefined.  The next
+ * ndc_fwd / ndc_bwd (or ..._rows) on that device after it has run returns NDC_ERR_TIMEOUT once, without
+ * launching anything; it looks at a word in host memory and does not synchronise.
+ * ndc_wait_expired: non-zero from then on, on the current device.  Synchronises with the device.
+ * ndc_probe_wait: launches one wait that runs out after `limit_us` microseconds (up to 1000000). */
 uint32_t ndc_wait_expired(void);
+int ndc_probe_wait(uint32_t limit_us, void *stream);
 
 /*
  * Whether a geometry is covered, and by which kernel family.  Returns NDC_OK and writes an

@@ -1,10 +1,14 @@
 """The tensor-core forward (bfloat16 tensors, filter and bias) against the FMA kernels, which take the
 same values as float32 parameters: edges of bands, chunks, blocks of eight columns and MMA tiles."""
 
+import subprocess
+import sys
+
 import pytest
 import torch
 
 import deconver_b200 as dcb
+from conftest import ROOT
 from deconver_b200 import _lib
 from deconver_b200 import functional as Fn
 from oracle import ndc_oracle as O
@@ -117,6 +121,26 @@ def test_rectified_sources_leave_no_rounding_behind(case, mixed, live):
     assert ((got - ref_t1).abs() <= (2.0 ** -8 + 2.0 ** -10) * ref_t1).all()
     ref = s * (O.A(x.double(), h.double(), C) + 1e-16) / (O.A(ref_t1, h.double(), C) + 1e-16)
     assert ((out.double().cpu() - ref).abs() <= (2.0 ** -7 + 2.0 ** -9) * ref).all()
+
+
+def test_a_wait_that_runs_out_is_reported():
+    """By the next call, once, and from then on by ndc_wait_expired (hence a process of its own)."""
+    program = """if True:
+        import torch, deconver_b200 as dcb
+        from deconver_b200 import _lib
+        lib = _lib.load()
+        mod, x = dcb.Deconv(4, (3, 3), ratio=4).cuda(), torch.rand(1, 4, 8, 8, device="cuda:0")
+        want = mod(x)
+        assert lib.ndc_probe_wait(2000, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        try:
+            mod(x)
+            raise SystemExit("not reported")
+        except RuntimeError as e:
+            assert "ran out" in str(e), e
+        assert torch.equal(mod(x), want) and lib.ndc_wait_expired()
+        """
+    subprocess.run([sys.executable, "-c", program], check=True, timeout=300, cwd=ROOT)
 
 
 @pytest.mark.parametrize("relu", [True, False])
