@@ -29,7 +29,14 @@ using torch::autograd::variable_list;
 
 int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? NDC_BF16 : NDC_F32; }
 bool kernel_dtype(const Tensor& t) { return t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16; }
-void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+// The tensor's memory.  A tensor may have none though it has elements (FakeTensor and other wrappers): library
+// calls would read at address zero.
+void* ptr(const Tensor& t) {
+    if (!t.defined()) return nullptr;
+    void* p = t.data_ptr();
+    TORCH_CHECK(p || !t.numel(), "deconver_b200: a tensor of ", t.sizes(), " has no memory; the kernels need one that does");
+    return p;
+}
 float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
 void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
@@ -109,8 +116,8 @@ void channel_gemm(const Tensor& w, bool transpose, const Tensor& x, Tensor& y, i
     cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
     // column-major view: (n x out) = (n x in) * (in x out)
     const cublasStatus_t st = cublasGemmStridedBatchedEx(
-        handle, CUBLAS_OP_N, transpose ? CUBLAS_OP_T : CUBLAS_OP_N, (int)n, (int)out, (int)in, &one, x.data_ptr(),
-        type, (int)n, (long long)(in * n), w.data_ptr(), type, (int)ci, 0LL, &beta, y.data_ptr(), type, (int)n,
+        handle, CUBLAS_OP_N, transpose ? CUBLAS_OP_T : CUBLAS_OP_N, (int)n, (int)out, (int)in, &one, ptr(x),
+        type, (int)n, (long long)(in * n), ptr(w), type, (int)ci, 0LL, &beta, ptr(y), type, (int)n,
         (long long)(out * n), (int)batch, compute, CUBLAS_GEMM_DEFAULT);
     TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection GEMM failed (cuBLAS status ", (int)st, ")");
 }
@@ -140,8 +147,8 @@ Tensor weight_grad(const Tensor& gy, const Tensor& x, const Tensor& w, int64_t b
             const size_t e = bf16 ? 2 : 4;
             const cublasStatus_t st = cublasGemmStridedBatchedEx(
                 handle, CUBLAS_OP_T, CUBLAS_OP_N, (int)ci, (int)co, (int)length, &one,
-                static_cast<const char*>(x.data_ptr()) + b * ci * n * e, type, (int)n, (long long)(slices > 1 ? length : ci * n),
-                static_cast<const char*>(gy.data_ptr()) + b * co * n * e, type, (int)n, (long long)(slices > 1 ? length : co * n),
+                static_cast<const char*>(ptr(x)) + b * ci * n * e, type, (int)n, (long long)(slices > 1 ? length : ci * n),
+                static_cast<const char*>(ptr(gy)) + b * co * n * e, type, (int)n, (long long)(slices > 1 ? length : co * n),
                 &zero, fptr(partial) + b * slices * co * ci, CUDA_R_32F, (int)ci, (long long)(co * ci),
                 (int)(slices > 1 ? slices : batch), compute, CUBLAS_GEMM_DEFAULT);
             TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection gradient failed (cuBLAS status ", (int)st, ")");

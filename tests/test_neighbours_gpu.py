@@ -6,6 +6,7 @@ import itertools
 import pytest
 import torch
 import torch.nn.functional as F
+from torch._subclasses.fake_tensor import FakeTensorMode
 
 import deconver_b200 as dcb
 from conftest import max_norm_error
@@ -101,3 +102,15 @@ def test_autocast(dtype):
     assert y.dtype == torch.bfloat16 and x.grad.dtype == dtype
     assert all(p.grad is not None and p.grad.dtype == torch.float32 for p in mlp.parameters())
     assert max_norm_error(y.detach().float().cpu().numpy(), mlp.cpu()(x.detach().float().cpu()).detach().numpy()) < 2e-2
+
+
+MODULES = {"linear": lambda: dcb.Linear(6, 10), "mlp": lambda: dcb.MLP(6), "norm": lambda: dcb.InstanceNorm2d(6, affine=True),
+           "deconv": lambda: dcb.Deconv(6, (3, 3), ratio=4, num_iters=2)}
+
+
+@pytest.mark.parametrize("module", MODULES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_tensors_without_memory_are_refused(module, dtype):
+    net, x = MODULES[module]().to(DEV, dtype), torch.rand(2, 6, 4, 8, device=DEV).to(dtype)
+    with FakeTensorMode(allow_non_fake_inputs=True) as mode, pytest.raises(RuntimeError, match="memory|NULL"):
+        net(mode.from_tensor(x))
