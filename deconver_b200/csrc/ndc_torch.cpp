@@ -44,6 +44,13 @@ void check(int status, const char* message) {
     TORCH_CHECK(status == NDC_OK, "ndc_b200 status ", status, ": ", message);
 }
 
+// The nodes have no forward-mode derivative.  Their own `apply` says so, but calls without reverse-mode
+// gradients do not go through it, and would drop the tangents.
+void refuse_tangents(std::initializer_list<const Tensor*> tensors) {
+    for (const Tensor* t : tensors)
+        TORCH_CHECK(!t->defined() || !t->_fw_grad(0).defined(), "deconver_b200: forward-mode differentiation is not implemented");
+}
+
 // ---- optional CUDA-event timing of ndc_fwd / ndc_bwd on the stream they are issued on ----------
 struct Timing {
     std::mutex mu;
@@ -389,6 +396,8 @@ Tensor layer(const Tensor& x_in, const Tensor& h0_in, const Tensor& w_in, const 
     TORCH_CHECK(!bias_in || (bias_in->device() == x_in.device() && bias_in->numel() == groups * sc),
                 "deconver_b200: the bias does not match the projection");
     c10::cuda::CUDAGuard guard(x_in.device());
+    refuse_tangents({&x_in, &h0_in, &w_in});
+    if (bias_in) refuse_tangents({&*bias_in});
     const Tensor x = x_in.contiguous(), h0 = h0_in.contiguous(), w = w_in.contiguous();
     const std::optional<Tensor> bias = bias_in ? std::optional<Tensor>(bias_in->contiguous()) : std::nullopt;
     const bool grad = at::GradMode::is_enabled() &&
@@ -522,6 +531,7 @@ Tensor linear(const Tensor& x_in, const Tensor& w_in, const std::optional<Tensor
                 "deconver_b200: the bias does not match the projection");
     c10::cuda::CUDAGuard guard(x_in.device());
     const Tensor x = x_in.contiguous(), w = w_in.contiguous(), b = bias_in ? *bias_in : Tensor();
+    refuse_tangents({&x, &w, &b});
     if (wants_grad({&x, &w, &b})) return LinearNode::apply(x, w, bias_in);
     at::AutoDispatchBelowADInplaceOrView below;
     return LinearNode::run(x, w, b);
@@ -577,6 +587,7 @@ Tensor bias_gelu(const Tensor& h_in, const std::optional<Tensor>& bias) {
                 "deconver_b200: the bias does not match the tensor");
     c10::cuda::CUDAGuard guard(h_in.device());
     const Tensor h = h_in.contiguous(), b = bias ? *bias : Tensor();
+    refuse_tangents({&h, &b});
     if (wants_grad({&h, &b})) return BiasGeluNode::apply(h, bias);
     at::AutoDispatchBelowADInplaceOrView below;
     return BiasGeluNode::run(h, as_f32(b));
@@ -647,6 +658,7 @@ Tensor instance_norm(const Tensor& x_in, const std::optional<Tensor>& weight, co
                     "deconver_b200: instance norm parameters do not match the input ", x_in.sizes());
     c10::cuda::CUDAGuard guard(x_in.device());
     const Tensor x = x_in.contiguous(), w = weight ? *weight : Tensor(), b = bias ? *bias : Tensor();
+    refuse_tangents({&x, &w, &b});
     if (wants_grad({&x, &w, &b})) return NormNode::apply(x, weight, bias, eps);
     at::AutoDispatchBelowADInplaceOrView below;
     Tensor stats;

@@ -7,6 +7,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 from torch._subclasses.fake_tensor import FakeTensorMode
+from torch.autograd import forward_ad
 
 import deconver_b200 as dcb
 from conftest import max_norm_error
@@ -114,3 +115,17 @@ def test_tensors_without_memory_are_refused(module, dtype):
     net, x = MODULES[module]().to(DEV, dtype), torch.rand(2, 6, 4, 8, device=DEV).to(dtype)
     with FakeTensorMode(allow_non_fake_inputs=True) as mode, pytest.raises(RuntimeError, match="memory|NULL"):
         net(mode.from_tensor(x))
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("module", MODULES)
+def test_tangents_are_refused(module, grad):
+    """Not dropped, whether or not anything asks for a gradient."""
+    net, x = MODULES[module]().to(DEV), torch.rand(2, 6, 4, 8, device=DEV)
+    net.requires_grad_(grad)
+    with forward_ad.dual_level():
+        with pytest.raises(RuntimeError, match="forward-mode|jvp"):
+            net(forward_ad.make_dual(x, torch.ones_like(x)))
+        p = next(net.parameters())
+        with torch.no_grad(), pytest.raises(RuntimeError, match="forward-mode|jvp"):
+            torch.func.functional_call(net, {next(iter(net.state_dict())): forward_ad.make_dual(p, torch.ones_like(p))}, x)
