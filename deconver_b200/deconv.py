@@ -16,8 +16,7 @@ import torch
 import torch.nn.functional as F
 from torch import Tensor, nn
 
-from ._lib import load_ext
-from .functional import current_flags, kernels_apply, warn_if_generic
+from .functional import current_flags, kernels_apply, native, warn_if_generic
 from .linear import Linear
 
 __all__ = ["Initializer", "Deconv", "NDC"]
@@ -146,10 +145,10 @@ class Deconv(nn.Module):
             warn_if_generic(x, self.groups, self.filter_channels, self.source_channels, self.kernel_size)
             if len(_checked) < 4096:
                 _checked.add(key)
-        init = self.init
-        projection = init.linear.linear
-        return load_ext().layer(x, init.h0, projection.weight, projection.bias, self.groups, self.filter_channels,
-                                self.source_channels, self.eps, self.num_iters, self.num_grad_iters, current_flags())
+        init = self._modules["init"]       # a third of the time of an attribute, which single small images notice
+        projection = init._modules["linear"]._modules["linear"]
+        return native("layer", (x, init.h0, projection.weight, projection.bias), self.groups, self.filter_channels, self.source_channels,
+                      self.eps, self.num_iters, self.num_grad_iters, current_flags())
 
     # ----------------------------------------------------------------- interface
 

@@ -21,6 +21,7 @@ from typing import Optional, Sequence
 
 import torch
 from torch import Tensor
+from torch.overrides import handle_torch_function, has_torch_function
 
 from . import _lib
 
@@ -145,6 +146,42 @@ def _warn_if_generic(desc, flags: int) -> None:
             f"({desc.D},{desc.H},{desc.W}) runs on the kernels for any geometry (several times slower per "
             "voxel); the depthwise ones cover 3x3x3 volumes up to 256 columns and 5x5 / 3x3 images up to 512",
             RuntimeWarning, stacklevel=3)
+
+
+class _Traced(torch.autograd.Function):
+    """A call of the host extension as one operator of a traced graph, which cannot look into it and would
+    otherwise keep the uninitialised outputs it sees being allocated."""
+
+    @staticmethod
+    def forward(ctx, name, *args):
+        inner = [a.detach().requires_grad_(a.requires_grad) if isinstance(a, Tensor) else a for a in args]
+        with torch.enable_grad():
+            out = getattr(_lib.load_ext(), name)(*inner)
+        ctx.inner, ctx.out = inner, out
+        return out.detach()
+
+    @staticmethod
+    def backward(ctx, gout):
+        if torch.is_grad_enabled():
+            raise RuntimeError("double backward through a traced call is not supported")
+        wanted = [i for i, a in enumerate(ctx.inner) if isinstance(a, Tensor) and a.requires_grad]
+        grads = dict(zip(wanted, torch.autograd.grad(ctx.out, [ctx.inner[i] for i in wanted], gout, retain_graph=True,
+                                                     allow_unused=True)))
+        return (None, *(grads.get(i) for i in range(len(ctx.inner))))
+
+
+_is_tracing = torch._C._is_tracing
+
+
+def native(name: str, tensors: tuple, *args) -> Tensor:
+    """Calls a function of the host extension (`csrc/ndc_torch.cpp`), which by itself is invisible to
+    tracing and to tensor subclasses, on `tensors` (or None) and further arguments."""
+    if _is_tracing():
+        return _Traced.apply(name, *tensors, *args)
+    fn = getattr(_lib._ext or _lib.load_ext(), name)
+    if type(tensors[0]) is not Tensor and has_torch_function(tensors):
+        return handle_torch_function(fn, tensors, *tensors, *args)
+    return fn(*tensors, *args)
 
 
 def current_flags() -> int:

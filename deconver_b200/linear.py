@@ -17,7 +17,7 @@ from typing import Optional
 import torch
 from torch import nn
 
-from ._lib import load_ext
+from .functional import native
 
 _DTYPES = (torch.float32, torch.bfloat16)
 
@@ -45,6 +45,6 @@ class Linear(nn.Module):
         bias = self.linear.bias
         operands = native_operands(x, self.linear.weight)
         if operands is not None and (bias is not None or operands[0].dtype == torch.bfloat16):
-            return load_ext().linear(*operands, bias)
+            return native("linear", (*operands, bias))
         shape = x.shape
         return self.linear(self.flatten(x)).view(shape[0], -1, *shape[2:])

@@ -17,7 +17,7 @@ import torch
 from torch import nn
 from torch.nn.modules.utils import _pair
 
-from ._lib import load_ext
+from .functional import native
 from .linear import _DTYPES, Linear, native_operands
 
 
@@ -25,7 +25,7 @@ def bias_gelu(h: torch.Tensor, bias: Optional[torch.Tensor]) -> torch.Tensor:
     """``gelu(h + bias)`` over the channel axis (dim 1) of a CUDA float32 / bfloat16 tensor."""
     if not h.is_cuda or h.dtype not in _DTYPES:
         raise RuntimeError("bias_gelu runs on CUDA float32 / bfloat16 tensors only")
-    return load_ext().bias_gelu(h, bias)
+    return native("bias_gelu", (h, bias))
 
 
 class MLP(nn.Module):
@@ -49,6 +49,5 @@ class MLP(nn.Module):
         operands = native_operands(x, first.linear.weight) if type(first) is Linear else None
         if operands is None or not isinstance(act, nn.GELU) or act.approximate != "none":
             return self.block(x)
-        ext = load_ext()
-        a = ext.bias_gelu(ext.linear(*operands, None), first.linear.bias)
+        a = native("bias_gelu", (native("linear", (*operands, None)), first.linear.bias))
         return drop2(second(drop1(a)))

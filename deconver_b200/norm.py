@@ -16,7 +16,7 @@ from typing import Optional
 import torch
 from torch import Tensor, nn
 
-from ._lib import load_ext
+from .functional import native
 
 __all__ = ["InstanceNorm1d", "InstanceNorm2d", "InstanceNorm3d", "instance_norm"]
 
@@ -32,7 +32,7 @@ def instance_norm(x: Tensor, weight: Optional[Tensor] = None, bias: Optional[Ten
         raise NotImplementedError(f"deconver_b200: instance norm of {x.dtype} is not supported")
     if x.dim() < 3:
         raise ValueError("instance norm expects (batch, channels, spatial...)")
-    return load_ext().instance_norm(x, weight, bias, float(eps))
+    return native("instance_norm", (x, weight, bias), float(eps))
 
 
 class _InstanceNorm(nn.Module):

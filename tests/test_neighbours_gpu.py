@@ -129,3 +129,33 @@ def test_tangents_are_refused(module, grad):
         p = next(net.parameters())
         with torch.no_grad(), pytest.raises(RuntimeError, match="forward-mode|jvp"):
             torch.func.functional_call(net, {next(iter(net.state_dict())): forward_ad.make_dual(p, torch.ones_like(p))}, x)
+
+
+@pytest.mark.filterwarnings("ignore::DeprecationWarning", "ignore::torch.jit.TracerWarning")
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("module", MODULES)
+def test_traced_modules_compute_what_the_modules_do(module, grad):
+    net, (x, y) = MODULES[module]().to(DEV), torch.rand(2, 2, 6, 4, 8, device=DEV)
+    with torch.set_grad_enabled(grad):
+        traced = torch.jit.trace(net, (x,))
+        assert torch.equal(traced(y), net(y))
+    if grad:
+        res = []
+        for f in (traced, net):
+            t = y.clone().requires_grad_(True)
+            net.zero_grad(set_to_none=True)
+            f(t).square().sum().backward()
+            res.append([t.grad] + [p.grad for p in net.parameters()])
+        assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
+@pytest.mark.parametrize("module", MODULES)
+def test_tensor_subclasses_stay(module):
+    class Tagged(torch.Tensor):
+        pass
+
+    net, x = MODULES[module]().to(DEV), torch.rand(2, 6, 4, 8, device=DEV, requires_grad=True)
+    y = net(x.as_subclass(Tagged))
+    assert type(y) is Tagged and torch.equal(y.as_subclass(torch.Tensor), net(x))
+    y.sum().backward()
+    assert x.grad is not None
