@@ -92,8 +92,14 @@ int check_pitch(const NdcDesc* d, int pitch, int out_pitch) {
     return NDC_OK;
 }
 
-bool tensor_cores(const NdcDesc* d, const ndc::Geo& g) {
-    return d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && !(d->flags & NDC_FLAG_RELU_FILTER) && ndc::tc::covers(g);
+// The kernels an update runs on; `at`: the OR of the addresses that decide about the tensor cores.
+int family_of(const NdcDesc* d, const ndc::Geo& g, uintptr_t at) {
+    const int path = path_of(d, g.W);   // g.W: the pitch
+    if (path == NDC_PATH_GENERIC) return tile_path(d, g) ? NDC_FAMILY_TILE : NDC_FAMILY_GENERIC;
+    // bfloat16 tensors with bfloat16 parameters: exact products on the tensor cores
+    if (d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && !(d->flags & NDC_FLAG_RELU_FILTER) && at % 8 == 0 && ndc::tc::covers(g))
+        return NDC_FAMILY_TENSOR;
+    return path == NDC_PATH_DEPTHWISE4_ROWS ? NDC_FAMILY_MARCH_ROWS : NDC_FAMILY_MARCH;
 }
 
 // Launches return long before their kernels run, so that a wait that ran out in one of them is
@@ -197,6 +203,13 @@ int ndc_query(const NdcDesc* desc, int32_t* path) {
     return NDC_OK;
 }
 
+int ndc_kernel_family(const NdcDesc* desc, int32_t pitch, int32_t* family) {
+    NDC_TRY(validate(desc));
+    NDC_TRY(check_pitch(desc, pitch, pitch));
+    if (family) *family = family_of(desc, ndc::make_geo(*desc, false, pitch, pitch), 0);
+    return NDC_OK;
+}
+
 int ndc_fwd(const NdcDesc* desc, const void* x, const void* z, const float* h, const float* bias,
             void* out, void* t1, void* stream) {
     NDC_TRY(validate(desc));
@@ -229,13 +242,13 @@ int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const vo
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
     typedef __nv_bfloat16 bf16;
-    if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
-        // bfloat16 tensors with bfloat16 parameters: exact products on the tensor cores
-        if (tensor_cores(desc, g) && (((uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0)) & 7) == 0) {
-            e = ndc::tc::forward(g, (const bf16*)x, (const bf16*)z, h, bias, (bf16*)out, (bf16*)t1, st);
-            if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (tensor core) launch");
-            return NDC_OK;
-        }
+    const int family = family_of(desc, g, (uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0));
+    if (family == NDC_FAMILY_TENSOR) {
+        e = ndc::tc::forward(g, (const bf16*)x, (const bf16*)z, h, bias, (bf16*)out, (bf16*)t1, st);
+        if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (tensor core) launch");
+        return NDC_OK;
+    }
+    if (family == NDC_FAMILY_MARCH || family == NDC_FAMILY_MARCH_ROWS) {
         bool handled = false;
         if (desc->dtype == NDC_F32)
             e = ndc::dw4::forward<float>(g, (const float*)x, (const float*)z, h, bias, (float*)out,
@@ -317,12 +330,12 @@ int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const v
     const ndc::Geo g = ndc::make_geo(*desc, bias != nullptr, pitch, gout_pitch);
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
-    if (path_of(desc, pitch) != NDC_PATH_GENERIC) {
+    const int family = family_of(desc, g, (uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (uintptr_t)gz | (gout_pitch == pitch ? (uintptr_t)gout : 0));
+    if (family != NDC_FAMILY_GENERIC && family != NDC_FAMILY_TILE) {
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) {
             typedef __nv_bfloat16 bf16;
-            if (tensor_cores(desc, g) && (((uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (uintptr_t)gz |
-                                           (gout_pitch == pitch ? (uintptr_t)gout : 0)) & 7) == 0) {
+            if (family == NDC_FAMILY_TENSOR) {
                 e = ndc::tc::backward_ratio(g, (const bf16*)x, (const bf16*)z, (const bf16*)t1, h, bias, (const bf16*)gout,
                                             (float*)((char*)workspace + p.off_gnum), (float*)((char*)workspace + p.off_gden),
                                             (bf16*)gz, p.pairs, st);

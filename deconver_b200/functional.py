@@ -126,7 +126,7 @@ _checked_tiled = set()     # geometries already known to run on the tiled kernel
 
 def _warn_if_generic(desc, flags: int) -> None:
     """Depthwise ratio-4 problems normally run on the tiled kernels; tell the user (once per
-    geometry class) when one falls outside them and takes the much slower generic kernels."""
+    geometry class) when one falls outside them and takes the slower tile or generic kernels."""
     if flags & _lib.FLAG_FORCE_GENERIC or desc.m != 1 or desc.sc != 4:
         return
     key = (desc.kD, desc.kH, desc.kW, desc.W > 256, desc.dtype)
@@ -135,17 +135,18 @@ def _warn_if_generic(desc, flags: int) -> None:
     seen = (desc.batch, desc.groups, desc.D, desc.H, desc.W, desc.kD, desc.kH, desc.kW, desc.dtype)
     if seen in _checked_tiled:
         return
-    path = ctypes.c_int32(-1)
-    status = _lib.load().ndc_query(desc, ctypes.byref(path))
-    if status == _lib.NDC_OK and path.value != _lib.PATH_GENERIC and len(_checked_tiled) < 4096:
+    family = ctypes.c_int32(-1)
+    status = _lib.load().ndc_kernel_family(desc, desc.W, ctypes.byref(family))
+    slower = {_lib.FAMILY_TILE: "the tile kernels (about half as fast per voxel)",
+              _lib.FAMILY_GENERIC: "the kernels for any geometry (several times slower per voxel)"}.get(family.value)
+    if status == _lib.NDC_OK and slower is None and len(_checked_tiled) < 4096:
         _checked_tiled.add(seen)
-    if status == _lib.NDC_OK and path.value == _lib.PATH_GENERIC:
+    if status == _lib.NDC_OK and slower is not None:
         _warned_generic.add(key)
         warnings.warn(
             f"deconver_b200: depthwise ratio-4 update with kernel ({desc.kD},{desc.kH},{desc.kW}) on "
-            f"({desc.D},{desc.H},{desc.W}) runs on the kernels for any geometry (several times slower per "
-            "voxel); the depthwise ones cover 3x3x3 volumes up to 256 columns and 5x5 / 3x3 images up to 512",
-            RuntimeWarning, stacklevel=3)
+            f"({desc.D},{desc.H},{desc.W}) runs on {slower}; the depthwise ones cover 3x3x3 volumes up to 256 "
+            "columns and 5x5 / 3x3 images up to 512", RuntimeWarning, stacklevel=3)
 
 
 class _Traced(torch.autograd.Function):

@@ -60,14 +60,25 @@ enum NdcFlags {
                                    launched, where the depthwise kernels do not apply        */
 };
 
-/* Which family of kernels a geometry runs on (informational; results are the same). */
+/* Whether the depthwise ratio-4 kernels take a geometry, and how they run over it.  (Which kernels
+ * an update runs on in the end, flags and type included: ndc_kernel_family.) */
 enum NdcPath {
-    NDC_PATH_GENERIC = 0, /* any m, sc <= 16, any odd kernel with <= 343 taps (3x3x3, 1x5x5 and
-                             1x3x3 kernels staged tile by tile)                              */
+    NDC_PATH_GENERIC = 0, /* no: any m, sc <= 16, any odd kernel with <= 343 taps             */
     NDC_PATH_DEPTHWISE4 = 1, /* m = 1, sc = 4, kernel 3x3x3, 1x5x5 or 1x3x3: tiled, fused    */
     NDC_PATH_DEPTHWISE4_ROWS = 2 /* the same kernels marching down the rows of 2-D images:
                                     5x5 or 3x3, up to 512 columns, at least 8 rows, enough
                                     images in the batch to fill a 32-thread CTA             */
+};
+
+/* The kernels an update runs on.  They compute the same sums of float32 products in different orders. */
+enum NdcFamily {
+    NDC_FAMILY_GENERIC = 0,    /* one thread per element, anything within the limits          */
+    NDC_FAMILY_TILE = 1,       /* any m, sc <= 16 with 3x3x3, 1x5x5 and 1x3x3 kernels          */
+    NDC_FAMILY_MARCH = 2,      /* NDC_PATH_DEPTHWISE4                                         */
+    NDC_FAMILY_MARCH_ROWS = 3, /* NDC_PATH_DEPTHWISE4_ROWS                                    */
+    NDC_FAMILY_TENSOR = 4      /* tensor cores: NDC_BF16 with NDC_FLAG_BF16_PARAMS, where large
+                                  enough; the forward and the first step of the backward, the rest
+                                  of which marches                                            */
 };
 
 /*
@@ -119,6 +130,10 @@ int ndc_probe_wait(uint32_t limit_us, void *stream);
  * (deconver/deconvolution/kernels.py:114-163).
  */
 int ndc_query(const NdcDesc *desc, int32_t *path);
+
+/* Writes the NdcFamily of ndc_fwd_rows / ndc_bwd_rows for rows of `pitch` elements (desc->W: no padding)
+ * and tensors aligned to 16 bytes; the entry points decide by the same function.  Host-only. */
+int ndc_kernel_family(const NdcDesc *desc, int32_t pitch, int32_t *family);
 
 /*
  * Forward of one update: writes `out` and `t1` (t1 is what backward needs, besides x and z).

@@ -1,16 +1,19 @@
 """The tensor-core forward (bfloat16 tensors, filter and bias) against the FMA kernels, which take the
 same values as float32 parameters: edges of bands, chunks, blocks of eight columns and MMA tiles."""
 
+import ctypes
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 import torch
 
 import deconver_b200 as dcb
-from conftest import ROOT
+from conftest import ROOT, max_norm_error
 from deconver_b200 import _lib
 from deconver_b200 import functional as Fn
+from oracle import c_oracle
 from oracle import ndc_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -84,6 +87,38 @@ def test_gradients_match_the_fma_kernels(case):
         assert ((a - r).norm() / r.norm()).item() < 5e-3, name
 
 
+def _family(C, ks, B, spatial, flags, relu=True):
+    lib, family = _lib.load(), ctypes.c_int32(-1)
+    desc = _lib.make_desc(B, C, 1, 4, spatial, ks, 1e-16, relu, _lib.NDC_BF16, flags)
+    assert lib.ndc_kernel_family(desc, lib.ndc_row_pitch(desc), ctypes.byref(family)) == _lib.NDC_OK
+    return family.value
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "C%d_k%d_b%d_%s" % (c[0], c[1][0], c[2], "x".join(map(str, c[3]))))
+def test_update_against_the_oracle(case):
+    """Forward and every gradient on the tensor cores against the C oracle in 64 bits on the same bfloat16
+    values.  `out`, of positive terms, element by element: t1 and out are each rounded once (2^-8).  The
+    gradients have sums that cancel: largest error over the largest value, as for every bfloat16 update."""
+    C, ks, B, spatial = case
+    assert _family(C, ks, B, spatial, _lib.FLAG_BF16_PARAMS) == _lib.FAMILY_TENSOR
+    assert _family(C, ks, B, spatial, 0) in (_lib.FAMILY_MARCH, _lib.FAMILY_MARCH_ROWS)
+    gen = torch.Generator().manual_seed(C)
+    x = torch.rand(B, C, *spatial, generator=gen).bfloat16()
+    z = (torch.randn(B, 4 * C, *spatial, generator=gen) * 0.5 + 0.3).bfloat16()
+    h = (torch.rand(C, 4, *ks, generator=gen) / 27).bfloat16()
+    bias = (torch.randn(4 * C, generator=gen) * 0.1).bfloat16()
+    g = torch.randn(B, 4 * C, *spatial, generator=gen).bfloat16()
+    t = [v.to("cuda:0").requires_grad_(True) for v in (x, z, h, bias)]
+    out = dcb.deconv_update(*t, groups=C, m=1, sc=4, eps=1e-16, relu_input=True)
+    out.backward(g.to("cuda:0"))
+    cfg = dict(groups=C, m=1, sc=4, eps=1e-16, relu_input=True)
+    args = [v.double().numpy() for v in (x, z, h, bias)]
+    ref, _ = c_oracle.forward(*args, **cfg)
+    assert (np.abs(out.detach().double().cpu().numpy() - ref) <= (2.0 ** -7 + 2.0 ** -9) * ref).all()
+    for name, a, r in zip(("gx", "gz", "gh", "gb"), (v.grad for v in t), c_oracle.backward(*args, g.double().numpy(), **cfg)):
+        assert max_norm_error(a.float().cpu().numpy(), r) < 2e-2, name
+
+
 # volumes and images, rows of whole blocks of eight columns and not, several bands and chunks of planes
 CANCELLING = [(150, (3, 3, 3), 1, (18, 17, 20)), (200, (3, 3, 3), 1, (7, 9, 64)), (50, (5, 5), 4, (130, 128)),
               (45, (5, 5), 14, (77, 68)), (70, (3, 3), 3, (60, 252))]
@@ -98,6 +133,7 @@ def test_rectified_sources_leave_no_rounding_behind(case, mixed, live):
     further off than its roundings to bfloat16 (2^-8 each) and a float32 sum's share of one.  `mixed`: the
     channels' biases differ by factors of ten, so that what is left is small beside what cancelled."""
     C, ks, B, spatial = case
+    assert _family(C, ks, B, spatial, _lib.FLAG_BF16_PARAMS) == _lib.FAMILY_TENSOR
     gen = torch.Generator().manual_seed(C)
     x = torch.rand(B, C, *spatial, generator=gen).bfloat16()
     bias = torch.rand(4 * C, generator=gen) * 0.2 + 0.9
@@ -152,6 +188,7 @@ def test_padding_of_the_source_is_not_read(ks, B, spatial, pitch, relu):
     x, z = (torch.zeros(B, n, *lead, pitch, device=dev, dtype=torch.bfloat16) for n in (C, 4 * C))
     x[..., :W] = torch.rand(B, C, *lead, W, device=dev, generator=gen)
     z[..., :W] = torch.rand(B, 4 * C, *lead, W, device=dev, generator=gen)
+    assert _family(C, ks, B, spatial, _lib.FLAG_BF16_PARAMS, relu) == _lib.FAMILY_TENSOR
     h = (torch.rand(C, 4, *ks, device=dev, generator=gen) / 27).bfloat16().float()
     desc = _lib.make_desc(B, C, 1, 4, spatial, ks, 1e-16, relu, _lib.NDC_BF16, _lib.FLAG_BF16_PARAMS)
     res = []
