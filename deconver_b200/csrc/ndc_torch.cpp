@@ -9,6 +9,7 @@
 // see the figures at their section.
 #include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/ops/convolution_backward.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/relu.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -16,7 +17,9 @@
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "ndc_b200.h"
@@ -129,45 +132,90 @@ void channel_gemm(const Tensor& w, bool transpose, const Tensor& x, Tensor& y, i
     TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection GEMM failed (cuBLAS status ", (int)st, ")");
 }
 
+// The weight gradient of a 1x1 projection is a product of two wide matrices along their positions, and no
+// one way is the fastest over the channels, batches and positions that occur:
+//   Kernel       ndc_proj_wgrad: any row length; its MMAs' rate and tiles of 128 x 64 bound it for many channels
+//   Product      one library product per sample, where samples and tiles of 128 x 128 fill the GPU
+//   Slices       a sample's positions in as many slices as fill the GPU, one batched library product each
+//   Convolution  the library's convolution backward, for rows that are not whole vectors and many channels
+// (Slices and Product are views of the tensors as they lie, float32 partial products, summed by ndc_proj_sum.)
+enum WgradRoute { kKernel = 0, kProduct = 1, kSlices = 2, kConvolution = 3 };
+struct WgradPlan { WgradRoute route; int64_t slices; };
+
+// Whole vectors: the least expected time, microseconds, of the first three.  The constants fit 1481
+// float32 and 1317 bfloat16 shapes (16 to 2048 channels, 1 to 16 samples of 343 to 262144 positions) to 11 - 33 %
+// rms; what they choose takes 1.07 times the best of all four ways and 0.66 (float32) and 0.76 (bfloat16) times
+// the library's convolution, which is up to 50 times slower than the best and cannot be foreseen.  (Fixed
+// limits on channels and batches, before: 1.29, 0.80 and 1.25, 0.88; 8 x (640 + 160) x 32768 in float32 took
+// 782 us, 217 now.)
+// Others (672 shapes): below the limit the kernel takes 0.05 - 0.9 times the library's convolution on the
+// average of a class of widths and batches, above it 1.0 - 3.5; a single sample is a plain product for the
+// library (1.3 - 3.8 from 20000 on).
+WgradPlan plan_weight_grad(int64_t batch, int64_t co, int64_t ci, int64_t n, bool bf16, int sms) {
+    if (n % (bf16 ? 8 : 4)) {
+        const int64_t limit = batch == 1 ? 20000 : batch <= 8 ? 200000 : bf16 ? 100000 : 30000;
+        return {co * ci >= limit ? kConvolution : kKernel, 1};
+    }
+    const auto tiles = [](int64_t v, int64_t t) { return (v + t - 1) / t; };
+    const double e = bf16 ? 2 : 4, bytes = (double)(co + ci) * n * e;                       // of a sample
+    const int64_t square = tiles(co, 128) * tiles(ci, 128);
+    // the library's products: CTAs of 128 x 128 outputs, each one chain along its positions
+    const double rate = bf16 ? 1180.0 : n % 8 ? 455.0 : 525.0;                              // positions per us
+    const double product = 14.0 + std::max((double)tiles(batch * square, sms) * n / rate, batch * bytes / 3.9e6);
+    const int64_t slices = std::min(tiles(sms, square), n / 1024);
+    const double sliced = slices < 2 ? product + 1.0
+                                     : 9.0 + batch * (5.5 + std::max(bytes / (bf16 ? 3.4e6 : 4.0e6),
+                                                                     bf16 ? 0.0 : std::max(1.0, (double)slices * square / sms) * n / slices / 770.0));
+    // ndc_proj_wgrad: see plan_wgrad there
+    const int64_t t = tiles(co, 128) * tiles(ci, 64), parts = std::max<int64_t>(1, std::min(tiles(4 * sms, t * batch), tiles(n, 512)));
+    const double flops = 2.0 * batch * n * t * 128 * 64, read = ((double)co * tiles(ci, 64) + (double)ci * tiles(co, 128)) * batch * n * e;
+    const double kernel = 7.3 + std::max(flops / (bf16 ? 272e6 : 134e6) / std::min(1.0, t * batch * parts / (2.0 * sms)), read / (bf16 ? 5.7e6 : 4.1e6)) +
+                          batch * parts * co * ci * 8 / (bf16 ? 1.8e6 : 1.4e6);
+    if (kernel <= product && kernel <= sliced) return {kKernel, 1};
+    return product <= sliced ? WgradPlan{kProduct, 1} : WgradPlan{kSlices, slices};
+}
+
 Tensor weight_grad(const Tensor& gy, const Tensor& x, const Tensor& w, int64_t batch, int64_t n) {
     Tensor gw = at::empty(w.sizes(), w.options());
     const int64_t co = w.size(0), ci = w.size(1);
-    if (!batch || !n) return gw.zero_();
+    if (!batch || !n || !co || !ci) return gw.zero_();
     const bool bf16 = gy.scalar_type() == at::kBFloat16;
-    // The library's tcgen05 GEMM is the faster one where it can load whole vectors and fill the GPU:
-    // its positions cut into `slices` per sample (views of the tensors as they lie), or, from 192
-    // input channels on, where the product is bound by the tensor cores (co * ci / (co + ci)
-    // multiply-adds per value read), one product per sample.  Everything else - rows that are not
-    // whole vectors, many samples of few channels - runs on the kernel of ndc_proj_wgrad.
-    int64_t slices = 1;
-    while (slices < 32 && n % (slices * 16) == 0 && n / (slices * 2) >= 2048) slices *= 2;
-    if (n % (bf16 ? 8 : 4) == 0 && (ci >= 192 || (batch <= 4 && slices >= 8))) {
-        if (ci >= 192 && batch * ((co + 127) / 128) * ((ci + 127) / 128) >= 64) slices = 1;
-        Tensor partial = at::empty({batch * slices, co, ci}, w.options().dtype(at::kFloat));
-        const float one = 1.0f, zero = 0.0f;
-        const cudaDataType_t type = bf16 ? CUDA_R_16BF : CUDA_R_32F;
-        const cublasComputeType_t compute = !bf16 && conv_tf32() ? CUBLAS_COMPUTE_32F_FAST_TF32 : CUBLAS_COMPUTE_32F;
-        at::NoTF32Guard plain;
-        cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
-        const int64_t calls = slices > 1 ? batch : 1, length = n / slices;
-        for (int64_t b = 0; b < calls; ++b) {
-            const size_t e = bf16 ? 2 : 4;
-            const cublasStatus_t st = cublasGemmStridedBatchedEx(
-                handle, CUBLAS_OP_T, CUBLAS_OP_N, (int)ci, (int)co, (int)length, &one,
-                static_cast<const char*>(ptr(x)) + b * ci * n * e, type, (int)n, (long long)(slices > 1 ? length : ci * n),
-                static_cast<const char*>(ptr(gy)) + b * co * n * e, type, (int)n, (long long)(slices > 1 ? length : co * n),
-                &zero, fptr(partial) + b * slices * co * ci, CUDA_R_32F, (int)ci, (long long)(co * ci),
-                (int)(slices > 1 ? slices : batch), compute, CUBLAS_GEMM_DEFAULT);
-            TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection gradient failed (cuBLAS status ", (int)st, ")");
-        }
-        if (batch * slices == 1 && !bf16) return partial.view(w.sizes());
-        check(ndc_proj_sum((int)(batch * slices), co * ci, dtype_code(gy), fptr(partial), ptr(gw), stream()), ndc_proj_last_error());
+    const WgradPlan plan = plan_weight_grad(batch, co, ci, n, bf16, at::cuda::getCurrentDeviceProperties()->multiProcessorCount);
+    if (plan.route == kConvolution)
+        return std::get<1>(at::convolution_backward(gy.view({batch, co, n}), x.view({batch, ci, n}), w.view({co, ci, 1}), at::nullopt, {1}, {0},
+                                                    {1}, false, {0}, 1, {false, true, false})).view(w.sizes());
+    if (plan.route == kKernel) {
+        const size_t bytes = ndc_proj_wgrad_workspace_bytes((int)batch, (int)co, (int)ci, n);
+        Tensor ws = at::empty({(int64_t)bytes}, w.options().dtype(at::kByte));
+        check(ndc_proj_wgrad((int)batch, (int)co, (int)ci, n, dtype_code(gy), conv_tf32() ? 1 : 0, ptr(gy), ptr(x),
+                             ptr(gw), ptr(ws), bytes, stream()), ndc_proj_last_error());
         return gw;
     }
-    const size_t bytes = ndc_proj_wgrad_workspace_bytes((int)batch, (int)co, (int)ci, n);
-    Tensor ws = at::empty({(int64_t)bytes}, w.options().dtype(at::kByte));
-    check(ndc_proj_wgrad((int)batch, (int)co, (int)ci, n, dtype_code(gy), conv_tf32() ? 1 : 0, ptr(gy), ptr(x),
-                         ptr(gw), ptr(ws), bytes, stream()), ndc_proj_last_error());
+    // slices of whole vectors, and what they leave
+    const int64_t slices = plan.slices, length = slices > 1 ? n / slices / 8 * 8 : n, rest = n - slices * length;
+    Tensor partial = at::empty({batch * slices, co, ci}, w.options().dtype(at::kFloat));
+    const cudaDataType_t type = bf16 ? CUDA_R_16BF : CUDA_R_32F;
+    const cublasComputeType_t compute = !bf16 && conv_tf32() ? CUBLAS_COMPUTE_32F_FAST_TF32 : CUBLAS_COMPUTE_32F;
+    at::NoTF32Guard plain;
+    cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
+    // `count` products along `k` positions, the first from position `at` of sample b on, the others
+    // further on in it (`length` apart) or in the samples after it
+    auto products = [&](int64_t b, int64_t at, int64_t k, bool samples, int64_t count, float beta) {
+        const float one = 1.0f;
+        const size_t e = bf16 ? 2 : 4;
+        const int64_t sx = samples ? ci * n : length, sy = samples ? co * n : length, out_step = samples ? slices : 1;
+        const cublasStatus_t st = cublasGemmStridedBatchedEx(
+            handle, CUBLAS_OP_T, CUBLAS_OP_N, (int)ci, (int)co, (int)k, &one, static_cast<const char*>(ptr(x)) + (b * ci * n + at) * e, type,
+            (int)n, (long long)sx, static_cast<const char*>(ptr(gy)) + (b * co * n + at) * e, type, (int)n, (long long)sy, &beta,
+            fptr(partial) + b * slices * co * ci, CUDA_R_32F, (int)ci, (long long)(out_step * co * ci), (int)count, compute, CUBLAS_GEMM_DEFAULT);
+        TORCH_CHECK(st == CUBLAS_STATUS_SUCCESS, "deconver_b200: projection gradient failed (cuBLAS status ", (int)st, ")");
+    };
+    if (slices == 1) products(0, 0, n, true, batch, 0.0f);
+    else
+        for (int64_t b = 0; b < batch; ++b) products(b, 0, length, false, slices, 0.0f);
+    if (rest) products(0, slices * length, rest, true, batch, 1.0f);
+    if (batch * slices == 1 && !bf16) return partial.view(w.sizes());
+    check(ndc_proj_sum((int)(batch * slices), co * ci, dtype_code(gy), fptr(partial), ptr(gw), stream()), ndc_proj_last_error());
     return gw;
 }
 
@@ -672,6 +720,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod) {
     mod.def("linear", &linear, py::call_guard<py::gil_scoped_release>());
     mod.def("bias_gelu", &bias_gelu, py::call_guard<py::gil_scoped_release>());
     mod.def("instance_norm", &instance_norm, py::call_guard<py::gil_scoped_release>());
+    mod.def("weight_grad_route", [](int64_t batch, int64_t co, int64_t ci, int64_t n, bool bf16, int sms) {
+        return (int)plan_weight_grad(batch, co, ci, n, bf16, sms).route;
+    });
     mod.def("timing_enable", &timing_enable);
     mod.def("timing_collect", &timing_collect);
 }

@@ -87,3 +87,33 @@ def test_row_padding(rows, W, pitch, dtype):
     assert lib.ndc_unpad_rows(rows, W, pitch, code, p.data_ptr(), y.data_ptr(), st) == 0
     assert torch.equal(p[:, :W], x) and torch.equal(y, x) and not p[:, W:].any()
     assert lib.ndc_pad_rows(rows, W, W - 1, code, x.data_ptr(), p.data_ptr(), st) == 1
+
+
+KERNEL, PRODUCT, SLICES, CONVOLUTION = range(4)      # WgradRoute
+
+
+@pytest.mark.parametrize("dtype,tf32,tol", [(torch.float32, True, 2e-3), (torch.float32, False, 1e-5), (torch.bfloat16, True, 6e-3)],
+                         ids=["tf32", "f32", "bf16"])
+@pytest.mark.parametrize("batch,co,ci,n,route", [
+    (4, 128, 32, 16384, KERNEL), (3, 40, 24, 1001, KERNEL), (2, 96, 24, 4095, KERNEL), (1, 192, 48, 4095, KERNEL),
+    (8, 640, 160, 4096, PRODUCT), (16, 288, 72, 4096, PRODUCT), (1, 2048, 512, 512, PRODUCT), (16, 48, 192, 4096, PRODUCT),
+    (1, 256, 64, 110592, SLICES), (1, 96, 384, 32768, SLICES), (3, 130, 70, 49992, SLICES),
+    (1, 384, 96, 4095, CONVOLUTION), (2, 512, 512, 343, CONVOLUTION), (9, 640, 160, 101, CONVOLUTION),
+])
+def test_weight_gradient_of_every_route(dtype, tf32, tol, batch, co, ci, n, route):
+    """Each side of each line of the dispatch, slices with a rest among them (49992 positions)."""
+    dev = torch.device("cuda:0")
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    assert _lib.load_ext().weight_grad_route(batch, co, ci, n, dtype == torch.bfloat16, sms) == route
+    gen = torch.Generator(device=dev).manual_seed(co + n)
+    lin = dcb.Linear(ci, co).to(dev, dtype)
+    x, g = torch.rand(batch, ci, n, device=dev, generator=gen).to(dtype), torch.randn(batch, co, n, device=dev, generator=gen).to(dtype)
+    old = torch.backends.cudnn.allow_tf32
+    torch.backends.cudnn.allow_tf32 = tf32
+    try:
+        (gw,) = torch.autograd.grad(lin(x), lin.linear.weight, g)
+    finally:
+        torch.backends.cudnn.allow_tf32 = old
+    ref = torch.einsum("bon,bcn->oc", g.double(), x.double())
+    assert gw.dtype == dtype and gw.shape == (co, ci, 1)
+    assert ((gw[:, :, 0].double() - ref).norm() / ref.norm()).item() < tol
