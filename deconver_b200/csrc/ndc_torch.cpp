@@ -136,18 +136,18 @@ void channel_gemm(const Tensor& w, bool transpose, const Tensor& x, Tensor& y, i
 // one way is the fastest over the channels, batches and positions that occur:
 //   Kernel       ndc_proj_wgrad: any row length; its MMAs' rate and tiles of 128 x 64 bound it for many channels
 //   Product      one library product per sample, where samples and tiles of 128 x 128 fill the GPU
-//   Slices       a sample's positions in as many slices as fill the GPU, one batched library product each
+//   Slices       a sample's positions in 32 or 16 slices (more were slower: 2 x (256 + 64) x 262144 takes 136 us
+//                with 32, 157 with 74), one batched library product per sample
 //   Convolution  the library's convolution backward, for rows that are not whole vectors and many channels
 // (Slices and Product are views of the tensors as they lie, float32 partial products, summed by ndc_proj_sum.)
 enum WgradRoute { kKernel = 0, kProduct = 1, kSlices = 2, kConvolution = 3 };
 struct WgradPlan { WgradRoute route; int64_t slices; };
 
-// Whole vectors: the least expected time, microseconds, of the first three.  The constants fit 1481
-// float32 and 1317 bfloat16 shapes (16 to 2048 channels, 1 to 16 samples of 343 to 262144 positions) to 11 - 33 %
-// rms; what they choose takes 1.07 times the best of all four ways and 0.66 (float32) and 0.76 (bfloat16) times
-// the library's convolution, which is up to 50 times slower than the best and cannot be foreseen.  (Fixed
-// limits on channels and batches, before: 1.29, 0.80 and 1.25, 0.88; 8 x (640 + 160) x 32768 in float32 took
-// 782 us, 217 now.)
+// Whole vectors: the least expected time, microseconds, of the first three, by constants fitted to 1481
+// float32 and 1317 bfloat16 shapes (16 to 2048 channels, 1 to 16 samples of 343 to 262144 positions).  On 400
+// other shapes of either type the choice takes 42 and 51 ms together, the library's convolution 88 and
+// 94, fixed limits on channels and batches (before) 55 and 57; by more than a tenth the convolution is
+// faster on 39 and 7 (before: 135 and 76), but it is up to 50 times slower on others, which cannot be foreseen.
 // Others (672 shapes): below the limit the kernel takes 0.05 - 0.9 times the library's convolution on the
 // average of a class of widths and batches, above it 1.0 - 3.5; a single sample is a plain product for the
 // library (1.3 - 3.8 from 20000 on).
@@ -162,10 +162,10 @@ WgradPlan plan_weight_grad(int64_t batch, int64_t co, int64_t ci, int64_t n, boo
     // the library's products: CTAs of 128 x 128 outputs, each one chain along its positions
     const double rate = bf16 ? 1180.0 : n % 8 ? 455.0 : 525.0;                              // positions per us
     const double product = 14.0 + std::max((double)tiles(batch * square, sms) * n / rate, batch * bytes / 3.9e6);
-    const int64_t slices = std::min(tiles(sms, square), n / 1024);
+    const int64_t slices = std::min<int64_t>(square < 4 ? 32 : 16, n / 1024);
     const double sliced = slices < 2 ? product + 1.0
-                                     : 9.0 + batch * (5.5 + std::max(bytes / (bf16 ? 3.4e6 : 4.0e6),
-                                                                     bf16 ? 0.0 : std::max(1.0, (double)slices * square / sms) * n / slices / 770.0));
+                                     : 9.0 + (n % (8 * slices) ? 8.0 : 0.0) +
+                                           batch * (5.5 + std::max(bytes / 5.0e6, 2.0 * co * ci * n / (bf16 ? 600e6 : 370e6)));
     // ndc_proj_wgrad: see plan_wgrad there
     const int64_t t = tiles(co, 128) * tiles(ci, 64), parts = std::max<int64_t>(1, std::min(tiles(4 * sms, t * batch), tiles(n, 512)));
     const double flops = 2.0 * batch * n * t * 128 * 64, read = ((double)co * tiles(ci, 64) + (double)ci * tiles(co, 128)) * batch * n * e;
