@@ -21,6 +21,21 @@ inline std::atomic<unsigned long long>& launch_counter() {
 // Call once after every kernel launch.
 inline void launched(int n = 1) { launch_counter().fetch_add(n, std::memory_order_relaxed); }
 
+// Multiprocessors of the current device (148 on B200), asked once per process; 148 where no
+// device answers (planning on a host without a GPU).
+inline int num_sms() {
+    static const int n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) {
+            (void)cudaGetLastError();   // planning must not leave an error behind
+            v = 148;
+        }
+        return v;
+    }();
+    return n;
+}
+
 // Geometry handed to every kernel by value.
 struct Geo {
     int B, G, m, sc;

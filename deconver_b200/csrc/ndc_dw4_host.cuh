@@ -10,20 +10,6 @@
 namespace ndc {
 namespace dw4 {
 
-// Multiprocessors of the current device (148 on B200), asked once per process; 148 where no
-// device answers (planning on a host without a GPU).
-inline int num_sms() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) {
-            (void)cudaGetLastError();   // planning must not leave an error behind
-            v = 148;
-        }
-        return v;
-    }();
-    return n;
-}
 constexpr size_t kSmemTwoPerSM = 112 * 1024;   // lets two CTAs share an SM
 constexpr size_t kSmemMax = 227 * 1024;
 
@@ -357,7 +343,7 @@ inline int rows_class(const Geo& g) {
     const int images = NQ > 64 ? 1 : std::min(g.B, 64 / NQ);   // per CTA
     const long long image = (long long)g.H * g.W;       // elements of one channel
     if ((images * (long long)g.G + 1) * SCH * image >= (1LL << 31)) return 0;
-    if (g.H < 32 && (long long)g.G * ((g.B + images - 1) / images) < 148) return 0;
+    if (g.H < 32 && (long long)g.G * ((g.B + images - 1) / images) < num_sms()) return 0;
     const int strips = images * NQ;
     if (g.kH == 5 && images == 1 && strips > 32 && strips <= 48) return 0;
     return strips > 64 ? 128 : strips > 32 ? 64 : strips >= 24 ? 32 : 0;

@@ -243,7 +243,7 @@ gb_kernel(Geo g, const T* __restrict__ gz, float* __restrict__ gb) {
 
 inline int grid_for(long long total) {
     long long blocks = (total + kThreads - 1) / kThreads;
-    const long long cap = 148LL * 64;  // grid-stride beyond 64 blocks per SM
+    const long long cap = 64LL * num_sms();  // grid-stride beyond 64 blocks per SM
     return (int)(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
 }
 

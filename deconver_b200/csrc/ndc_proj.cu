@@ -259,7 +259,7 @@ void plan_wgrad(int batch, int co, int ci, long long n, WgradParams& P) {
     P.tiles_o = (co + TO - 1) / TO;
     P.tiles_c = (ci + TC - 1) / TC;
     const long long tiles = (long long)P.tiles_o * P.tiles_c * batch;
-    long long want = (4LL * 148 + tiles - 1) / tiles;
+    long long want = (4LL * ndc::num_sms() + tiles - 1) / tiles;
     const long long most = (n + 511) / 512;
     if (want > most) want = most;
     if (want < 1) want = 1;

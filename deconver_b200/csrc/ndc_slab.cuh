@@ -69,13 +69,7 @@ __device__ __forceinline__ void cta_sum2(float& a, float& b, float* scratch) {
 
 // parts per slab: enough CTAs for about four per multiprocessor, parts of at least 4096 elements
 inline int choose_split(long long slabs, long long sp) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-        (void)cudaGetLastError();
-        sms = 148;
-    }
-    long long want = (4LL * sms + slabs - 1) / slabs;
+    long long want = (4LL * num_sms() + slabs - 1) / slabs;
     const long long most = sp / 4096 > 0 ? sp / 4096 : 1;
     if (want > most) want = most;
     if (want > kMaxSplit) want = kMaxSplit;

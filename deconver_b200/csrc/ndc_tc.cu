@@ -79,12 +79,12 @@ bool plan(const Geo& g, bool source, Band& b) {
     if ((b.TH + KH - 1) * row >= (1LL << 31)) return false;
     const long long per = (long long)g.B * g.G * b.nth;
     long long ndc = 1;
-    const long long want = (4 * 148 + per - 1) / per, finest = std::max(1, g.D / (6 * (KD / 2)));
+    const long long sms = num_sms(), want = (4 * sms + per - 1) / per, finest = std::max(1, g.D / (6 * (KD / 2)));
     ndc = std::max(ndc, std::min(want, finest));
     if (source || (g.W % 8 == 0 && g.Wv == g.W)) {
         const float halo = source ? 7.0f : KD > 3 ? 12.0f : 4.0f;
         auto time = [&](long long n) {
-            const long long planes = (g.D + n - 1) / n, ctas = (per * ((g.D + planes - 1) / planes) + 147) / 148;
+            const long long planes = (g.D + n - 1) / n, ctas = (per * ((g.D + planes - 1) / planes) + sms - 1) / sms;
             return ((float)planes + halo) * (source ? (float)(ctas / 2) + (ctas % 2 ? 0.65f : 0.0f) : (float)ctas);
         };
         float least = 0.98f * time(ndc);

@@ -694,7 +694,7 @@ inline long long tiles_of(const TileGeo& t) { return (long long)t.ntw * t.nth * 
 inline int corr_splits(const Geo& g, const TileGeo& t) {
     const long long combos = (long long)g.G * g.m * source_blocks(g), work = (long long)g.B * tiles_of(t);
     // one CTA of 240 registers per thread fits a multiprocessor: one full round of the GPU
-    long long s = 148 / combos;
+    long long s = num_sms() / combos;
     if (s > work) s = work;
     return (int)std::max(1LL, s);
 }
