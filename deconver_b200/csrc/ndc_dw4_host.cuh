@@ -331,8 +331,10 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
 // the CTA size class (strips of 4 per CTA), or 0 where the band kernels stay:
 //  - a batch too small to fill even the small CTA, or a band whose 32-bit offsets would overflow;
 //  - fewer than 32 rows and fewer CTAs than SMs: so short a march is not cut, and the band
-//    kernels have more blocks (bf16 8 x 40 groups of 28x30, 5x5: 213 -> 181 us for a training
-//    update of which ~100 us are launches; 16 x 512 of 16x16 stays, 403 against 671 us);
+//    kernels have more blocks (bf16 8 x 40 groups of 28x30, 5x5: 159 -> 107 us for a training
+//    update; 16 x 512 of 16x16 stays, 403 against 671 us).  3x3 likewise (73 shapes of several images
+//    per CTA: 1.13 of the bands' time, 0.83 - 1.58), but one image that fills a CTA marches in 0.84 of it
+//    (17 shapes, 0.51 - 1.09) and keeps its rows;
 //  - 5x5 on images of 129..192 columns, where one image leaves a quarter or more of the 64 lanes
 //    idle and a second does not fit (5 x 24 of 203x171: 878 -> 708 us; 3x3 there is 563 against
 //    580 us for the bands and keeps its rows).
@@ -343,7 +345,7 @@ inline int rows_class(const Geo& g) {
     const int images = NQ > 64 ? 1 : std::min(g.B, 64 / NQ);   // per CTA
     const long long image = (long long)g.H * g.W;       // elements of one channel
     if ((images * (long long)g.G + 1) * SCH * image >= (1LL << 31)) return 0;
-    if (g.H < 32 && (long long)g.G * ((g.B + images - 1) / images) < num_sms()) return 0;
+    if (g.H < 32 && (g.kH == 5 || images > 1) && (long long)g.G * ((g.B + images - 1) / images) < num_sms()) return 0;
     const int strips = images * NQ;
     if (g.kH == 5 && images == 1 && strips > 32 && strips <= 48) return 0;
     return strips > 64 ? 128 : strips > 32 ? 64 : strips >= 24 ? 32 : 0;

@@ -41,6 +41,12 @@ def test_image_kernels_match_the_generic_ones(case, dtype, tol):
         assert max_norm_error(a.float().cpu().numpy(), r.float().cpu().numpy()) < tol, name
 
 
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)], ids=["f32", "bf16"])
+@pytest.mark.parametrize("case", [(1, 5, 3, 20, 200), (2, 3, 3, 31, 129), (2, 3, 3, 31, 128), (1, 3, 3, 8, 96)], ids=lambda c: "x".join(map(str, c)))
+def test_short_3x3_images_of_one_per_cta(case, dtype, tol):
+    test_image_kernels_match_the_generic_ones(case, dtype, tol)
+
+
 @pytest.mark.parametrize("k,spatial", [(5, (16, 16)), (5, (40, 128)), (3, (40, 171)), (3, (8, 8, 8)), (3, (9, 20, 33)), (7, (12, 12))])
 def test_inference_rectifies_the_filter_as_training_does(k, spatial):
     torch.manual_seed(0)
