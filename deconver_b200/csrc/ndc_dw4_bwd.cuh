@@ -18,8 +18,6 @@
 
 #include <type_traits>
 
-#include <type_traits>
-
 #include "ndc_dw4_common.cuh"
 
 namespace ndc {
@@ -682,7 +680,7 @@ __device__ __forceinline__ int swz2(int chunk) {
 // CTAs per SM the packed K kernel is built for: 256 threads in all.
 template <int NT> constexpr int kconv2_min_blocks() { return NT >= 256 ? 1 : NT >= 128 ? 2 : NT >= 64 ? 4 : 8; }
 
-template <typename T, int KD, int KH, int KW, int NT, int VK, int MAXC, int AL, bool WGRAD, int WQ>
+template <typename T, int KD, int KH, int KW, int NT, int MAXC, int AL, bool WGRAD, int WQ>
 __global__ void __launch_bounds__(NT, kconv2_min_blocks<NT>()) kconv2_kernel(const Kconv2Params P) {
     constexpr bool VEC = AL != kScalar, PADDED = AL == kPadded;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;

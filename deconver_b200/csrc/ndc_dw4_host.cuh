@@ -123,10 +123,6 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
                      (g.Wo != g.W || aligned_for_vec(out, dtype)) && aligned_for_vec(t1, dtype);
     const bool whole = vec && g.Wv == g.W && g.Wo == g.W;   // no padding: compile-time widths apply
     // widths that occur in the published configurations get kernels with a compile-time width
-    if constexpr (KD > 1 && KH > 1 && S::NT == 256) {
-        if (whole && g.W == 64) return launch_fwd<T, KD, KH, KW, S, kVector, 16>(P, smem, BC, st);
-        if (whole && g.W == 128) return launch_fwd<T, KD, KH, KW, S, kVector, 32>(P, smem, BC, st);
-    }
     if constexpr (KD > 1 && KH == 1) {   // rows kernels: 256, 128 and 64 columns
         if (whole && g.W == 4 * S::NT) return launch_fwd<T, KD, KH, KW, S, kVector, S::NT>(P, smem, BC, st);
         if (whole && S::NT == 64 && g.W == 128) return launch_fwd<T, KD, KH, KW, S, kVector, 32>(P, smem, BC, st);
@@ -141,28 +137,28 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
 
 // Threads (and prefetch registers, in quads per thread) of the three backward kernels.
 // Bands: a CTA owns a band of rows of every plane.  kconv: 48 strip slots x 4 channel lanes.
-// Kconv2NT / Kconv2VK: threads and strip length of the packed K kernel (3x3x3 volumes): a strip
-// of VK voxels per group of 4 channel lanes.  Kconv2WideNT: the CTA used instead for rows of more
+// Kconv2NT: threads of the packed K kernel (3x3x3 volumes): a strip of VK voxels per group of 4 channel
+// lanes.  Kconv2WideNT: the CTA used instead for rows of more
 // than 64 voxels (0: none), where the narrow one would be left with bands of one or two rows.
 // Kconv2MAXC: 16-byte source chunks a thread copies per plane, at most (bands shrink to fit).
 struct BwdBands {
     static constexpr int RatioNT = 128, RatioMAXX = 2, KconvNT = 192, GzNT = 128, GzMAXX = 4;
-    static constexpr int Kconv2NT = 128, Kconv2VK = 8, Kconv2MAXC = 6, Kconv2WideNT = 256, Kconv2WideMAXC = 6;
+    static constexpr int Kconv2NT = 128, Kconv2MAXC = 6, Kconv2WideNT = 256, Kconv2WideMAXC = 6;
 };
 // Rows: one-row planes of NQ 4-voxel strips (2-D images run as volumes, see FwdRows).
 template <int NQ_> struct BwdRows {
     static constexpr int RatioNT = NQ_, RatioMAXX = 1, KconvNT = 2 * NQ_, GzNT = NQ_, GzMAXX = 1;
-    static constexpr int Kconv2VK = 8, Kconv2MAXC = 4, Kconv2WideNT = 0, Kconv2WideMAXC = 0;   // 3x3: kconv2_threads
+    static constexpr int Kconv2MAXC = 4, Kconv2WideNT = 0, Kconv2WideMAXC = 0;   // 3x3: kconv2_threads
 };
 // Small volumes (3x3x3): narrower CTAs where they cover the same bands as the default ones
 // (a wide CTA would mostly idle on a band of 16 or 8 short rows).
 struct BwdSmall16 {   // bands of up to 64 strips of 4 (16 x 16 rows)
     static constexpr int RatioNT = 64, RatioMAXX = 2, KconvNT = 128, GzNT = 64, GzMAXX = 2;
-    static constexpr int Kconv2NT = 128, Kconv2VK = 8, Kconv2MAXC = 6, Kconv2WideNT = 0, Kconv2WideMAXC = 0;
+    static constexpr int Kconv2NT = 128, Kconv2MAXC = 6, Kconv2WideNT = 0, Kconv2WideMAXC = 0;
 };
 struct BwdSmall8 {    // bands of up to 32 strips of 4 (8 x 8 rows)
     static constexpr int RatioNT = 32, RatioMAXX = 1, KconvNT = 32, GzNT = 32, GzMAXX = 1;
-    static constexpr int Kconv2NT = 32, Kconv2VK = 8, Kconv2MAXC = 5, Kconv2WideNT = 0, Kconv2WideMAXC = 0;
+    static constexpr int Kconv2NT = 32, Kconv2MAXC = 5, Kconv2WideNT = 0, Kconv2WideMAXC = 0;
 };
 constexpr int kGzCS = 1;        // channel split of gz_kernel (2 was measured no faster)
 
@@ -241,7 +237,7 @@ template <int KD> constexpr bool packed_kconv() { return KD == 3; }
 template <int KH, typename S>
 constexpr int kconv2_threads() { if constexpr (KH == 1) return 2 * S::RatioNT; else return S::Kconv2NT; }
 
-template <int KD, int KH, int KW, int NT, int VK, int MAXC>
+template <int KD, int KH, int KW, int NT, int MAXC>
 inline bool plan_kconv2(int D, int H, int W, long long BC, Tiling& t, size_t& smem_bytes) {
     constexpr int PH = KH / 2;
     if ((long long)D * H * W >= (1LL << 29) || W > (KH == 1 ? 512 : 256)) return false;
@@ -291,11 +287,11 @@ inline bool plan_bwd(const Geo& g, BwdPlan& p) {
         bool ok = false;
         if constexpr (S::Kconv2WideNT > 0) {
             if (g.W > 64) {
-                ok = plan_kconv2<KD, KH, KW, S::Kconv2WideNT, S::Kconv2VK, S::Kconv2WideMAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv);
+                ok = plan_kconv2<KD, KH, KW, S::Kconv2WideNT, S::Kconv2WideMAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv);
                 p.kconv_wide = ok ? 1 : 0;
             }
         }
-        if (!ok && !plan_kconv2<KD, KH, KW, kconv2_threads<KH, S>(), S::Kconv2VK, S::Kconv2MAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv))
+        if (!ok && !plan_kconv2<KD, KH, KW, kconv2_threads<KH, S>(), S::Kconv2MAXC>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv))
             return false;
     } else {
         if (!plan_kconv<KD, KH, KW, S::KconvNT>(g.D, g.H, g.W, BC, p.kconv, p.smem_kconv)) return false;
@@ -435,13 +431,13 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.partial = gh ? pa : nullptr;
         P.h = h; P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.kconv; P.Wv = g.Wv;
         auto run = [&](auto nt, auto maxc) -> cudaError_t {
-            constexpr int NT = decltype(nt)::value, VK = S::Kconv2VK, MAXC = decltype(maxc)::value;
+            constexpr int NT = decltype(nt)::value, MAXC = decltype(maxc)::value;
             if (gh) {
-                auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, AL, true, WQ>;
+                auto kern = kconv2_kernel<T, KD, KH, KW, NT, MAXC, AL, true, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
                 kern<<<(unsigned)p.n_kconv, NT, p.smem_kconv, st>>>(P);
             } else {
-                auto kern = kconv2_kernel<T, KD, KH, KW, NT, VK, MAXC, AL, false, WQ>;
+                auto kern = kconv2_kernel<T, KD, KH, KW, NT, MAXC, AL, false, WQ>;
                 NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
                 kern<<<(unsigned)p.n_kconv, NT, p.smem_kconv, st>>>(P);
             }

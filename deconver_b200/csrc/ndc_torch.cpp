@@ -480,7 +480,8 @@ Tensor from_f32(const Tensor& g, at::ScalarType type) {
 }
 
 // The gradients of a node whose backward is not itself differentiable: they are computed without a
-// graph, and differentiating them raises an error.
+// graph, and differentiating them raises an error.  What torch.autograd.function.once_differentiable does
+// for Python nodes, which these were, message included.
 variable_list once(const variable_list& grads, variable_list out) {
     bool any = false;
     for (const Tensor& g : grads) any = any || (g.defined() && g.requires_grad());
