@@ -13,8 +13,8 @@
 // What bounds them: at 8 groups of 4 channels and 8 sources, 2 x 32^3 (a training step, float32) they
 // take 0.67 ms where the one-thread-per-element kernels took 4.5 ms; the multiply-adds alone are
 // 0.13 ms, the rest is staging (a 4-byte copy and its address per staged element, 2.4 of them per
-// output voxel and channel with the halo) and, in corr_kernel, one CTA of 200 registers per
-// thread on a multiprocessor.  For depthwise ratio-4 filters the marching kernels of ndc_dw4_*.cuh
+// output voxel and channel with the halo) and, in corr_kernel, one CTA of 194 - 221 registers per
+// thread (3x3x3) on a multiprocessor.  For depthwise ratio-4 filters the marching kernels of ndc_dw4_*.cuh
 // stage each element once and are twice as fast.
 //
 //   adjoint_kernel   A of x and t1 (forward output, backward ratio terms) or of gt1 (source gradient)
@@ -689,11 +689,10 @@ template <int KD, int KH, int KW>
 inline TileGeo plan_corr(const Geo& g) { return plan<KD, KH, KW>(g, 1, 256); }
 inline long long tiles_of(const TileGeo& t) { return (long long)t.ntw * t.nth * t.ntd; }
 
-// CTAs per (group, output channel, block of source channels) of corr_kernel: two rounds of the GPU,
-// but no more than there are tiles.
+// CTAs per (group, output channel, block of source channels) of corr_kernel: one round of the GPU, of
+// which a multiprocessor takes one CTA, but no more than there are tiles.
 inline int corr_splits(const Geo& g, const TileGeo& t) {
     const long long combos = (long long)g.G * g.m * source_blocks(g), work = (long long)g.B * tiles_of(t);
-    // one CTA of 240 registers per thread fits a multiprocessor: one full round of the GPU
     long long s = num_sms() / combos;
     if (s > work) s = work;
     return (int)std::max(1LL, s);
