@@ -82,7 +82,10 @@ struct WgradParams {
 
 // VEC: bytes of one copy: 16 (rows on 16-byte boundaries), 4 (float32 rows of any length, or
 // bfloat16 rows of even length), 0 (element loads: bfloat16 rows of odd length).  EXACT: float32
-// as the sum of two tf32 terms, three products (used where TF32 products are not allowed).
+// as the sum of two tf32 terms, three products (used where TF32 products are not allowed).  The MMA rounds its
+// accumulators towards zero, which adds up along a slice, so a stage's twelve are added to sums
+// that round to nearest: 3.6e-7 of the result against 64 bits where one chain was off by 3.6e-6
+// (5 x (96 + 24) x 34916; the library's float32 5.8e-7).
 template <typename T, int VEC, bool EXACT>
 __global__ void __launch_bounds__(WNT, 2) wgrad1x1_kernel(const WgradParams P) {
     constexpr int PPW = 4 / (int)sizeof(T);    // positions per word
@@ -133,13 +136,13 @@ __global__ void __launch_bounds__(WNT, 2) wgrad1x1_kernel(const WgradParams P) {
 
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int wo = (warp >> 1) * 32, wc = (warp & 1) * 32;   // 4 x 2 warps of 32 x 32 outputs
-    float acc[2][4][4];
+    float acc[2][4][4], sum[2][4][4];           // sum: EXACT
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.0f;
+            for (int k = 0; k < 4; ++k) acc[i][j][k] = sum[i][j][k] = 0.0f;
 
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
@@ -205,6 +208,14 @@ __global__ void __launch_bounds__(WNT, 2) wgrad1x1_kernel(const WgradParams P) {
                     }
             }
         }
+        if (EXACT) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) { sum[i][j][q] += acc[i][j][q]; acc[i][j][q] = 0.0f; }
+        }
     }
     if (!busy) return;
     float* out = P.partial + (long long)slice * P.co * P.ci;
@@ -215,7 +226,7 @@ __global__ void __launch_bounds__(WNT, 2) wgrad1x1_kernel(const WgradParams P) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int o = o0 + wo + 16 * i + g + (q >> 1) * 8, c = c0 + wc + 8 * j + 2 * t + (q & 1);
-                if (o < P.co && c < P.ci) out[(long long)o * P.ci + c] = acc[i][j][q];
+                if (o < P.co && c < P.ci) out[(long long)o * P.ci + c] = EXACT ? sum[i][j][q] : acc[i][j][q];
             }
 }
 

@@ -92,9 +92,11 @@ def test_row_padding(rows, W, pitch, dtype):
 KERNEL, PRODUCT, SLICES, CONVOLUTION = range(4)      # WgradRoute
 
 
-@pytest.mark.parametrize("dtype,tf32,tol", [(torch.float32, True, 2e-3), (torch.float32, False, 1e-5), (torch.bfloat16, True, 6e-3)],
+# f32: products of two-term operands, off by 2^-22 each at random, and sums rounded to nearest
+@pytest.mark.parametrize("dtype,tf32,tol", [(torch.float32, True, 2e-3), (torch.float32, False, 1e-6), (torch.bfloat16, True, 6e-3)],
                          ids=["tf32", "f32", "bf16"])
 @pytest.mark.parametrize("batch,co,ci,n,route", [
+    (5, 96, 24, 34916, KERNEL),
     (4, 128, 32, 16384, KERNEL), (3, 40, 24, 1001, KERNEL), (2, 96, 24, 4095, KERNEL), (1, 192, 48, 4095, KERNEL),
     (8, 640, 160, 4096, PRODUCT), (16, 288, 72, 4096, PRODUCT), (1, 2048, 512, 512, PRODUCT), (16, 48, 192, 4096, PRODUCT),
     (1, 256, 64, 110592, SLICES), (1, 96, 384, 32768, SLICES), (3, 130, 70, 49992, SLICES),
@@ -104,7 +106,8 @@ def test_weight_gradient_of_every_route(dtype, tf32, tol, batch, co, ci, n, rout
     """Each side of each line of the dispatch, slices with a rest among them (49992 positions)."""
     dev = torch.device("cuda:0")
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    assert _lib.load_ext().weight_grad_route(batch, co, ci, n, dtype == torch.bfloat16, sms) == route
+    exact = dtype == torch.float32 and not tf32
+    assert _lib.load_ext().weight_grad_route(batch, co, ci, n, dtype == torch.bfloat16, exact, sms) == (KERNEL if exact else route)
     gen = torch.Generator(device=dev).manual_seed(co + n)
     lin = dcb.Linear(ci, co).to(dev, dtype)
     x, g = torch.rand(batch, ci, n, device=dev, generator=gen).to(dtype), torch.randn(batch, co, n, device=dev, generator=gen).to(dtype)
