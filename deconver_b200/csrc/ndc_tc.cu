@@ -163,10 +163,12 @@ cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1
 }
 
 // How large a problem has to be, and how much of the MMAs' rows it has to fill, for the tensor cores to be the
-// faster way (measured on 46 shapes of either kind): volumes from 0.8 M group-voxels on, rows of 128 at
-// least 30 % full (16^3 fills 25 % and takes 0.90x the FMA kernels' speed, 20^3 39 % and 1.22x); images from 3 M on
-// and 45 % (8 images of 64 columns; 4 take 0.58x), 80 % for 3x3 filters at the widths the FMA kernels
-// have compile-time instances for (0.88x at 50 %, 1.06x - 1.11x at 89 %).
+// faster way: volumes from 0.8 M group-voxels on, rows of 128 at least 30 % full (16^3 fills 25 % and its forward
+// takes 0.93x the FMA kernels' speed, 20^3 39 % and 1.23x - 1.36x); images from 3 M on and 45 % (8 images of 64
+// columns 1.29x, 4 of them 0.79x), 80 % for 3x3 filters at the widths the FMA kernels have compile-time
+// instances for (4 x 64 of 128^2 0.81x).  On 31 shapes about the lines nothing that goes to the tensor cores is
+// slower there (forward 1.19x - 1.70x, a whole update 1.04x - 1.19x); some that stays would gain (16 x 128 of 32^2
+// 1.49x, 16 x 32 of 256^2 with 3x3 filters 1.43x): the lines are older than the source kernel's present form.
 template <int KD, int KH, int KW>
 bool worth(const Geo& g) {
     Band a, s;
