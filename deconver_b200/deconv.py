@@ -145,8 +145,11 @@ class Deconv(nn.Module):
             warn_if_generic(x, self.groups, self.filter_channels, self.source_channels, self.kernel_size)
             if len(_checked) < 4096:
                 _checked.add(key)
-        init = self._modules["init"]       # a third of the time of an attribute, which single small images notice
-        projection = init._modules["linear"]._modules["linear"]
+        init = self._modules["init"]
+        try:      # a third of the time of attributes, which single small images notice
+            projection = init._modules["linear"]._modules["linear"]
+        except KeyError:      # a wrapper around one of them, which passes attributes on
+            projection = init.linear.linear
         return native("layer", (x, init.h0, projection.weight, projection.bias), self.groups, self.filter_channels, self.source_channels,
                       self.eps, self.num_iters, self.num_grad_iters, current_flags())
 

@@ -159,3 +159,24 @@ def test_tensor_subclasses_stay(module):
     assert type(y) is Tagged and torch.equal(y.as_subclass(torch.Tensor), net(x))
     y.sum().backward()
     assert x.grad is not None
+
+
+def test_wrapped_submodules():
+    """As sharding and checkpointing wrappers do: a module of another structure that passes attributes on."""
+    class Wrapper(torch.nn.Module):
+        def __init__(self, module):
+            super().__init__()
+            self.wrapped = module
+
+        def __getattr__(self, name):
+            try:
+                return super().__getattr__(name)
+            except AttributeError:
+                return getattr(self.wrapped, name)
+
+    net, x = MODULES["deconv"]().to(DEV), torch.rand(2, 6, 4, 8, device=DEV)
+    want = net(x)
+    net.init.linear = Wrapper(net.init.linear)
+    assert torch.equal(net(x), want)
+    net.init = Wrapper(net.init)
+    assert torch.equal(net(x), want)
