@@ -63,7 +63,11 @@ def is_stale():
 def ext_target():
     """The PyTorch and Python that an extension built now is for: it uses their C++ interfaces, which
     hold for one version only."""
-    return "torch %s, %s" % (importlib.metadata.version("torch"), sys.implementation.cache_tag)
+    try:
+        version = importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:      # a source tree on the path
+        version = "of unknown version"
+    return "torch %s, %s" % (version, sys.implementation.cache_tag)
 
 
 def ext_built_for():
