@@ -289,7 +289,7 @@ size_t ndc_bwd_rows_workspace_bytes(const NdcDesc* desc, int32_t pitch) {
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) return p.bytes;
     }
-    if (tile_path(desc, g)) return ndc::tile::bwd_scratch(g).bytes;
+    if (tile_path(desc, g)) return ndc::tile::bwd_scratch(g);
     return ndc::generic::bwd_scratch(g).bytes;
 }
 

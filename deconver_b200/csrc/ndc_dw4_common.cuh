@@ -357,6 +357,15 @@ __device__ __forceinline__ void unpack2(f32x2 p, float& lo, float& hi) {
 __device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+// A pair put together from two registers that many multiply-adds will read.  The compiler keeps the two
+// registers and makes the pair again at every use, at one to two moves per multiply-add; the product of
+// an instruction stays where it is.  (x 1 is exact for every value.)  On a loop of 27 taps x 4 channels x 8 voxels
+// per thread, as in the correlations: 36 -> 53 TFLOP/s.
+__device__ __forceinline__ f32x2 make_pair2(float lo, float hi) {
+    f32x2 r;
+    asm volatile("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(lo, hi)), "l"(pack2(1.0f, 1.0f)));
+    return r;
+}
 // lane `hi` (0 or 1, a compile-time value after unrolling) of a pair
 __device__ __forceinline__ float lane_of(f32x2 p, int hi) {
     float lo, up;

@@ -1,4 +1,5 @@
-// Tile kernels: any grouping (m, sc <= 16) with 3x3x3, 5x5 and 3x3 filters, 1 <= m, sc <= 16.
+// Tile kernels: any grouping with 3x3x3, 5x5 and 3x3 filters, 1 <= m, sc <= 16.  Rows and tensors of whole
+// vectors go to those of ndc_pairs.cuh; these take the others.
 //
 // A CTA owns a tile of one (sample, group) pair: TD planes x TH rows x TW columns of the output.
 // One input channel at a time (or a few) is staged in shared memory with its halo, as float32 rows
@@ -27,6 +28,7 @@
 
 #include "ndc_common.cuh"
 #include "ndc_dw4_common.cuh"
+#include "ndc_pairs.cuh"
 
 namespace ndc {
 namespace tile {
@@ -587,7 +589,7 @@ __global__ void __launch_bounds__(256, 1) corr_kernel(const CorrParams P) {
 #pragma unroll
             for (int j = 0; j < CB / 2; ++j)
 #pragma unroll
-                for (int v = 0; v < V; ++v) a[j][v] = pack2(av[2 * j][v], av[2 * j + 1][v]);
+                for (int v = 0; v < V; ++v) a[j][v] = dw4::make_pair2(av[2 * j][v], av[2 * j + 1][v]);
         }
         __syncthreads();       // everybody's part of the tile has landed
         if (!at.active) continue;
@@ -711,10 +713,16 @@ inline BwdScratch scratch_shape(const Geo& g) {
     s.bytes = s.corr + up256((size_t)g.G * g.m * source_blocks(g) * corr_splits(g, tc) * g.KT * CB * sizeof(float));
     return s;
 }
-inline BwdScratch bwd_scratch(const Geo& g) {
-    if (g.kD == 3) return scratch_shape<3, 3, 3>(g);
-    if (g.kH == 5) return scratch_shape<1, 5, 5>(g);
-    return scratch_shape<1, 3, 3>(g);
+// Bytes of it for either kind of kernel: which one runs depends on the tensors' alignment too.
+template <int KD, int KH, int KW>
+inline size_t scratch_bytes(const Geo& g) {
+    const size_t n = scratch_shape<KD, KH, KW>(g).bytes;
+    return pairs::covers(g) ? std::max(n, pairs::scratch_shape<KD, KH, KW>(g).bytes) : n;
+}
+inline size_t bwd_scratch(const Geo& g) {
+    if (g.kD == 3) return scratch_bytes<3, 3, 3>(g);
+    if (g.kH == 5) return scratch_bytes<1, 5, 5>(g);
+    return scratch_bytes<1, 3, 3>(g);
 }
 
 template <typename Kern, typename P>
@@ -763,6 +771,7 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 template <typename T, int KD, int KH, int KW>
 cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, const float* bias, T* out, T* t1,
                           cudaStream_t st) {
+    if (pairs::covers(g) && pairs::whole<T>({x, z, out, t1})) return pairs::forward_shape<T, KD, KH, KW>(g, x, z, h, bias, out, t1, st);
     const bool vec = g.W % V == 0 && aligned16(z) && aligned16(out) && aligned16(t1);
     KParams K{};
     K.in[0] = z; K.out[0] = t1; K.out_f32[0] = 0; K.count = 1; K.h = h; K.bias = bias; K.relu = g.relu;
@@ -776,6 +785,8 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
 template <typename T, int KD, int KH, int KW>
 cudaError_t backward_shape(const Geo& g, const T* x, const T* z, const T* t1, const float* h, const float* bias,
                            const T* gout, T* gx, T* gz, float* gh, float* gb, void* ws, cudaStream_t st) {
+    if (pairs::covers(g) && pairs::whole<T>({x, z, t1, gout, gx, gz}))
+        return pairs::backward_shape<T, KD, KH, KW>(g, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
     const BwdScratch sc = scratch_shape<KD, KH, KW>(g);
     float* gnum = (float*)((char*)ws + sc.gnum);
     float* gden = (float*)((char*)ws + sc.gden);
