@@ -9,7 +9,8 @@
 // accumulators of KD output planes, which lie next to each other in TMEM.  So a source plane is read
 // once, when the CTA's march through the depth comes to it, and a filter row kh is a shift of the start
 // address.  Batches of images march down their rows the same way (planes = image rows, plane rows =
-// images, KH = 1: see SlabAddr).  An MMA of up to 128 columns takes 64 cycles here, whatever its width
+// images, KH = 1: see SlabAddr); the rows of their bands never meet, so a band takes any of them, of several
+// chunks at once (see At), and fills its 128 blocks whatever the batch.  An MMA of up to 128 columns takes 64 cycles here, whatever its width
 // (reading 4 KB of A operand), hence the wide ones.  With KW = 3 most of the products meet a zero of the
 // band; the tensor cores do them 30 times faster than the FMA pipe does the useful ones.  What K = 16
 // holds differs:
@@ -36,6 +37,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ndc_common.cuh"
 #include "ndc_dw4_common.cuh"
@@ -51,7 +53,7 @@ struct Band {
     int C, D, H, W;               // W: row pitch (a multiple of 4)
     int Wv, Wo;                   // columns of the volume, row pitch of out (see Geo)
     int NB, PB;                   // blocks that hold columns, blocks per row in shared memory
-    int TH, nth, DC, ndc;         // rows and bands, planes and chunks
+    int TH, nth, DC, ndc;         // rows and bands, planes and chunks (KH = 1: bands of rows of all chunks)
     float eps;
     int relu;
 };
@@ -162,7 +164,8 @@ __device__ __forceinline__ unsigned instr_desc(int n) { return 1u << 4 | 1u << 7
 // turns as well), one warp that issues the MMAs.  The source kernel, whose epilogue is short and whose
 // source planes have four channels, has one epilogue group and stages with two groups of five warps.  The
 // adjoint kernel: two and two groups of two warps, two CTAs per multiprocessor; with five depth taps, whose
-// accumulators leave room for one, four and four.
+// accumulators leave room for one, four and four.  (Two CTAs of two channels each, 16 x 64 images of 128^2, 5x5: 203 us
+// for the forward's 211, but 4 x 64 of them 78 for 71.)
 constexpr int kSourceThreads = 32 * (4 + 10 + 1), kSourceStagers = 160;
 template <int KD> struct AdjointShape {
     static constexpr int EPI = KD > 3 ? 4 : 2, GROUPS = KD > 3 ? 4 : 2, STAGERS = 64, BLOCKS = KD > 3 ? 2 : 3;
@@ -173,15 +176,33 @@ constexpr int kSourceSlots = 4;   // of the source kernel, which stages two term
 constexpr int kHeader = 1024;     // bytes: barriers and the TMEM address (512), the filter as float32
 
 // Place of a CTA: (sample, channel), band of rows, chunk of planes; all addresses in elements.
+// ROWS: row v of the band is image v % H of chunk v / H, and its planes count from the chunk's first one; `d0` is 0.
+// (Bands of the images of one chunk left blocks idle: 16 images of 128 columns fill 7 + 7 + 2 of the adjoint's
+// rows, 16 of 64 columns 14 + 2.)
 template <bool ROWS>
 struct At {
     int bc, c, h0, TH, d0, DC;
     __device__ __forceinline__ At(const Band& b, int blk) {
         const int th = blk % b.nth; blk /= b.nth;
-        const int dc = blk % b.ndc; blk /= b.ndc;
+        const int dc = ROWS ? 0 : blk % b.ndc;
+        if (!ROWS) blk /= b.ndc;
         bc = blk; c = bc % b.C;
-        h0 = th * b.TH; TH = min(b.TH, b.H - h0);
+        h0 = th * b.TH; TH = min(b.TH, (ROWS ? b.H * b.ndc : b.H) - h0);
         d0 = dc * b.DC; DC = min(b.DC, b.D - d0);
+    }
+};
+// ROWS: the image that the 32-bit offsets of a band that begins at row h0 count from.  (Bands of several chunks jump
+// back to the first image; the host sees to it that the offsets fit.)
+__device__ __forceinline__ long long base_row(const Band& b, int h0) { return b.ndc == 1 ? h0 : 0; }
+// Where row h of a plane lies: its offset, and for ROWS the first plane of its chunk (else 0).
+template <bool ROWS>
+struct RowAt {
+    long long off;
+    int d;
+    __device__ __forceinline__ RowAt(const Band& b, int h, long long row_stride, long long plane) {
+        const int chunk = ROWS ? h / b.H : 0;
+        d = chunk * b.DC;
+        off = (h - chunk * b.H) * row_stride + d * plane;
     }
 };
 
@@ -211,10 +232,11 @@ __device__ __forceinline__ uint4 to_places(const unsigned (&a)[5]) {
 
 // A group's planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are passed
 // on without data.  `S`: load, prefetch and store a plane.
-template <int SLOTS, int GROUPS, typename S, typename F>
+template <int SLOTS, int GROUPS, bool ROWS, typename S, typename F>
 __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int PD, int planes, unsigned full, unsigned empty, int group,
                                              int lane) {
-    const int first = max(0, PD - d0), last = min(planes - 1, D - 1 + PD - d0);   // those inside
+    // those inside; the stager knows which rows of several chunks are
+    const int first = ROWS ? 0 : max(0, PD - d0), last = ROWS ? planes - 1 : min(planes - 1, D - 1 + PD - d0);
     if (group >= first && group <= last) st.load(d0 - PD + group);
     for (int p = group; p < planes; p += GROUPS) {
         const int s = p % SLOTS;
@@ -237,41 +259,58 @@ __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int 
 // from L2.  Addresses are a base that is the same for the whole CTA and a 32-bit offset.
 template <int KH, int KW, int NCH, bool WIDE, int NTHR, int U>
 struct Stager {
+    static constexpr bool ROWS = KH == 1;
     const Band& b;
-    const bf16* src;               // row h0 - KH / 2 of plane 0
+    const bf16* src;               // row h0 - KH / 2 of plane 0 (ROWS: see base_row)
     long long stride, plane;
     int blocks;                    // per channel of a slot
     unsigned off[U];               // this thread's blocks: offset of the first column
     bool in[U];                    // inside the volume (else zero)
     int w[U], at[U];               // column; block, or -1
+    int d0[U];                     // ROWS: first plane of the row's chunk
     unsigned a[U][NCH][5];
 
-    __device__ __forceinline__ Stager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, int h0,
+    __device__ __forceinline__ Stager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, const At<ROWS>& place,
                                       int tid)
-        : b(b_), src(src_ + (h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB) {
+        : b(b_), src(src_ + (ROWS ? base_row(b_, place.h0) : place.h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int i = tid + u * NTHR, row = i / b.PB, q = i - row * b.PB, h = h0 - KH / 2 + row;
+            const int i = tid + u * NTHR, row = i / b.PB, q = i - row * b.PB, h = place.h0 - KH / 2 + row;
             at[u] = i < blocks ? i : -1;
             w[u] = 8 * q;
-            off[u] = (unsigned)(row * row_stride) + w[u];
-            in[u] = i < blocks && h >= 0 && h < b.H;
+            if (ROWS) {
+                const RowAt<ROWS> r(b, h, row_stride, plane);
+                d0[u] = r.d;
+                off[u] = (unsigned)(r.off - base_row(b, place.h0) * row_stride) + w[u];
+                in[u] = i < blocks && row < place.TH;
+            } else {
+                d0[u] = 0;
+                off[u] = (unsigned)(row * row_stride) + w[u];
+                in[u] = i < blocks && h >= 0 && h < b.H;
+            }
         }
     }
+    __device__ __forceinline__ bool has(int u, int d) const { return in[u] && (!ROWS || (unsigned)(d + d0[u]) < (unsigned)b.D); }
     __device__ __forceinline__ void load(int d) {
         const bf16* p = src + d * plane;
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (in[u]) {
+        for (int u = 0; u < U; ++u) {
+            if (has(u, d)) {
 #pragma unroll
                 for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride, off[u], w[u], b.W, a[u][ch]);
+            } else if (ROWS) {
+#pragma unroll
+                for (int ch = 0; ch < NCH; ++ch)
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) a[u][ch][i] = 0u;
             }
+        }
     }
     __device__ __forceinline__ void prefetch(int d) const {
         const bf16* p = src + d * plane;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (in[u] && (w[u] & 63) == 0 && w[u] < b.W) {
+            if (has(u, d) && (w[u] & 63) == 0 && w[u] < b.W) {
 #pragma unroll
                 for (int ch = 0; ch < NCH; ++ch)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off[u]));
@@ -441,7 +480,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
             if (p >= RING && p < at.DC) ok = mbar_wait_thread(aempty + 8 * (p % RING), (p / RING - 1) & 1, kWaitLimit) && ok;
             tc_fence_after();
             if (ok) {
-                if (d >= 0 && d < b.D) {
+                if (ROWS || (d >= 0 && d < b.D)) {
                     // groups g of output planes o = p - (KD - 1) + g inside the chunk
                     const int g0 = max(0, KD - 1 - p), g1 = min(KD - 1, at.DC - 1 + KD - 1 - p), o0 = p - (KD - 1) + g0;
                     const int r0 = o0 % RING, n = g1 - g0 + 1, n0 = min(n, RING - r0);
@@ -466,12 +505,14 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         // x and t1 as two channels: the distance between the tensors takes the place of the stride
         const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
         Stager<KH, KW, 2, AL == kWide, Shape::STAGERS, Shape::BLOCKS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x,
-                                                                         at.h0, (tid - 32 * kEpilogueWarps) % Shape::STAGERS);
-        ok = stage_planes<kSlots, Shape::GROUPS>(st, [&](int s) { st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, planes, sfull, sempty,
+                                                                         at, (tid - 32 * kEpilogueWarps) % Shape::STAGERS);
+        ok = stage_planes<kSlots, Shape::GROUPS, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, planes, sfull, sempty,
                                                  (tid - 32 * kEpilogueWarps) / Shape::STAGERS, lane);
     } else {
         const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q;
-        const bool valid = r < at.TH && q < b.NB;
+        const RowAt<ROWS> zat(b, at.h0 + r, addr.row_z, addr.plane), oat(b, at.h0 + r, oaddr.row_z, oaddr.plane);
+        // this row's output planes in the march
+        const int count = r < at.TH && q < b.NB ? (ROWS ? min(b.DC, b.D - zat.d) : at.DC) : 0;
         const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
         f32x2 b2[SC];
 #pragma unroll
@@ -479,15 +520,17 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
             const float v = P.bias ? P.bias[at.c * SC + j] : 0.0f;
             b2[j] = pack2(v, v);
         }
-        const long long zrow = (long long)at.bc * SC * addr.chan + (at.h0 + r) * addr.row_z;
-        const long long orow = (long long)at.bc * SC * oaddr.chan + (at.h0 + r) * oaddr.row_z;
+        const long long zrow = (long long)at.bc * SC * addr.chan + zat.off;
+        const long long orow = (long long)at.bc * SC * oaddr.chan + oat.off;
         const bf16* const zb = P.z + zrow;
         const bf16* const gb = MODE == kOut ? nullptr : P.gout + orow;
         for (int o = warp >> 2; o < at.DC && ok; o += Shape::EPI) {
             const int slot = o % RING;
             const long long d = at.d0 + o;
+            const bool valid = o < count;
             // z of all channels, or z and gout of two (the registers do not hold more), are on their way
             // while the accumulators are waited for; their lines of this group's next plane come to L2
+            // (one plane further ahead, in registers: 2.88 ms for 2.35 at 4 x 64 x 128^3, spills)
             constexpr int AHEAD = MODE == kOut ? SC : 2;
             uint4 zr[AHEAD], gr[AHEAD];
             auto fetch = [&](int j) {
@@ -495,7 +538,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                 gr[j % AHEAD] = make_uint4(0u, 0u, 0u, 0u);
                 if (!valid) return;
                 const bf16* zp = zb + j * addr.chan + d * addr.plane;
-                const bool more = (q & 7) == 0 && o + Shape::EPI < at.DC;
+                const bool more = (q & 7) == 0 && o + Shape::EPI < count;
                 zr[j % AHEAD] = load8<AL>(zp, w, b.W);
                 if (more) asm volatile("prefetch.global.L2 [%0];" ::"l"(zp + Shape::EPI * addr.plane + w));
                 if (MODE == kOut) return;
@@ -622,32 +665,43 @@ template <int KD> __host__ __device__ constexpr int source_ring() { return kSour
 // block of a plane; see Stager.
 template <int KH, bool WIDE>
 struct SourceStager {
+    static constexpr bool ROWS = KH == 1;
     const Band& b;
     const bf16* src;
     long long stride, plane;
     int blocks;
     unsigned off;
-    bool in;
-    int w, at;
+    bool row_in, in;               // the row is the band's; and its plane is inside the volume
+    int w, at, d0;
     uint4 a[SC];
 
-    __device__ __forceinline__ SourceStager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, int h0,
-                                            int i)
-        : b(b_), src(src_ + (h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.NB) {
-        const int row = i / b.NB, h = h0 - KH / 2 + row;
+    __device__ __forceinline__ SourceStager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride,
+                                            const At<ROWS>& place, int i)
+        : b(b_), src(src_ + (ROWS ? base_row(b_, place.h0) : place.h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.NB) {
+        const int row = i / b.NB, h = place.h0 - KH / 2 + row;
         at = i < blocks ? i : -1;
         w = 8 * (i - row * b.NB);
-        off = (unsigned)(row * row_stride) + w;
-        in = i < blocks && h >= 0 && h < b.H;
+        if (ROWS) {
+            const RowAt<ROWS> r(b, h, row_stride, plane);
+            d0 = r.d;
+            off = (unsigned)(r.off - base_row(b, place.h0) * row_stride) + w;
+            row_in = i < blocks && row < place.TH;
+        } else {
+            d0 = 0;
+            off = (unsigned)(row * row_stride) + w;
+            row_in = i < blocks && h >= 0 && h < b.H;
+        }
+        in = row_in;
     }
     __device__ __forceinline__ void load(int d) {
+        if (ROWS) in = row_in && (unsigned)(d + d0) < (unsigned)b.D;
         if (!in) return;
         const bf16* p = src + d * plane;
 #pragma unroll
         for (int ch = 0; ch < SC; ++ch) a[ch] = load8<WIDE ? kWide : kQuad>(p + ch * stride + (off - w), w, b.W);
     }
     __device__ __forceinline__ void prefetch(int d) const {
-        if (!in || (w & 63)) return;
+        if (!row_in || (w & 63) || (ROWS && (unsigned)(d + d0) >= (unsigned)b.D)) return;
         const bf16* p = src + d * plane;
 #pragma unroll
         for (int ch = 0; ch < SC; ++ch) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off));
@@ -737,7 +791,7 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
             if (p >= RING) ok = mbar_wait_thread(aempty + 8 * (p % RING), (p / RING - 1) & 1, kWaitLimit) && ok;
             tc_fence_after();
             if (ok) {
-                if (d >= 0 && d < b.D) {
+                if (ROWS || (d >= 0 && d < b.D)) {
                     const int g0 = max(0, KD - 1 - p);       // output planes of the chunk only
                     const unsigned long long a0 = ad + s * slot_blocks, m0 = md + g0 * kGroup * 2;
                     const unsigned idesc = instr_desc(NCOL - g0 * kGroup), acc = tmem + kGroup * (p % RING + g0);
@@ -757,16 +811,18 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
             const __nv_bfloat162 v = __float2bfloat162_rn(P.bias ? P.bias[at.c * SC + j] : 0.0f);
             bias[j] = *reinterpret_cast<const unsigned*>(&v);
         }
-        SourceStager<KH, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at.h0,
+        SourceStager<KH, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at,
                                          (tid - 32 * kEpilogueWarps) % kSourceStagers);
-        ok = stage_planes<kSourceSlots, 2>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, sfull,
+        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, sfull,
                                            sempty, (warp - kEpilogueWarps) / 5, lane);
     } else {
-        const int m = warp * 32 + lane, r = m / b.NB, q = m - r * b.NB, w = 8 * q, h = at.h0 + r;
-        const bool valid = r < at.TH, left = q > 0, right = q + 1 < b.NB;
+        const int m = warp * 32 + lane, r = m / b.NB, q = m - r * b.NB, w = 8 * q;
+        const RowAt<ROWS> row(b, at.h0 + r, addr.row_x, addr.plane);
+        const int count = r < at.TH ? (ROWS ? min(b.DC, b.D - row.d) : at.DC) : 0;      // this row's output planes in the march
+        const bool left = q > 0, right = q + 1 < b.NB;
         const bool split = 32 % b.NB != 0;              // rows go on in another warp's lanes
         const unsigned lanes = tmem + ((unsigned)warp << 21);
-        bf16* const tb = P.t1 + (long long)at.bc * addr.chan + h * addr.row_x;
+        bf16* const tb = P.t1 + (long long)at.bc * addr.chan + row.off;
         for (int o = 0; o < at.DC && ok; ++o) {
             const int place = (o + KD - 1) % RING;
             ok = mbar_wait(afull + 8 * (o % RING), (o / RING) & 1);
@@ -814,7 +870,7 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
                 v[8 - PW + i] += right ? from_right[i] : 0.0f;
                 v[i] += left ? from_left[i] : 0.0f;
             }
-            if (valid) {
+            if (o < count) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (AL != kWide && w + i >= b.Wv) v[i] = 0.0f;
