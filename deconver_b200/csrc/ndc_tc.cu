@@ -71,11 +71,18 @@ bool plan(const Geo& g, bool source, Band& b) {
     b.C = g.G; b.D = g.D; b.H = g.H; b.W = g.W; b.Wv = g.Wv; b.Wo = g.Wo; b.eps = g.eps; b.relu = g.relu;
     b.NB = (g.Wv + 7) / 8;
     b.PB = source ? b.NB : (g.Wv + KW / 2 + 7) / 8;
+    // The adjoint's CTAs that are alone on their multiprocessor (five depth taps) go on from place to place where there
+    // are several for each: nobody else fills their gaps (16 x 64 images of 128^2: 127 -> 105 us for three each).  With one
+    // each that form is 5 % slower; and of two CTAs on a multiprocessor either fills the other's gaps.
+    const bool alone = !source && AdjointShape<KD>::CTAS == 1;
+    const bool waits = !(g.W % 8 == 0 && g.Wv == g.W);      // for its loads, of 8 bytes
     const long long sms = num_sms(), finest = std::max(1, g.D / (6 * (KD / 2)));
-    const float halo = source ? 7.0f : KD > 3 ? 12.0f : 4.0f;
-    auto march = [&](int planes, long long ctas) {      // expected time of chunks of so many planes
-        const long long on_one = (ctas + sms - 1) / sms;
-        return ((float)planes + halo) * (source ? (float)(on_one / 2) + (on_one % 2 ? 0.65f : 0.0f) : (float)on_one);
+    // expected time of so many places of chunks of so many planes
+    auto time = [&](int planes, long long items) {
+        const long long on_one = (items + sms - 1) / sms;
+        if (alone) return (float)on_one * ((float)planes + (KD - 1) + 1.5f) + 12.0f;
+        const float pairs = (float)(on_one / 2) + (on_one % 2 ? 0.65f : 0.0f);
+        return ((float)planes + (source ? 7.0f : 4.0f)) * (source ? pairs : (float)on_one);
     };
     b.TH = std::min(MB / b.PB, kSourceStagers / b.PB - (KH - 1));
     if (b.TH < 1) return false;
@@ -86,7 +93,7 @@ bool plan(const Geo& g, bool source, Band& b) {
         for (long long n = 1; n <= std::min(finest, 32LL); ++n) {
             const int planes = (int)((g.D + n - 1) / n);
             const long long chunks = (g.D + planes - 1) / planes, rows = g.H * chunks, bands = (rows + most - 1) / most;
-            const float t = march(planes, (long long)g.B * g.G * bands);
+            const float t = time(planes, (long long)g.B * g.G * bands);
             if (rows > 0x7fffffffLL || (chunks > 1 ? g.H : std::min(g.H, most)) * row >= (1LL << 31) || (least >= 0.0f && t >= 0.99f * least)) continue;
             least = t;
             b.DC = planes; b.ndc = (int)chunks;
@@ -95,7 +102,10 @@ bool plan(const Geo& g, bool source, Band& b) {
         }
         if (least < 0.0f) return false;
         b.nth = (int)(((long long)g.H * b.ndc + b.TH - 1) / b.TH);
-        return true;
+        const long long items = (long long)g.B * g.G * b.nth;
+        b.items = (int)std::min(items, 0x7fffffffLL);
+        b.march = alone && items > sms;
+        return items <= 0x7fffffffLL;
     }
     b.TH = std::min(g.H, b.TH);
     b.nth = (g.H + b.TH - 1) / b.TH;
@@ -107,18 +117,21 @@ bool plan(const Geo& g, bool source, Band& b) {
     long long ndc = 1;
     const long long want = (4 * sms + per - 1) / per;
     ndc = std::max(ndc, std::min(want, finest));
-    if (source || (g.W % 8 == 0 && g.Wv == g.W)) {
-        auto time = [&](long long n) {
+    if (source || !waits) {
+        auto cut = [&](long long n) {
             const int planes = (int)((g.D + n - 1) / n);
-            return march(planes, per * ((g.D + planes - 1) / planes));
+            return time(planes, per * ((g.D + planes - 1) / planes));
         };
-        float least = 0.98f * time(ndc);
+        float least = 0.98f * cut(ndc);
         const long long last = std::min(2 * ndc + 2, (long long)finest);
         for (long long n = std::max(1LL, ndc / 6), from = ndc; n <= last; ++n)
-            if (n != from && time(n) < least) { least = time(n); ndc = n; }
+            if (n != from && cut(n) < least) { least = cut(n); ndc = n; }
     }
     b.DC = (int)((g.D + ndc - 1) / ndc);
     b.ndc = (g.D + b.DC - 1) / b.DC;
+    if (per * b.ndc > 0x7fffffffLL) return false;
+    b.items = (int)(per * b.ndc);
+    b.march = 0;
     return true;
 }
 
@@ -135,25 +148,30 @@ template <int KD, int KH, int KW> size_t source_smem(const Band& b) {
 }
 
 template <typename K, typename P>
-cudaError_t launch(K kern, int threads, const Band& b, const Geo& g, size_t smem, cudaStream_t st, const P& p) {
-    const long long grid = (long long)g.B * g.G * b.nth * (g.kH == 1 ? 1 : b.ndc);
-    if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+cudaError_t launch(K kern, int threads, const Band& b, size_t smem, cudaStream_t st, const P& p) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)grid, threads, smem, st>>>(p);
+    kern<<<(unsigned)(b.march ? num_sms() : b.items), threads, smem, st>>>(p);
     launched();
     return cudaGetLastError();
 }
 
 bool on16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-template <int KD, int KH, int KW, int MODE>
+template <int KD, int KH, int KW, int MODE, bool MARCH>
 cudaError_t launch_adjoint(const Geo& g, const AdjointArgs& A, bool wide, cudaStream_t st) {
     const size_t smem = adjoint_smem<KD, KH, KW>(A.b);
     constexpr int NT = AdjointShape<KD>::THREADS;
-    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut, MODE>, NT, A.b, g, smem, st, A);
-    return wide ? launch(tc_adjoint_kernel<KD, KH, KW, kWide, MODE>, NT, A.b, g, smem, st, A)
-                : launch(tc_adjoint_kernel<KD, KH, KW, kQuad, MODE>, NT, A.b, g, smem, st, A);
+    if (g.Wo != g.W) return launch(tc_adjoint_kernel<KD, KH, KW, kPaddedOut, MODE, MARCH>, NT, A.b, smem, st, A);
+    return wide ? launch(tc_adjoint_kernel<KD, KH, KW, kWide, MODE, MARCH>, NT, A.b, smem, st, A)
+                : launch(tc_adjoint_kernel<KD, KH, KW, kQuad, MODE, MARCH>, NT, A.b, smem, st, A);
+}
+template <int KD, int KH, int KW, int MODE>
+cudaError_t launch_adjoint(const Geo& g, const AdjointArgs& A, bool wide, cudaStream_t st) {
+    if constexpr (AdjointShape<KD>::CTAS == 1) {
+        if (A.b.march) return launch_adjoint<KD, KH, KW, MODE, true>(g, A, wide, st);
+    }
+    return launch_adjoint<KD, KH, KW, MODE, false>(g, A, wide, st);
 }
 
 template <int KD, int KH, int KW>
@@ -168,8 +186,8 @@ cudaError_t run(const Geo& g, const bf16* x, const bf16* z, const float* h, cons
     if (e != cudaSuccess) return e;
     A.expired = S.expired;
     const bool wide = g.W % 8 == 0 && g.Wv == g.W && on16(x) && on16(z) && on16(t1);
-    e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, g, ss, st, S)
-             : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, g, ss, st, S);
+    e = wide ? launch(tc_source_kernel<KD, KH, KW, kWide>, kSourceThreads, S.b, ss, st, S)
+             : launch(tc_source_kernel<KD, KH, KW, kQuad>, kSourceThreads, S.b, ss, st, S);
     if (e != cudaSuccess) return e;
     return launch_adjoint<KD, KH, KW, kOut>(g, A, wide && on16(out), st);
 }

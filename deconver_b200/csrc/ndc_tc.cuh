@@ -54,6 +54,8 @@ struct Band {
     int Wv, Wo;                   // columns of the volume, row pitch of out (see Geo)
     int NB, PB;                   // blocks that hold columns, blocks per row in shared memory
     int TH, nth, DC, ndc;         // rows and bands, planes and chunks (KH = 1: bands of rows of all chunks)
+    int items;                    // places of work (see Items)
+    int march;                    // CTAs that have several, one after the other
     float eps;
     int relu;
 };
@@ -166,7 +168,7 @@ __device__ __forceinline__ unsigned instr_desc(int n) { return 1u << 4 | 1u << 7
 // adjoint kernel: two and two groups of two warps, two CTAs per multiprocessor; with five depth taps, whose
 // accumulators leave room for one, four and four.  (Two CTAs of two channels each, 16 x 64 images of 128^2, 5x5: 203 us
 // for the forward's 211, but 4 x 64 of them 78 for 71.)
-constexpr int kSourceThreads = 32 * (4 + 10 + 1), kSourceStagers = 160;
+constexpr int kSourceThreads = 32 * (4 + 10 + 1), kSourceStagers = 160, kSourceCtas = 2;
 template <int KD> struct AdjointShape {
     static constexpr int EPI = KD > 3 ? 4 : 2, GROUPS = KD > 3 ? 4 : 2, STAGERS = 64, BLOCKS = KD > 3 ? 2 : 3;
     static constexpr int THREADS = 32 * (4 * EPI + 2 * GROUPS + 1), CTAS = KD > 3 ? 1 : 2;
@@ -194,6 +196,17 @@ struct At {
 // ROWS: the image that the 32-bit offsets of a band that begins at row h0 count from.  (Bands of several chunks jump
 // back to the first image; the host sees to it that the offsets fit.)
 __device__ __forceinline__ long long base_row(const Band& b, int h0) { return b.ndc == 1 ? h0 : 0; }
+// The places of a CTA: its own, or (MARCH) a contiguous share of all, one after the other without emptying the pipeline
+// in between; their channel (and with it the banded matrices) seldom changes.
+template <bool MARCH>
+struct Items {
+    int first, last;               // [first, last)
+    __device__ __forceinline__ Items(const Band& b) {
+        first = MARCH ? (int)((long long)b.items * blockIdx.x / gridDim.x) : blockIdx.x;
+        last = MARCH ? (int)((long long)b.items * (blockIdx.x + 1) / gridDim.x) : first + 1;
+    }
+};
+
 // Where row h of a plane lies: its offset, and for ROWS the first plane of its chunk (else 0).
 template <bool ROWS>
 struct RowAt {
@@ -207,11 +220,11 @@ struct RowAt {
 };
 
 // Columns w-2 .. w+7 of a global row as five words, w = 8 q at `p[off]`; zero outside the row of W.
-template <bool WIDE>
-__device__ __forceinline__ void load_words(const bf16* p, unsigned off, int w, int W, unsigned (&a)[5]) {
+template <bool WIDE, typename Offset>
+__device__ __forceinline__ void load_words(const bf16* p, Offset off, int w, int W, unsigned (&a)[5]) {
 #pragma unroll
     for (int i = 0; i < 5; ++i) a[i] = 0u;
-    if (w > 0 && w - 4 < W) a[0] = __ldg(reinterpret_cast<const unsigned*>(p + (off - 2u)));
+    if (w > 0 && w - 4 < W) a[0] = __ldg(reinterpret_cast<const unsigned*>(p + (off - (Offset)2)));
     if (WIDE) {
         if (w < W) {
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + off));
@@ -219,7 +232,7 @@ __device__ __forceinline__ void load_words(const bf16* p, unsigned off, int w, i
         }
     } else {
         if (w < W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + off)); a[1] = v.x; a[2] = v.y; }
-        if (w + 4 < W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (off + 4u))); a[3] = v.x; a[4] = v.y; }
+        if (w + 4 < W) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (off + (Offset)4))); a[3] = v.x; a[4] = v.y; }
     }
 }
 // The eight places of block q of a shared row (columns 8 q - PW .. 8 q + 7 - PW) from those words.
@@ -230,17 +243,18 @@ __device__ __forceinline__ uint4 to_places(const unsigned (&a)[5]) {
                       __funnelshift_l(a[3], a[4], 16));
 }
 
-// A group's planes of a chunk: p counts source planes from d0 - PD; planes outside the volume are passed
-// on without data.  `S`: load, prefetch and store a plane.
+// A group's planes of a chunk: p counts source planes from d0 - PD, `base` those of the places before; planes
+// outside the volume are passed on without data.  `S`: load, prefetch and store a plane.
 template <int SLOTS, int GROUPS, bool ROWS, typename S, typename F>
-__device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int PD, int planes, unsigned full, unsigned empty, int group,
+__device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int PD, int planes, int base, unsigned full, unsigned empty, int group,
                                              int lane) {
     // those inside; the stager knows which rows of several chunks are
     const int first = ROWS ? 0 : max(0, PD - d0), last = ROWS ? planes - 1 : min(planes - 1, D - 1 + PD - d0);
-    if (group >= first && group <= last) st.load(d0 - PD + group);
-    for (int p = group; p < planes; p += GROUPS) {
-        const int s = p % SLOTS;
-        if (p >= SLOTS && !mbar_wait(empty + 8 * s, (p / SLOTS - 1) & 1)) return false;
+    const int begin = (group - base % GROUPS + GROUPS) % GROUPS;
+    if (begin >= first && begin <= last) st.load(d0 - PD + begin);
+    for (int p = begin; p < planes; p += GROUPS) {
+        const int s = (base + p) % SLOTS, use = (base + p) / SLOTS;
+        if (use && !mbar_wait(empty + 8 * s, (use - 1) & 1)) return false;
         if (p >= first && p <= last) {
             store(s);
             fence_async_proxy();
@@ -297,7 +311,12 @@ struct Stager {
         for (int u = 0; u < U; ++u) {
             if (has(u, d)) {
 #pragma unroll
-                for (int ch = 0; ch < NCH; ++ch) load_words<WIDE>(p + ch * stride, off[u], w[u], b.W, a[u][ch]);
+                for (int ch = 0; ch < NCH; ++ch) {
+                    // a pointer per block and tensor, or a base and 32-bit offsets: rows that are not whole blocks
+                    // make several loads of a pointer (64 x 5 images of 203x171, 3x3, forward: 257 -> 237 us)
+                    if (ROWS && !WIDE) load_words<WIDE>(p + ch * stride + off[u], 0, w[u], b.W, a[u][ch]);
+                    else load_words<WIDE>(p + ch * stride, off[u], w[u], b.W, a[u][ch]);
+                }
             } else if (ROWS) {
 #pragma unroll
                 for (int ch = 0; ch < NCH; ++ch)
@@ -354,9 +373,10 @@ __device__ __forceinline__ unsigned word_of(const uint4& v, int i) { return i ==
 
 // The banded matrices of a kernel: `value(t, n, k)` is what place k of matrix t, column n is multiplied by.
 // Layout of one matrix: groups of eight columns, then the two halves of K, eight 16-byte rows each.
+// Done by the `threads` threads of a group of stagers, of which this is number `tid`.
 template <int NCOL, typename F>
-__device__ __forceinline__ void build_bands(bf16* bmat, int mats, F value) {
-    for (int e = threadIdx.x; e < mats * NCOL * 2; e += blockDim.x) {
+__device__ __forceinline__ void build_bands(bf16* bmat, int mats, int tid, int threads, F value) {
+    for (int e = tid; e < mats * NCOL * 2; e += threads) {
         const int n = e % 8, half = (e / 8) % 2, g = (e / 16) % (NCOL / 8), t = e / (2 * NCOL);
         unsigned words[4];
 #pragma unroll
@@ -423,7 +443,7 @@ struct AdjointArgs {
 // columns, two CTAs per multiprocessor; five: eight planes, all 512.
 template <int KD> __host__ __device__ constexpr int adjoint_ring() { return KD > 3 ? 8 : 4; }
 
-template <int KD, int KH, int KW, int AL, int MODE>
+template <int KD, int KH, int KW, int AL, int MODE, bool MARCH>
 __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::CTAS) tc_adjoint_kernel(const AdjointArgs P) {
     constexpr bool ROWS = KH == 1;
     typedef AdjointShape<KD> Shape;
@@ -431,33 +451,41 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
     constexpr int PD = KD / 2, NC = SC * 8, RING = adjoint_ring<KD>(), TCOLS = RING * 2 * NC, KT = KD * KH * KW;
     extern __shared__ __align__(128) unsigned char smem_tc[];
     const Band& b = P.b;
-    const At<ROWS> at(b, blockIdx.x);
+    const Items<MARCH> items(b);
+    const At<ROWS> first(b, items.first);
     const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W), oaddr(b.C, b.D, b.H, b.Wo);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned base = smem_u32(smem_tc);
     const unsigned sfull = base, sempty = base + 8 * kSlots, afull = base + 16 * kSlots, aempty = afull + 8 * RING;
-    constexpr int kTmemAt = 16 * kSlots + 16 * RING;
+    const unsigned bfull = aempty + 8 * RING, bfree = bfull + 8;      // the banded matrices are there; are no longer read
+    constexpr int kTmemAt = 16 * kSlots + 16 * RING + 16;
     bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader);
     uint4* const slots = reinterpret_cast<uint4*>(smem_tc + kHeader + KH * KD * NC * 32);
     const int blocks = (b.TH + KH - 1) * b.PB, slot_blocks = 2 * blocks;
-    const int planes = at.DC + KD - 1;
 
     if (warp == kMmaWarp) tmem_alloc(base + kTmemAt, TCOLS);
     if (tid == 0) {
         for (int i = 0; i < kSlots; ++i) { mbar_init(sfull + 8 * i, Shape::STAGERS / 32); mbar_init(sempty + 8 * i, 1); }
         for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, 4); }
+        mbar_init(bfull, Shape::STAGERS / 32);
+        mbar_init(bfree, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // windows of valid blocks may touch blocks that no plane has been staged to: those have to be numbers
     for (int i = tid; i < kSlots * slot_blocks + slack_blocks(b); i += kThreads) slots[i] = make_uint4(0u, 0u, 0u, 0u);
-    float* const hs = reinterpret_cast<float*>(smem_tc + 512);
-    for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)at.c * SC * KT + e];
-    __syncthreads();
     // [kh][output plane p - (KD - 1) + kd: groups of 32 columns][channel, column]
-    build_bands<KD * NC>(bmat, KH, [&](int kh, int n, int k) {
-        const int kd = n / NC, j = n % NC / 8, kw = n % 8 + KW - 1 - k;
-        return kw >= 0 && kw < KW ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
-    });
+    auto bands = [&](const float* h, int own, int threads) {
+        build_bands<KD * NC>(bmat, KH, own, threads, [&](int kh, int n, int k) {
+            const int kd = n / NC, j = n % NC / 8, kw = n % 8 + KW - 1 - k;
+            return kw >= 0 && kw < KW ? h[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
+        });
+    };
+    if (!MARCH) {
+        float* const hs = reinterpret_cast<float*>(smem_tc + 512);
+        for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)first.c * SC * KT + e];
+        __syncthreads();
+        bands(hs, tid, kThreads);
+    }
     fence_async_proxy();
     tc_fence_before();
     __syncthreads();
@@ -473,17 +501,21 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
     bool ok = true;
     if (warp == kMmaWarp) {
         const unsigned long long ad = mat_desc(smem_u32(slots), 16, 128), md = mat_desc(smem_u32(bmat), 128, 256);
-        for (int p = 0; p < planes && ok && lane == 0; ++p) {
-            const int s = p % kSlots, d = at.d0 - PD + p;
-            ok = mbar_wait_thread(sfull + 8 * s, (p / kSlots) & 1, kWaitLimit);
-            // a new output plane begins: its accumulators have been read and zeroed
-            if (p >= RING && p < at.DC) ok = mbar_wait_thread(aempty + 8 * (p % RING), (p / RING - 1) & 1, kWaitLimit) && ok;
-            tc_fence_after();
-            if (ok) {
+        // base, out: planes and output planes of the places before
+        auto place = [&](const At<ROWS>& at, int base, int out) {
+            const int planes = at.DC + KD - 1;
+            for (int p = 0; p < planes && ok && lane == 0; ++p) {
+                const int s = (base + p) % kSlots, d = at.d0 - PD + p;
+                ok = mbar_wait_thread(sfull + 8 * s, ((base + p) / kSlots) & 1, kWaitLimit);
+                // a new output plane begins: its accumulators have been read and filled again
+                const int begun = out + p;
+                if (begun >= RING && p < at.DC) ok = mbar_wait_thread(aempty + 8 * (begun % RING), (begun / RING - 1) & 1, kWaitLimit) && ok;
+                tc_fence_after();
+                if (!ok) break;
                 if (ROWS || (d >= 0 && d < b.D)) {
                     // groups g of output planes o = p - (KD - 1) + g inside the chunk
                     const int g0 = max(0, KD - 1 - p), g1 = min(KD - 1, at.DC - 1 + KD - 1 - p), o0 = p - (KD - 1) + g0;
-                    const int r0 = o0 % RING, n = g1 - g0 + 1, n0 = min(n, RING - r0);
+                    const int r0 = (out + o0) % RING, n = g1 - g0 + 1, n0 = min(n, RING - r0);
                     // descriptors differ in their start address alone, in units of 16 bytes
                     const unsigned long long a0 = ad + s * slot_blocks, m0 = md + g0 * NC * 2;
                     const unsigned i0 = instr_desc(n0 * NC), i1 = instr_desc((n - n0) * NC);
@@ -498,22 +530,62 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                 }
                 mma_commit(sempty + 8 * s);
                 const int o = p - (KD - 1);
-                if (o >= 0) mma_commit(afull + 8 * (o % RING));
+                if (o >= 0) mma_commit(afull + 8 * ((out + o) % RING));
             }
+        };
+        if (MARCH) {
+            int base = 0, out = 0, channel = -1, built = 0;
+            for (int item = items.first; item < items.last && ok && lane == 0; ++item) {
+                const At<ROWS> at(b, item);
+                if (at.c != channel) {
+                    if (channel >= 0) mma_commit(bfree);
+                    channel = at.c;
+                    ok = mbar_wait_thread(bfull, built++ & 1, kWaitLimit);
+                }
+                place(at, base, out);
+                base += at.DC + KD - 1;
+                out += at.DC;
+            }
+        } else {
+            place(first, 0, 0);
         }
     } else if (warp >= kEpilogueWarps) {
         // x and t1 as two channels: the distance between the tensors takes the place of the stride
         const long long apart = ((long long)(uintptr_t)P.t1 - (long long)(uintptr_t)P.x) / 2;
-        Stager<KH, KW, 2, AL == kWide, Shape::STAGERS, Shape::BLOCKS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x,
-                                                                         at, (tid - 32 * kEpilogueWarps) % Shape::STAGERS);
-        ok = stage_planes<kSlots, Shape::GROUPS, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, planes, sfull, sempty,
-                                                 (tid - 32 * kEpilogueWarps) / Shape::STAGERS, lane);
+        const int group = (tid - 32 * kEpilogueWarps) / Shape::STAGERS, own = (tid - 32 * kEpilogueWarps) % Shape::STAGERS;
+        auto place = [&](const At<ROWS>& at, int base) {
+            Stager<KH, KW, 2, AL == kWide, Shape::STAGERS, Shape::BLOCKS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at, own);
+            ok = stage_planes<kSlots, Shape::GROUPS, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, at.DC + KD - 1, base,
+                                                           sfull, sempty, group, lane);
+        };
+        if (MARCH) {
+            int base = 0, channel = -1, built = 0;
+            for (int item = items.first; item < items.last && ok; ++item) {
+                const At<ROWS> at(b, item);
+                if (at.c != channel) {
+                    channel = at.c;
+                    if (group == 0) {      // always the same one: it sees every phase of the barrier
+                        if (built) ok = mbar_wait(bfree, (built - 1) & 1);
+                        bands(P.h + (long long)channel * SC * KT, own, Shape::STAGERS);
+                        fence_async_proxy();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bfull);
+                    }
+                    ++built;
+                }
+                if (ok) place(at, base);
+                base += at.DC + KD - 1;
+            }
+        } else {
+            place(first, 0);
+        }
     } else {
         const int m = (warp & 3) * 32 + lane, r = m / b.PB, q = m - r * b.PB, w = 8 * q;
+        const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
+        auto place = [&](const At<ROWS>& at, int out) {
         const RowAt<ROWS> zat(b, at.h0 + r, addr.row_z, addr.plane), oat(b, at.h0 + r, oaddr.row_z, oaddr.plane);
         // this row's output planes in the march
         const int count = r < at.TH && q < b.NB ? (ROWS ? min(b.DC, b.D - zat.d) : at.DC) : 0;
-        const unsigned lanes = tmem + ((unsigned)(warp & 3) << 21);
         f32x2 b2[SC];
 #pragma unroll
         for (int j = 0; j < SC; ++j) {
@@ -524,8 +596,8 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         const long long orow = (long long)at.bc * SC * oaddr.chan + oat.off;
         const bf16* const zb = P.z + zrow;
         const bf16* const gb = MODE == kOut ? nullptr : P.gout + orow;
-        for (int o = warp >> 2; o < at.DC && ok; o += Shape::EPI) {
-            const int slot = o % RING;
+        for (int o = ((warp >> 2) - out % Shape::EPI + Shape::EPI) % Shape::EPI; o < at.DC && ok; o += Shape::EPI) {
+            const int slot = (out + o) % RING;
             const long long d = at.d0 + o;
             const bool valid = o < count;
             // z of all channels, or z and gout of two (the registers do not hold more), are on their way
@@ -554,7 +626,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
             };
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j) fetch(j);
-            ok = mbar_wait(afull + 8 * slot, (o / RING) & 1);
+            ok = mbar_wait(afull + 8 * slot, ((out + o) / RING) & 1);
             tc_fence_after();
             const unsigned acc = lanes + slot * NC;
 #pragma unroll
@@ -629,6 +701,17 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
                     }
                 }
             }
+        }
+        };
+        if (MARCH) {
+            int out = 0;
+            for (int item = items.first; item < items.last && ok; ++item) {
+                const At<ROWS> at(b, item);
+                place(at, out);
+                out += at.DC;
+            }
+        } else {
+            place(first, 0);
         }
     }
     if (!ok && lane == 0) report_expired(P.expired);
@@ -732,7 +815,7 @@ struct SourceStager {
 };
 
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const SourceArgs P) {
+__global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(const SourceArgs P) {
     constexpr bool ROWS = KH == 1;
     constexpr int kThreads = kSourceThreads, kEpilogueWarps = 4, kMmaWarp = 14;
     constexpr int PD = KD / 2, PW = KW / 2, KT = KD * KH * KW, RING = source_ring<KD>();
@@ -764,7 +847,7 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
     for (int e = tid; e < SC * KT; e += kThreads) hs[e] = P.h[(long long)at.c * SC * KT + e];
     __syncthreads();
     // [channel, kh][output plane p - kd, kd = KD - 1 - g: groups of 16 columns][own eight columns, left, right]
-    build_bands<NCOL>(bmat, NMAT, [&](int t, int n, int k) {
+    build_bands<NCOL>(bmat, NMAT, tid, kThreads, [&](int t, int n, int k) {
         const int j = t / KH, kh = t % KH, kd = KD - 1 - n / kGroup, i = n % kGroup;
         const int o = i < 8 ? i : i < 8 + PW ? i - 8 - PW : i - PW, kw = k % 8 - o + PW;
         return i < 8 + 2 * PW && kw >= 0 && kw < KW ? hs[j * KT + (kd * KH + kh) * KW + kw] : 0.0f;
@@ -813,7 +896,7 @@ __global__ void __launch_bounds__(kSourceThreads, 2) tc_source_kernel(const Sour
         }
         SourceStager<KH, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at,
                                          (tid - 32 * kEpilogueWarps) % kSourceStagers);
-        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, sfull,
+        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, 0, sfull,
                                            sempty, (warp - kEpilogueWarps) / 5, lane);
     } else {
         const int m = warp * 32 + lane, r = m / b.NB, q = m - r * b.NB, w = 8 * q;
