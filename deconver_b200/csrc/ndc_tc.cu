@@ -208,20 +208,21 @@ cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1
 }
 
 // How large a problem has to be, and how much of the MMAs' rows it has to fill, for the tensor cores to be the
-// faster way: volumes from 0.8 M group-voxels on, rows of 128 at least 30 % full (16^3 fills 25 % and its forward
-// takes 0.93x the FMA kernels' speed, 20^3 39 % and 1.23x - 1.36x); images from 3 M on and 45 % (8 images of 64
-// columns 1.29x, 4 of them 0.79x), 80 % for 3x3 filters at the widths the FMA kernels have compile-time
-// instances for (4 x 64 of 128^2 0.81x).  On 31 shapes about the lines nothing that goes to the tensor cores is
-// slower there (forward 1.19x - 1.70x, a whole update 1.04x - 1.19x); some that stays would gain (16 x 128 of 32^2
-// 1.49x, 16 x 32 of 256^2 with 3x3 filters 1.43x): the lines are older than the source kernel's present form.
+// faster way.  Device time of an update against the FMA kernels', on 76 shapes about the lines:
+//   volumes    from 0.4 M group-voxels on (0.4 - 0.8 M: forward 0.94x - 1.45x, with the backward 1.00x - 1.20x), rows of 128
+//              at least 30 % full (16^3 fills 25 %: 0.90x - 0.94x)
+//   images     from 0.7 M on, 45 % full (0.7 - 3 M: forward 1.00x - 2.1x, with the backward 0.96x - 1.29x); below
+//              3 M from 10 rows on, 20 with 5x5 filters (16 x 512 of 16^2: 0.79x; 16 x 128 of 20^2: 1.04x); 3x3 filters at the widths that the FMA kernels
+//              have compile-time instances for from 3 M on, 70 % full (2 x 64 of 128^2: 1.04x, 0.98x; 16 x 32 of 256^2, 75 %
+//              full: 1.49x, 1.13x)
 template <int KD, int KH, int KW>
 bool worth(const Geo& g) {
     Band a, s;
     if (!plan<KD, KH, KW>(g, false, a) || !plan<KD, KH, KW>(g, true, s)) return false;
     const double voxels = (double)g.B * g.G * g.D * g.H * g.Wv, use = std::min(useful<KH>(a), useful<KH>(s));
-    if (KH > 1) return voxels >= 0.8e6 && use >= 0.3;
+    if (KH > 1) return voxels >= 0.4e6 && use >= 0.3;
     const bool tuned = KW == 3 && (g.W == 64 || g.W == 128 || g.W == 256);
-    return voxels >= 3e6 && use >= (tuned ? 0.8 : 0.45);
+    return tuned ? voxels >= 3e6 && use >= 0.7 : use >= 0.45 && (voxels >= 3e6 || (voxels >= 0.7e6 && g.D >= 10 * (KD / 2)));
 }
 
 // Image batches as volumes whose planes are the image rows and whose plane rows are the images.
