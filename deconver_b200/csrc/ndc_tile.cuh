@@ -713,11 +713,18 @@ inline BwdScratch scratch_shape(const Geo& g) {
     s.bytes = s.corr + up256((size_t)g.G * g.m * source_blocks(g) * corr_splits(g, tc) * g.KT * CB * sizeof(float));
     return s;
 }
+// Whether whole vectors go to the pairs kernels: not where their scratch alone would be too large for
+// ndc_bwd_static, whose results are those of ndc_bwd.
+template <int KD, int KH, int KW>
+inline bool use_pairs(const Geo& g, size_t own) {
+    if (!pairs::covers(g)) return false;
+    return own > NDC_STATIC_WORKSPACE_BYTES || pairs::scratch_shape<KD, KH, KW>(g).bytes <= NDC_STATIC_WORKSPACE_BYTES;
+}
 // Bytes of it for either kind of kernel: which one runs depends on the tensors' alignment too.
 template <int KD, int KH, int KW>
 inline size_t scratch_bytes(const Geo& g) {
     const size_t n = scratch_shape<KD, KH, KW>(g).bytes;
-    return pairs::covers(g) ? std::max(n, pairs::scratch_shape<KD, KH, KW>(g).bytes) : n;
+    return use_pairs<KD, KH, KW>(g, n) ? std::max(n, pairs::scratch_shape<KD, KH, KW>(g).bytes) : n;
 }
 inline size_t bwd_scratch(const Geo& g) {
     if (g.kD == 3) return scratch_bytes<3, 3, 3>(g);
@@ -785,9 +792,9 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
 template <typename T, int KD, int KH, int KW>
 cudaError_t backward_shape(const Geo& g, const T* x, const T* z, const T* t1, const float* h, const float* bias,
                            const T* gout, T* gx, T* gz, float* gh, float* gb, void* ws, cudaStream_t st) {
-    if (pairs::covers(g) && pairs::whole<T>({x, z, t1, gout, gx, gz}))
-        return pairs::backward_shape<T, KD, KH, KW>(g, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
     const BwdScratch sc = scratch_shape<KD, KH, KW>(g);
+    if (use_pairs<KD, KH, KW>(g, sc.bytes) && pairs::whole<T>({x, z, t1, gout, gx, gz}))
+        return pairs::backward_shape<T, KD, KH, KW>(g, x, z, t1, h, bias, gout, gx, gz, gh, gb, ws, st);
     float* gnum = (float*)((char*)ws + sc.gnum);
     float* gden = (float*)((char*)ws + sc.gden);
     float* gt1 = (float*)((char*)ws + sc.gt1);

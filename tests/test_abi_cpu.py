@@ -173,3 +173,20 @@ def test_bias_entry_points_validate_without_a_gpu(lib):
     assert b"positive" in lib.ndc_bias_last_error()
     assert lib.ndc_bias_gelu_fwd(2, 64, 4096, 7, 16, None, 16, None) == 1
     assert b"dtype" in lib.ndc_bias_last_error()
+
+
+def test_grouped_scratch_near_the_built_in_array():
+    """Grouped geometries whose scratch fits the array of `ndc_bwd_static` with the tile kernels keep fitting: the pairs
+    kernels' records are larger, and where they alone would exceed it the tile kernels stay."""
+    lib = _lib.load()
+    limit, near = _lib.STATIC_WORKSPACE_BYTES, 0
+    for planes in range(20, 60):
+        for rows in range(8, 40, 2):
+            desc = _lib.make_desc(1, 4, 2, 8, (planes, rows, 32), (3, 3, 3), 1e-16, True, _lib.NDC_F32)
+            need = lib.ndc_bwd_workspace_bytes(desc)
+            tensors = 4 * (2 * 8 + 2) * planes * rows * 32 * 4      # gnum, gden and gt1, float32
+            assert need >= tensors
+            if limit - 300000 < tensors + 150000 <= limit:          # the tile kernels' records are below 150 kB here
+                near += 1
+                assert need <= limit
+    assert near
