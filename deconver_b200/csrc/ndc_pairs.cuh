@@ -16,7 +16,7 @@
 // four 16-byte words serves all channels and up to three filter rows; weights are read by broadcast).  With
 // one stream per pass, neighbouring voxels in the lanes and four channels per thread it was 2.3 - 5:
 // lanes moved to make odd pairs, windows read once per filter row, and each tile staged once per four channels.
-// A training step with 8 groups of 4 channels and 8 sources, 2 x 32^3, float32: 733 -> 502 us.
+// A training step with 8 groups of 4 channels and 8 sources, 2 x 32^3, float32: 733 -> 489 us.
 //
 //   conv_kernel      A of x and t1 (forward output, backward ratio terms) or of gt1 (source gradient); K of the
 //                    source, or of the two backward ratio tensors
@@ -643,7 +643,7 @@ struct ConvPlan { TileGeo t; int cb, blocks, units; long long grid; size_t smem;
 
 // The CTA size (tiles of as many strips) of least expected time: instructions of a CTA and channel, its sweep
 // and its staged quads, times the CTAs of the fullest multiprocessor, which few warps leave waiting (by 6 /
-// warps).
+// warps; as many as fit its shared memory: counted so, the training step above takes 489 us for 501).
 template <int KD, int KH, int KW>
 inline ConvPlan plan_conv(const Geo& g, bool adjoint, bool two_tiles) {
     ConvPlan best;
@@ -662,7 +662,8 @@ inline ConvPlan plan_conv(const Geo& g, bool adjoint, bool two_tiles) {
         const int warps = p.t.threads / 32;
         const double cta = warps * 1.25 * g.KT * 8 * V + p.t.chunks / 32.0 * 30.0;
         const long long per_sm = (p.grid + num_sms() - 1) / num_sms();
-        const double resident = (double)std::min(per_sm * warps, 16LL);
+        const long long fit = std::max((size_t)1, (size_t)225 * 1024 / (p.smem + 1024));
+        const double resident = (double)std::min(std::min(per_sm, fit) * warps, 16LL);
         const double time = cta * (double)per_sm * (1.0 + 6.0 / resident);
         if (least < 0 || time < 0.97 * least) { least = time; best = p; }
     }
