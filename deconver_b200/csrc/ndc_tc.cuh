@@ -9,8 +9,8 @@
 // accumulators of KD output planes, which lie next to each other in TMEM.  So a source plane is read
 // once, when the CTA's march through the depth comes to it, and a filter row kh is a shift of the start
 // address.  Batches of images march down their rows the same way (planes = image rows, plane rows =
-// images, KH = 1: see SlabAddr); the rows of their bands never meet, so a band takes any of them, of several
-// chunks at once (see At), and fills its 128 blocks whatever the batch.  An MMA of up to 128 columns takes 64 cycles here, whatever its width
+// images, KH = 1: see SlabAddr); no filter row takes a row of their bands to another, so a band takes any of them, of
+// several chunks at once (see At), and fills its 128 blocks whatever the batch.  An MMA of up to 128 columns takes 64 cycles here, whatever its width
 // (reading 4 KB of A operand), hence the wide ones.  With KW = 3 most of the products meet a zero of the
 // band; the tensor cores do them 30 times faster than the FMA pipe does the useful ones.  What K = 16
 // holds differs:
@@ -244,10 +244,11 @@ __device__ __forceinline__ uint4 to_places(const unsigned (&a)[5]) {
 }
 
 // A group's planes of a chunk: p counts source planes from d0 - PD, `base` those of the places before; planes
-// outside the volume are passed on without data.  `S`: load, prefetch and store a plane.
+// outside the volume are passed on without data.  `S`: load, prefetch and store a plane; `again`: set where one of its
+// values is not finite (see look()).
 template <int SLOTS, int GROUPS, bool ROWS, typename S, typename F>
 __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int PD, int planes, int base, unsigned full, unsigned empty, int group,
-                                             int lane) {
+                                             int lane, volatile unsigned* again) {
     // those inside; the stager knows which rows of several chunks are
     const int first = ROWS ? 0 : max(0, PD - d0), last = ROWS ? planes - 1 : min(planes - 1, D - 1 + PD - d0);
     const int begin = (group - base % GROUPS + GROUPS) % GROUPS;
@@ -256,7 +257,7 @@ __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int 
         const int s = (base + p) % SLOTS, use = (base + p) / SLOTS;
         if (use && !mbar_wait(empty + 8 * s, (use - 1) & 1)) return false;
         if (p >= first && p <= last) {
-            store(s);
+            if (store(s)) *again = 1u;
             fence_async_proxy();
         }
         __syncwarp();
@@ -265,6 +266,20 @@ __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int 
         if (p + 2 * GROUPS <= last) st.prefetch(d0 - PD + p + 2 * GROUPS);
     }
     return true;
+}
+
+// Infinities and NaN.  A zero of the band times one of them is NaN, and a window reaches into its row's next block and, past
+// its last one, into the next row's: what the taps never see would become NaN, in another image too.  So the stagers look
+// at what they stage, and a CTA that has met one computes what became NaN once more after its march, tap by tap on the FMA
+// pipe (adjoint_again, source_again).  Looking takes an instruction for two values: 131 us for 128 in the source kernel at
+// 2 x 64 x 64^3, nothing measurable in the adjoint.  Where every value is one the forward takes 7.0 ms there, not 0.33.
+// (A block of zeros between the rows would keep images apart, and NaN spread over blocks of eight columns all the same.)
+// Not zero where one of the eight values is not finite.
+__device__ __forceinline__ unsigned look(const uint4& v) {
+    unsigned seen = 0u;
+    asm("fma.rn.bf16x2 %0, %1, %5, %0;\n\tfma.rn.bf16x2 %0, %2, %5, %0;\n\tfma.rn.bf16x2 %0, %3, %5, %0;\n\tfma.rn.bf16x2 %0, %4, %5, %0;"
+        : "+r"(seen) : "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(0u));
+    return seen;
 }
 
 // Stages planes of NCH channels (`src + ch * stride`), halo rows included; rows outside the volume are
@@ -279,32 +294,32 @@ struct Stager {
     long long stride, plane;
     int blocks;                    // per channel of a slot
     unsigned off[U];               // this thread's blocks: offset of the first column
-    bool in[U];                    // inside the volume (else zero)
-    int w[U], at[U];               // column; block, or -1
+    unsigned in;                   // bit u: inside the volume (else zero)
+    int w[U], own;                 // columns; the first block
     int d0[U];                     // ROWS: first plane of the row's chunk
     unsigned a[U][NCH][5];
 
     __device__ __forceinline__ Stager(const Band& b_, const bf16* src_, long long stride_, long long plane_, long long row_stride, const At<ROWS>& place,
                                       int tid)
-        : b(b_), src(src_ + (ROWS ? base_row(b_, place.h0) : place.h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB) {
+        : b(b_), src(src_ + (ROWS ? base_row(b_, place.h0) : place.h0 - KH / 2) * row_stride), stride(stride_), plane(plane_), blocks((b_.TH + KH - 1) * b_.PB),
+          in(0u), own(tid) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int i = tid + u * NTHR, row = i / b.PB, q = i - row * b.PB, h = place.h0 - KH / 2 + row;
-            at[u] = i < blocks ? i : -1;
             w[u] = 8 * q;
             if (ROWS) {
                 const RowAt<ROWS> r(b, h, row_stride, plane);
                 d0[u] = r.d;
                 off[u] = (unsigned)(r.off - base_row(b, place.h0) * row_stride) + w[u];
-                in[u] = i < blocks && row < place.TH;
+                in |= (i < blocks && row < place.TH ? 1u : 0u) << u;
             } else {
                 d0[u] = 0;
                 off[u] = (unsigned)(row * row_stride) + w[u];
-                in[u] = i < blocks && h >= 0 && h < b.H;
+                in |= (i < blocks && h >= 0 && h < b.H ? 1u : 0u) << u;
             }
         }
     }
-    __device__ __forceinline__ bool has(int u, int d) const { return in[u] && (!ROWS || (unsigned)(d + d0[u]) < (unsigned)b.D); }
+    __device__ __forceinline__ bool has(int u, int d) const { return (in >> u & 1) && (!ROWS || (unsigned)(d + d0[u]) < (unsigned)b.D); }
     __device__ __forceinline__ void load(int d) {
         const bf16* p = src + d * plane;
 #pragma unroll
@@ -335,14 +350,20 @@ struct Stager {
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off[u]));
             }
     }
-    __device__ __forceinline__ void store(uint4* dst) {
+    __device__ __forceinline__ unsigned store(uint4* dst) {
+        unsigned seen = 0u;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (at[u] < 0) continue;
+            const int i = own + u * NTHR;
+            if (i >= blocks) continue;
 #pragma unroll
-            for (int ch = 0; ch < NCH; ++ch)
-                dst[ch * blocks + at[u]] = in[u] ? to_places<KW / 2>(a[u][ch]) : make_uint4(0u, 0u, 0u, 0u);
+            for (int ch = 0; ch < NCH; ++ch) {
+                const uint4 v = in >> u & 1 ? to_places<KW / 2>(a[u][ch]) : make_uint4(0u, 0u, 0u, 0u);
+                dst[ch * blocks + i] = v;
+                seen |= look(v);
+            }
         }
+        return seen;
     }
 };
 
@@ -354,11 +375,6 @@ __host__ __device__ inline int slack_blocks(const Band& b) { return MB + 1 - b.T
 using dw4::f32x2;
 using dw4::pack2;
 using dw4::unpack2;
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -443,8 +459,73 @@ struct AdjointArgs {
 // columns, two CTAs per multiprocessor; five: eight planes, all 512.
 template <int KD> __host__ __device__ constexpr int adjoint_ring() { return KD > 3 ? 8 : 4; }
 
+// What became NaN of a place's outputs (out; gden where any of the three did) tap by tap (see look()), by all threads of the
+// CTA.  A function of its own: inline, it costs the kernel's loops registers.
+template <int KD, int KH, int KW, int MODE>
+__device__ __noinline__ void adjoint_again(const AdjointArgs& P, int item) {
+    constexpr bool ROWS = KH == 1;
+    constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
+    const Band& b = P.b;
+    const At<ROWS> at(b, item);
+    const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W), oaddr(b.C, b.D, b.H, b.Wo);
+    const float* const hc = P.h + (long long)at.c * SC * KT;
+#pragma unroll 1
+    for (int o = 0; o < at.DC; ++o)
+#pragma unroll 1
+        for (int e = threadIdx.x; e < at.TH * b.Wv; e += blockDim.x) {
+            const int r = e / b.Wv, w = e - r * b.Wv, h = at.h0 + r;
+            const RowAt<ROWS> xat(b, h, addr.row_x, addr.plane), zat(b, h, addr.row_z, addr.plane), oat(b, h, oaddr.row_z, oaddr.plane);
+            const int d = at.d0 + o;                 // from the row's chunk on
+            if (d + xat.d >= b.D) continue;
+            const long long ze0 = (long long)at.bc * SC * addr.chan + zat.off + d * addr.plane + w;
+            const long long oe0 = (long long)at.bc * SC * oaddr.chan + oat.off + d * oaddr.plane + w;
+            bool nan = false;
+#pragma unroll
+            for (int j = 0; j < SC; ++j) {
+                const long long ze = ze0 + j * addr.chan;
+                nan |= isnan(MODE == kOut ? to_f32(P.out[oe0 + j * oaddr.chan]) : MODE == kPairs ? P.gnum[2 * ze] : P.gden[ze]);
+            }
+            if (!nan) continue;
+            float n[SC], dn[SC];
+#pragma unroll
+            for (int j = 0; j < SC; ++j) n[j] = dn[j] = b.eps;
+            const long long row = (long long)at.bc * addr.chan + xat.off + w + PW;
+#pragma unroll 1
+            for (int t = 0; t < KT; t += KW) {
+                const int kh = t / KW % KH, kd = t / (KW * KH), dd = d + PD - kd, hh = h + PH - kh;
+                if ((unsigned)(dd + xat.d) >= (unsigned)b.D || (!ROWS && (unsigned)hh >= (unsigned)b.H)) continue;
+                const long long off = row + dd * addr.plane + (PH - kh) * addr.row_x;
+#pragma unroll
+                for (int kw = 0; kw < KW; ++kw) {
+                    const bool here = (unsigned)(w + PW - kw) < (unsigned)b.Wv;
+                    const float xv = here ? to_f32(P.x[off - kw]) : 0.0f, tv = here ? to_f32(P.t1[off - kw]) : 0.0f;
+#pragma unroll
+                    for (int j = 0; j < SC; ++j) {
+                        n[j] = fmaf(xv, hc[j * KT + t + kw], n[j]);
+                        dn[j] = fmaf(tv, hc[j * KT + t + kw], dn[j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < SC; ++j) {
+                const long long ze = ze0 + j * addr.chan, oe = oe0 + j * oaddr.chan;
+                float s = to_f32(P.z[ze]) + (P.bias ? P.bias[at.c * SC + j] : 0.0f);
+                if (b.relu) s = fmaxf(s, 0.0f);
+                const float rd = rcp(dn[j]);
+                if (MODE == kOut) {
+                    P.out[oe] = from_f32<bf16>(s * n[j] * rd);
+                } else {
+                    const float g = to_f32(P.gout[oe]) * rd, gn = g * s, gd = -(gn * n[j] * rd);
+                    if (P.out) P.out[ze] = from_f32<bf16>(g * n[j]);
+                    P.gnum[MODE == kPairs ? 2 * ze + 1 : ze] = gn;
+                    if (MODE == kPairs) P.gnum[2 * ze] = gd; else P.gden[ze] = gd;
+                }
+            }
+        }
+}
+
 template <int KD, int KH, int KW, int AL, int MODE, bool MARCH>
-__global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::CTAS) tc_adjoint_kernel(const AdjointArgs P) {
+__global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::CTAS) tc_adjoint_kernel(const __grid_constant__ AdjointArgs P) {
     constexpr bool ROWS = KH == 1;
     typedef AdjointShape<KD> Shape;
     constexpr int kThreads = Shape::THREADS, kEpilogueWarps = 4 * Shape::EPI, kMmaWarp = kThreads / 32 - 1;
@@ -453,12 +534,13 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
     const Band& b = P.b;
     const Items<MARCH> items(b);
     const At<ROWS> first(b, items.first);
-    const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W), oaddr(b.C, b.D, b.H, b.Wo);
+    const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W), oaddr(b.C, b.D, b.H, AL == kPaddedOut ? b.Wo : b.W);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned base = smem_u32(smem_tc);
     const unsigned sfull = base, sempty = base + 8 * kSlots, afull = base + 16 * kSlots, aempty = afull + 8 * RING;
     const unsigned bfull = aempty + 8 * RING, bfree = bfull + 8;      // the banded matrices are there; are no longer read
     constexpr int kTmemAt = 16 * kSlots + 16 * RING + 16;
+    volatile unsigned* const again = reinterpret_cast<unsigned*>(smem_tc + kTmemAt + 4);      // see look()
     bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader);
     uint4* const slots = reinterpret_cast<uint4*>(smem_tc + kHeader + KH * KD * NC * 32);
     const int blocks = (b.TH + KH - 1) * b.PB, slot_blocks = 2 * blocks;
@@ -469,6 +551,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, 4); }
         mbar_init(bfull, Shape::STAGERS / 32);
         mbar_init(bfree, 1);
+        *again = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // windows of valid blocks may touch blocks that no plane has been staged to: those have to be numbers
@@ -555,8 +638,8 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         const int group = (tid - 32 * kEpilogueWarps) / Shape::STAGERS, own = (tid - 32 * kEpilogueWarps) % Shape::STAGERS;
         auto place = [&](const At<ROWS>& at, int base) {
             Stager<KH, KW, 2, AL == kWide, Shape::STAGERS, Shape::BLOCKS> st(b, P.x + (long long)at.bc * addr.chan, apart, addr.plane, addr.row_x, at, own);
-            ok = stage_planes<kSlots, Shape::GROUPS, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, at.DC + KD - 1, base,
-                                                           sfull, sempty, group, lane);
+            ok = stage_planes<kSlots, Shape::GROUPS, ROWS>(st, [&](int s) { return st.store(slots + s * slot_blocks); }, b.D, at.d0, PD, at.DC + KD - 1, base,
+                                                           sfull, sempty, group, lane, again);
         };
         if (MARCH) {
             int base = 0, channel = -1, built = 0;
@@ -586,12 +669,9 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         const RowAt<ROWS> zat(b, at.h0 + r, addr.row_z, addr.plane), oat(b, at.h0 + r, oaddr.row_z, oaddr.plane);
         // this row's output planes in the march
         const int count = r < at.TH && q < b.NB ? (ROWS ? min(b.DC, b.D - zat.d) : at.DC) : 0;
-        f32x2 b2[SC];
+        float bj[SC];          // (as pairs for two-lane additions: four registers more, 2.65 ms for 2.42 at 4 x 64 x 128^3)
 #pragma unroll
-        for (int j = 0; j < SC; ++j) {
-            const float v = P.bias ? P.bias[at.c * SC + j] : 0.0f;
-            b2[j] = pack2(v, v);
-        }
+        for (int j = 0; j < SC; ++j) bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
         const long long zrow = (long long)at.bc * SC * addr.chan + zat.off;
         const long long orow = (long long)at.bc * SC * oaddr.chan + oat.off;
         const bf16* const zb = P.z + zrow;
@@ -647,9 +727,7 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const unsigned u = word_of(zr[j % AHEAD], i);
-                    f32x2 s2 = add2(pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)), b2[j]);
-                    float lo, hi;
-                    unpack2(s2, lo, hi);
+                    float lo = __uint_as_float(u << 16) + bj[j], hi = __uint_as_float(u & 0xffff0000u) + bj[j];
                     if (b.relu) { lo = fmaxf(lo, 0.0f); hi = fmaxf(hi, 0.0f); }
                     const f32x2 n2 = pack2(n[2 * i], n[2 * i + 1]), r2 = pack2(rcp(dn[2 * i]), rcp(dn[2 * i + 1]));
                     if (MODE == kOut) {
@@ -719,6 +797,8 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
     __syncthreads();
     __syncwarp();
     if (warp == kMmaWarp) tmem_free(tmem, TCOLS);
+    if (*again)
+        for (int item = items.first; item < items.last; ++item) adjoint_again<KD, KH, KW, MODE>(P, item);
 }
 
 // ---- t1 = K(relu(z + b)) ------------------------------------------------------------------------
@@ -790,8 +870,9 @@ struct SourceStager {
         for (int ch = 0; ch < SC; ++ch) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off));
     }
     // `bias`: two copies of b per channel
-    __device__ __forceinline__ void store(uint4* dst, const unsigned (&bias)[SC], bool relu) {
-        if (at < 0) return;
+    __device__ __forceinline__ unsigned store(uint4* dst, const unsigned (&bias)[SC], bool relu) {
+        if (at < 0) return 0u;
+        unsigned seen = 0u;
 #pragma unroll
         for (int ch = 0; ch < SC; ++ch) {
             unsigned z[4], c[4];
@@ -808,14 +889,58 @@ struct SourceStager {
                 z[i] &= m;
                 c[i] = bias[ch] & m;
             }
-            dst[2 * ch * blocks + at] = make_uint4(z[0], z[1], z[2], z[3]);
+            const uint4 v = make_uint4(z[0], z[1], z[2], z[3]);
+            dst[2 * ch * blocks + at] = v;
+            seen |= look(v);
             dst[(2 * ch + 1) * blocks + at] = make_uint4(c[0], c[1], c[2], c[3]);
         }
+        return seen;
     }
 };
 
+// What became NaN of a place's t1 tap by tap (see look()), by all threads of the CTA.
+template <int KD, int KH, int KW>
+__device__ __noinline__ void source_again(const SourceArgs& P, int item) {
+    constexpr bool ROWS = KH == 1;
+    constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
+    const Band& b = P.b;
+    const At<ROWS> at(b, item);
+    const dw4::SlabAddr<ROWS> addr(b.C, b.D, b.H, b.W);
+#pragma unroll 1
+    for (int o = 0; o < at.DC; ++o)
+#pragma unroll 1
+        for (int e = threadIdx.x; e < at.TH * b.Wv; e += blockDim.x) {
+            const int r = e / b.Wv, w = e - r * b.Wv, h = at.h0 + r;
+            const RowAt<ROWS> xat(b, h, addr.row_x, addr.plane), zat(b, h, addr.row_z, addr.plane);
+            const int d = at.d0 + o;                 // from the row's chunk on
+            if (d + xat.d >= b.D) continue;
+            bf16* const out = P.t1 + (long long)at.bc * addr.chan + xat.off + d * addr.plane + w;
+            if (!isnan(to_f32(*out))) continue;
+            const bf16* const zc = P.z + (long long)at.bc * SC * addr.chan + zat.off + w - PW;
+            float sum = 0.0f;
+#pragma unroll 1
+            for (int t = 0; t < KT; t += KW) {
+                const int kh = t / KW % KH, kd = t / (KW * KH), dd = d + kd - PD, hh = h + kh - PH;
+                if ((unsigned)(dd + xat.d) >= (unsigned)b.D || (!ROWS && (unsigned)hh >= (unsigned)b.H)) continue;
+                const long long off = dd * addr.plane + (kh - PH) * addr.row_z;
+#pragma unroll
+                for (int j = 0; j < SC; ++j) {
+                    const float bj = P.bias ? P.bias[at.c * SC + j] : 0.0f;
+#pragma unroll
+                    for (int kw = 0; kw < KW; ++kw) {
+                        if ((unsigned)(w + kw - PW) >= (unsigned)b.Wv) continue;
+                        float s = to_f32(zc[j * addr.chan + off + kw]) + bj;
+                        if (b.relu) s = fmaxf(s, 0.0f);
+                        sum = fmaf(s, P.h[(long long)(at.c * SC + j) * KT + t + kw], sum);
+                    }
+                }
+            }
+            *out = from_f32<bf16>(sum);
+        }
+}
+
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(const SourceArgs P) {
+__global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(const __grid_constant__ SourceArgs P) {
     constexpr bool ROWS = KH == 1;
     constexpr int kThreads = kSourceThreads, kEpilogueWarps = 4, kMmaWarp = 14;
     constexpr int PD = KD / 2, PW = KW / 2, KT = KD * KH * KW, RING = source_ring<KD>();
@@ -830,6 +955,7 @@ __global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(
                    edges = aempty + 8 * RING;
     constexpr int kEdgesAt = 320, kTmemAt = 504;
     static_assert(8 * (2 * kSourceSlots + 2 * RING + 1) <= kEdgesAt && kEdgesAt + 64 * PW <= kTmemAt, "header");
+    volatile unsigned* const again = reinterpret_cast<unsigned*>(smem_tc + kTmemAt + 4);      // see look()
     float* const edge = reinterpret_cast<float*>(smem_tc + kEdgesAt);      // [parity][warp][side][PW]
     bf16* const bmat = reinterpret_cast<bf16*>(smem_tc + kHeader);
     uint4* const slots = reinterpret_cast<uint4*>(bmat + NMAT * NCOL * 16);
@@ -841,6 +967,7 @@ __global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(
         for (int i = 0; i < kSourceSlots; ++i) { mbar_init(sfull + 8 * i, kSourceStagers / 32); mbar_init(sempty + 8 * i, 1); }
         for (int i = 0; i < RING; ++i) { mbar_init(afull + 8 * i, 1); mbar_init(aempty + 8 * i, kEpilogueWarps); }
         mbar_init(edges, kEpilogueWarps);
+        *again = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     float* const hs = reinterpret_cast<float*>(smem_tc + 512);
@@ -894,10 +1021,11 @@ __global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(
             const __nv_bfloat162 v = __float2bfloat162_rn(P.bias ? P.bias[at.c * SC + j] : 0.0f);
             bias[j] = *reinterpret_cast<const unsigned*>(&v);
         }
+        if (look(make_uint4(bias[0], bias[1], bias[2], bias[3]))) *again = 1u;
         SourceStager<KH, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at,
                                          (tid - 32 * kEpilogueWarps) % kSourceStagers);
-        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, 0, sfull,
-                                           sempty, (warp - kEpilogueWarps) / 5, lane);
+        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { return st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, 0, sfull,
+                                           sempty, (warp - kEpilogueWarps) / 5, lane, again);
     } else {
         const int m = warp * 32 + lane, r = m / b.NB, q = m - r * b.NB, w = 8 * q;
         const RowAt<ROWS> row(b, at.h0 + r, addr.row_x, addr.plane);
@@ -967,6 +1095,7 @@ __global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(
     __syncthreads();
     __syncwarp();
     if (warp == kMmaWarp) tmem_free(tmem, kSourceCols);
+    if (*again) source_again<KD, KH, KW>(P, blockIdx.x);
 }
 
 }  // namespace tc
