@@ -20,7 +20,7 @@ FLAG_FORCE_GENERIC, FLAG_BF16_PARAMS = 1, 2
 # every symbol `include/ndc_b200.h` declares
 SYMBOLS = (
     "ndc_version", "ndc_last_error", "ndc_status_string", "ndc_launch_count", "ndc_query",
-    "ndc_kernel_family",
+    "ndc_kernel_family", "ndc_backward_family",
     "ndc_fwd", "ndc_bwd_workspace_bytes", "ndc_bwd", "ndc_bwd_static", "ndc_gconv",
     "ndc_probe_fp32_fma", "ndc_inorm_workspace_bytes", "ndc_inorm_last_error", "ndc_inorm_fwd",
     "ndc_inorm_bwd", "ndc_bias_grad_workspace_bytes", "ndc_bias_last_error", "ndc_bias_add",
@@ -72,8 +72,9 @@ def load():
     lib.ndc_launch_count.restype = ctypes.c_uint64
     lib.ndc_query.restype = ctypes.c_int
     lib.ndc_query.argtypes = [dp, ctypes.POINTER(ctypes.c_int32)]
-    lib.ndc_kernel_family.restype = ctypes.c_int
-    lib.ndc_kernel_family.argtypes = [dp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32)]
+    for name in ("ndc_kernel_family", "ndc_backward_family"):
+        getattr(lib, name).restype = ctypes.c_int
+        getattr(lib, name).argtypes = [dp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32)]
     lib.ndc_fwd.restype = ctypes.c_int
     lib.ndc_fwd.argtypes = [dp, vp, vp, fp, fp, vp, vp, vp]
     lib.ndc_bwd_workspace_bytes.restype = ctypes.c_size_t

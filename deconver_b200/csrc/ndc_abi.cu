@@ -92,12 +92,13 @@ int check_pitch(const NdcDesc* d, int pitch, int out_pitch) {
     return NDC_OK;
 }
 
-// The kernels an update runs on; `at`: the OR of the addresses that decide about the tensor cores.
-int family_of(const NdcDesc* d, const ndc::Geo& g, uintptr_t at) {
+// The kernels that one direction of an update runs on; `at`: the OR of the addresses that decide about the tensor cores.
+int family_of(const NdcDesc* d, const ndc::Geo& g, uintptr_t at, bool backward) {
     const int path = path_of(d, g.W);   // g.W: the pitch
     if (path == NDC_PATH_GENERIC) return tile_path(d, g) ? NDC_FAMILY_TILE : NDC_FAMILY_GENERIC;
     // bfloat16 tensors with bfloat16 parameters: exact products on the tensor cores
-    if (d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && !(d->flags & NDC_FLAG_RELU_FILTER) && at % 8 == 0 && ndc::tc::covers(g))
+    if (d->dtype == NDC_BF16 && (d->flags & NDC_FLAG_BF16_PARAMS) && !(d->flags & NDC_FLAG_RELU_FILTER) && at % 8 == 0 &&
+        ndc::tc::covers(g, backward))
         return NDC_FAMILY_TENSOR;
     return path == NDC_PATH_DEPTHWISE4_ROWS ? NDC_FAMILY_MARCH_ROWS : NDC_FAMILY_MARCH;
 }
@@ -206,7 +207,14 @@ int ndc_query(const NdcDesc* desc, int32_t* path) {
 int ndc_kernel_family(const NdcDesc* desc, int32_t pitch, int32_t* family) {
     NDC_TRY(validate(desc));
     NDC_TRY(check_pitch(desc, pitch, pitch));
-    if (family) *family = family_of(desc, ndc::make_geo(*desc, false, pitch, pitch), 0);
+    if (family) *family = family_of(desc, ndc::make_geo(*desc, false, pitch, pitch), 0, false);
+    return NDC_OK;
+}
+
+int ndc_backward_family(const NdcDesc* desc, int32_t pitch, int32_t* family) {
+    NDC_TRY(validate(desc));
+    NDC_TRY(check_pitch(desc, pitch, pitch));
+    if (family) *family = family_of(desc, ndc::make_geo(*desc, false, pitch, pitch), 0, true);
     return NDC_OK;
 }
 
@@ -242,7 +250,7 @@ int ndc_fwd_rows(const NdcDesc* desc, int32_t pitch, int32_t out_pitch, const vo
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
     typedef __nv_bfloat16 bf16;
-    const int family = family_of(desc, g, (uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0));
+    const int family = family_of(desc, g, (uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (out_pitch == pitch ? (uintptr_t)out : 0), false);
     if (family == NDC_FAMILY_TENSOR) {
         e = ndc::tc::forward(g, (const bf16*)x, (const bf16*)z, h, bias, (bf16*)out, (bf16*)t1, st);
         if (e != cudaSuccess) return cuda_fail(e, "ndc_fwd (tensor core) launch");
@@ -330,7 +338,8 @@ int ndc_bwd_rows(const NdcDesc* desc, int32_t pitch, int32_t gout_pitch, const v
     const ndc::Geo g = ndc::make_geo(*desc, bias != nullptr, pitch, gout_pitch);
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
-    const int family = family_of(desc, g, (uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (uintptr_t)gz | (gout_pitch == pitch ? (uintptr_t)gout : 0));
+    const int family = family_of(desc, g, (uintptr_t)x | (uintptr_t)z | (uintptr_t)t1 | (uintptr_t)gz | (gout_pitch == pitch ? (uintptr_t)gout : 0),
+                                 true);
     if (family != NDC_FAMILY_GENERIC && family != NDC_FAMILY_TILE) {
         ndc::dw4::BwdPlan p;
         if (ndc::dw4::plan_bwd_any(g, p)) {

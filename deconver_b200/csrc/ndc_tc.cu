@@ -207,22 +207,33 @@ cudaError_t run_ratio(const Geo& g, const bf16* x, const bf16* z, const bf16* t1
     return launch_adjoint<KD, KH, KW, kPairs>(g, A, wide, st);
 }
 
-// How large a problem has to be, and how much of the MMAs' rows it has to fill, for the tensor cores to be the
-// faster way.  Device time of an update against the FMA kernels', on 76 shapes about the lines:
-//   volumes    from 0.4 M group-voxels on (0.4 - 0.8 M: forward 0.94x - 1.45x, with the backward 1.00x - 1.20x), rows of 128
-//              at least 30 % full (16^3 fills 25 %: 0.90x - 0.94x)
-//   images     from 0.7 M on, 45 % full (0.7 - 3 M: forward 1.00x - 2.1x, with the backward 0.96x - 1.29x); below
-//              3 M from 10 rows on, 20 with 5x5 filters (16 x 512 of 16^2: 0.79x; 16 x 128 of 20^2: 1.04x); 3x3 filters at the widths that the FMA kernels
-//              have compile-time instances for from 3 M on, 70 % full (2 x 64 of 128^2: 1.04x, 0.98x; 16 x 32 of 256^2, 75 %
-//              full: 1.49x, 1.13x)
+// How large a problem has to be, and how much of the MMAs' rows it has to fill, for the tensor cores to be the faster way:
+// for a forward update, or (`ratio`) for the first step of its backward, whose FMA kernel is the better one of the two, so that
+// its lines lie higher.  560 shapes about the lines, in CUDA graphs over more than the L2,
+// against the FMA kernels: of the 399 beyond the forward's lines none takes longer (1.61x in the mean), and a backward with
+// this first step takes 0.99x - 1.5x (1.14x).  The lines that cost something:
+//   volumes    0.4 M group-voxels, rows of 128 at least 30 % full (16^3 fills 25 %: forward 0.84x - 1.09x, backward 0.92x - 0.97x)
+//   images     0.7 M, 45 % full, 10 rows, with 5x5 filters 20 (16 x 512 of 16^2: 0.86x, 0.93x)
+//   below 3 M with rows of whole quads, which the FMA kernels take fastest:
+//     3x3      forward under 2 M: few rows in bands half full stay (8 x 188 of 16x32: 0.91x); ratio from 1.2 M (8 x 172 of
+//              28^2: 0.97x), from 1.6 M under 20 rows (24 x 192 of 12x28, 1.55 M: 0.98x)
+//     5x5      ratio from 0.85 M (16 x 64 of 28^2, 0.80 M: 0.89x), from 1.5 M in bands half full (14 x 88 of 30x36: 0.97x),
+//              unless an image has 46 rows (2 x 128 of 64^2, 1.05 M: 1.09x)
+//   3x3 at the widths that the FMA kernels have compile-time instances for: from 3 M, 70 % full (1 x 64 of 128^2: 0.98x); the ratio of
+//              128 and 256 columns from 5.5 M (3 x 172 of 24x256: 0.97x, 2 x 44 of 256^2: 1.02x)
 template <int KD, int KH, int KW>
-bool worth(const Geo& g) {
+bool worth(const Geo& g, bool ratio) {
     Band a, s;
     if (!plan<KD, KH, KW>(g, false, a) || !plan<KD, KH, KW>(g, true, s)) return false;
     const double voxels = (double)g.B * g.G * g.D * g.H * g.Wv, use = std::min(useful<KH>(a), useful<KH>(s));
     if (KH > 1) return voxels >= 0.4e6 && use >= 0.3;
-    const bool tuned = KW == 3 && (g.W == 64 || g.W == 128 || g.W == 256);
-    return tuned ? voxels >= 3e6 && use >= 0.7 : use >= 0.45 && (voxels >= 3e6 || (voxels >= 0.7e6 && g.D >= 10 * (KD / 2)));
+    if (KW == 3 && (g.W == 64 || g.W == 128 || g.W == 256)) return use >= 0.7 && voxels >= (ratio && g.W > 64 ? 5.5e6 : 3e6);
+    if (use < 0.45 || voxels < 0.7e6) return false;
+    if (voxels >= 3e6) return true;
+    if (g.D < 10 * (KD / 2)) return false;                // rows of an image
+    if (g.Wv != g.W) return true;
+    if (KW == 3) return ratio ? voxels >= (g.D >= 20 ? 1.2e6 : 1.6e6) : voxels >= 2e6 || use >= 0.65 || g.D >= 24;
+    return !ratio || voxels >= 1.5e6 || g.D >= 46 || (voxels >= 0.85e6 && use >= 0.5);
 }
 
 // Image batches as volumes whose planes are the image rows and whose plane rows are the images.
@@ -236,12 +247,12 @@ Geo as_rows(const Geo& g) {
 
 }  // namespace
 
-bool covers(const Geo& g) {
+bool covers(const Geo& g, bool ratio) {
     if (g.m != 1 || g.sc != SC || g.W % 4 || g.SP >= (1LL << 29)) return false;
-    if (g.kD == 3 && g.kH == 3 && g.kW == 3) return worth<3, 3, 3>(g);
+    if (g.kD == 3 && g.kH == 3 && g.kW == 3) return worth<3, 3, 3>(g, ratio);
     if (g.kD != 1 || g.D != 1 || g.kH != g.kW) return false;
-    if (g.kH == 5) return worth<5, 1, 5>(as_rows(g));
-    if (g.kH == 3) return worth<3, 1, 3>(as_rows(g));
+    if (g.kH == 5) return worth<5, 1, 5>(as_rows(g), ratio);
+    if (g.kH == 3) return worth<3, 1, 3>(as_rows(g), ratio);
     return false;
 }
 

@@ -6,8 +6,8 @@
 namespace ndc {
 namespace tc {
 
-// Whether the tensor-core kernels take this geometry and are the faster ones for it.
-bool covers(const Geo& g);
+// Whether the tensor-core kernels take this geometry and are the faster ones for it: for `forward`, or for `backward_ratio`.
+bool covers(const Geo& g, bool ratio);
 cudaError_t forward(const Geo& g, const __nv_bfloat16* x, const __nv_bfloat16* z, const float* h, const float* bias,
                     __nv_bfloat16* out, __nv_bfloat16* t1, cudaStream_t st);
 // First step of the backward: gnum, gden (two tensors, or (gden, gnum) pairs at `gnum`) and the direct term,

@@ -131,9 +131,11 @@ int ndc_probe_wait(uint32_t limit_us, void *stream);
  */
 int ndc_query(const NdcDesc *desc, int32_t *path);
 
-/* Writes the NdcFamily of ndc_fwd_rows / ndc_bwd_rows for rows of `pitch` elements (desc->W: no padding)
- * and tensors aligned to 16 bytes; the entry points decide by the same function.  Host-only. */
+/* Writes the NdcFamily of ndc_fwd_rows for rows of `pitch` elements (desc->W: no padding) and tensors aligned
+ * to 16 bytes, and that of ndc_bwd_rows: the same, but for NDC_FAMILY_TENSOR, whose backward has lines of its own
+ * (and of which it is the first step alone).  The entry points decide by the same function.  Host-only. */
 int ndc_kernel_family(const NdcDesc *desc, int32_t pitch, int32_t *family);
+int ndc_backward_family(const NdcDesc *desc, int32_t pitch, int32_t *family);
 
 /*
  * Forward of one update: writes `out` and `t1` (t1 is what backward needs, besides x and z).
