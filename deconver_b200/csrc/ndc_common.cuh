@@ -36,6 +36,14 @@ inline int num_sms() {
     return n;
 }
 
+// Lets a kernel have all the shared memory that a CTA can have (227 KB, for those that declare none).  That is state of the
+// kernel, for all threads of the process: set to the need of each launch, one thread's small one would have another's
+// large one refused between its setting and its launch.
+template <typename K>
+inline cudaError_t allow_smem(K kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 // Geometry handed to every kernel by value.
 struct Geo {
     int B, G, m, sc;

@@ -98,8 +98,7 @@ inline bool aligned_for_vec(const void* p, int dtype) {
 template <typename T, int KD, int KH, int KW, typename S, int AL, int WQ>
 cudaError_t launch_fwd(const FwdParams& P, size_t smem_bytes, long long BC, cudaStream_t st) {
     auto kern = fwd_kernel<T, KD, KH, KW, S::NT, S::MAXZ, S::MAXX, S::MINB, AL, WQ>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_bytes);
+    const cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     const long long grid = BC * P.t.ndc * P.t.nth;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -388,11 +387,6 @@ inline bool plan_bwd_any(const Geo& g, BwdPlan& p) {
     return false;
 }
 
-template <typename K>
-inline cudaError_t set_smem(K kern, size_t bytes) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 #define NDC_CUDA_TRY(expr)                      \
     do {                                        \
         cudaError_t _e = (expr);                \
@@ -418,7 +412,7 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.ratio; P.eps = g.eps; P.relu = g.relu;
         P.Wv = g.Wv; P.Wo = g.Wo;
         auto kern = ratio_kernel<T, KD, KH, KW, S::RatioNT, S::RatioMAXX, AL, WQ, packed_kconv<KD>() ? kRatioPairs : kRatioPlanar>;
-        NDC_CUDA_TRY(set_smem(kern, p.smem_ratio));
+        NDC_CUDA_TRY(allow_smem(kern));
         kern<<<(unsigned)p.n_ratio, S::RatioNT, p.smem_ratio, st>>>(P);
         launched();
     }
@@ -434,11 +428,11 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
             constexpr int NT = decltype(nt)::value, MAXC = decltype(maxc)::value;
             if (gh) {
                 auto kern = kconv2_kernel<T, KD, KH, KW, NT, MAXC, AL, true, WQ>;
-                NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
+                NDC_CUDA_TRY(allow_smem(kern));
                 kern<<<(unsigned)p.n_kconv, NT, p.smem_kconv, st>>>(P);
             } else {
                 auto kern = kconv2_kernel<T, KD, KH, KW, NT, MAXC, AL, false, WQ>;
-                NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
+                NDC_CUDA_TRY(allow_smem(kern));
                 kern<<<(unsigned)p.n_kconv, NT, p.smem_kconv, st>>>(P);
             }
             return cudaSuccess;
@@ -474,11 +468,11 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
             dim3 grid((unsigned)p.n_kconv, n);
             if (gh) {
                 auto kern = kconv_kernel<T, KD, KH, KW, S::KconvNT, AL, true, WQ>;
-                NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
+                NDC_CUDA_TRY(allow_smem(kern));
                 kern<<<grid, S::KconvNT, p.smem_kconv, st>>>(P);
             } else {
                 auto kern = kconv_kernel<T, KD, KH, KW, S::KconvNT, AL, false, WQ>;
-                NDC_CUDA_TRY(set_smem(kern, p.smem_kconv));
+                NDC_CUDA_TRY(allow_smem(kern));
                 kern<<<grid, S::KconvNT, p.smem_kconv, st>>>(P);
             }
             launched();
@@ -490,11 +484,11 @@ cudaError_t backward_launch(const Geo& g, const BwdPlan& p, const T* x, const T*
         P.C = g.G; P.D = g.D; P.H = g.H; P.W = g.W; P.t = p.gz; P.relu = g.relu; P.Wv = g.Wv;
         if (gh) {
             auto kern = gz_kernel<T, KD, KH, KW, S::GzNT, S::GzMAXX, AL, true, WQ, kGzCS>;
-            NDC_CUDA_TRY(set_smem(kern, p.smem_gz));
+            NDC_CUDA_TRY(allow_smem(kern));
             kern<<<(unsigned)p.n_gz, S::GzNT, p.smem_gz, st>>>(P);
         } else {
             auto kern = gz_kernel<T, KD, KH, KW, S::GzNT, S::GzMAXX, AL, false, WQ, kGzCS>;
-            NDC_CUDA_TRY(set_smem(kern, p.smem_gz));
+            NDC_CUDA_TRY(allow_smem(kern));
             kern<<<(unsigned)p.n_gz, S::GzNT, p.smem_gz, st>>>(P);
         }
         launched();
@@ -608,7 +602,7 @@ cudaError_t launch_ksrc(const KsrcParams& P, size_t smem_bytes, long long BC, bo
     const long long grid = BC * P.t.ndc * P.t.nth;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     auto go = [&](auto kern) -> cudaError_t {
-        NDC_CUDA_TRY(set_smem(kern, smem_bytes));
+        NDC_CUDA_TRY(allow_smem(kern));
         kern<<<(unsigned)grid, S::NT, smem_bytes, st>>>(P);
         launched();
         return cudaSuccess;
@@ -626,7 +620,7 @@ cudaError_t launch_ratio_forward(const RatioForwardParams& P, size_t smem_bytes,
                                  cudaStream_t st) {
     if (n_ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     auto go = [&](auto kern) -> cudaError_t {
-        NDC_CUDA_TRY(set_smem(kern, smem_bytes));
+        NDC_CUDA_TRY(allow_smem(kern));
         kern<<<(unsigned)n_ctas, S::RatioNT, smem_bytes, st>>>(P);
         launched();
         return cudaSuccess;

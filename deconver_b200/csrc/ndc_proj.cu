@@ -286,7 +286,7 @@ void plan_wgrad(int batch, int co, int ci, long long n, WgradParams& P) {
 template <typename T, int VEC, bool EXACT>
 cudaError_t launch_wgrad(const WgradParams& P, unsigned grid, cudaStream_t st) {
     auto kern = wgrad1x1_kernel<T, VEC, EXACT>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgradSmem);
+    const cudaError_t e = ndc::allow_smem(kern);
     if (e != cudaSuccess) return e;
     kern<<<grid, WNT, kWgradSmem, st>>>(P);
     ndc::launched();

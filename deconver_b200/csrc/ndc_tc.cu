@@ -149,7 +149,7 @@ template <int KD, int KH, int KW> size_t source_smem(const Band& b) {
 
 template <typename K, typename P>
 cudaError_t launch(K kern, int threads, const Band& b, size_t smem, cudaStream_t st, const P& p) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)(b.march ? num_sms() : b.items), threads, smem, st>>>(p);
     launched();

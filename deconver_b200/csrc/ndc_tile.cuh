@@ -736,7 +736,7 @@ template <typename Kern, typename P>
 inline cudaError_t launch(Kern kern, long long grid, int threads, size_t smem, cudaStream_t st, const P& p) {
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_smem(kern);
         if (e != cudaSuccess) return e;
     }
     kern<<<(unsigned)grid, threads, smem, st>>>(p);
