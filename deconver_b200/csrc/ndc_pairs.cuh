@@ -155,14 +155,19 @@ struct ConvParams {
     int relu, blocks, units;             // blocks of CB output channels; tiles (pairs of tiles) of a group, all samples
 };
 
-// Rows and threads that go with CB channels: 32 sums of either stream per thread.
-template <int CB> struct ConvShape {
-    static constexpr int R = 8 / CB;
-    static constexpr int THREADS = CB >= 4 ? 128 : 64, CTAS = 512 / THREADS;
-};
+// Rows that go with CB channels: 32 sums of either stream per thread.
+template <int CB> struct ConvShape { static constexpr int R = 8 / CB; };
+
+// Strips whose operands a thread of A loads at once (see the epilogue), as far as registers go without spilling.
+template <int ROLE, int CB> __host__ __device__ constexpr int conv_batch() {
+    return 8 / (ROLE == kForward ? (CB == 1 ? 1 : 2) : ROLE == kRatio && CB > 1 ? 4 : 2);
+}
+// CTAs of 128 threads a multiprocessor holds: four, of 128 registers; the compiler needs more for one instance (400 bytes
+// of spills, 22.4 us for 17.6 at 32 groups of 2 channels and sources, 4 x 64^2).
+template <int ROLE, int KH, int CB> __host__ __device__ constexpr int conv_ctas() { return ROLE == kRatio && KH == 5 && CB == 2 ? 3 : 4; }
 
 template <typename T, int KD, int KH, int KW, int ROLE, int CB>
-__global__ void __launch_bounds__(ConvShape<CB>::THREADS, ConvShape<CB>::CTAS) conv_kernel(const ConvParams P) {
+__global__ void __launch_bounds__(128, conv_ctas<ROLE, KH, CB>()) conv_kernel(const ConvParams P) {
     constexpr bool ADJOINT = ROLE <= kSource, TWO_TILES = ROLE == kSource || ROLE == kTerm;
     constexpr int R = ConvShape<CB>::R, KT = KD * KH * KW, NWC = 4;     // chunks of a window
     typedef typename std::conditional<ROLE == kSource || ROLE == kBack, float, T>::type TI;
@@ -200,14 +205,6 @@ __global__ void __launch_bounds__(ConvShape<CB>::THREADS, ConvShape<CB>::CTAS) c
         place[e] = ((code & 255u) * t.plane + ((code >> 8) & 0xffffu) * t.pitch + ((c ^ ((c >> 3) & 1)) << 2)) | code & 0xff000000u;
     }
     auto offset = [&](int e, int s) { return have[s] ? offsets[(TWO_TILES ? s * t.table : 0) + e] : -1; };
-    for (int e = threadIdx.x; e < nin * KT * CB; e += blockDim.x) {
-        const int j = e % CB, tau = (e / CB) % KT, i = e / (CB * KT);
-        float v = 0.0f;
-        if (j < nch)
-            v = ADJOINT ? P.h[(((long long)g * t.m + i) * t.sc + j0 + j) * KT + KT - 1 - tau]
-                        : P.h[(((long long)g * t.m + j0 + j) * t.sc + i) * KT + tau];
-        w[e] = dup(v);
-    }
     f32x2 acc[R][CB][V];
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -218,7 +215,6 @@ __global__ void __launch_bounds__(ConvShape<CB>::THREADS, ConvShape<CB>::CTAS) c
     int chunk[NWC];                  // places of the window's chunks in a row
 #pragma unroll
     for (int i = 0; i < NWC; ++i) { const int c = 2 * spot.strip + 1 + i; chunk[i] = (c ^ ((c >> 3) & 1)) << 2; }
-    __syncthreads();
 
     // Quads come by cp.async, each thread its own, while the channel before is swept, and are then interleaved: a
     // quad of either stream makes two chunks of two pairs.
@@ -266,7 +262,15 @@ __global__ void __launch_bounds__(ConvShape<CB>::THREADS, ConvShape<CB>::CTAS) c
             *reinterpret_cast<float4*>(tile + (at ^ 4)) = make_float4(v[0].z, v[1].z, v[0].w, v[1].w);
         }
     };
-    request(0);
+    request(0);            // before the filter: a thread needs its own part of the tables alone
+    for (int e = threadIdx.x; e < nin * KT * CB; e += blockDim.x) {
+        const int j = e % CB, tau = (e / CB) % KT, i = e / (CB * KT);
+        float v = 0.0f;
+        if (j < nch)
+            v = ADJOINT ? P.h[(((long long)g * t.m + i) * t.sc + j0 + j) * KT + KT - 1 - tau]
+                        : P.h[(((long long)g * t.m + j0 + j) * t.sc + i) * KT + tau];
+        w[e] = dup(v);
+    }
     for (int i = 0; i < nin; ++i) {
         fill(i);
         if (i + 1 < nin) request(i + 1);
@@ -316,46 +320,73 @@ __global__ void __launch_bounds__(ConvShape<CB>::THREADS, ConvShape<CB>::CTAS) c
     for (int j = 0; j < CB; ++j) gbs[j] = 0.0f;
 #pragma unroll
     for (int s = 0; s < (TWO_TILES ? 2 : 1); ++s) {
-        const int d = origin[s].d0 + spot.dz, wcol = origin[s].w0 + V * spot.strip;
+        const int d = origin[s].d0 + spot.dz, wcol = origin[s].w0 + V * spot.strip, h0 = origin[s].h0 + spot.group * R;
         if (!spot.any || !have[TWO_TILES ? s : 0] && ROLE != kBack || d >= t.D || wcol >= t.W) continue;
+        if constexpr (!ADJOINT) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int hrow = origin[s].h0 + spot.group * R + r;
-            if (hrow >= t.H) continue;
-            const long long off = ((long long)d * t.H + hrow) * t.W + wcol;
+            for (int r = 0; r < R; ++r) {
+                if (h0 + r >= t.H) continue;
+                const long long off = ((long long)d * t.H + h0 + r) * t.W + wcol;
 #pragma unroll
-            for (int j = 0; j < CB; ++j) {
-                if (j >= nch) continue;
-                const long long e = (bg[s] * nout + j0 + j) * t.SP + off;
+                for (int j = 0; j < CB; ++j) {
+                    if (j >= nch) continue;
+                    const long long e = (bg[s] * nout + j0 + j) * t.SP + off;
+                    float lo[V], up[V];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) unpack2(acc[r][j][v], lo[v], up[v]);
+                    if (ROLE == kTerm) {
+                        store_strip<T>(reinterpret_cast<T*>(P.out) + e, s ? up : lo);
+                    } else {
+                        if (P.gt1) store_strip<float>(P.gt1 + e, lo);
+                        if (P.out) store_strip<T>(reinterpret_cast<T*>(P.out) + e, up);
+                    }
+                }
+            }
+            continue;
+        }
+        // Strips by rows, then channels.  What a batch of them reads is asked for ahead of its first store, or each would wait
+        // for the memory in turn: at 8 groups of one channel, 4 x 20x44, 3x3, 7.5 -> 6.3 us for the forward's A and 11.3 -> 6.8
+        // for the source gradient's.
+        constexpr int STRIPS = R * CB, BATCH = conv_batch<ROLE, CB>();
+        const long long e0 = (bg[s] * nout + j0) * t.SP + ((long long)d * t.H + h0) * t.W + wcol;
+        auto here = [&](int i) { return h0 + i / CB < t.H && i % CB < nch; };
+        auto at = [&](int i) { return e0 + (long long)(i % CB) * t.SP + (i / CB) * t.W; };
+#pragma unroll
+        for (int i0 = 0; i0 < STRIPS; i0 += BATCH) {
+            float bj[CB];
+#pragma unroll
+            for (int j = 0; j < CB; ++j) bj[j] = P.bias && j < nch ? P.bias[g * t.sc + j0 + j] : 0.0f;
+            dw4::Raw4<T> zr[BATCH], gr[BATCH];       // z; gout (kRatio) or the direct term (kSource)
+#pragma unroll
+            for (int i = i0; i < i0 + BATCH; ++i) {
+                if (!here(i)) continue;
+                zr[i - i0] = dw4::load4_raw<T, true>(reinterpret_cast<const T*>(P.z) + at(i), V);
+                if (ROLE != kForward)
+                    gr[i - i0] = dw4::load4_raw<T, true>(reinterpret_cast<const T*>(ROLE == kRatio ? P.gout : P.out) + at(i), V);
+            }
+#pragma unroll
+            for (int i = i0; i < i0 + BATCH; ++i) {
+                if (!here(i)) continue;
+                const int r = i / CB, j = i % CB;
+                const long long e = at(i);
                 float lo[V], up[V], out[V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) unpack2(acc[r][j][v], lo[v], up[v]);
-                if (ROLE == kTerm) {
-                    store_strip<T>(reinterpret_cast<T*>(P.out) + e, s ? up : lo);
-                    continue;
-                }
-                if (ROLE == kBack) {
-                    if (P.gt1) store_strip<float>(P.gt1 + e, lo);
-                    if (P.out) store_strip<T>(reinterpret_cast<T*>(P.out) + e, up);
-                    continue;
-                }
-                const float b = P.bias ? P.bias[g * t.sc + j0 + j] : 0.0f;
-                float zv[V];
-                load_strip<T>(reinterpret_cast<const T*>(P.z) + e, zv);
+                const float4 z4 = dw4::to_float4(zr[i - i0]), g4 = ROLE == kForward ? z4 : dw4::to_float4(gr[i - i0]);
+                const float zv[V] = {z4.x, z4.y, z4.z, z4.w}, gv[V] = {g4.x, g4.y, g4.z, g4.w};
                 if (ROLE == kForward) {
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        float sv = zv[v] + b;
+                        float sv = zv[v] + bj[j];
                         if (P.relu) sv = fmaxf(sv, 0.0f);
                         out[v] = __fdiv_rn(sv * lo[v], up[v]);
                     }
                     store_strip<T>(reinterpret_cast<T*>(P.out) + e, out);
                 } else if (ROLE == kRatio) {
-                    float gv[V], gn[V], gd[V];
-                    load_strip<T>(reinterpret_cast<const T*>(P.gout) + e, gv);
+                    float gn[V], gd[V];
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        float sv = zv[v] + b;
+                        float sv = zv[v] + bj[j];
                         if (P.relu) sv = fmaxf(sv, 0.0f);
                         gn[v] = __fdiv_rn(gv[v] * sv, up[v]);
                         gd[v] = -__fdiv_rn(gn[v] * lo[v], up[v]);
@@ -365,17 +396,14 @@ __global__ void __launch_bounds__(ConvShape<CB>::THREADS, ConvShape<CB>::CTAS) c
                     store_strip<float>(P.gden + e, gd);
                     if (P.out) store_strip<T>(reinterpret_cast<T*>(P.out) + e, out);
                 } else {
-                    float dv[V];
-                    T* gz = reinterpret_cast<T*>(P.out) + e;
-                    load_strip<T>(gz, dv);
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        float a = dv[v] + (s ? up[v] : lo[v]);
-                        if (P.relu && !(zv[v] + b > 0.0f)) a = 0.0f;
+                        float a = gv[v] + (s ? up[v] : lo[v]);
+                        if (P.relu && !(zv[v] + bj[j] > 0.0f)) a = 0.0f;
                         out[v] = a;
                         gbs[j] += to_f32(from_f32<T>(a));      // the values as stored
                     }
-                    store_strip<T>(gz, out);
+                    store_strip<T>(reinterpret_cast<T*>(P.out) + e, out);
                 }
             }
         }
@@ -639,8 +667,9 @@ inline size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
 inline int block_of(int channels) { return channels > 4 && (channels % 8 == 0 || channels % 8 > 4) ? 8 : channels > 2 ? 4 : channels; }
 inline int corr_block(const Geo& g) { return g.sc > 2 ? 4 : 2; }
 
-struct ConvPlan { TileGeo t; int cb, blocks, units; long long grid; size_t smem; };
+struct ConvPlan { TileGeo t; int cb, blocks, units, threads; long long grid; size_t smem; };
 
+// `threads`: of a CTA, those of the tile or more.
 // The CTA size (tiles of as many strips) of least expected time: instructions of a CTA and channel, its sweep
 // and its staged quads, times the CTAs of the fullest multiprocessor, which few warps leave waiting (by 6 /
 // warps; as many as fit its shared memory: counted so, the training step above takes 489 us for 501).
@@ -667,6 +696,13 @@ inline ConvPlan plan_conv(const Geo& g, bool adjoint, bool two_tiles) {
         const double time = cta * (double)per_sm * (1.0 + 6.0 / resident);
         if (least < 0 || time < 0.97 * least) { least = time; best = p; }
     }
+    // Warps that only stage, where every CTA has a multiprocessor to itself: a warp that stages eight rows for each of its own
+    // alone takes longer for that than for the sweep (8 groups of one channel, 64^2, 3x3, forward: 18.0 -> 12.1 us, with the
+    // batches of the epilogue).  Of several CTAs the same warps sweep, and meet on the same schedulers (16 groups of 4, 16 x
+    // 32^2, 5x5, A: 29 us for 23).
+    best.threads = best.t.threads;
+    if (best.grid <= num_sms())
+        while (best.threads < 128 && best.t.chunks > 2 * best.threads) best.threads += 32;
     return best;
 }
 
@@ -727,10 +763,10 @@ cudaError_t run_conv(const Geo& g, ConvParams& P, cudaStream_t st) {
     const ConvPlan p = plan_conv<KD, KH, KW>(g, ROLE <= kSource, ROLE == kSource || ROLE == kTerm);
     P.t = p.t; P.blocks = p.blocks; P.units = p.units; P.eps = g.eps;
     switch (p.cb) {
-        case 8: return launch(conv_kernel<T, KD, KH, KW, ROLE, 8>, p.grid, p.t.threads, p.smem, st, P);
-        case 4: return launch(conv_kernel<T, KD, KH, KW, ROLE, 4>, p.grid, p.t.threads, p.smem, st, P);
-        case 2: return launch(conv_kernel<T, KD, KH, KW, ROLE, 2>, p.grid, p.t.threads, p.smem, st, P);
-        default: return launch(conv_kernel<T, KD, KH, KW, ROLE, 1>, p.grid, p.t.threads, p.smem, st, P);
+        case 8: return launch(conv_kernel<T, KD, KH, KW, ROLE, 8>, p.grid, p.threads, p.smem, st, P);
+        case 4: return launch(conv_kernel<T, KD, KH, KW, ROLE, 4>, p.grid, p.threads, p.smem, st, P);
+        case 2: return launch(conv_kernel<T, KD, KH, KW, ROLE, 2>, p.grid, p.threads, p.smem, st, P);
+        default: return launch(conv_kernel<T, KD, KH, KW, ROLE, 1>, p.grid, p.threads, p.smem, st, P);
     }
 }
 

@@ -21,6 +21,11 @@ CASES = [
     (2, 1, 2, (5, 5), 1, (21, 68)),
     (1, 5, 16, (5, 5), 2, (35, 12)),
     (2, 8, 3, (3, 3), 1, (33, 132)),
+    # warps that only stage; the last grid that has them, and the first without
+    (8, 1, 1, (3, 3), 2, (41, 44)),
+    (1, 1, 1, (3, 3, 3), 3, (9, 13, 20)),
+    (4, 1, 2, (5, 5), 37, (16, 32)),
+    (149, 1, 1, (3, 3), 1, (16, 32)),
 ]
 
 
