@@ -269,10 +269,12 @@ __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int 
 }
 
 // Infinities and NaN.  A zero of the band times one of them is NaN, and a window reaches into its row's next block and, past
-// its last one, into the next row's: what the taps never see would become NaN, in another image too.  So the stagers look
-// at what they stage, and a CTA that has met one computes what became NaN once more after its march, tap by tap on the FMA
-// pipe (adjoint_again, source_again).  Looking takes an instruction for two values: 131 us for 128 in the source kernel at
-// 2 x 64 x 64^3, nothing measurable in the adjoint.  Where every value is one the forward takes 7.0 ms there, not 0.33.
+// its last one, into the next row's: what the taps never see would become NaN, in another image too.  So a CTA that has met
+// one computes what became NaN once more after its march, tap by tap on the FMA pipe (adjoint_again, source_again).  The
+// adjoint's stagers look at what they stage, which costs nothing measurable; the source kernel looks at what it stores, one
+// channel for the four that it stages (12 bfloat16 forwards, 0.4 % in the mean; at 2 x 64 x 64^3 the stagers' look took 131 us
+// for 128).  Looking at all takes 1 % of a volume's forward (2 x 64 x 64^3: 307 -> 315 us, the most).  Where every value
+// is not finite the forward takes 7.0 ms there, not 0.33.
 // (A block of zeros between the rows would keep images apart, and NaN spread over blocks of eight columns all the same.)
 // Not zero where one of the eight values is not finite.
 __device__ __forceinline__ unsigned look(const uint4& v) {
@@ -870,9 +872,8 @@ struct SourceStager {
         for (int ch = 0; ch < SC; ++ch) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + ch * stride + off));
     }
     // `bias`: two copies of b per channel
-    __device__ __forceinline__ unsigned store(uint4* dst, const unsigned (&bias)[SC], bool relu) {
-        if (at < 0) return 0u;
-        unsigned seen = 0u;
+    __device__ __forceinline__ void store(uint4* dst, const unsigned (&bias)[SC], bool relu) {
+        if (at < 0) return;
 #pragma unroll
         for (int ch = 0; ch < SC; ++ch) {
             unsigned z[4], c[4];
@@ -889,12 +890,9 @@ struct SourceStager {
                 z[i] &= m;
                 c[i] = bias[ch] & m;
             }
-            const uint4 v = make_uint4(z[0], z[1], z[2], z[3]);
-            dst[2 * ch * blocks + at] = v;
-            seen |= look(v);
+            dst[2 * ch * blocks + at] = make_uint4(z[0], z[1], z[2], z[3]);
             dst[(2 * ch + 1) * blocks + at] = make_uint4(c[0], c[1], c[2], c[3]);
         }
-        return seen;
     }
 };
 
@@ -1021,10 +1019,9 @@ __global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(
             const __nv_bfloat162 v = __float2bfloat162_rn(P.bias ? P.bias[at.c * SC + j] : 0.0f);
             bias[j] = *reinterpret_cast<const unsigned*>(&v);
         }
-        if (look(make_uint4(bias[0], bias[1], bias[2], bias[3]))) *again = 1u;
         SourceStager<KH, AL == kWide> st(b, P.z + (long long)at.bc * SC * addr.chan, addr.chan, addr.plane, addr.row_z, at,
                                          (tid - 32 * kEpilogueWarps) % kSourceStagers);
-        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { return st.store(slots + s * slot_blocks, bias, b.relu); }, b.D, at.d0, PD, planes, 0, sfull,
+        ok = stage_planes<kSourceSlots, 2, ROWS>(st, [&](int s) { st.store(slots + s * slot_blocks, bias, b.relu); return 0u; }, b.D, at.d0, PD, planes, 0, sfull,
                                            sempty, (warp - kEpilogueWarps) / 5, lane, again);
     } else {
         const int m = warp * 32 + lane, r = m / b.NB, q = m - r * b.NB, w = 8 * q;
@@ -1085,8 +1082,9 @@ __global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (AL != kWide && w + i >= b.Wv) v[i] = 0.0f;
-                store8<AL>(tb + (at.d0 + o) * addr.plane, w, b.W,
-                           make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])));
+                const uint4 t = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                if (look(t)) *again = 1u;
+                store8<AL>(tb + (at.d0 + o) * addr.plane, w, b.W, t);
             }
         }
     }
