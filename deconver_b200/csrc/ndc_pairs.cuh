@@ -710,14 +710,18 @@ template <int KD, int KH, int KW>
 inline TileGeo plan_corr(const Geo& g) { return plan<KD, KH, KW>(g, kCorrRows, kCorrThreads, 1); }
 
 // CTAs per (group, output channel, block of source channels) of corr_kernel: as many tiles as one of them
-// walks, and its combine (about one tile's worth), times the rounds of two CTAs per multiprocessor.
+// walks, and its combine (about one tile's worth), times the rounds of two CTAs per multiprocessor.  Of those that
+// leave a CTA as many tiles only the fewest is a candidate.
 inline int corr_splits(const Geo& g, const TileGeo& t) {
     const int cb = corr_block(g);
     const long long combos = (long long)g.G * g.m * ((g.sc + cb - 1) / cb), work = (long long)g.B * t.tiles(), slots = 2LL * num_sms();
+    const long long most = std::min(work, std::max(1LL, 2 * slots / combos));
     long long best = 1, least = -1;
-    for (long long s = 1; s <= std::min(work, std::max(1LL, 2 * slots / combos)); ++s) {
-        const long long time = (combos * s + slots - 1) / slots * ((work + s - 1) / s + 1);
+    for (long long s = 1; s <= most;) {
+        const long long walked = (work + s - 1) / s, time = (combos * s + slots - 1) / slots * (walked + 1);
         if (least < 0 || time < least) { least = time; best = s; }
+        if (walked == 1) break;
+        s = (work + walked - 2) / (walked - 1);
     }
     return (int)best;
 }
