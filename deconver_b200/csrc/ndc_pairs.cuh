@@ -726,28 +726,31 @@ inline int corr_splits(const Geo& g, const TileGeo& t) {
     return (int)best;
 }
 
-// Scratch of the backward: gnum | gden | gt1 | bias-gradient records | correlation records.
-struct BwdScratch { size_t gnum, gden, gt1, gb, corr, bytes; };
+// Scratch of the backward: gnum | gden | gt1 | bias-gradient records | correlation records, and the correlation's plan.
+struct BwdScratch { size_t gnum, gden, gt1, gb, corr, bytes; TileGeo tc; int splits; };
 
+// `limit`: bytes that there are.  The correlation makes do with fewer splits to keep to them, but with half as many as it
+// wants at least: false where that does not help.
 template <int KD, int KH, int KW>
-inline BwdScratch scratch_shape(const Geo& g) {
-    BwdScratch s;
+inline bool scratch_shape(const Geo& g, size_t limit, BwdScratch& s) {
     const size_t src = (size_t)g.B * g.G * g.sc * g.SP * sizeof(float);
     const ConvPlan pa = plan_conv<KD, KH, KW>(g, true, true);
-    const TileGeo tc = plan_corr<KD, KH, KW>(g);
     const int cb = corr_block(g);
+    s.tc = plan_corr<KD, KH, KW>(g);
     s.gnum = 0;
     s.gden = up256(src);
     s.gt1 = s.gden + up256(src);
     s.gb = s.gt1 + up256((size_t)g.B * g.G * g.m * g.SP * sizeof(float));
     s.corr = s.gb + up256((size_t)pa.grid * pa.cb * sizeof(float));
-    s.bytes = s.corr + up256((size_t)g.G * g.m * ((g.sc + cb - 1) / cb) * corr_splits(g, tc) * g.KT * cb * sizeof(float));
-    return s;
-}
-inline BwdScratch bwd_scratch(const Geo& g) {
-    if (g.kD == 3) return scratch_shape<3, 3, 3>(g);
-    if (g.kH == 5) return scratch_shape<1, 5, 5>(g);
-    return scratch_shape<1, 3, 3>(g);
+    const size_t split = (size_t)g.G * g.m * ((g.sc + cb - 1) / cb) * g.KT * cb * sizeof(float);
+    const int wanted = corr_splits(g, s.tc);
+    s.splits = wanted;
+    if (s.corr + up256(wanted * split) > limit) {
+        s.splits = s.corr < limit ? (int)std::min((size_t)wanted, (limit - s.corr) / 256 * 256 / split) : 0;
+        if (2 * s.splits < wanted) return false;
+    }
+    s.bytes = s.corr + up256(s.splits * split);
+    return true;
 }
 
 template <typename Kern, typename P>
@@ -788,8 +791,7 @@ cudaError_t forward_shape(const Geo& g, const T* x, const T* z, const float* h, 
 
 template <typename T, int KD, int KH, int KW>
 cudaError_t backward_shape(const Geo& g, const T* x, const T* z, const T* t1, const float* h, const float* bias,
-                           const T* gout, T* gx, T* gz, float* gh, float* gb, void* ws, cudaStream_t st) {
-    const BwdScratch sc = scratch_shape<KD, KH, KW>(g);
+                           const T* gout, T* gx, T* gz, float* gh, float* gb, void* ws, const BwdScratch& sc, cudaStream_t st) {
     float* gnum = (float*)((char*)ws + sc.gnum);
     float* gden = (float*)((char*)ws + sc.gden);
     float* gt1 = (float*)((char*)ws + sc.gt1);
@@ -807,11 +809,11 @@ cudaError_t backward_shape(const Geo& g, const T* x, const T* z, const T* t1, co
     }
     if (gh) {
         CorrParams C{};
-        C.t = plan_corr<KD, KH, KW>(g);
+        C.t = sc.tc;
         const int cb = corr_block(g);
         C.gden = gden; C.gnum = gnum; C.z = z; C.bias = bias; C.t1 = t1; C.x = x; C.gt1 = gt1;
         C.partial = (float*)((char*)ws + sc.corr); C.relu = g.relu; C.blocks = (g.sc + cb - 1) / cb;
-        C.splits = corr_splits(g, C.t);
+        C.splits = sc.splits;
         const size_t rec = (size_t)(C.t.threads / 32) * g.KT * cb;
         const size_t til = (size_t)C.t.table + 2 * ((size_t)C.t.planes * C.t.plane + (size_t)kCorrRows * cb * V * C.t.threads);
         const long long grid = (long long)g.G * g.m * C.blocks * C.splits;

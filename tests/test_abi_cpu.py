@@ -175,18 +175,23 @@ def test_bias_entry_points_validate_without_a_gpu(lib):
     assert b"dtype" in lib.ndc_bias_last_error()
 
 
-def test_grouped_scratch_near_the_built_in_array():
-    """Grouped geometries whose scratch fits the array of `ndc_bwd_static` with the tile kernels keep fitting: the pairs
-    kernels' records are larger, and where they alone would exceed it the tile kernels stay."""
-    lib = _lib.load()
-    limit, near = _lib.STATIC_WORKSPACE_BYTES, 0
-    for planes in range(20, 60):
-        for rows in range(8, 40, 2):
-            desc = _lib.make_desc(1, 4, 2, 8, (planes, rows, 32), (3, 3, 3), 1e-16, True, _lib.NDC_F32)
-            need = lib.ndc_bwd_workspace_bytes(desc)
-            tensors = 4 * (2 * 8 + 2) * planes * rows * 32 * 4      # gnum, gden and gt1, float32
-            assert need >= tensors
-            if limit - 300000 < tensors + 150000 <= limit:          # the tile kernels' records are below 150 kB here
-                near += 1
-                assert need <= limit
-    assert near
+# Grouped geometries (at 148 multiprocessors) whose tile scratch fits the built-in array and whose pairs scratch, with as many
+# records as the correlation wants, does not: batch, groups, m, sc, spatial, kernel, and those two sizes.
+NEAR = [
+    (1, 8, 4, 4, (23, 59, 32), (3, 3, 3), 16733184, 16796928),
+    (1, 4, 2, 8, (35, 46, 36), (3, 3, 3), 16759296, 16826112),
+    (1, 4, 2, 8, (37, 49, 32), (3, 3, 3), 16775936, 16841472),
+    (1, 8, 4, 4, (678, 64), (5, 5), 16716544, 16788736),
+    (1, 8, 4, 4, (145, 300), (5, 5), 16758528, 16825344),
+    (1, 2, 1, 16, (661, 96), (3, 3), 16777216, 16800256),
+    (1, 3, 16, 16, (453, 64), (3, 3), 16730112, 16804352),
+]
+
+
+@pytest.mark.parametrize("case", NEAR, ids=lambda c: "g%d_m%d_sc%d_k%d_%s" % (c[1], c[2], c[3], c[5][0], "x".join(map(str, c[4]))))
+def test_grouped_scratch_near_the_built_in_array(lib, case):
+    """What fits the array of `ndc_bwd_static` with the tile kernels keeps fitting: the pairs kernels make do with fewer records, or
+    the tile kernels stay."""
+    batch, groups, m, sc, spatial, ks, tile, pairs = case
+    need = lib.ndc_bwd_workspace_bytes(_lib.make_desc(batch, groups, m, sc, spatial, ks, 1e-16, True, _lib.NDC_F32))
+    assert tile <= need <= _lib.STATIC_WORKSPACE_BYTES < pairs

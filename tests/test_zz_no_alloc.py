@@ -24,6 +24,9 @@ CASES = [
     (2, 8, 1, 4, (10, 12, 16), (3, 3, 3)),
     (1, 6, 1, 4, (33, 40), (5, 5)),
     (2, 3, 2, 3, (6, 7, 5), (3, 3, 3)),
+    # grouped, just below the array's size: the pairs kernels with fewer records, and the tile kernels
+    (1, 8, 4, 4, (23, 59, 32), (3, 3, 3)),
+    (1, 4, 2, 8, (37, 49, 32), (3, 3, 3)),
 ]
 
 
@@ -43,7 +46,7 @@ def _outputs(x, z, h, bias):
     return (torch.empty_like(x), torch.empty_like(z), torch.empty_like(h), torch.empty_like(bias))
 
 
-@pytest.mark.parametrize("case", CASES, ids=["dw3d", "dw2d", "generic"])
+@pytest.mark.parametrize("case", CASES, ids=["dw3d", "dw2d", "generic", "pairs_limit", "tile_limit"])
 def test_static_workspace_backward_matches_regular_backward(case):
     assert torch.cuda.is_available()
     dev = torch.device("cuda:0")
