@@ -73,3 +73,38 @@ def test_shifted_tensors_take_the_other_kernels(case):
         res.append([out.detach()] + [v.grad for v in t])
     for name, a, r in zip(("out", "gx", "gz", "gh", "gb"), *res):
         assert max_norm_error(a.cpu().numpy(), r.cpu().numpy()) < 1e-4, name
+    assert not all(torch.equal(a, r) for a, r in zip(*res))
+
+
+@pytest.mark.parametrize("mask", range(1, 16))
+def test_partial_gradient_requests(mask):
+    """Either stream of K may be missing, and the direct term."""
+    t, gout = _data((2, 3, 5, (3, 3, 3), 2, (5, 6, 8)), torch.float32)
+
+    def run(bits):
+        v = [a.detach().requires_grad_(bool(bits >> i & 1)) for i, a in enumerate(t)]
+        dcb.deconv_update(*v, groups=2, m=3, sc=5, eps=1e-16, relu_input=True).backward(gout)
+        return [a.grad for a in v]
+
+    full = run(15)
+    for i, a in enumerate(run(mask)):
+        assert (a is None) if not mask >> i & 1 else torch.equal(a, full[i])
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)], ids=["f32", "bf16"])
+@pytest.mark.parametrize("case", [CASES[2], CASES[5], CASES[7]], ids=["volume", "5x5", "3x3"])
+def test_x_alone_off_a_vector_address(case, dtype, tol):
+    """The tile kernels with whole vectors of everything else."""
+    t, gout = _data(case, dtype)
+    flat = torch.empty(t[0].numel() + 1, dtype=dtype, device="cuda:0")
+    flat[1:] = t[0].detach().flatten()
+    aligned, t[0] = t[0].detach(), flat[1:].view(t[0].shape).requires_grad_(True)
+    cfg = dict(groups=case[0], m=case[1], sc=case[2], eps=1e-16, relu_input=True)
+    out = dcb.deconv_update(*t, **cfg)
+    out.backward(gout)
+    args = [v.detach().cpu().double().numpy() for v in t]
+    ref = [c_oracle.forward(*args, **cfg)[0], *c_oracle.backward(*args, gout.cpu().double().numpy(), **cfg)]
+    for name, a, r in zip(("out", "gx", "gz", "gh", "gb"), [out.detach()] + [v.grad for v in t], ref):
+        assert max_norm_error(a.float().cpu().numpy(), r) < tol, name
+    if dtype == torch.float32:      # summed in another order
+        assert not torch.equal(out.detach(), dcb.deconv_update(aligned, *t[1:], **cfg).detach())
