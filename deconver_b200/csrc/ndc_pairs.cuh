@@ -16,7 +16,7 @@
 // four 16-byte words serves all channels and up to three filter rows; weights are read by broadcast).  With
 // one stream per pass, neighbouring voxels in the lanes and four channels per thread it was 2.3 - 5:
 // lanes moved to make odd pairs, windows read once per filter row, and each tile staged once per four channels.
-// A training step with 8 groups of 4 channels and 8 sources, 2 x 32^3, float32: 733 -> 489 us.
+// A training step with 8 groups of 4 channels and 8 sources, 2 x 32^3, float32: 733 -> 478 us.
 //
 //   conv_kernel      A of x and t1 (forward output, backward ratio terms) or of gt1 (source gradient); K of the
 //                    source, or of the two backward ratio tensors
@@ -651,9 +651,11 @@ static __global__ void __launch_bounds__(128) gb_sum_kernel(const float* __restr
 }
 
 // ---- host side ------------------------------------------------------------------------------
-// Rows and tensors of whole vectors: others come by elements, and took 1.1 - 1.4 times as long as with the
-// tile kernels (5 x 37x203 and 13x25x19, one to sixteen channels a group; on whole vectors these take 1.0 - 1.75
-// times as long as these).
+// Rows and tensors of whole vectors: others would come by elements, and took 1.1 - 1.4 times as long as with the
+// tile kernels (5 x 37x203 and 13x25x19, one to sixteen channels a group).  On whole vectors 836 updates of 64 to 65536
+// voxels, one to sixteen channels a group, take 1 / 1.83 of the tile kernels' device time forward and 1 / 1.37 backward in the
+// mean.  16 forwards and 49 backwards take longer, 1.15 times at most: grids that leave most multiprocessors idle, where the
+// tile kernels' threads have fewer rows each.
 inline bool covers(const Geo& g) { return g.W % V == 0; }
 template <typename T> inline bool whole(std::initializer_list<const void*> tensors) {
     for (const void* p : tensors)
@@ -672,7 +674,7 @@ struct ConvPlan { TileGeo t; int cb, blocks, units, threads; long long grid; siz
 // `threads`: of a CTA, those of the tile or more.
 // The CTA size (tiles of as many strips) of least expected time: instructions of a CTA and channel, its sweep
 // and its staged quads, times the CTAs of the fullest multiprocessor, which few warps leave waiting (by 6 /
-// warps; as many as fit its shared memory: counted so, the training step above takes 489 us for 501).
+// warps; as many as fit its shared memory: counted so, the training step above took 489 us for 501).
 template <int KD, int KH, int KW>
 inline ConvPlan plan_conv(const Geo& g, bool adjoint, bool two_tiles) {
     ConvPlan best;

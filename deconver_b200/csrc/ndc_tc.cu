@@ -57,15 +57,14 @@ __global__ void probe_wait_kernel(unsigned limit, unsigned* expired) {
 
 // Bands: as many rows as fill the 128 blocks of an MMA; rows of images (KH = 1) of all chunks together, so that the last
 // band alone is partly filled: on 46 shapes of 1 to 20 images, forward and training step, 1.10x in the mean (16 x
-// 64 of 128^2, 3x3 filter, forward: 255 -> 184 us; one of 300^2: 172 -> 97).  Chunks of planes: all of them, but for a grid that
-// would leave multiprocessors idle; from there, the cut of least expected time, if that is 2 % less: the
-// CTAs of the fullest multiprocessor times a chunk's planes and `halo` more (its filling of the pipeline and
-// its neighbours' planes).  The adjoint's CTAs take turns on the tensor core, so two together need twice the
-// time (halo 4 planes of volumes, 12 of image rows; not for rows that are not whole 8-column blocks, which
-// wait for their loads); of the source's two, one alone needs 0.65 of their time (halo 7).  The adjoint's figures
-// fit sweeps of DC within 10 %; against the starting point they took the adjoint of 16 x 64 images of 128^2
-// from 147 to 126 us, of 12 x 128 of 60x64 from 68 to 41, and of 2 x 64 volumes of 64^3 from 201 to 188 (its
-// ratio step 428 to 394).  The source's choose a cut within 2 % of the best of ten on each of twelve shapes.
+// 64 of 128^2, 3x3 filter, forward: 255 -> 184 us; one of 300^2: 172 -> 97).  Chunks of planes: the cut of least
+// expected time, the CTAs of the fullest multiprocessor times a chunk's planes and some more (its filling of the pipeline
+// and its neighbours' planes).  Two adjoint CTAs share the tensor core and need twice the time of one (4 planes more); of the
+// source's two, one alone needs 0.65 of their time (7 planes more); adjoint CTAs that are alone fill the pipeline once (12
+// planes) and pay each chunk's neighbours and a plane and a half between places.  Images: any cut, the coarsest within 1 %.
+// Volumes: from the cut that gives every multiprocessor four CTAs, another if it is 2 % better; the adjoint of rows that are
+// not whole 8-column blocks waits for its loads instead, and keeps that one.  2 x 64 volumes of 64^3: adjoint 201 -> 188 us,
+// its ratio step 428 -> 394; 12 x 128 images of 60x64, 68 -> 41.
 template <int KD, int KH, int KW>
 bool plan(const Geo& g, bool source, Band& b) {
     b.C = g.G; b.D = g.D; b.H = g.H; b.W = g.W; b.Wv = g.Wv; b.Wo = g.Wo; b.eps = g.eps; b.relu = g.relu;

@@ -10,8 +10,9 @@
 // once, when the CTA's march through the depth comes to it, and a filter row kh is a shift of the start
 // address.  Batches of images march down their rows the same way (planes = image rows, plane rows =
 // images, KH = 1: see SlabAddr); no filter row takes a row of their bands to another, so a band takes any of them, of
-// several chunks at once (see At), and fills its 128 blocks whatever the batch.  An MMA of up to 128 columns takes 64 cycles here, whatever its width
-// (reading 4 KB of A operand), hence the wide ones.  With KW = 3 most of the products meet a zero of the
+// several chunks at once (see At), and fills its 128 blocks whatever the batch.  An MMA of N columns takes 32 + N / 4
+// cycles here, N / 2 from 128 on (measured; its A operand is 4 KB), and a thread whose descriptors change issues one
+// every 80, hence the wide ones.  With KW = 3 most of the products meet a zero of the
 // band; the tensor cores do them 30 times faster than the FMA pipe does the useful ones.  What K = 16
 // holds differs:
 //
@@ -37,7 +38,6 @@
 #pragma once
 
 #include <algorithm>
-#include <type_traits>
 
 #include "ndc_common.cuh"
 #include "ndc_dw4_common.cuh"
@@ -818,8 +818,8 @@ struct SourceArgs {
 // ring's end, so that no MMA is split there: the sums of an output plane at one of the first KD - 1 places
 // are then in two parts, P places apart, which the epilogue adds.
 //
-// What bounds the kernel is the issue of these MMAs: 12 x 64 cycles a plane and band, 1.38 ms at
-// 4 x 64 x 128^3.  A block of places for each of two terms takes as many of them as a window of one
+// What bounds the kernel: these MMAs, 12 x 44 cycles a plane and band at best (0.95 of 1.66 ms at 4 x 64 x 128^3), and the
+// loads, of which two groups are in flight.  A block of places for each of two terms takes as many of them as a window of one
 // term, and rows without zeros between them fill the 128 blocks better (16 rows of 64 columns, not 14), so
 // that the exact form is the faster one too: the forward 4.66 -> 3.95 ms there, 368 -> 316 us at 2 x 64 x 64^3,
 // 228 -> 181 on 16 x 64 images of 128^2, 5x5 (one term, chunks of up to 27 planes: before).

@@ -1,5 +1,6 @@
 // Tile kernels: any grouping with 3x3x3, 5x5 and 3x3 filters, 1 <= m, sc <= 16.  Rows and tensors of whole
-// vectors go to those of ndc_pairs.cuh; these take the others.
+// vectors go to those of ndc_pairs.cuh; these take the others: rows that are not (VEC = false), and whole ones where x or t1
+// alone is off a vector address, or where a backward's scratch is within a hundredth of the built-in array's size (see use_pairs).
 //
 // A CTA owns a tile of one (sample, group) pair: TD planes x TH rows x TW columns of the output.
 // One input channel at a time (or a few) is staged in shared memory with its halo, as float32 rows
@@ -11,12 +12,11 @@
 // Multiply-adds are two-lane `fma.rn.f32x2` over neighbouring voxels; the filter is staged as
 // duplicated (w, w) pairs.
 //
-// What bounds them: at 8 groups of 4 channels and 8 sources, 2 x 32^3 (a training step, float32) they
-// take 0.67 ms where the one-thread-per-element kernels took 4.5 ms; the multiply-adds alone are
-// 0.13 ms, the rest is staging (a 4-byte copy and its address per staged element, 2.4 of them per
-// output voxel and channel with the halo) and, in corr_kernel, one CTA of 194 - 221 registers per
-// thread (3x3x3) on a multiprocessor.  For depthwise ratio-4 filters the marching kernels of ndc_dw4_*.cuh
-// stage each element once and are twice as fast.
+// What bounds them: at 8 groups of 4 channels and 8 sources, 2 x 32x32x31 (an update and its backward, float32) they
+// take 159 + 503 us, of which the multiply-adds alone are 0.13 ms; the rest is staging (a 4-byte copy and its address
+// per staged element, 2.4 of them per output voxel and channel with the halo) and, in corr_kernel, one CTA of 194 - 221
+// registers per thread (3x3x3) on a multiprocessor.  For depthwise ratio-4 filters the marching kernels of
+// ndc_dw4_*.cuh stage each element once and are twice as fast.
 //
 //   adjoint_kernel   A of x and t1 (forward output, backward ratio terms) or of gt1 (source gradient)
 //   k_kernel         K of the source, or of the two backward ratio tensors
@@ -639,22 +639,6 @@ __global__ void __launch_bounds__(256, 1) corr_kernel(const CorrParams P) {
     }
 }
 
-// gh[g*m + o][i][tau] = sum over splits; one thread per element.
-static __global__ void __launch_bounds__(128) corr_sum_kernel(const float* __restrict__ partial, int GM, int sc, int blocks,
-                                                       int splits, int KT, float* __restrict__ gh) {
-    const int e = blockIdx.x * 128 + threadIdx.x;
-    if (e >= GM * sc * KT) return;
-    const int tau = e % KT, i = (e / KT) % sc, go = e / (KT * sc);
-    const float* p = partial + ((size_t)(go * blocks + i / CB) * splits) * KT * CB + tau * CB + i % CB;
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    int k = 0;
-    for (; k + 4 <= splits; k += 4)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] += p[(size_t)(k + u) * KT * CB];
-    for (; k < splits; ++k) s[0] += p[(size_t)k * KT * CB];
-    gh[e] = (s[0] + s[1]) + (s[2] + s[3]);
-}
-
 // gb[g*sc + i] = sum over samples and tiles; one warp per channel, lanes in a fixed partition.
 static __global__ void __launch_bounds__(128) gb_sum_kernel(const float* __restrict__ partial, int B, int G, int sc, int blocks,
                                                      int ntiles, float* __restrict__ gb) {
@@ -825,7 +809,7 @@ cudaError_t backward_shape(const Geo& g, const T* x, const T* z, const T* t1, co
                 : launch(corr_kernel<T, KD, KH, KW, false>, grid, C.t.threads, sizeof(float) * std::max(rec, til), st, C);
         if (e != cudaSuccess) return e;
         const int n = g.G * g.m * g.sc * g.KT;
-        corr_sum_kernel<<<(n + 127) / 128, 128, 0, st>>>(C.partial, g.G * g.m, g.sc, C.blocks, C.splits, g.KT, gh);
+        pairs::corr_sum_kernel<<<(n + 127) / 128, 128, 0, st>>>(C.partial, g.G * g.m, g.sc, C.blocks, CB, C.splits, g.KT, gh);
         launched();
     }
     if (gz) {
