@@ -152,24 +152,22 @@ struct ConvParams {
     float* gt1;                          // kBack
     float* gb_partial;                   // kSource: [g][block][unit][CB] bias-gradient sums, or NULL
     float eps;
-    int relu, blocks, units;             // blocks of CB output channels; tiles (pairs of tiles) of a group, all samples
+    int relu, cb, blocks, units;         // CB; blocks of CB output channels; tiles (pairs of tiles) of a group, all samples
 };
 
-// Rows that go with CB channels: 32 sums of either stream per thread.
-template <int CB> struct ConvShape { static constexpr int R = 8 / CB; };
-
+// A thread has R rows x CB channels: eight, 32 sums of either stream, or four where the grid is small (see plan_conv).
 // Strips whose operands a thread of A loads at once (see the epilogue), as far as registers go without spilling.
-template <int ROLE, int CB> __host__ __device__ constexpr int conv_batch() {
-    return 8 / (ROLE == kForward ? (CB == 1 ? 1 : 2) : ROLE == kRatio && CB > 1 ? 4 : 2);
+template <int ROLE, int CB, int R> __host__ __device__ constexpr int conv_batch() {
+    return R * CB < 8 ? R * CB : 8 / (ROLE == kForward ? (CB == 1 ? 1 : 2) : ROLE == kRatio && CB > 1 ? 4 : 2);
 }
 // CTAs of 128 threads a multiprocessor holds: four, of 128 registers; the compiler needs more for one instance (400 bytes
 // of spills, 22.4 us for 17.6 at 32 groups of 2 channels and sources, 4 x 64^2).
-template <int ROLE, int KH, int CB> __host__ __device__ constexpr int conv_ctas() { return ROLE == kRatio && KH == 5 && CB == 2 ? 3 : 4; }
+template <int ROLE, int KH, int CB, int R> __host__ __device__ constexpr int conv_ctas() { return ROLE == kRatio && KH == 5 && CB == 2 && R == 4 ? 3 : 4; }
 
-template <typename T, int KD, int KH, int KW, int ROLE, int CB>
-__global__ void __launch_bounds__(128, conv_ctas<ROLE, KH, CB>()) conv_kernel(const ConvParams P) {
+template <typename T, int KD, int KH, int KW, int ROLE, int CB, int R>
+__global__ void __launch_bounds__(128, conv_ctas<ROLE, KH, CB, R>()) conv_kernel(const ConvParams P) {
     constexpr bool ADJOINT = ROLE <= kSource, TWO_TILES = ROLE == kSource || ROLE == kTerm;
-    constexpr int R = ConvShape<CB>::R, KT = KD * KH * KW, NWC = 4;     // chunks of a window
+    constexpr int KT = KD * KH * KW, NWC = 4;     // chunks of a window
     typedef typename std::conditional<ROLE == kSource || ROLE == kBack, float, T>::type TI;
     extern __shared__ __align__(16) float smem[];
     const TileGeo& t = P.t;
@@ -347,7 +345,7 @@ __global__ void __launch_bounds__(128, conv_ctas<ROLE, KH, CB>()) conv_kernel(co
         // Strips by rows, then channels.  What a batch of them reads is asked for ahead of its first store, or each would wait
         // for the memory in turn: at 8 groups of one channel, 4 x 20x44, 3x3, 7.5 -> 6.3 us for the forward's A and 11.3 -> 6.8
         // for the source gradient's.
-        constexpr int STRIPS = R * CB, BATCH = conv_batch<ROLE, CB>();
+        constexpr int STRIPS = R * CB, BATCH = conv_batch<ROLE, CB, R>();
         const long long e0 = (bg[s] * nout + j0) * t.SP + ((long long)d * t.H + h0) * t.W + wcol;
         auto here = [&](int i) { return h0 + i / CB < t.H && i % CB < nch; };
         auto at = [&](int i) { return e0 + (long long)(i % CB) * t.SP + (i / CB) * t.W; };
@@ -653,9 +651,8 @@ static __global__ void __launch_bounds__(128) gb_sum_kernel(const float* __restr
 // ---- host side ------------------------------------------------------------------------------
 // Rows and tensors of whole vectors: others would come by elements, and took 1.1 - 1.4 times as long as with the
 // tile kernels (5 x 37x203 and 13x25x19, one to sixteen channels a group).  On whole vectors 836 updates of 64 to 65536
-// voxels, one to sixteen channels a group, take 1 / 1.83 of the tile kernels' device time forward and 1 / 1.37 backward in the
-// mean.  16 forwards and 49 backwards take longer, 1.15 times at most: grids that leave most multiprocessors idle, where the
-// tile kernels' threads have fewer rows each.
+// voxels, one to sixteen channels a group, take 1 / 2.27 of the tile kernels' device time forward and 1 / 1.62 backward in the
+// mean; two forwards take longer, by 3 %.
 inline bool covers(const Geo& g) { return g.W % V == 0; }
 template <typename T> inline bool whole(std::initializer_list<const void*> tensors) {
     for (const void* p : tensors)
@@ -669,7 +666,7 @@ inline size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
 inline int block_of(int channels) { return channels > 4 && (channels % 8 == 0 || channels % 8 > 4) ? 8 : channels > 2 ? 4 : channels; }
 inline int corr_block(const Geo& g) { return g.sc > 2 ? 4 : 2; }
 
-struct ConvPlan { TileGeo t; int cb, blocks, units, threads; long long grid; size_t smem; };
+struct ConvPlan { TileGeo t; int cb, rows, blocks, units, threads; long long grid; size_t smem; };
 
 // `threads`: of a CTA, those of the tile or more.
 // The CTA size (tiles of as many strips) of least expected time: instructions of a CTA and channel, its sweep
@@ -677,18 +674,24 @@ struct ConvPlan { TileGeo t; int cb, blocks, units, threads; long long grid; siz
 // warps; as many as fit its shared memory: counted so, the training step above took 489 us for 501).
 template <int KD, int KH, int KW>
 inline ConvPlan plan_conv(const Geo& g, bool adjoint, bool two_tiles) {
-    ConvPlan best;
-    double least = -1.0;
-    const int nin = adjoint ? g.m : g.sc, nout = adjoint ? g.sc : g.m, cb = block_of(nout), R = 8 / cb;
-    for (int threads = cb >= 4 ? 128 : 64; threads >= 32; threads /= 2) {
+    const int nin = adjoint ? g.m : g.sc, nout = adjoint ? g.sc : g.m;
+    auto shape = [&](int cb, int rows, int threads) {
         ConvPlan p;
-        p.t = plan<KD, KH, KW>(g, R, threads, 2);
-        p.cb = cb; p.blocks = (nout + cb - 1) / cb;
+        p.t = plan<KD, KH, KW>(g, rows, threads, 2);
+        p.cb = cb; p.rows = rows; p.blocks = (nout + cb - 1) / cb;
         const long long tiles = (long long)p.t.tiles() * g.B;
         p.units = (int)(two_tiles ? (tiles + 1) / 2 : tiles);
         p.grid = (long long)g.G * p.blocks * (two_tiles ? (tiles + 1) / 2 : tiles);
         p.smem = sizeof(float) * ((2 * (size_t)nin * g.KT * cb + 3) / 4 * 4 + (size_t)(two_tiles ? 3 : 2) * p.t.table +
                                   (size_t)p.t.planes * p.t.plane + 2 * V * (size_t)p.t.table);
+        p.threads = p.t.threads;
+        return p;
+    };
+    ConvPlan best;
+    double least = -1.0;
+    const int cb = block_of(nout);
+    for (int threads = cb >= 4 ? 128 : 64; threads >= 32; threads /= 2) {
+        const ConvPlan p = shape(cb, 8 / cb, threads);
         if (p.smem > 220 * 1024 && threads > 32) continue;
         const int warps = p.t.threads / 32;
         const double cta = warps * 1.25 * g.KT * 8 * V + p.t.chunks / 32.0 * 30.0;
@@ -698,13 +701,18 @@ inline ConvPlan plan_conv(const Geo& g, bool adjoint, bool two_tiles) {
         const double time = cta * (double)per_sm * (1.0 + 6.0 / resident);
         if (least < 0 || time < 0.97 * least) { least = time; best = p; }
     }
-    // Warps that only stage, where every CTA has a multiprocessor to itself: a warp that stages eight rows for each of its own
-    // alone takes longer for that than for the sweep (8 groups of one channel, 64^2, 3x3, forward: 18.0 -> 12.1 us, with the
-    // batches of the epilogue).  Of several CTAs the same warps sweep, and meet on the same schedulers (16 groups of 4, 16 x
-    // 32^2, 5x5, A: 29 us for 23).
-    best.threads = best.t.threads;
-    if (best.grid <= num_sms())
+    // Where every CTA has a multiprocessor to itself, what counts is how long a thread takes.
+    if (best.grid <= num_sms()) {
+        // Half as much per thread: half of the rows, or of eight channels.  836 updates of 64 to 65536 voxels, most of which
+        // have such grids: forward 1.23 times as fast in the mean, backward 1.18 (4 groups of 4 channels and 16 sources, 20x44,
+        // 5x5, backward: 82 -> 62 us).
+        const ConvPlan p = shape(std::min(cb, 4), cb == 8 ? 1 : 4 / cb, std::min(128, cb == 8 ? best.t.threads : 2 * best.t.threads));
+        if (p.grid <= num_sms() && p.smem <= 220 * 1024) best = p;
+        // Warps that only stage: one that stages eight rows for each of its own alone takes longer for that than for the sweep
+        // (8 groups of one channel, 64^2, 3x3, forward: 18.0 -> 12.1 us, with the batches of the epilogue).  (Of several CTAs
+        // the same warps sweep, and meet on the same schedulers: 16 groups of 4, 16 x 32^2, 5x5, A: 29 us for 23.)
         while (best.threads < 128 && best.t.chunks > 2 * best.threads) best.threads += 32;
+    }
     return best;
 }
 
@@ -770,12 +778,15 @@ inline cudaError_t launch(Kern kern, long long grid, int threads, size_t smem, c
 template <typename T, int KD, int KH, int KW, int ROLE>
 cudaError_t run_conv(const Geo& g, ConvParams& P, cudaStream_t st) {
     const ConvPlan p = plan_conv<KD, KH, KW>(g, ROLE <= kSource, ROLE == kSource || ROLE == kTerm);
-    P.t = p.t; P.blocks = p.blocks; P.units = p.units; P.eps = g.eps;
-    switch (p.cb) {
-        case 8: return launch(conv_kernel<T, KD, KH, KW, ROLE, 8>, p.grid, p.threads, p.smem, st, P);
-        case 4: return launch(conv_kernel<T, KD, KH, KW, ROLE, 4>, p.grid, p.threads, p.smem, st, P);
-        case 2: return launch(conv_kernel<T, KD, KH, KW, ROLE, 2>, p.grid, p.threads, p.smem, st, P);
-        default: return launch(conv_kernel<T, KD, KH, KW, ROLE, 1>, p.grid, p.threads, p.smem, st, P);
+    P.t = p.t; P.cb = p.cb; P.blocks = p.blocks; P.units = p.units; P.eps = g.eps;
+    switch (10 * p.cb + p.rows) {
+        case 81: return launch(conv_kernel<T, KD, KH, KW, ROLE, 8, 1>, p.grid, p.threads, p.smem, st, P);
+        case 42: return launch(conv_kernel<T, KD, KH, KW, ROLE, 4, 2>, p.grid, p.threads, p.smem, st, P);
+        case 41: return launch(conv_kernel<T, KD, KH, KW, ROLE, 4, 1>, p.grid, p.threads, p.smem, st, P);
+        case 24: return launch(conv_kernel<T, KD, KH, KW, ROLE, 2, 4>, p.grid, p.threads, p.smem, st, P);
+        case 22: return launch(conv_kernel<T, KD, KH, KW, ROLE, 2, 2>, p.grid, p.threads, p.smem, st, P);
+        case 18: return launch(conv_kernel<T, KD, KH, KW, ROLE, 1, 8>, p.grid, p.threads, p.smem, st, P);
+        default: return launch(conv_kernel<T, KD, KH, KW, ROLE, 1, 4>, p.grid, p.threads, p.smem, st, P);
     }
 }
 
@@ -833,8 +844,7 @@ cudaError_t backward_shape(const Geo& g, const T* x, const T* z, const T* t1, co
         e = run_conv<T, KD, KH, KW, kSource>(g, S, st);
         if (e != cudaSuccess) return e;
         if (gb) {
-            const int cb = block_of(g.sc);
-            gb_sum_kernel<<<(g.G * g.sc + 3) / 4, 128, 0, st>>>(S.gb_partial, g.G, g.sc, S.blocks, cb, S.units, gb);
+            gb_sum_kernel<<<(g.G * g.sc + 3) / 4, 128, 0, st>>>(S.gb_partial, g.G, g.sc, S.blocks, S.cb, S.units, gb);
             launched();
         }
     }

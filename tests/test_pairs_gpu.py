@@ -21,11 +21,20 @@ CASES = [
     (2, 1, 2, (5, 5), 1, (21, 68)),
     (1, 5, 16, (5, 5), 2, (35, 12)),
     (2, 8, 3, (3, 3), 1, (33, 132)),
-    # warps that only stage; the last grid that has them, and the first without
+    # warps that only stage, on the last grid that has them; the first without
     (8, 1, 1, (3, 3), 2, (41, 44)),
     (1, 1, 1, (3, 3, 3), 3, (9, 13, 20)),
     (4, 1, 2, (5, 5), 37, (16, 32)),
     (149, 1, 1, (3, 3), 1, (16, 32)),
+    # more CTAs than multiprocessors: as much per thread as there is (half of it in the cases above)
+    (300, 1, 1, (3, 3, 3), 1, (2, 9, 8)),
+    (300, 2, 2, (3, 3, 3), 1, (3, 5, 8)),
+    (300, 8, 4, (3, 3, 3), 1, (2, 5, 4)),
+    (300, 1, 2, (5, 5), 1, (9, 12)),
+    (300, 3, 8, (5, 5), 1, (7, 8)),
+    (300, 1, 1, (5, 5), 1, (17, 8)),
+    (300, 4, 8, (3, 3), 1, (10, 12)),
+    (300, 1, 2, (3, 3), 1, (13, 4)),
 ]
 
 
