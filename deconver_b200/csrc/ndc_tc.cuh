@@ -377,6 +377,11 @@ __host__ __device__ inline int slack_blocks(const Band& b) { return MB + 1 - b.T
 using dw4::f32x2;
 using dw4::pack2;
 using dw4::unpack2;
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -671,9 +676,16 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
         const RowAt<ROWS> zat(b, at.h0 + r, addr.row_z, addr.plane), oat(b, at.h0 + r, oaddr.row_z, oaddr.plane);
         // this row's output planes in the march
         const int count = r < at.TH && q < b.NB ? (ROWS ? min(b.DC, b.D - zat.d) : at.DC) : 0;
-        float bj[SC];          // (as pairs for two-lane additions: four registers more, 2.65 ms for 2.42 at 4 x 64 x 128^3)
+        // as single values (as pairs for two-lane additions four registers more: forward 2.65 ms for 2.42 at 4 x 64 x 128^3); as pairs
+        // in the volumes' ratio step, which spills with single ones (3 x 216 of 19x25x25: 178 us for 148)
+        constexpr bool PAIRED = MODE == kPairs && KH > 1;
+        float bj[SC];
+        f32x2 b2[SC];
 #pragma unroll
-        for (int j = 0; j < SC; ++j) bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
+        for (int j = 0; j < SC; ++j) {
+            bj[j] = P.bias ? P.bias[at.c * SC + j] : 0.0f;
+            b2[j] = pack2(bj[j], bj[j]);
+        }
         const long long zrow = (long long)at.bc * SC * addr.chan + zat.off;
         const long long orow = (long long)at.bc * SC * oaddr.chan + oat.off;
         const bf16* const zb = P.z + zrow;
@@ -729,7 +741,9 @@ __global__ void __launch_bounds__(AdjointShape<KD>::THREADS, AdjointShape<KD>::C
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const unsigned u = word_of(zr[j % AHEAD], i);
-                    float lo = __uint_as_float(u << 16) + bj[j], hi = __uint_as_float(u & 0xffff0000u) + bj[j];
+                    float lo = __uint_as_float(u << 16), hi = __uint_as_float(u & 0xffff0000u);
+                    if (PAIRED) unpack2(add2(pack2(lo, hi), b2[j]), lo, hi);
+                    else { lo += bj[j]; hi += bj[j]; }
                     if (b.relu) { lo = fmaxf(lo, 0.0f); hi = fmaxf(hi, 0.0f); }
                     const f32x2 n2 = pack2(n[2 * i], n[2 * i + 1]), r2 = pack2(rcp(dn[2 * i]), rcp(dn[2 * i + 1]));
                     if (MODE == kOut) {
