@@ -271,10 +271,9 @@ __device__ __forceinline__ bool stage_planes(S& st, F store, int D, int d0, int 
 // Infinities and NaN.  A zero of the band times one of them is NaN, and a window reaches into its row's next block and, past
 // its last one, into the next row's: what the taps never see would become NaN, in another image too.  So a CTA that has met
 // one computes what became NaN once more after its march, tap by tap on the FMA pipe (adjoint_again, source_again).  The
-// adjoint's stagers look at what they stage, which costs nothing measurable; the source kernel looks at what it stores, one
-// channel for the four that it stages (12 bfloat16 forwards, 0.4 % in the mean; at 2 x 64 x 64^3 the stagers' look took 131 us
-// for 128).  Looking at all takes 1 % of a volume's forward (2 x 64 x 64^3: 307 -> 315 us, the most).  Where every value
-// is not finite the forward takes 7.0 ms there, not 0.33.
+// adjoint's stagers look at what they stage, which costs up to 2 % of it; the source kernel looks at what it stores, one
+// channel for the four that it stages, which costs nothing measurable (its stagers' look 2 %).  Where no value is finite
+// the forward takes 7.0 ms at 2 x 64 x 64^3, not 0.31.
 // (A block of zeros between the rows would keep images apart, and NaN spread over blocks of eight columns all the same.)
 // Not zero where one of the eight values is not finite.
 __device__ __forceinline__ unsigned look(const uint4& v) {
@@ -910,9 +909,10 @@ struct SourceStager {
     }
 };
 
-// What became NaN of a place's t1 tap by tap (see look()), by all threads of the CTA.
+// What became NaN of a place's t1 tap by tap (see look()), by all threads of the CTA.  Its arguments by value: their address,
+// which a reference needs, costs the kernel 2 - 4 % (3 x 32 of 33x40x39: 34.5 us for 33.4; 2 x 64 x 64^3: 125.5 for 123.9).
 template <int KD, int KH, int KW>
-__device__ __noinline__ void source_again(const SourceArgs& P, int item) {
+__device__ __noinline__ void source_again(const SourceArgs P, int item) {
     constexpr bool ROWS = KH == 1;
     constexpr int PD = KD / 2, PH = KH / 2, PW = KW / 2, KT = KD * KH * KW;
     const Band& b = P.b;
@@ -952,7 +952,7 @@ __device__ __noinline__ void source_again(const SourceArgs& P, int item) {
 }
 
 template <int KD, int KH, int KW, int AL>
-__global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(const __grid_constant__ SourceArgs P) {
+__global__ void __launch_bounds__(kSourceThreads, kSourceCtas) tc_source_kernel(const SourceArgs P) {
     constexpr bool ROWS = KH == 1;
     constexpr int kThreads = kSourceThreads, kEpilogueWarps = 4, kMmaWarp = 14;
     constexpr int PD = KD / 2, PW = KW / 2, KT = KD * KH * KW, RING = source_ring<KD>();
